@@ -129,6 +129,40 @@ int reskv_decode_compact(int bits, int nnz, const void* q, const void* k_centroi
                          const void* recent_q, const void* recent_k, const void* recent_v, int recent_tokens,
                          void* workspace, size_t workspace_bytes, void* out, float* out_m, float* out_l, void* stream);
 
+/* ---- any layout, arguments in a struct --------------------------------------------------
+ * What reskv_decode_bitmap_fp16 (layout UNSTRUCTURED, bits 16), reskv_decode_packed and
+ * reskv_decode_compact (layout COMPACT) do, behind one entry point.  nnz is read for the
+ * bitmap and the compact layouts.  The dense window may be the leading recent_tokens of a
+ * longer buffer: recent_tok_stride is the number of tokens between its (sequence, head)
+ * units (0: recent_tokens).  device_memory != 0: the caller vouches that every pointer is
+ * memory of the current device, and the pointer queries of the call are left out.
+ * workspace_bytes has to be at least reskv_decode_args_workspace_bytes(args), which reads
+ * the sizes and the metadata pointers only. */
+typedef struct reskv_decode_args {
+    int layout, bits, nnz;
+    const void *q, *k_centroids, *k_ids, *k_payload, *k_meta, *k_scale;
+    const void *v_centroids, *v_ids, *v_payload, *v_meta, *v_scale;
+    int batch, kv_heads, q_heads, tokens;
+    int64_t tok_stride;
+    int k_clusters, v_clusters, start_pos, pos_q;
+    float rope_theta;
+    const float* inv_freq;
+    float scaling;
+    int splits;
+    const void *recent_q, *recent_k, *recent_v;
+    int recent_tokens;
+    int64_t recent_tok_stride;
+    void* workspace;
+    size_t workspace_bytes;
+    void* out;
+    float *out_m, *out_l;
+    void* stream;
+    int device_memory;
+} reskv_decode_args;
+
+size_t reskv_decode_args_workspace_bytes(const reskv_decode_args* args);
+int reskv_decode_run(const reskv_decode_args* args);
+
 /* ---- decode steps that can be captured in a CUDA graph --------------------------------
  * No counterpart in the reference (its decode loop is eager Python,
  * benchmarks/timing.py:105-145, and passes positions by value).

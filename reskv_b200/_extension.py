@@ -7,8 +7,10 @@ ahead-of-time ``libreskv_b200.so`` (sm_100a, C ABI, see
 ``include/reskv_b200.h``) is opened with ``ctypes``; ``load_extension`` keeps the
 reference's signature and returns an object that exposes the same operator
 names with the same positional arguments and return values.  Tensors stay
-torch-owned: outputs and scratch memory are allocated here with ``torch.empty``
-and the kernels run on the current CUDA stream.
+torch-owned: outputs and scratch memory come from torch's allocator and the
+kernels run on the current CUDA stream.  The calls of a decode step go through
+``_host.so`` (``csrc/host.cpp``), which does the tensor checks, the allocations
+and the call of the C ABI natively.
 
 There is no CPU or eager fallback: a missing library, a device that is not
 compute capability 10.x, or a failing kernel call raises.
@@ -17,9 +19,10 @@ compute capability 10.x, or a failing kernel call raises.
 from __future__ import annotations
 
 import ctypes
-import os
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 from functools import lru_cache
+from importlib.machinery import ExtensionFileLoader
+from importlib.util import module_from_spec, spec_from_file_location
 from pathlib import Path
 
 import torch
@@ -27,6 +30,7 @@ import torch
 from .config import KernelPlan
 
 _LIB_PATH = Path(__file__).resolve().parent / "csrc" / "libreskv_b200.so"
+_HOST_PATH = _LIB_PATH.parent / "_host.so"
 _FAMILIES = ("compression", "attention", "cluster_mass")
 
 ERR_INVALID, ERR_WORKSPACE, ERR_CUDA, ERR_LIMIT = -1, -2, -3, -4
@@ -54,6 +58,8 @@ SIGNATURES = {
         _I,
         [_I, _I] + [_P] * 11 + [_I, _I, _I, _I, _L, _I, _I, _I, _I, _F, _P, _F, _I, _P, _P, _P, _I, _P, _Z, _P, _P, _P, _P],
     ),
+    "reskv_decode_args_workspace_bytes": (_Z, [_P]),
+    "reskv_decode_run": (_I, [_P]),
     "reskv_window_append": (_I, [_P] * 6 + [_I, _I, _I, _P, _P]),
     "reskv_window_write": (_I, [_P] * 6 + [_I, _I, _I, _I, _P]),
     "reskv_decode_step": (
@@ -101,8 +107,26 @@ def library() -> ctypes.CDLL:
     return lib
 
 
-# Kernels launched through this module since import (bench.py reports it).
-launch_count = 0
+@lru_cache(maxsize=1)
+def host():
+    """The native host module (``csrc/host.cpp``).  Raises if it was not built."""
+    library()
+    if not _HOST_PATH.exists():
+        raise RuntimeError(f"{_HOST_PATH} is missing: build it with `python -m reskv_b200.csrc.build`")
+    loader = ExtensionFileLoader("_host", str(_HOST_PATH))
+    module = module_from_spec(spec_from_file_location("_host", str(_HOST_PATH), loader=loader))
+    loader.exec_module(module)
+    return module
+
+
+# Kernels launched through `check` since import; `launch_count` (bench.py reports it) adds those of the native module.
+_launches = 0
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _launches + host().launches()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def check(rc: int, launches: int = 1) -> None:
@@ -111,8 +135,8 @@ def check(rc: int, launches: int = 1) -> None:
     RuntimeError subclasses, its Python checks as ValueError; callers match on
     the message), everything else ``RuntimeError``."""
     if rc >= 0:
-        global launch_count
-        launch_count += launches
+        global _launches
+        _launches += launches
         return
     msg = library().reskv_last_error().decode()
     if rc in (ERR_INVALID, ERR_LIMIT):
@@ -126,9 +150,6 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 def _stream(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
-
-
-_CHECK_STATUS = os.environ.get("RESKV_CHECK_STATUS") == "1"
 
 
 def device_index_of(device) -> int:
@@ -298,8 +319,7 @@ class CompressionOps(_Ops):
         xs = token_stride_of(x_k)
         if x_k.dtype != torch.float16 or x_v.dtype != torch.float16 or xs is None or xs != token_stride_of(x_v):
             raise ValueError("compress_group expects FP16 x[B,H,T,128] of one token stride")
-        layout = {"unstructured": LAYOUT_UNSTRUCTURED, "tiled": LAYOUT_TILED, "structured": LAYOUT_STRUCTURED,
-                  "compact": LAYOUT_COMPACT}[plan.layout]
+        layout = LAYOUT_IDS[plan.layout]
         args = []
         for old, new, buffers in sides:
             _same_device(self.device.index, old, new, *buffers)
@@ -331,66 +351,19 @@ def token_stride_of(x: torch.Tensor):
     return step // 128
 
 
-def _token_stride(rows: torch.Tensor, width: int) -> int:
-    """Tokens between units of a ``[units, T, width]`` (or ``[units, T]``) view."""
-    if rows.shape[0] == 1:
-        return rows.shape[1]
-    return rows.stride(0) // width
-
-
 LAYOUT_UNSTRUCTURED, LAYOUT_TILED, LAYOUT_STRUCTURED, LAYOUT_COMPACT = 0, 1, 2, 3
 
 
-def _decode(lib, layout, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta, scale,
-            splits, inv_freq, return_stats=True, recent=None):
-    """Allocate outputs and scratch, call the decode entry point of a layout.
+LAYOUT_IDS = {"unstructured": LAYOUT_UNSTRUCTURED, "tiled": LAYOUT_TILED, "structured": LAYOUT_STRUCTURED,
+              "compact": LAYOUT_COMPACT}
 
-    ``layout is None`` selects the unstructured FP16 bitmap kernel, ``LAYOUT_COMPACT``
-    ``reskv_decode_compact``, anything else ``reskv_decode_packed``.  ``recent = (q_rot [B*nh,128], k_rot, v [B,kh,Tr,128])``
-    folds a dense window into the same launch pair.
-    """
-    _same_device(lib._index, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, inv_freq, *(recent or ()))
-    bnh = q.shape[0]
-    b = bnh // nh
-    t, width = kp.shape[1], kp.shape[2]
-    stride = _token_stride(kp, width)
-    for rows in (ki, km, ks, vi, vp, vm, vs):
-        if rows is not None and rows.numel() and _token_stride(rows, rows.shape[2] if rows.ndim == 3 else 1) != stride:
-            raise ValueError("K and V cache tensors must share one token stride")
-    dev = q.device
-    need = lib.reskv_decode_bitmap_fp16_workspace_bytes(b, kh, nh, t, int(splits))
-    ws = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
-    if _CHECK_STATUS:
-        ws[:256].zero_()
-    out = torch.empty((bnh, 128), dtype=torch.float16, device=dev)
-    m = torch.empty(bnh, dtype=torch.float32, device=dev) if return_stats else None
-    l = torch.empty(bnh, dtype=torch.float32, device=dev) if return_stats else None
-    rq = rk = rv = None
-    tr = 0
-    if recent is not None and recent[1].shape[2] > 0:
-        rq, rk, rv = (x.contiguous() for x in recent)
-        tr = rk.shape[2]
-    tail = (b, kh, nh, t, stride, kc.shape[1], vc.shape[1])
-    rest = (int(start_pos), int(pos_q), float(rope_theta), _ptr(inv_freq), float(scale), int(splits), _ptr(rq),
-            _ptr(rk), _ptr(rv), tr, ws.data_ptr(), ws.numel(), out.data_ptr(), _ptr(m), _ptr(l), _stream(dev))
-    if layout is None:
-        rc = lib.reskv_decode_bitmap_fp16(q.data_ptr(), kc.data_ptr(), ki.data_ptr(), kp.data_ptr(), km.data_ptr(),
-                                          vc.data_ptr(), vi.data_ptr(), vp.data_ptr(), vm.data_ptr(), *tail, width,
-                                          *rest)
-    elif layout == LAYOUT_COMPACT:
-        rc = lib.reskv_decode_compact(bits, width * 32 // bits, q.data_ptr(), kc.data_ptr(), ki.data_ptr(), kp.data_ptr(),
-                                      _ptr(km), _ptr(ks), vc.data_ptr(), vi.data_ptr(), vp.data_ptr(), _ptr(vm),
-                                      _ptr(vs), *tail, *rest)
-    else:
-        rc = lib.reskv_decode_packed(layout, bits, q.data_ptr(), kc.data_ptr(), ki.data_ptr(), kp.data_ptr(),
-                                     _ptr(km), _ptr(ks), vc.data_ptr(), vi.data_ptr(), vp.data_ptr(), _ptr(vm),
-                                     _ptr(vs), *tail, *rest)
-    check(rc, launches=2)
-    if _CHECK_STATUS:
-        status = int(ws[:4].view(torch.int32).item())
-        if status:
-            raise RuntimeError(f"decode: device status {status:#x} (bounded wait ran out)")
-    return (out, m, l) if return_stats else (out,)
+
+def _decode(device, layout, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta, scale,
+            splits, inv_freq, return_stats=True, recent=None):
+    """The decode call of an operator table: outputs and scratch are allocated and the kernels of the layout launched
+    natively.  ``recent = (q_rot [B*nh,128], k_rot, v [B,kh,Tr,128])`` folds a dense window into the same launch pair."""
+    return host().decode(layout, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta,
+                         scale, splits, inv_freq, return_stats, recent, device.index)
 
 
 class ClusterMassOps(_Ops):
@@ -401,17 +374,17 @@ class ClusterMassOps(_Ops):
         """Unstructured FP16 bitmap decode -> ``(out, m, l)`` (``(out,)`` without
         stats), as cluster_mass.cu:1177-1296.  ``recent`` (not part of the
         reference signature) fuses the dense window into the same call."""
-        return _decode(self.lib, None, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh, start_pos, pos_q,
+        return _decode(self.device, LAYOUT_UNSTRUCTURED, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh, start_pos, pos_q,
                        rope_theta, scale, splits, inv_freq, return_stats, recent)
 
     def decode_structured_fp16(self, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta,
                                scale, return_stats=True, splits=0, inv_freq=None, recent=None):
-        return _decode(self.lib, LAYOUT_STRUCTURED, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh,
+        return _decode(self.device, LAYOUT_STRUCTURED, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh,
                        start_pos, pos_q, rope_theta, scale, splits, inv_freq, return_stats, recent)
 
     def decode_structured_int4(self, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta,
                                scale, return_stats=True, splits=0, inv_freq=None, recent=None):
-        return _decode(self.lib, LAYOUT_STRUCTURED, 4, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
+        return _decode(self.device, LAYOUT_STRUCTURED, 4, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
                        pos_q, rope_theta, scale, splits, inv_freq, return_stats, recent)
 
     def merge_recent(self, out, m, l, scores, v_recent, kh, nh):
@@ -431,25 +404,25 @@ class AttentionOps(_Ops):
                     splits=0, inv_freq=None, recent=None):
         """Tiled (64 values per token) or 4:16 structured (32 values) FP16 decode."""
         layout = LAYOUT_TILED if kp.shape[2] == 64 else LAYOUT_STRUCTURED
-        return _decode(self.lib, layout, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh, start_pos, pos_q,
+        return _decode(self.device, layout, 16, q, kc, ki, kp, km, None, vc, vi, vp, vm, None, kh, nh, start_pos, pos_q,
                        rope_theta, scale, splits, inv_freq, True, recent)
 
     def decode_int4(self, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta, scale,
                     splits=0, inv_freq=None, recent=None):
-        return _decode(self.lib, LAYOUT_STRUCTURED, 4, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
+        return _decode(self.device, LAYOUT_STRUCTURED, 4, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
                        pos_q, rope_theta, scale, splits, inv_freq, True, recent)
 
     def decode_quantized(self, q, kc, ki, kp, ks, vc, vi, vp, vs, kh, nh, start_pos, pos_q, rope_theta, scale, k_bits,
                          v_bits, splits=0, inv_freq=None, recent=None):
         if k_bits != v_bits or k_bits not in (2, 4):
             raise ValueError("decode_quantized expects equal key and value bit widths of 2 or 4")
-        return _decode(self.lib, LAYOUT_UNSTRUCTURED, k_bits, q, kc, ki, kp, None, ks, vc, vi, vp, None, vs, kh, nh,
+        return _decode(self.device, LAYOUT_UNSTRUCTURED, k_bits, q, kc, ki, kp, None, ks, vc, vi, vp, None, vs, kh, nh,
                        start_pos, pos_q, rope_theta, scale, splits, inv_freq, True, recent)
 
     def decode_compact(self, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos, pos_q, rope_theta, scale,
                        bits, splits=0, inv_freq=None, recent=None):
         """Compact quantised layout (not in the reference): bitmap + codes of the retained coordinates."""
-        return _decode(self.lib, LAYOUT_COMPACT, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
+        return _decode(self.device, LAYOUT_COMPACT, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start_pos,
                        pos_q, rope_theta, scale, splits, inv_freq, True, recent)
 
     def merge_recent(self, out, m, l, q_rope, k_recent, v_recent, kh, nh, scale):
@@ -481,6 +454,13 @@ def _load_extension(family: str, plan: KernelPlan | None = None, device_index: i
     template instances inside the prebuilt library at call time."""
     if family not in _FAMILIES:
         raise ValueError(f"unknown native family: {family}")
+    require_device(device_index)
+    return _TABLES[family](plan, device_index or 0)
+
+
+@lru_cache(maxsize=64)
+def require_device(device_index: int | None) -> None:
+    """Raises unless ``device_index`` is a GPU these kernels were built for."""
     if not torch.cuda.is_available():
         raise RuntimeError("ResKV B200 kernels need a CUDA device (there is no CPU path)")
     capability = torch.cuda.get_device_capability(device_index)
@@ -489,4 +469,3 @@ def _load_extension(family: str, plan: KernelPlan | None = None, device_index: i
             f"libreskv_b200 is built for sm_100a only; device {device_index} has compute capability "
             f"{capability[0]}.{capability[1]}"
         )
-    return _TABLES[family](plan, device_index or 0)

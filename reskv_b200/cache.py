@@ -100,7 +100,7 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         else:
             self._take_token(key_states, raw, value_states)
         self.length += q_len
-        return self.keys[:, :, : self.live], self.values[:, :, : self.live]
+        return self.keys.narrow(2, 0, self.live), self.values.narrow(2, 0, self.live)
 
     def _take_prompt(self, keys, raw, values):
         """Split a prompt of T tokens into sinks [0, s), a compressed run [s, s + n) and the dense tail."""
@@ -120,13 +120,11 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
     def _take_token(self, key, raw, value):
         """One launch writes the token's rotated key, raw key and value into slot ``live`` of the three
         buffers; a full window then gives its oldest group to the compressed segment."""
-        from ._extension import _stream, check
+        from ._extension import host
 
-        b, h, cap, _ = self.keys.shape
+        cap = self.keys.shape[2]
         if key.dtype == torch.float16 and key.is_cuda:
-            check(self._lib.reskv_window_write(self.keys.data_ptr(), self.raw_keys.data_ptr(), self.values.data_ptr(),
-                                               key.contiguous().data_ptr(), raw.contiguous().data_ptr(),
-                                               value.contiguous().data_ptr(), b, h, cap, self.live, _stream(key.device)))
+            host().window_write(self.keys, self.raw_keys, self.values, key, raw, value, self.live)
         else:  # other dtypes (a BF16 model before its cast): plain slice copies
             at = self.live
             for buf, src in ((self.keys, key), (self.raw_keys, raw), (self.values, value)):

@@ -3,23 +3,27 @@
     python -m reskv_b200.csrc.build [--force] [--verbose]
 
 One ``nvcc`` invocation per ``.cu`` file (object files under ``build/``), then a
-shared link next to this file.  Nothing links against torch or Python: the
-library is plain CUDA runtime code behind the C ABI of ``include/reskv_b200.h``.
-nvcc cross-compiles, so no GPU is needed to build.  ``RESKV_NVCC_FLAGS`` (environment) adds compiler flags for
+shared link next to this file.  The library does not link against torch or Python: it
+is plain CUDA runtime code behind the C ABI of ``include/reskv_b200.h``.  Next to it
+``_host.so`` is built from ``host.cpp``: the CPython module that takes torch tensors
+and calls that ABI.  nvcc cross-compiles, so no GPU is needed to build.  ``RESKV_NVCC_FLAGS`` (environment) adds compiler flags for
 experiment builds, e.g. ``RESKV_NVCC_FLAGS="-DRESKV_MMA_CTAS_PER_SM=3" python -m reskv_b200.csrc.build --force``.
 """
 
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 LIB = HERE / "libreskv_b200.so"
+HOST = HERE / "_host.so"
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
@@ -67,8 +71,22 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         list(pool.map(run, jobs))
     objs = [objdir / (s.stem + ".o") for s in sources()]
     if force or jobs or _stale(LIB, objs):
-        run([nvcc, *ARCH_FLAGS, "-shared", "-o", str(LIB), *map(str, objs), "-lcudart"])
+        run([nvcc, *ARCH_FLAGS, "-shared", "-Xlinker=-soname=libreskv_b200.so", "-o", str(LIB), *map(str, objs), "-lcudart"])
+    if force or _stale(HOST, [HERE / "host.cpp", headers[-1]]):
+        run(_host_command(nvcc))
     return LIB
+
+
+def _host_command(nvcc: str) -> list[str]:
+    """g++ for the tensor-facing module.  torch is only located, not imported: its headers and libraries sit in the
+    package, and at run time they are already loaded."""
+    torch = Path(importlib.util.find_spec("torch").origin).parent
+    cuda = Path(nvcc).resolve().parent.parent
+    includes = [torch / "include", torch / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    libs = ["c10", "c10_cuda", "torch_cpu", "torch_cuda", "torch_python"]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in includes), str(HERE / "host.cpp"), "-o",
+            str(HOST), f"-L{torch / 'lib'}", *(f"-l{lib}" for lib in libs), f"-L{cuda / 'lib64'}", "-lcudart", f"-L{HERE}",
+            "-lreskv_b200", "-Wl,-rpath,$ORIGIN"]
 
 
 if __name__ == "__main__":

@@ -443,7 +443,7 @@ struct MergeParams {
     int kh, nh, splits, cv, tr;
     float scaling;
     const int32_t* dyn;  // device step state: dyn[1] = recent tokens (overrides tr), or null
-    int recent_cap;      // tokens between units in rk / rv (== tr for contiguous windows)
+    int64_t recent_cap;  // tokens between units in rk / rv (== tr for contiguous windows)
     uint32_t* status;    // device status word of the call's workspace, or null
 };
 
@@ -856,8 +856,9 @@ struct DecodeArgs {
     float *out_m, *out_l;
     void* stream;
     const int32_t* dyn = nullptr;  // device step state {pos_q, recent tokens}
-    int recent_cap = 0;            // window capacity in tokens when dyn is given
+    int64_t recent_cap = 0;        // tokens between units of the window buffers (0: recent_tokens)
     bool clear_status = false;     // zero the workspace's status header once the arguments are accepted
+    bool device_memory = false;    // the caller vouches for the pointers: no pointer queries
 };
 
 // Which partial kernel dispatch_layout will pick for this call (its partial plan differs).
@@ -894,14 +895,18 @@ int decode_common(const DecodeArgs& a, LayoutId layout, bool has_meta, bool has_
         return fail(RESKV_ERR_INVALID, "%s: misaligned centroid (16 bytes) or query pointer", who);
     if ((a.rk && !aligned16(a.rk)) || (a.rv && !aligned16(a.rv)))
         return fail(RESKV_ERR_INVALID, "%s: recent keys and values must be 16-byte aligned", who);
-    if (int rc = check_device_pointer(a.q, who, "q")) return rc;
-    if (int rc = check_device_pointer(a.kp, who, "k_payload")) return rc;
-    if (int rc = check_device_pointer(a.out, who, "out")) return rc;
+    if (!a.device_memory) {
+        if (int rc = check_device_pointer(a.q, who, "q")) return rc;
+        if (int rc = check_device_pointer(a.kp, who, "k_payload")) return rc;
+        if (int rc = check_device_pointer(a.out, who, "out")) return rc;
+    }
     const bool has_recent = a.recent_tokens > 0;
     if (a.recent_tokens < 0 || (has_recent && (!a.rq || !a.rk || !a.rv)))
         return fail(RESKV_ERR_INVALID, "%s: recent window needs rotated q, rotated k and v", who);
     if (a.recent_tokens > kMaxRecent)
         return fail(RESKV_ERR_LIMIT, "%s: at most %d recent tokens, got %d", who, kMaxRecent, a.recent_tokens);
+    if (!a.dyn && a.recent_cap != 0 && a.recent_cap < a.recent_tokens)
+        return fail(RESKV_ERR_INVALID, "%s: window token stride smaller than the window", who);
 
     const int units = a.batch * a.kv_heads;
     const PartialPlan pp = plan_partials(units, a.tokens, a.splits, tensor_core_variant(layout, a), a.dyn != nullptr, a.tok_stride);
@@ -957,11 +962,65 @@ int decode_common(const DecodeArgs& a, LayoutId layout, bool has_meta, bool has_
     mp.out_m = a.out_m, mp.out_l = a.out_l;
     mp.kh = a.kv_heads, mp.nh = a.q_heads, mp.splits = splits, mp.cv = a.cv, mp.tr = a.recent_tokens;
     mp.scaling = a.scaling;
-    mp.dyn = a.dyn, mp.recent_cap = a.dyn ? a.recent_cap : a.recent_tokens;
+    mp.dyn = a.dyn, mp.recent_cap = a.recent_cap ? a.recent_cap : a.recent_tokens;
     mp.status = p.status;
-    return launch_merge(mp, units, a.dyn ? a.recent_cap : a.recent_tokens, s);
+    return launch_merge(mp, units, a.dyn ? static_cast<int>(a.recent_cap) : a.recent_tokens, s);
+}
+
+// The kernel layout of (layout, bits, nnz) and which per-token tensors it has; false when there is none.
+bool resolve_layout(int layout, int bits, int nnz, LayoutId& id, bool& meta, bool& scale) {
+    meta = true, scale = false;
+    if (layout == RESKV_LAYOUT_UNSTRUCTURED && bits == 16 && (nnz == 32 || nnz == 64)) {
+        id = nnz == 32 ? kBitmap32 : kBitmap64;
+    } else if (layout == RESKV_LAYOUT_UNSTRUCTURED && (bits == 4 || bits == 2)) {
+        id = bits == 4 ? kQuant4 : kQuant2, meta = false, scale = true;
+    } else if (layout == RESKV_LAYOUT_TILED && bits == 16) {
+        id = kTiled64;
+    } else if (layout == RESKV_LAYOUT_STRUCTURED && bits == 16) {
+        id = kStruct32;
+    } else if (layout == RESKV_LAYOUT_STRUCTURED && bits == 4) {
+        id = kStructInt4, scale = true;
+    } else if (layout == RESKV_LAYOUT_COMPACT && bits == 4 && (nnz == 64 || nnz == 32)) {
+        id = nnz == 64 ? kCompact4x64 : kCompact4x32, scale = true;
+    } else if (layout == RESKV_LAYOUT_COMPACT && bits == 2 && nnz == 64) {
+        id = kCompact2x64, scale = true;
+    } else {
+        return false;
+    }
+    return true;
+}
+
+DecodeArgs from_struct(const reskv_decode_args& s) {
+    DecodeArgs a{s.q, s.k_centroids, s.k_ids, s.k_payload, s.k_meta, s.k_scale, s.v_centroids, s.v_ids, s.v_payload, s.v_meta,
+                 s.v_scale, s.batch, s.kv_heads, s.q_heads, s.tokens, s.tok_stride, s.k_clusters, s.v_clusters, s.start_pos,
+                 s.pos_q, s.rope_theta, s.inv_freq, s.scaling, s.splits, s.recent_q, s.recent_k, s.recent_v, s.recent_tokens,
+                 s.workspace, s.workspace_bytes, s.out, s.out_m, s.out_l, s.stream};
+    a.recent_cap = s.recent_tok_stride;
+    a.device_memory = s.device_memory != 0;
+    return a;
 }
 }  // namespace
+
+extern "C" size_t reskv_decode_args_workspace_bytes(const reskv_decode_args* args) {
+    LayoutId id;
+    bool meta, scale;
+    if (!args || args->batch < 1 || args->kv_heads < 1 || args->q_heads < 1 || args->tokens < 1 ||
+        !resolve_layout(args->layout, args->bits, args->nnz, id, meta, scale))
+        return 0;
+    const DecodeArgs a = from_struct(*args);
+    const PartialPlan pp = plan_partials(a.batch * a.kv_heads, a.tokens, a.splits, tensor_core_variant(id, a), false, a.tok_stride);
+    return workspace_bytes(a.batch * a.q_heads, pp.slots);
+}
+
+extern "C" int reskv_decode_run(const reskv_decode_args* args) {
+    if (!args) return fail(RESKV_ERR_INVALID, "decode_run: null arguments");
+    LayoutId id;
+    bool meta, scale;
+    if (!resolve_layout(args->layout, args->bits, args->nnz, id, meta, scale))
+        return fail(RESKV_ERR_INVALID, "decode_run: no kernel for layout %d with %d-bit residuals (nnz %d)", args->layout,
+                    args->bits, args->nnz);
+    return decode_common(from_struct(*args), id, meta, scale, "decode");
+}
 
 extern "C" int reskv_decode_bitmap_fp16(const void* q, const void* k_centroids, const void* k_ids,
                                         const void* k_payload, const void* k_bitmap, const void* v_centroids,
@@ -1047,23 +1106,8 @@ extern "C" int reskv_decode_step(int layout, int bits, int nnz, const void* q, c
     if (!step_state) return fail(RESKV_ERR_INVALID, "decode_step: null step state");
     LayoutId id;
     bool meta = true, scale = false;
-    if (layout == RESKV_LAYOUT_UNSTRUCTURED && bits == 16 && (nnz == 32 || nnz == 64)) {
-        id = nnz == 32 ? kBitmap32 : kBitmap64;
-    } else if (layout == RESKV_LAYOUT_UNSTRUCTURED && (bits == 4 || bits == 2)) {
-        id = bits == 4 ? kQuant4 : kQuant2, meta = false, scale = true;
-    } else if (layout == RESKV_LAYOUT_TILED && bits == 16) {
-        id = kTiled64;
-    } else if (layout == RESKV_LAYOUT_STRUCTURED && bits == 16) {
-        id = kStruct32;
-    } else if (layout == RESKV_LAYOUT_STRUCTURED && bits == 4) {
-        id = kStructInt4, scale = true;
-    } else if (layout == RESKV_LAYOUT_COMPACT && bits == 4 && (nnz == 64 || nnz == 32)) {
-        id = nnz == 64 ? kCompact4x64 : kCompact4x32, scale = true;
-    } else if (layout == RESKV_LAYOUT_COMPACT && bits == 2 && nnz == 64) {
-        id = kCompact2x64, scale = true;
-    } else {
+    if (!resolve_layout(layout, bits, nnz, id, meta, scale))
         return fail(RESKV_ERR_INVALID, "decode_step: no kernel for layout %d with %d-bit residuals (nnz %d)", layout, bits, nnz);
-    }
     DecodeArgs a{q, k_centroids, k_ids, k_payload, k_meta, k_scale, v_centroids, v_ids, v_payload, v_meta, v_scale,
                  batch, kv_heads, q_heads, tokens, tok_stride, k_clusters, v_clusters, start_pos, 0, rope_theta,
                  inv_freq, scaling, splits, recent_q, window_k, window_v, 0, workspace, workspace_bytes_given, out,

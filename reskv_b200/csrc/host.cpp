@@ -1,0 +1,351 @@
+// Native host path of the decode-step calls: a CPython module (`_host`) that takes torch tensors, checks them,
+// allocates results and scratch from torch's caching allocator and calls the C ABI of libreskv_b200.so.
+//
+// Why native: a batch-1 decode attention is two kernels of ~8 us each, and the same work in Python (30 tensor
+// attribute reads, four allocations, a 30-argument ctypes call) took 65 us per call, so the GPU waited for the host
+// up to batch 8.  Nothing is kept between calls here: every pointer and size is read from the tensors of the call.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <Python.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdlib>
+#include <optional>
+#include <string>
+
+#include "../../include/reskv_b200.h"
+
+namespace {
+
+struct PyError {};  // a Python exception is set
+
+[[noreturn]] void value_error(const char* msg) {
+    PyErr_SetString(PyExc_ValueError, msg);
+    throw PyError{};
+}
+
+// The exception a failed library call stands for: argument problems are ValueError, the rest RuntimeError.
+void check(int rc) {
+    if (rc >= 0) return;
+    PyErr_SetString(rc == RESKV_ERR_INVALID || rc == RESKV_ERR_LIMIT ? PyExc_ValueError : PyExc_RuntimeError, reskv_last_error());
+    throw PyError{};
+}
+
+long long g_launches = 0;  // kernels launched through this module (the interpreter lock serialises the calls)
+bool g_check_status = false;
+
+const at::Tensor& tensor(PyObject* o, const char* what) {
+    if (!THPVariable_Check(o)) {
+        PyErr_Format(PyExc_TypeError, "%s must be a tensor", what);
+        throw PyError{};
+    }
+    return THPVariable_Unpack(o);
+}
+// None -> undefined tensor
+at::Tensor optional_tensor(PyObject* o, const char* what) { return o == Py_None ? at::Tensor() : tensor(o, what); }
+
+long long integer(PyObject* o) {  // int(o)
+    PyObject* i = PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o);
+    const long long v = i ? PyLong_AsLongLong(i) : -1;
+    Py_XDECREF(i);
+    if (v == -1 && PyErr_Occurred()) throw PyError{};
+    return v;
+}
+double number(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw PyError{};
+    return v;
+}
+PyObject* item(PyObject* tuple, Py_ssize_t i) {
+    PyObject* o = PyTuple_Check(tuple) ? PyTuple_GetItem(tuple, i) : nullptr;
+    if (!o) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "expected a tuple");
+        throw PyError{};
+    }
+    return o;
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+const void* data(const at::Tensor& t) { return t.defined() && t.numel() ? t.const_data_ptr() : nullptr; }
+
+void same_device(c10::DeviceIndex dev, const at::Tensor& t) {
+    if (t.defined() && (!t.is_cuda() || t.get_device() != dev)) {
+        const std::string at = t.device().str();
+        PyErr_Format(PyExc_ValueError, "all tensors of this call must live on cuda:%d, got one on %s", static_cast<int>(dev), at.c_str());
+        throw PyError{};
+    }
+}
+
+// Tokens between (sequence, head) units of x[B,H,T,128] when it is dense or a token slice of a dense
+// [B,H,capacity,128] buffer, else -1 (same rule as `token_stride_of` of the Python module).
+int64_t token_stride_of(const at::Tensor& x) {
+    const int64_t b = x.size(0), h = x.size(1), t = x.size(2);
+    if (x.size(3) != 128 || x.stride(3) != 1 || (t > 1 && x.stride(2) != 128)) return -1;
+    int64_t step;
+    if (h > 1)
+        step = x.stride(1);
+    else if (b > 1)
+        step = x.stride(0);
+    else
+        return t;
+    if (step % 128 || step / 128 < t || (h > 1 && b > 1 && x.stride(0) != h * step)) return -1;
+    return step / 128;
+}
+
+// One side of a compressed cache as the kernels take it: (centroids [U,C,128], ids [U,T], payload [U,T,w],
+// metadata [U,T,m] or None, scale [U,T] or None).
+struct Side {
+    at::Tensor centroids, ids, payload, meta, scale;
+    explicit Side(PyObject* native)
+        : centroids(tensor(item(native, 0), "centroids")), ids(tensor(item(native, 1), "ids")),
+          payload(tensor(item(native, 2), "payload")), meta(optional_tensor(item(native, 3), "metadata")),
+          scale(optional_tensor(item(native, 4), "scale")) {}
+    Side(PyObject* c, PyObject* i, PyObject* p, PyObject* m, PyObject* s)
+        : centroids(tensor(c, "centroids")), ids(tensor(i, "ids")), payload(tensor(p, "payload")),
+          meta(optional_tensor(m, "metadata")), scale(optional_tensor(s, "scale")) {}
+};
+
+int64_t rows_stride(const at::Tensor& rows) {  // tokens between units
+    const int64_t width = rows.dim() == 3 ? rows.size(2) : 1;
+    return rows.size(0) == 1 ? rows.size(1) : rows.stride(0) / width;
+}
+
+struct Decode {
+    int layout, bits, nnz;
+    const Side *k, *v;
+    int64_t kv_heads, q_heads, start, position;
+    double theta, scaling;
+    int64_t splits;
+    at::Tensor inv_freq;  // f32 [64], contiguous, or undefined
+    at::Tensor rq, rk, rv;  // dense window: rotated query, rotated keys, values; undefined for none
+    bool stats;
+};
+
+struct Result {
+    at::Tensor out, m, l;
+};
+
+// Outputs and scratch, then the library call.  q: contiguous [B*NH,128].
+Result run_decode(const Decode& d, const at::Tensor& q) {
+    const c10::DeviceIndex dev = q.get_device();
+    for (const Side* s : {d.k, d.v})
+        for (const at::Tensor* t : {&s->centroids, &s->ids, &s->payload, &s->meta, &s->scale}) same_device(dev, *t);
+    for (const at::Tensor* t : {&d.inv_freq, &d.rq, &d.rk, &d.rv}) same_device(dev, *t);
+    const int64_t tokens = d.k->payload.size(1), stride = rows_stride(d.k->payload);
+    for (const at::Tensor* t : {&d.k->ids, &d.k->meta, &d.k->scale, &d.v->ids, &d.v->payload, &d.v->meta, &d.v->scale})
+        if (t->defined() && t->numel() && rows_stride(*t) != stride) value_error("K and V cache tensors must share one token stride");
+    const c10::cuda::CUDAGuard guard(dev);
+    const int64_t rows = q.size(0);
+    reskv_decode_args a{};
+    a.layout = d.layout, a.bits = d.bits, a.nnz = d.nnz;
+    a.q = data(q);
+    a.k_centroids = data(d.k->centroids), a.k_ids = data(d.k->ids), a.k_payload = data(d.k->payload);
+    a.k_meta = data(d.k->meta), a.k_scale = data(d.k->scale);
+    a.v_centroids = data(d.v->centroids), a.v_ids = data(d.v->ids), a.v_payload = data(d.v->payload);
+    a.v_meta = data(d.v->meta), a.v_scale = data(d.v->scale);
+    a.batch = static_cast<int>(rows / d.q_heads), a.kv_heads = static_cast<int>(d.kv_heads), a.q_heads = static_cast<int>(d.q_heads);
+    a.tokens = static_cast<int>(tokens), a.tok_stride = stride;
+    a.k_clusters = static_cast<int>(d.k->centroids.size(1)), a.v_clusters = static_cast<int>(d.v->centroids.size(1));
+    a.start_pos = static_cast<int>(d.start), a.pos_q = static_cast<int>(d.position);
+    a.rope_theta = static_cast<float>(d.theta);
+    a.inv_freq = static_cast<const float*>(data(d.inv_freq));
+    a.scaling = static_cast<float>(d.scaling);
+    a.splits = static_cast<int>(d.splits);
+    at::Tensor rq, rk, rv;  // keep copies alive until the launch
+    if (d.rk.defined() && d.rk.size(2) > 0) {
+        rq = d.rq.contiguous(), rk = d.rk, rv = d.rv;
+        // window views of one token stride and 16-byte alignment are read in place
+        int64_t step = token_stride_of(rk);
+        if (step < 0 || step != token_stride_of(rv) || !aligned16(rk.const_data_ptr()) || !aligned16(rv.const_data_ptr())) {
+            rk = rk.contiguous(), rv = rv.contiguous();
+            step = rk.size(2);
+        }
+        a.recent_q = data(rq), a.recent_k = data(rk), a.recent_v = data(rv);
+        a.recent_tokens = static_cast<int>(rk.size(2)), a.recent_tok_stride = step;
+    }
+    a.device_memory = 1;
+    Result r;
+    const auto f32 = q.options().dtype(at::kFloat);
+    r.out = at::empty({rows, 128}, q.options());
+    if (d.stats) r.m = at::empty({rows}, f32), r.l = at::empty({rows}, f32);
+    const size_t need = reskv_decode_args_workspace_bytes(&a);
+    const at::Tensor ws = at::empty({static_cast<int64_t>(need < 256 ? 256 : need)}, q.options().dtype(at::kByte));
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+    if (g_check_status) cudaMemsetAsync(ws.data_ptr(), 0, 256, stream);
+    a.workspace = ws.data_ptr(), a.workspace_bytes = static_cast<size_t>(ws.numel());
+    a.out = r.out.data_ptr();
+    a.out_m = d.stats ? static_cast<float*>(r.m.data_ptr()) : nullptr;
+    a.out_l = d.stats ? static_cast<float*>(r.l.data_ptr()) : nullptr;
+    a.stream = stream;
+    check(reskv_decode_run(&a));
+    g_launches += 2;
+    if (g_check_status) {
+        unsigned status = 0;
+        cudaMemcpyAsync(&status, ws.data_ptr(), sizeof(status), cudaMemcpyDeviceToHost, stream);
+        cudaStreamSynchronize(stream);
+        if (status) {
+            PyErr_Format(PyExc_RuntimeError, "decode: device status 0x%x (bounded wait ran out)", status);
+            throw PyError{};
+        }
+    }
+    return r;
+}
+
+// Runs `f`, turning C++ exceptions into Python ones.
+template <class F>
+PyObject* guarded(F&& f) {
+    try {
+        return f();
+    } catch (const PyError&) {
+    } catch (const c10::OutOfMemoryError& e) {
+        PyObject* torch = PyImport_ImportModule("torch");
+        PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+        PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
+        Py_XDECREF(type);
+        Py_XDECREF(torch);
+    } catch (const c10::Error& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return nullptr;
+}
+
+void expect(Py_ssize_t got, Py_ssize_t want) {
+    if (got == want) return;
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, got);
+    throw PyError{};
+}
+
+// The two integers (layout, nnz) of an operator call: the retained count of the layouts that need one follows
+// from the payload width.
+int retained(int layout, int bits, const at::Tensor& payload) {
+    const int width = static_cast<int>(payload.size(2));
+    if (layout == RESKV_LAYOUT_COMPACT) return width * 32 / bits;
+    return bits == 16 ? width : 0;
+}
+
+// decode(layout, bits, q, kc, ki, kp, km, ks, vc, vi, vp, vm, vs, kh, nh, start, position, theta, scaling, splits,
+//        inv_freq, stats, recent, device) -> (out, m, l) or (out,).  The operator tables' calls; `device`: theirs.
+PyObject* py_decode(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 24);
+        const at::Tensor& q = tensor(o[2], "q");
+        same_device(static_cast<c10::DeviceIndex>(integer(o[23])), q);
+        const Side k(o[3], o[4], o[5], o[6], o[7]), v(o[8], o[9], o[10], o[11], o[12]);
+        Decode d{};
+        d.layout = static_cast<int>(integer(o[0])), d.bits = static_cast<int>(integer(o[1])), d.nnz = retained(d.layout, d.bits, k.payload);
+        d.k = &k, d.v = &v;
+        d.kv_heads = integer(o[13]), d.q_heads = integer(o[14]), d.start = integer(o[15]), d.position = integer(o[16]);
+        d.theta = number(o[17]), d.scaling = number(o[18]), d.splits = integer(o[19]);
+        d.inv_freq = optional_tensor(o[20], "inv_freq");
+        d.stats = PyObject_IsTrue(o[21]);
+        if (o[22] != Py_None) {
+            d.rq = tensor(item(o[22], 0), "recent query"), d.rk = tensor(item(o[22], 1), "recent keys");
+            d.rv = tensor(item(o[22], 2), "recent values");
+        }
+        const Result r = run_decode(d, q);
+        if (!d.stats) {
+            PyObject* t = PyTuple_New(1);
+            PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(r.out));
+            return t;
+        }
+        PyObject* t = PyTuple_New(3);
+        PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(r.out));
+        PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(r.m));
+        PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(r.l));
+        return t;
+    });
+}
+
+// attention(query, k_table [B,H,C,128], k_native, v_native, layout, bits, position, start, theta, inv_freq, scaling,
+//           recent, splits) -> [B,NH,1,128].  The tensor checks of the public `attention` (reskv/_attention.py:24-57).
+PyObject* py_attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 13);
+        if (!THPVariable_Check(o[0])) value_error("query must be FP16 CUDA [batch, query_heads, 1, 128]");
+        const at::Tensor& query = THPVariable_Unpack(o[0]);
+        if (query.dim() != 4 || query.size(2) != 1 || query.size(3) != 128 || !query.is_cuda() || query.scalar_type() != at::kHalf)
+            value_error("query must be FP16 CUDA [batch, query_heads, 1, 128]");
+        const int64_t b = query.size(0), nh = query.size(1);
+        const at::Tensor& table = tensor(o[1], "centroids");
+        const Side k(o[2]), v(o[3]);
+        const int64_t kh = table.size(1);
+        if (query.device() != k.payload.device() || query.device() != v.payload.device())
+            value_error("query and cache must be on the same CUDA device");
+        if (b != table.size(0) || k.ids.size(1) != v.ids.size(1)) value_error("query/cache batch or K/V sequence lengths differ");
+        if (nh % kh || (nh / kh != 1 && nh / kh != 4 && nh / kh != 8)) value_error("supported query/kv head ratios are 1, 4, and 8");
+        Decode d{};
+        d.layout = static_cast<int>(integer(o[4])), d.bits = static_cast<int>(integer(o[5])), d.nnz = retained(d.layout, d.bits, k.payload);
+        d.k = &k, d.v = &v, d.kv_heads = kh, d.q_heads = nh;
+        d.position = integer(o[6]), d.start = integer(o[7]);
+        if (d.position < d.start + k.ids.size(1) - 1) value_error("query position precedes compressed tokens");
+        d.theta = number(o[8]);
+        if (o[9] != Py_None) {
+            d.inv_freq = tensor(o[9], "inv_freq");
+            if (d.inv_freq.dim() != 1 || d.inv_freq.size(0) != 64 || d.inv_freq.device() != query.device())
+                value_error("inv_freq must be [64] on the query CUDA device");
+            if (d.inv_freq.scalar_type() != at::kFloat || !d.inv_freq.is_contiguous()) d.inv_freq = d.inv_freq.to(at::kFloat).contiguous();
+        }
+        d.scaling = o[10] == Py_None ? 0.08838834764831845 : number(o[10]);  // 128 ** -0.5
+        if (o[11] != Py_None) {
+            const at::Tensor& rk = tensor(item(o[11], 1), "recent keys");
+            if (rk.dim() < 3 || rk.size(2) > 0) {
+                const at::Tensor &rq = tensor(item(o[11], 0), "recent query"), &rv = tensor(item(o[11], 2), "recent values");
+                if (rq.sizes() != query.sizes() || rk.sizes() != rv.sizes() || rk.dim() != 4 || rk.size(0) != b || rk.size(1) != kh)
+                    value_error("recent Q/K/V shapes do not match the compressed cache");
+                for (const at::Tensor* t : {&rq, &rk, &rv})
+                    if (t->device() != query.device() || t->scalar_type() != at::kHalf)
+                        value_error("recent tensors must be FP16 on the query device");
+                d.rq = rq, d.rk = rk, d.rv = rv;
+            }
+        }
+        d.splits = integer(o[12]);
+        // only the memory order of q matters to the kernels: [B,NH,1,128] dense is [B*NH,128] dense
+        const at::Tensor q = (query.is_contiguous() ? query : query.contiguous()).view({b * nh, 128});
+        return THPVariable_Wrap(run_decode(d, q).out.view({b, nh, 1, 128}));
+    });
+}
+
+// window_write(keys, raw_keys, values, key, raw_key, value, slot): the new token's three rows into slot `slot`.
+PyObject* py_window_write(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 7);
+        const at::Tensor &wk = tensor(o[0], "keys"), &wr = tensor(o[1], "raw keys"), &wv = tensor(o[2], "values");
+        at::Tensor rows[3];
+        for (int i = 0; i < 3; ++i) {
+            rows[i] = tensor(o[3 + i], "token").contiguous();
+            same_device(wk.get_device(), rows[i]);
+            if (rows[i].scalar_type() != at::kHalf || rows[i].numel() != wk.size(0) * wk.size(1) * 128)
+                value_error("window_write expects FP16 rows [B,H,1,128]");
+        }
+        const c10::cuda::CUDAGuard guard(wk.get_device());
+        check(reskv_window_write(wk.data_ptr(), wr.data_ptr(), wv.data_ptr(), rows[0].const_data_ptr(), rows[1].const_data_ptr(),
+                                 rows[2].const_data_ptr(), static_cast<int>(wk.size(0)), static_cast<int>(wk.size(1)),
+                                 static_cast<int>(wk.size(2)), static_cast<int>(integer(o[6])),
+                                 c10::cuda::getCurrentCUDAStream(wk.get_device()).stream()));
+        ++g_launches;
+        Py_RETURN_NONE;
+    });
+}
+
+PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
+
+#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f))
+PyMethodDef g_methods[] = {
+    {"decode", FAST(py_decode), METH_FASTCALL, "decode attention on given operands"},
+    {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
+    {"window_write", FAST(py_window_write), METH_FASTCALL, "append one token to the dense window"},
+    {"launches", py_launches, METH_NOARGS, "kernels launched through this module"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, g_methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() {
+    const char* v = std::getenv("RESKV_CHECK_STATUS");
+    g_check_status = v && std::string(v) == "1";
+    return PyModule_Create(&g_module);
+}
