@@ -216,12 +216,18 @@ int reskv_step_advance(int32_t* step_state, int position_increment, int window_i
  *                   the key rotated, the raw key and the value go to slot step_state[1] - 1 of
  *                   the window buffers ([batch*kv_heads,window_capacity,128]) when those are
  *                   given, and / or to k_rot / v_out ([batch*kv_heads,128]).
+ * reskv_rope_prompt: the same split and rotation for a whole prompt: qkv [batch, tokens, (q | k | v heads) * 128],
+ *                   cos_table / sin_table f32 [tokens, 64]; writes q_rot, k_raw, k_rot, v as
+ *                   [batch, heads, tokens, 128].
  * reskv_silu_mul:   out[r][j] = silu(gate_up[r][j]) * gate_up[r][ffn + j]; gate_up [rows, 2 ffn]. */
 int reskv_rms_norm(const void* x, const void* weight, void* out, int rows, int dim, float eps, void* stream);
 
 int reskv_rope_split(const void* qkv, int batch, int q_heads, int kv_heads, const float* inv_freq,
                      const int32_t* step_state, void* q_raw, void* q_rot, void* k_rot, void* v_out, void* window_k,
                      void* window_raw, void* window_v, int window_capacity, void* stream);
+
+int reskv_rope_prompt(const void* qkv, int batch, int tokens, int q_heads, int kv_heads, const float* cos_table,
+                      const float* sin_table, void* q_rot, void* k_raw, void* k_rot, void* v, void* stream);
 
 int reskv_silu_mul(const void* gate_up, void* out, int rows, int ffn, void* stream);
 

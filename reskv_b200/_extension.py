@@ -69,6 +69,7 @@ SIGNATURES = {
     "reskv_step_advance": (_I, [_P, _I, _I, _P]),
     "reskv_rms_norm": (_I, [_P, _P, _P, _I, _I, _F, _P]),
     "reskv_rope_split": (_I, [_P, _I, _I, _I, _P, _P] + [_P] * 7 + [_I, _P]),
+    "reskv_rope_prompt": (_I, [_P, _I, _I, _I, _I] + [_P] * 7),
     "reskv_silu_mul": (_I, [_P, _P, _I, _I, _P]),
     "reskv_decode_auto_splits": (_I, [_I, _I, _I]),
     "reskv_decode_noalloc_status": (_I, [_P, _P]),

@@ -137,6 +137,11 @@ class ResKVLlama:
         self.scaling = hd**-0.5
         self.caches = None
         self.length = 0
+        self._lib = None
+        # graph decode: stream of the captures, the last captured graph (owner of their memory pool), batch sizes whose
+        # step has run once
+        self._capture_stream = self._last_graph = None
+        self._warm = set()
 
     # -- helpers -----------------------------------------------------------------------------
     def _all_reduce(self, x):
@@ -148,22 +153,59 @@ class ResKVLlama:
         ang = torch.arange(start, start + n, device=self.device).float()[:, None] * self.inv_freq[None, :]
         return ang.cos(), ang.sin()
 
-    def _mlp(self, layer, x):
-        out = torch.empty_like(x)
-        flat, oflat = x.reshape(-1, x.shape[-1]), out.reshape(-1, x.shape[-1])
-        for i in range(0, flat.shape[0], self.prefill_chunk):
-            gu = F.linear(flat[i:i + self.prefill_chunk], layer["w_gate_up"])
-            gate = F.silu(gu[:, :self.ffn])
-            gate.mul_(gu[:, self.ffn:])
-            oflat[i:i + self.prefill_chunk] = F.linear(gate, layer["w_down"])
-        return self._all_reduce(out)
+    def _native(self):
+        """The library with the model's device current, or ``None`` for a model on the CPU (dense cache only)."""
+        from .._extension import bound_library
 
-    def _qkv(self, layer, x):
+        if self._lib is None and self.device.type == "cuda":
+            self._lib = bound_library(self.device)
+        return self._lib
+
+    def _norm(self, x, weight):
+        # tensor operations, not the decode step's kernel: what is kept of a prompt's keys hangs on their last bit, and
+        # the order of this sum decides it
+        return _rms_norm(x, weight, self.shape.rms_eps)
+
+    def _add_projection(self, x, inp, weight):
+        """``x += inp @ weight^T`` in place (residual branch), summed over the tensor-parallel group."""
+        x += self._all_reduce(F.linear(inp, weight))
+
+    def _add_mlp(self, layer, x):
+        """``x += MLP(norm(x))`` in place, at most ``prefill_chunk`` tokens at a time."""
+        lib, flat = self._native(), x.view(-1, x.shape[-1])
+        for i in range(0, flat.shape[0], self.prefill_chunk):
+            part = flat[i:i + self.prefill_chunk]
+            gu = F.linear(self._norm(part, layer["norm2"]), layer["w_gate_up"])
+            if lib is None or self.ffn % 2:
+                act = F.silu(gu[:, :self.ffn])
+                act.mul_(gu[:, self.ffn:])
+            else:
+                from .._extension import _stream, check
+
+                act = torch.empty((gu.shape[0], self.ffn), dtype=gu.dtype, device=gu.device)
+                check(lib.reskv_silu_mul(gu.data_ptr(), act.data_ptr(), gu.shape[0], self.ffn, _stream(self.device)))
+            del gu
+            self._add_projection(part, act, layer["w_down"])
+
+    def _qkv(self, layer, x, trig, k_raw, k_rot, v_all):
+        """Projections of ``x [B,T,hidden]``: raw keys, rotated keys and values into the given ``[B,Hkv,T,128]``
+        tensors; returns raw and rotated queries ``[B,Hq,T,128]``."""
         b, t, _ = x.shape
-        qkv = F.linear(_rms_norm(x, layer["norm1"], self.shape.rms_eps), layer["wqkv"])
-        q, k, v = qkv.split((self.h_q * 128, self.h_kv * 128, self.h_kv * 128), dim=-1)
-        return (q.reshape(b, t, self.h_q, 128).transpose(1, 2), k.reshape(b, t, self.h_kv, 128).transpose(1, 2),
-                v.reshape(b, t, self.h_kv, 128).transpose(1, 2).contiguous())
+        cos, sin = trig
+        qkv = F.linear(self._norm(x, layer["norm1"]), layer["wqkv"])
+        lib = self._native()
+        if lib is not None:
+            from .._extension import _stream, check
+
+            q_rot = torch.empty((b, self.h_q, t, 128), dtype=torch.float16, device=self.device)
+            check(lib.reskv_rope_prompt(qkv.data_ptr(), b, t, self.h_q, self.h_kv, cos.data_ptr(), sin.data_ptr(),
+                                        q_rot.data_ptr(), k_raw.data_ptr(), k_rot.data_ptr(), v_all.data_ptr(),
+                                        _stream(self.device)))
+            return qkv[..., :self.h_q * 128].unflatten(-1, (self.h_q, 128)).transpose(1, 2), q_rot
+        q, k, v = (part.reshape(b, t, -1, 128).transpose(1, 2) for part in
+                   qkv.split((self.h_q * 128, self.h_kv * 128, self.h_kv * 128), dim=-1))
+        k_raw.copy_(k), v_all.copy_(v), k_rot.copy_(_rope(k, cos, sin))
+        return q, _rope(q, cos, sin)
 
     # -- prefill / decode ----------------------------------------------------------------------
     @torch.no_grad()
@@ -174,7 +216,7 @@ class ResKVLlama:
         ``prefill_chunk`` tokens at a time) so that their FP32 temporaries stay small at long contexts;
         the cache of a layer receives the whole batch at once."""
         b, t = ids.shape
-        cos, sin = self._trig(0, t)
+        trig = self._trig(0, t)
         x = self.embed[ids]
         self.caches = []
         rows = max(1, self.prefill_chunk // t)  # sequences per slice
@@ -182,14 +224,13 @@ class ResKVLlama:
         for layer in self.layers:
             k_raw = torch.empty((b, self.h_kv, t, 128), **half)
             k_rot, v_all = torch.empty_like(k_raw), torch.empty_like(k_raw)
-            att = torch.empty((b, t, self.h_q * 128), **half)
             for i in range(0, b, rows):
-                q, k, v = self._qkv(layer, x[i:i + rows])
-                qr, kr = _rope(q, cos, sin), _rope(k, cos, sin)
-                out = F.scaled_dot_product_attention(qr, kr, v, is_causal=t > 1, enable_gqa=True, scale=self.scaling)
-                att[i:i + rows] = out.transpose(1, 2).reshape(-1, t, self.h_q * 128)
-                k_raw[i:i + rows], k_rot[i:i + rows], v_all[i:i + rows] = k, kr, v
-                del q, k, v, qr, kr, out
+                part = slice(i, i + rows)
+                _, qr = self._qkv(layer, x[part], trig, k_raw[part], k_rot[part], v_all[part])
+                att = F.scaled_dot_product_attention(qr, k_rot[part], v_all[part], is_causal=t > 1, enable_gqa=True,
+                                                     scale=self.scaling)
+                self._add_projection(x[part], att.transpose(1, 2).reshape(-1, t, self.h_q * 128), layer["wo"])
+                del qr, att
             if self.cache_kind == "reskv":
                 cache = ResKVLayerCache(self.kernel_config, self.sink_tokens)
                 cache.update(k_rot, v_all, {"raw_keys": k_raw})
@@ -200,29 +241,25 @@ class ResKVLlama:
                 cache.append(k_rot, v_all)
             self.caches.append(cache)
             del k_raw, k_rot, v_all
-            for i in range(0, b, rows):
-                x[i:i + rows] += self._all_reduce(F.linear(att[i:i + rows], layer["wo"]))
-            del att
-            for i in range(0, b, rows):
-                x[i:i + rows] += self._mlp(layer, _rms_norm(x[i:i + rows], layer["norm2"], self.shape.rms_eps))
+            self._add_mlp(layer, x)
         self.length = t
         return self._logits(x[:, -1:])
 
     def _logits(self, x):
-        return F.linear(_rms_norm(x, self.final_norm, self.shape.rms_eps), self.lm_head)[:, 0].float()
+        return F.linear(self._norm(x, self.final_norm), self.lm_head)[:, 0].float()
 
     @torch.no_grad()
     def decode(self, tokens: torch.Tensor) -> torch.Tensor:
         """One step for ``tokens [B]``; returns logits ``[B, vocab]``."""
         b = tokens.shape[0]
         pos = self.length
-        cos, sin = self._trig(pos, 1)
+        trig = self._trig(pos, 1)
         x = self.embed[tokens].unsqueeze(1)
         for layer, cache in zip(self.layers, self.caches):
-            q, k, v = self._qkv(layer, x)
-            qr, kr = _rope(q, cos, sin), _rope(k, cos, sin)
+            k, kr, v = torch.empty((3, b, self.h_kv, 1, 128), dtype=torch.float16, device=self.device)
+            q, qr = self._qkv(layer, x, trig, k, kr, v)
             if self.cache_kind == "reskv":
-                keys, values = cache.update(kr, v, {"raw_keys": k.contiguous()})
+                keys, values = cache.update(kr, v, {"raw_keys": k})
                 if cache.compressed is not None:
                     att = attention(q.contiguous(), cache.compressed, position=pos, start_position=cache.start_position,
                                     inv_freq=self.inv_freq, scaling=self.scaling, recent=(qr, keys, values))
@@ -231,8 +268,8 @@ class ResKVLlama:
             else:
                 keys, values = cache.append(kr, v)
                 att = F.scaled_dot_product_attention(qr, keys, values, enable_gqa=True, scale=self.scaling)
-            x = x + self._all_reduce(F.linear(att.transpose(1, 2).reshape(b, 1, -1), layer["wo"]))
-            x = x + self._mlp(layer, _rms_norm(x, layer["norm2"], self.shape.rms_eps))
+            self._add_projection(x, att.transpose(1, 2).reshape(b, 1, -1), layer["wo"])
+            self._add_mlp(layer, x)
         self.length += 1
         return self._logits(x)
 
@@ -336,8 +373,9 @@ class ResKVLlama:
         from .._extension import library
 
         self._tok_in = torch.zeros(batch, dtype=torch.long, device=self.device)
-        self._graph = None
-        self._warmed = False
+        self._graph = self._logits_out = None
+        if self._capture_stream is None:
+            self._capture_stream = torch.cuda.Stream(device=self.device)
         if self.cache_kind == "reskv":
             self._state = torch.zeros(4, dtype=torch.int32, device=self.device)
             # centroid tables at their final shape (zero rows beyond the live count), one pair per layer
@@ -375,6 +413,35 @@ class ResKVLlama:
             self._graph_addresses = addresses
             self._graph = None
 
+    def _capture_step(self):
+        """Capture one decode step as a CUDA graph.
+
+        ``torch.cuda.graph`` would collect garbage and empty the allocator's cache first, and everything a server
+        allocates next would go back to ``cudaMalloc`` (72 of 114 ms for a prompt of 4 x 1024 tokens and 72 steps).  The
+        step's temporaries come from one pool per model: the graph captured last stays alive, and with it the pool,
+        until the next capture has taken the pool over."""
+        side, main = self._capture_stream, torch.cuda.current_stream(self.device)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            if self._tok_in.shape[0] not in self._warm:
+                # once per batch size: a step outside capture (library handles, lazy inits), on a state that is restored
+                reskv = self.cache_kind == "reskv"
+                counts = self._state if reskv else self._seqlens
+                saved, saved_state = counts.clone(), self._state.clone()
+                self._step_body(self._tok_in)
+                self._state.copy_(saved_state)
+                if not reskv:
+                    counts.copy_(saved)
+                self._warm.add(self._tok_in.shape[0])
+            graph = torch.cuda.CUDAGraph()
+            graph.capture_begin(pool=None if self._last_graph is None else self._last_graph.pool())
+            try:
+                self._logits_out = self._step_body(self._tok_in)
+            finally:
+                graph.capture_end()
+        main.wait_stream(side)
+        self._graph = self._last_graph = graph
+
     @torch.no_grad()
     def decode_graph(self, tokens: torch.Tensor) -> torch.Tensor:
         """Same result as ``decode`` but replaying a captured CUDA graph of the step."""
@@ -387,23 +454,8 @@ class ResKVLlama:
                 cache._compress_oldest_group()
             self._sync_graph_inputs()
         self._tok_in.copy_(tokens)
-        if self._graph is None and not self._warmed:
-            # once: a warm-up outside capture (library handles, lazy inits), on a state copy that is restored
-            self._warmed = True
-            saved = self._state.clone()
-            saved_len = None if self.cache_kind == "reskv" else self._seqlens.clone()
-            side = torch.cuda.Stream(device=self.device)
-            side.wait_stream(torch.cuda.current_stream(self.device))
-            with torch.cuda.stream(side):
-                self._step_body(self._tok_in)
-            torch.cuda.current_stream(self.device).wait_stream(side)
-            self._state.copy_(saved)
-            if saved_len is not None:
-                self._seqlens.copy_(saved_len)
         if self._graph is None:
-            self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph):
-                self._logits_out = self._step_body(self._tok_in)
+            self._capture_step()
         self._graph.replay()
         self.length += 1
         if self.cache_kind == "reskv":
