@@ -22,9 +22,9 @@
 // shared by all query heads of the KV head (GQA); RoPE sin/cos advance by a
 // fixed rotation per token and are re-seeded every 16 tiles.
 //
-// Kernel 2 (merge): one CTA per query head reduces the split partials, applies
-// the value centroids, and -- when a dense recent window is given -- folds its
-// tokens into the same softmax.
+// Kernel 2 (merge, decode_merge.cu) reduces the split partials, applies the value
+// centroids, and -- when a dense recent window is given -- folds its tokens into
+// the same softmax.
 #include "decode_common.cuh"
 
 namespace reskv {
@@ -424,242 +424,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_simt_partial_kernel(const 
 }
 
 #include "decode_mma.cuh"
-
-// ---- merge -----------------------------------------------------------------------
-struct MergeParams {
-    const float* ws_m;      // log2-domain maxima [BNH][splits], or natural-log m [BNH] when splits == 0
-    const float* ws_l;
-    const float* ws_delta;
-    const float* ws_beta;
-    const __half* vc;       // [B*KH,CV,128]
-    const __half* comp_out; // splits == 0: finished compressed result to merge with
-    const __half* rq;       // rotated query [BNH,128] or null
-    const __half* rk;       // rotated recent keys [B*KH,Tr,128] or null
-    const __half* rv;       // recent values
-    const float* rscores;   // precomputed scaled scores [BNH,Tr] (natural units) or null
-    __half* out;
-    float* out_m;
-    float* out_l;
-    int kh, nh, splits, cv, tr;
-    float scaling;
-    const int32_t* dyn;  // device step state: dyn[1] = recent tokens (overrides tr), or null
-    int64_t recent_cap;  // tokens between units in rk / rv (== tr for contiguous windows)
-    uint32_t* status;    // device status word of the call's workspace, or null
-};
-
-constexpr int kMergeThreads = 128;
-constexpr int kMaxRecent = 1024;  // recent tokens whose scores fit the shared buffer
-constexpr int kRecentChunk = 32;  // recent tokens staged in shared memory at a time
-
-// rows x 128 FP16 values, global -> shared, 16 bytes per thread and copy (all in flight at once)
-__device__ __forceinline__ void stage_rows(__half* dst, const __half* src, int rows, int tid, int threads) {
-    for (int i = tid; i < rows * (kHeadDim / 8); i += threads) cp_async16(dst + i * 8, src + i * 8);
-}
-
-// dynamic shared memory of the merge kernel: value centroids, one chunk of recent keys and of recent
-// values (shared by the unit's query heads), recent scores per head
-constexpr int kMergePartStride = kHeadDim + kMaxClusters + 4;
-size_t merge_smem_bytes(int cv, int gqa, int recent_max) {
-    return (static_cast<size_t>(cv) + 2 * kRecentChunk) * kHeadDim * sizeof(__half) +
-           static_cast<size_t>(gqa) * ((kMergeThreads / 32) * kMergePartStride + (recent_max + 3) / 4 * 4) * sizeof(float);
-}
-
-// One CTA per (sequence, KV head) unit, 128 threads per query head of the unit; thread (h, d) owns
-// output coordinate d of head h.  Everything that is read with a stride or by several heads (value
-// centroids, recent keys and values) is staged in shared memory by 16-byte asynchronous copies
-// issued up front, so the kernel pays a few memory round trips instead of one per centroid and
-// per recent token.
-__global__ void __launch_bounds__(1024) decode_merge_kernel(const MergeParams p, int recent_max) {
-    extern __shared__ __align__(16) unsigned char merge_smem[];
-    __shared__ float beta_s[8][kMaxClusters];
-    __shared__ float red[8][kMergeThreads / 32];
-    constexpr int kPartStride = kMergePartStride;  // per (head, warp): delta, cluster masses, max, sum
-    const int gqa = p.nh / p.kh, threads = gqa * kMergeThreads;
-    const int unit = blockIdx.x, tid = threadIdx.x;
-    const int h = tid / kMergeThreads, d = tid % kMergeThreads, lane = d & 31, warp = d >> 5;
-    const int fq = unit * gqa + h;  // (b * kh + hkv) * gqa + h == b * nh + hkv * gqa + h
-    const int sc_stride = (recent_max + 3) / 4 * 4;
-    __half* vc_s = reinterpret_cast<__half*>(merge_smem);
-    __half* rk_s = vc_s + static_cast<size_t>(p.cv) * kHeadDim;
-    __half* rv_s = rk_s + kRecentChunk * kHeadDim;
-    float* part_s = reinterpret_cast<float*>(rv_s + kRecentChunk * kHeadDim);  // [gqa][4 warps][kPartStride]
-    float* sc_s = part_s + gqa * (kMergeThreads / 32) * kPartStride + h * sc_stride;
-    const int tr = p.dyn ? min(p.dyn[1], recent_max) : p.tr;
-    // a window count beyond the buffers is cut (the newest tokens are then missing from the result): tell the host
-    if (p.dyn && p.status && tid == 0 && unit == 0 && (p.dyn[1] > recent_max || p.dyn[1] < 0))
-        atomicOr(p.status, RESKV_STATUS_STATE_RANGE);
-    const bool dot_scores = tr > 0 && !p.rscores;
-    const __half* rk_g = p.rk ? p.rk + static_cast<size_t>(unit) * p.recent_cap * kHeadDim : nullptr;
-    const __half* rv_g = p.rv ? p.rv + static_cast<size_t>(unit) * p.recent_cap * kHeadDim : nullptr;
-
-    // group 0: value centroids + first chunk of recent keys; group 1: first chunk of recent values
-    if (p.splits > 0) stage_rows(vc_s, p.vc + static_cast<size_t>(unit) * p.cv * kHeadDim, p.cv, tid, threads);
-    if (dot_scores) stage_rows(rk_s, rk_g, min(tr, kRecentChunk), tid, threads);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (tr > 0) stage_rows(rv_s, rv_g, min(tr, kRecentChunk), tid, threads);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-
-    // rotated query of this head, requested together with everything else the kernel reads
-    float qv[4] = {0.f, 0.f, 0.f, 0.f};
-    if (dot_scores) {
-        const __half* qrow = p.rq + static_cast<size_t>(fq) * kHeadDim;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) qv[i] = __half2float(qrow[lane + 32 * i]);
-    }
-
-    // compressed part: numerator `num`, max `m2` (log2 domain), sum `l`
-    float m2, l, num;
-    if (p.splits > 0) {
-        // The four warps of a head share the splits (warp w takes splits w, w + 4, ...) and read each
-        // partial row with 16-byte loads (lane: coordinates 4 lane .. 4 lane + 3; lanes 0..15 also four
-        // cluster masses), so all loads of a warp are in flight together; the four partial results are
-        // combined through shared memory.
-        const float* pm = p.ws_m + static_cast<size_t>(fq) * p.splits;
-        const float* pl = p.ws_l + static_cast<size_t>(fq) * p.splits;
-        float wm = -INFINITY;
-        for (int s = warp; s < p.splits; s += kMergeThreads / 32) wm = fmaxf(wm, pm[s]);
-        float wl = 0.f;
-        float4 wn = make_float4(0.f, 0.f, 0.f, 0.f), wb = wn;
-#pragma unroll 4
-        for (int s = warp; s < p.splits; s += kMergeThreads / 32) {
-            if (pm[s] == -INFINITY) continue;  // empty slot: its delta / beta rows were never written
-            const float w = fast_exp2(pm[s] - wm);
-            const size_t row = static_cast<size_t>(fq) * p.splits + s;
-            const float4 dv = *reinterpret_cast<const float4*>(p.ws_delta + row * kHeadDim + 4 * lane);
-            wl += pl[s] * w;
-            wn.x += dv.x * w, wn.y += dv.y * w, wn.z += dv.z * w, wn.w += dv.w * w;
-            if (lane < kMaxClusters / 4) {
-                const float4 bv = *reinterpret_cast<const float4*>(p.ws_beta + row * kMaxClusters + 4 * lane);
-                wb.x += bv.x * w, wb.y += bv.y * w, wb.z += bv.z * w, wb.w += bv.w * w;
-            }
-        }
-        float* slot = part_s + (h * (kMergeThreads / 32) + warp) * kPartStride;  // [delta 128 | beta 64 | m | l]
-        *reinterpret_cast<float4*>(slot + 4 * lane) = wn;
-        if (lane < kMaxClusters / 4) *reinterpret_cast<float4*>(slot + kHeadDim + 4 * lane) = wb;
-        if (lane == 0) slot[kHeadDim + kMaxClusters] = wm, slot[kHeadDim + kMaxClusters + 1] = wl;
-        __syncthreads();
-        const float* mine = part_s + h * (kMergeThreads / 32) * kPartStride;
-        m2 = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kMergeThreads / 32; ++w) m2 = fmaxf(m2, mine[w * kPartStride + kHeadDim + kMaxClusters]);
-        l = 0.f, num = 0.f;
-        float bsum = 0.f;
-#pragma unroll
-        for (int w = 0; w < kMergeThreads / 32; ++w) {
-            const float* ps = mine + w * kPartStride;
-            const float pmw = ps[kHeadDim + kMaxClusters];
-            const float sc = (pmw == -INFINITY) ? 0.f : fast_exp2(pmw - m2);
-            l += ps[kHeadDim + kMaxClusters + 1] * sc;
-            num += ps[d] * sc;
-            if (d < p.cv) bsum += ps[kHeadDim + d] * sc;
-        }
-        if (d < kMaxClusters) beta_s[h][d] = (d < p.cv) ? bsum : 0.f;
-        if (d == 0) {
-            if (p.out_m) p.out_m[fq] = m2 * kLn2;
-            if (p.out_l) p.out_l[fq] = l;
-        }
-    } else {
-        m2 = p.ws_m[fq] * kLog2e;
-        l = p.ws_l[fq];
-        num = __half2float(p.comp_out[static_cast<size_t>(fq) * kHeadDim + d]) * l;
-    }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();  // beta_s, vc_s and the first key chunk are in place
-    if (p.splits > 0) {
-#pragma unroll 8
-        for (int c = 0; c < p.cv; ++c) num = fmaf(beta_s[h][c], __half2float(vc_s[c * kHeadDim + d]), num);
-    }
-
-    if (tr > 0) {
-        // scores of the recent tokens (log2 domain) into shared memory
-        if (p.rscores) {
-            for (int t = d; t < tr; t += kMergeThreads)
-                sc_s[t] = p.rscores[static_cast<size_t>(fq) * tr + t] * kLog2e;
-        } else {
-            const float mul = p.scaling * kLog2e;
-            for (int c0 = 0; c0 < tr; c0 += kRecentChunk) {
-                const int n = min(kRecentChunk, tr - c0);
-                if (c0 > 0) {  // later chunks: plain staging, one round trip each
-                    __syncthreads();
-                    stage_rows(rk_s, rk_g + static_cast<size_t>(c0) * kHeadDim, n, tid, threads);
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                    asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    __syncthreads();
-                }
-                for (int t = warp; t < n; t += kMergeThreads / 32) {
-                    const __half* krow = rk_s + t * kHeadDim;
-                    float dot = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) dot = fmaf(qv[i], __half2float(krow[lane + 32 * i]), dot);
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
-                    if (lane == 0) sc_s[c0 + t] = dot * mul;
-                }
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // scores and the first value chunk are in place
-        float rm = -INFINITY;
-        for (int t = d; t < tr; t += kMergeThreads) rm = fmaxf(rm, sc_s[t]);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xffffffffu, rm, off));
-        if (lane == 0) red[h][warp] = rm;
-        __syncthreads();
-        rm = fmaxf(fmaxf(red[h][0], red[h][1]), fmaxf(red[h][2], red[h][3]));
-        const float jm = fmaxf(rm, m2);
-        const float cw = (m2 == -INFINITY) ? 0.f : fast_exp2(m2 - jm);
-        float rnum = 0.f, rl = 0.f;
-        for (int c0 = 0; c0 < tr; c0 += kRecentChunk) {
-            const int n = min(kRecentChunk, tr - c0);
-            if (c0 > 0) {
-                __syncthreads();
-                stage_rows(rv_s, rv_g + static_cast<size_t>(c0) * kHeadDim, n, tid, threads);
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                __syncthreads();
-            }
-#pragma unroll 8
-            for (int t = 0; t < n; ++t) {
-                const float w = fast_exp2(sc_s[c0 + t] - jm);
-                rl += w;
-                rnum = fmaf(w, __half2float(rv_s[t * kHeadDim + d]), rnum);
-            }
-        }
-        num = num * cw + rnum;
-        l = l * cw + rl;
-    }
-    p.out[static_cast<size_t>(fq) * kHeadDim + d] = __float2half_rn(num / fmaxf(l, 1e-20f));
-}
-
-// cudaFuncSetAttribute(max dynamic shared memory) once per kernel instance and device, not per call.
-// `done` is a per-instantiation bit mask over device ordinals (< 64); a race between host threads only
-// repeats the idempotent call.
-template <class Kernel>
-int allow_smem(Kernel kern, size_t smem, unsigned long long& done, const char* what) {
-    int dev = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
-    const bool tracked = dev >= 0 && dev < 64;
-    if (tracked && (done >> dev & 1ull)) return RESKV_OK;
-    if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), what))
-        return rc;
-    if (tracked) done |= 1ull << dev;
-    return RESKV_OK;
-}
-
-// one CTA per unit with 128 threads per query head of the unit
-int launch_merge(const MergeParams& mp, int units, int recent_max, cudaStream_t s) {
-    const int gqa = mp.nh / mp.kh;
-    if (gqa < 1 || gqa > 8) return fail(RESKV_ERR_INVALID, "merge: at most 8 query heads per KV head");
-    const size_t smem = merge_smem_bytes(mp.splits > 0 ? mp.cv : 0, gqa, recent_max);
-    if (smem > 48 * 1024) {
-        static unsigned long long done = 0;
-        if (int rc = allow_smem(decode_merge_kernel, merge_smem_bytes(kMaxClusters, 8, kMaxRecent), done,
-                                "cudaFuncSetAttribute(decode_merge)"))
-            return rc;
-    }
-    decode_merge_kernel<<<units, gqa * kMergeThreads, smem, s>>>(mp, recent_max);
-    return check_cuda(cudaGetLastError(), "decode_merge launch");
-}
 
 template <int GQA, class L, int CVS>
 int launch_simt_cvs(const DecodeParams& p, int units, cudaStream_t stream) {

@@ -55,6 +55,32 @@ struct DecodeParams {
     const int32_t* dyn;
 };
 
+struct MergeParams {
+    const float* ws_m;      // log2-domain maxima [BNH][splits], or natural-log m [BNH] when splits == 0
+    const float* ws_l;
+    const float* ws_delta;
+    const float* ws_beta;
+    const __half* vc;       // [B*KH,CV,128]
+    const __half* comp_out; // splits == 0: finished compressed result to merge with
+    const __half* rq;       // rotated query [BNH,128] or null
+    const __half* rk;       // rotated recent keys [B*KH,Tr,128] or null
+    const __half* rv;       // recent values
+    const float* rscores;   // precomputed scaled scores [BNH,Tr] (natural units) or null
+    __half* out;
+    float* out_m;
+    float* out_l;
+    int kh, nh, splits, cv, tr;
+    float scaling;
+    const int32_t* dyn;  // device step state: dyn[1] = recent tokens (overrides tr), or null
+    int64_t recent_cap;  // tokens between units in rk / rv (== tr for contiguous windows)
+    uint32_t* status;    // device status word of the call's workspace, or null
+};
+
+constexpr int kMaxRecent = 1024;  // window tokens of one call
+
+// Launches the merge kernel (decode_merge.cu): one CTA per unit; recent_max bounds a device-side window count.
+int launch_merge(const MergeParams& mp, int units, int recent_max, cudaStream_t stream);
+
 // compressed tokens of this launch: from the device step state when it carries a count
 __device__ __forceinline__ int token_count(const DecodeParams& p) {
     if (p.dyn) {
@@ -76,6 +102,29 @@ namespace {
 
 __device__ __forceinline__ float rope_freq(const float* inv_freq, float theta, int i) {
     return inv_freq ? inv_freq[i] : powf(theta, -static_cast<float>(i) / 64.0f);
+}
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// cudaFuncSetAttribute(max dynamic shared memory) once per kernel instance and device, not per call.
+// `done` is a per-instantiation bit mask over device ordinals (< 64); a race between host threads only
+// repeats the idempotent call.
+template <class Kernel>
+int allow_smem(Kernel kern, size_t smem, unsigned long long& done, const char* what) {
+    int dev = 0;
+    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
+    const bool tracked = dev >= 0 && dev < 64;
+    if (tracked && (done >> dev & 1ull)) return RESKV_OK;
+    if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), what))
+        return rc;
+    if (tracked) done |= 1ull << dev;
+    return RESKV_OK;
 }
 
 }  // namespace
