@@ -6,8 +6,8 @@ One ``nvcc`` invocation per ``.cu`` file (object files under ``build/``), then a
 shared link next to this file.  The library does not link against torch or Python: it
 is plain CUDA runtime code behind the C ABI of ``include/reskv_b200.h``.  Next to it
 ``_host.so`` is built from ``host.cpp``: the CPython module that takes torch tensors
-and calls that ABI.  nvcc cross-compiles, so no GPU is needed to build.  ``RESKV_NVCC_FLAGS`` (environment) adds compiler flags for
-experiment builds, e.g. ``RESKV_NVCC_FLAGS="-DRESKV_MMA_CTAS_PER_SM=3" python -m reskv_b200.csrc.build --force``.
+and calls that ABI.  nvcc cross-compiles, so no GPU is needed to build.  ``RESKV_NVCC_FLAGS`` (environment) adds compiler flags; use it
+together with ``--force``.
 """
 
 from __future__ import annotations
@@ -51,7 +51,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objdir = HERE / "build"
     objdir.mkdir(exist_ok=True)
     headers = sorted(HERE.glob("*.cuh")) + [HERE.parent.parent / "include" / "reskv_b200.h"]
-    # extra compiler flags for experiment builds (e.g. -DRESKV_MMA_CTAS_PER_SM=3); use together with --force
     extra = os.environ.get("RESKV_NVCC_FLAGS", "").split()
     jobs = []
     for src in sources():

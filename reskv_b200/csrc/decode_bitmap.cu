@@ -449,10 +449,10 @@ int launch_simt(const DecodeParams& p, int units, cudaStream_t s) {
 template <int GQA, int NNZ, int BETA>
 int launch_partial_mma_beta(const DecodeParams& p, cudaStream_t stream) {
     using ML = mma::LayoutMmaBitmap<NNZ>;
-    const size_t smem = mma::smem_bytes<GQA, ML>(p.ck);
+    const size_t smem = mma::Smem<GQA, ML>::bytes(p.ck);
     auto kern = mma::decode_mma_kernel<GQA, ML, BETA>;
     static unsigned long long done = 0;
-    if (int rc = allow_smem(kern, mma::smem_bytes<GQA, ML>(kMaxClusters), done, "cudaFuncSetAttribute(decode_bitmap_mma)"))
+    if (int rc = allow_smem(kern, mma::Smem<GQA, ML>::bytes(kMaxClusters), done, "cudaFuncSetAttribute(decode_bitmap_mma)"))
         return rc;
     kern<<<p.grid, mma::kThreadsM, smem, stream>>>(p);
     return check_cuda(cudaGetLastError(), "decode_bitmap_mma launch");
@@ -470,6 +470,9 @@ int g_variant = 0;
 cudaEvent_t g_ev_start = nullptr, g_ev_stop = nullptr;
 
 enum LayoutId { kBitmap32, kBitmap64, kQuant4, kQuant2, kTiled64, kStruct32, kStructInt4, kCompact4x64, kCompact4x32, kCompact2x64 };
+
+// 8-byte metadata rows are copied in whole rows
+bool aligned8(const void* a, const void* b) { return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 7u) == 0; }
 
 template <int GQA>
 int dispatch_layout(const DecodeParams& p, LayoutId layout, int units, cudaStream_t s) {
@@ -494,12 +497,9 @@ int dispatch_layout(const DecodeParams& p, LayoutId layout, int units, cudaStrea
             if (g_variant != 0)
                 return fail(RESKV_ERR_INVALID, "the compact quantised layout has no warp-per-token kernel");
             return launch_packed_mma(p, 5 + (layout - kCompact4x64), GQA, units, s);
-        default: {
-            // 8-byte metadata rows can only be bulk-copied when every tile starts 16-byte aligned
-            const bool bulk_ok = p.tokens % 2 == 0 && p.tok_stride % 2 == 0 && aligned16(p.kb) && aligned16(p.vb);
-            return (g_variant == 0 && bulk_ok) ? launch_packed_mma(p, 4, GQA, units, s)
-                                               : launch_simt<GQA, LayoutStructInt4>(p, units, s);
-        }
+        default:
+            return g_variant == 0 && aligned8(p.kb, p.vb) ? launch_packed_mma(p, 4, GQA, units, s)
+                                                          : launch_simt<GQA, LayoutStructInt4>(p, units, s);
     }
 }
 
@@ -530,38 +530,37 @@ size_t workspace_bytes(int bnh, int splits) {
 // How a decode call is cut into partial results.
 struct PartialPlan {
     int slots;     // partial results per query head in the workspace
-    int chunk;     // tiles per CTA
+    int chunk;     // granules (tensor-core kernel) or tiles (warp-per-token kernel) per CTA
     int grid;      // CTAs of the tensor-core kernel (the warp-per-token kernel runs slots x units)
-    int balanced;  // 1: equal share of all tiles per CTA, 0: one CTA per (unit, split)
+    int balanced;  // 1: equal share of all granules per CTA, 0: one CTA per (unit, split)
 };
 
 // splits_req > 0 (caller's choice) or the warp-per-token kernel: fixed splits per unit.  Otherwise the balanced
-// schedule: at most two CTAs per SM, every CTA streams ceil(all tiles / CTAs) consecutive tiles, so the per-CTA
-// tables are built once per CTA and no SM idles on a partial last wave.  A unit of n tiles is then touched by at
-// most (n - 1) / chunk + 2 CTAs.  With a device-side token count (`dyn`) chunk is recomputed on the device as
-// ceil(units * n / grid), which keeps that figure below ceil(grid / units) + 1 for any n.
+// schedule: at most one CTA per SM, every CTA streams ceil(all granules / CTAs) consecutive granules, so the per-CTA
+// tables are built once per CTA and no SM idles on a partial last wave.  A unit of n granules is then touched by at
+// most (n - 1) / chunk + 2 CTAs.  With a device-side token count (`dyn`) chunk is recomputed on the device, which keeps
+// that figure below ceil(grid / units) + 1 for any n.
 PartialPlan plan_partials(int units, int tokens, int splits_req, bool tensor_core, bool dyn, int64_t tok_stride) {
-    const int tiles = (tokens + kTile - 1) / kTile;
+    const int step = tensor_core ? kGranule : kTile, steps = (tokens + step - 1) / step;
     PartialPlan pp{};
     if (splits_req > 0 || !tensor_core) {
         int splits = splits_req > 0 ? splits_req : pick_splits(units, tokens);
-        if (splits > tiles) splits = tiles;
-        const int per = (tiles + splits - 1) / splits;
-        splits = (tiles + per - 1) / per;  // drop splits that would get no tile
+        if (splits > steps) splits = steps;
+        const int per = (steps + splits - 1) / splits;
+        splits = (steps + per - 1) / per;  // drop splits that would get nothing
         pp.slots = splits, pp.chunk = per, pp.grid = units * splits, pp.balanced = 0;
         return pp;
     }
-    const long long max_tiles = dyn ? (tok_stride + kTile - 1) / kTile : tiles;
-    const long long all = static_cast<long long>(units) * (dyn ? max_tiles : tiles);
-    long long grid = static_cast<long long>(RESKV_MMA_CTAS_PER_SM) * sm_count();
-    if (grid > all) grid = all;
-    const long long chunk = (static_cast<long long>(units) * tiles + grid - 1) / grid;
+    const long long most = dyn ? (tok_stride + step - 1) / step : steps, all = units * most;
+    long long grid = sm_count();
+    if (grid * kMinChunk > all) grid = (all + kMinChunk - 1) / kMinChunk;
+    const long long chunk = (static_cast<long long>(units) * steps + grid - 1) / grid;
     if (dyn) {
         pp.slots = static_cast<int>((grid + units - 1) / units) + 1;
     } else {
-        grid = (static_cast<long long>(units) * tiles + chunk - 1) / chunk;  // CTAs that get tiles
-        const long long s = (tiles - 1) / chunk + 2;
-        pp.slots = static_cast<int>(s < tiles ? s : tiles);
+        grid = (static_cast<long long>(units) * steps + chunk - 1) / chunk;  // CTAs that get granules
+        const long long s = (steps - 1) / chunk + 2;
+        pp.slots = static_cast<int>(s < steps ? s : steps);
     }
     pp.chunk = static_cast<int>(chunk), pp.grid = static_cast<int>(grid), pp.balanced = 1;
     return pp;
@@ -627,10 +626,7 @@ struct DecodeArgs {
 
 // Which partial kernel dispatch_layout will pick for this call (its partial plan differs).
 bool tensor_core_variant(LayoutId layout, const DecodeArgs& a) {
-    if (layout == kStructInt4) {
-        const bool bulk_ok = a.tokens % 2 == 0 && a.tok_stride % 2 == 0 && aligned16(a.km) && aligned16(a.vm);
-        return g_variant == 0 && bulk_ok;
-    }
+    if (layout == kStructInt4) return g_variant == 0 && aligned8(a.km, a.vm);
     if (layout == kCompact4x64 || layout == kCompact4x32 || layout == kCompact2x64) return true;
     return g_variant == 0;
 }
@@ -673,6 +669,9 @@ int decode_common(const DecodeArgs& a, LayoutId layout, bool has_meta, bool has_
         return fail(RESKV_ERR_INVALID, "%s: window token stride smaller than the window", who);
 
     const int units = a.batch * a.kv_heads;
+    if (static_cast<long long>(units) * (a.tok_stride / kGranule + 2) >= (1ll << 30))
+        return fail(RESKV_ERR_LIMIT, "%s: %d units of up to %lld tokens are more than a call takes", who, units,
+                    static_cast<long long>(a.tok_stride));
     const PartialPlan pp = plan_partials(units, a.tokens, a.splits, tensor_core_variant(layout, a), a.dyn != nullptr, a.tok_stride);
     const int splits = pp.slots, per = pp.chunk;
     const size_t need = workspace_bytes(a.batch * a.q_heads, splits);
@@ -703,7 +702,7 @@ int decode_common(const DecodeArgs& a, LayoutId layout, bool has_meta, bool has_
     p.inv_freq = a.inv_freq;
     p.tok_stride = a.tok_stride;
     p.kh = a.kv_heads, p.nh = a.q_heads, p.tokens = a.tokens, p.ck = a.ck, p.cv = a.cv;
-    p.start_pos = a.start_pos, p.pos_q = a.pos_q, p.splits = splits, p.tiles_per_split = per;
+    p.start_pos = a.start_pos, p.pos_q = a.pos_q, p.splits = splits, p.chunk = per;
     p.theta = a.theta, p.scaling = a.scaling;
     p.dyn = a.dyn;
     p.units = units, p.balanced = pp.balanced, p.grid = pp.grid;

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tmem.cuh"
 
 namespace reskv {
 
@@ -13,7 +14,9 @@ int launch_packed_mma(const DecodeParams& p, int layout, int gqa, int units, cud
 
 namespace {
 
-constexpr int kTile = 64;    // tokens per pipeline stage
+constexpr int kGranule = 32;  // tokens: the tensor-core kernel's segments start and end at multiples of this
+constexpr int kMinChunk = 2;  // granules a CTA takes at least: 64 tokens, one warp per scheduler
+constexpr int kTile = 64;     // tokens per pipeline stage of the warp-per-token kernel
 constexpr int kWarps = 8;    // warps per CTA
 constexpr int kThreads = kWarps * 32;
 constexpr int kTokPerWarp = kTile / kWarps;
@@ -41,11 +44,12 @@ struct DecodeParams {
     const float* inv_freq;
     int64_t tok_stride;
     int kh, nh, tokens, ck, cv;
-    // splits = partial slots per query head in the workspace; tiles_per_split = tiles per CTA (see `balanced`)
-    int start_pos, pos_q, splits, tiles_per_split;
+    // splits = partial slots per query head in the workspace; chunk = granules (tensor-core kernel) or tiles (warp-per-
+    // token kernel) per CTA
+    int start_pos, pos_q, splits, chunk;
     // units = batch * kv heads.  balanced != 0: the tensor-core kernel runs a 1-D grid whose CTAs each take an
-    // equal share of all units' tiles (a CTA may finish one unit and start the next); balanced == 0: one CTA per
-    // (unit, split) with `tiles_per_split` tiles each.
+    // equal share of all units' granules (a CTA may finish one unit and start the next); balanced == 0: one CTA per
+    // (unit, split) with `chunk` granules or tiles each.
     int units, balanced, grid;  // grid = CTAs of the tensor-core kernel
     float theta, scaling;
     // optional device-resident step state {query position, dense-window tokens, compressed tokens
@@ -92,7 +96,7 @@ __device__ __forceinline__ int token_count(const DecodeParams& p) {
 
 // tiles per split: the host's figure, or the same formula on the device-side token count
 __device__ __forceinline__ int split_tiles(const DecodeParams& p, int total_tiles) {
-    return p.dyn ? (total_tiles + p.splits - 1) / p.splits : p.tiles_per_split;
+    return p.dyn ? (total_tiles + p.splits - 1) / p.splits : p.chunk;
 }
 
 // query position of this launch: from the device step state when one is attached

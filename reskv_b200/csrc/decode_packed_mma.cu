@@ -9,7 +9,7 @@ namespace {
 
 template <int GQA, class ML, int BETA>
 int launch_beta(const DecodeParams& p, cudaStream_t stream) {
-    const size_t smem = mma::smem_bytes<GQA, ML>(p.ck);
+    const size_t smem = mma::Smem<GQA, ML>::bytes(p.ck);
     auto kern = mma::decode_mma_kernel<GQA, ML, BETA>;
     // allowed once per kernel instance and device (bit mask over device ordinals), for the largest centroid table
     static unsigned long long done = 0;
@@ -17,7 +17,7 @@ int launch_beta(const DecodeParams& p, cudaStream_t stream) {
     if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
     if (dev < 0 || dev >= 64 || !(done >> dev & 1ull)) {
         if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(mma::smem_bytes<GQA, ML>(kMaxClusters))),
+                                                     static_cast<int>(mma::Smem<GQA, ML>::bytes(kMaxClusters))),
                                 "cudaFuncSetAttribute(decode_mma packed)"))
             return rc;
         if (dev >= 0 && dev < 64) done |= 1ull << dev;
