@@ -357,6 +357,14 @@ int reskv_compress_group(int layout, int bits, int nnz, const void* x_k, const v
                          void* v_centroids_new, int v_clusters_new, void* v_ids, void* v_payload, void* v_meta,
                          void* v_scale, int64_t v_tok_stride, int seq_len, int32_t* ids_scratch, void* stream);
 
+/* Cluster ids given by the caller, [units, tokens] integers of 1, 2, 4 or 8 bytes for K and for V (count = units *
+ * tokens): int32 copies (wide, 2 * count, K first) for the packers, int8 copies (k_narrow, v_narrow) for the cache; *bad, zeroed
+ * by the caller (device memory, or mapped host memory that is read once the call's stream has got there), becomes 1 when
+ * an id of K lies outside [0, k_clusters) or one of V outside [0, v_clusters).  The packers clamp ids, so they may be
+ * launched before *bad has been read. */
+int reskv_take_ids(const void* k_ids, const void* v_ids, int k_bytes, int v_bytes, int64_t count, int k_clusters,
+                   int v_clusters, int32_t* wide, void* k_narrow, void* v_narrow, uint32_t* bad, void* stream);
+
 /* Moves tokens [src, src + count) of every unit of the three window buffers (f16
  * [B*KH,window_capacity,128], 16-byte aligned) to [dst, dst + count), dst <= src; the ranges may
  * overlap.  Replaces the slice copies that slide the window after a group left it

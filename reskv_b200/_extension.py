@@ -85,6 +85,7 @@ SIGNATURES = {
         _I,
         [_I, _I, _I, _P, _P, _I, _I, _I, _L] + [_P, _I, _P, _I, _P, _P, _P, _P, _L] * 2 + [_I, _P, _P],
     ),
+    "reskv_take_ids": (_I, [_P, _P, _I, _I, _L, _I, _I] + [_P] * 5),
     "reskv_window_shift": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     "reskv_kmeans_workspace_bytes": (_Z, [_I, _I, _I]),
     "reskv_kmeans": (_I, [_P, _I, _I, _I, _L, _I, _I, _I, _P, _Z, _P, _P, _P]),
@@ -310,6 +311,13 @@ class CompressionOps(_Ops):
                                                 new, ids.data_ptr(), _stream(x.device)))
         return out, ids
 
+
+    def take_ids(self, ids_k, ids_v, clusters_k, clusters_v):
+        """Given cluster ids of K and V -> int32 ids ``[2,B,H,T]``, the two int8 ids and a check that waits for the
+        verdict: ``check()`` is False when an id was out of range.  Meanwhile the packers, which clamp ids, can run."""
+        _same_device(self.device.index, ids_k, ids_v)
+        wide, narrow_k, narrow_v, ticket = host().take_ids(ids_k, ids_v, clusters_k, clusters_v)
+        return wide, (narrow_k, narrow_v), lambda: host().ids_in_range(ticket)
 
     def compress_group(self, plan: KernelPlan, x_k, x_v, sides, seq_len: int):
         """One decode group of K and V clustered, packed and written behind token ``seq_len`` of the capacity

@@ -76,10 +76,10 @@ def _incremental_cluster(x, centers, config, *, value=False):
 
 
 @torch.no_grad()
-def _encode(x, centers, ids, plan: KernelPlan, *, value=False):
+def _encode(x, centers, ids, plan: KernelPlan, *, value=False, stored_ids=None):
     """Residuals of ``x`` to its centres in the layout of ``plan``
     (reference compression.py:72-101).  ``value`` is accepted for signature
-    compatibility: K and V use the same selection rule here."""
+    compatibility: K and V use the same selection rule here.  ``stored_ids``: the ids as int8, when there."""
     ids = ids.int().contiguous()
     centers = centers.half().contiguous()
     x = _dense_or_slice(x)
@@ -95,7 +95,7 @@ def _encode(x, centers, ids, plan: KernelPlan, *, value=False):
         payload, metadata, scale = ops.compress_structured_int4(x, centers, ids)
     else:
         payload, scale = ops.compress_quantized(x, centers, ids, plan.nnz, plan.bits)
-    return CompressedTensor(centers, ids, payload, metadata, scale, plan)
+    return CompressedTensor(centers, ids if stored_ids is None else stored_ids, payload, metadata, scale, plan)
 
 
 def _plan_for(config: ResKVKernelConfig, previous, plan, batch: int) -> KernelPlan:
@@ -128,7 +128,7 @@ def _check_previous(previous: CompressedKV, key: torch.Tensor, limit: int) -> No
 
 def _check_external(centres, ids, key: torch.Tensor, limit: int) -> None:
     """One side of ``clustering=``: a centroid table ``[B,H,C,128]`` with ``1 <= C <= limit`` and integer
-    ids ``[B,H,T]`` inside ``[0, C)``, both next to K / V."""
+    ids ``[B,H,T]``, both next to K / V.  That the ids lie inside ``[0, C)`` is checked on the device (``take_ids``)."""
     if centres.ndim != 4 or tuple(centres.shape[:2]) != tuple(key.shape[:2]) or centres.shape[-1] != 128:
         raise ValueError("external centers must have shape [B,H,C,128]")
     count = centres.shape[2]
@@ -138,9 +138,6 @@ def _check_external(centres, ids, key: torch.Tensor, limit: int) -> None:
         raise ValueError("external clustering must share the K/V device")
     if ids.dtype not in _INT_DTYPES:
         raise ValueError("cluster IDs must be integer tensors")
-    lo, hi = torch.aminmax(ids)
-    if int(lo) < 0 or int(hi) >= count:
-        raise ValueError("external cluster IDs are out of range")
 
 
 def _append_group_in_place(key, value, previous: CompressedKV, config, plan: KernelPlan):
@@ -214,12 +211,21 @@ def compress(
         if extended is not None:
             return extended
 
+    if clustering is not None:
+        # one pass over the ids of both sides checks and converts them; its verdict is read after the packers have
+        # been launched behind it, so the device does not wait for the host
+        (k_centres, k_ids), (v_centres, v_ids) = clustering
+        ids_wide, ids_narrow, in_range = _ops(key).take_ids(k_ids, v_ids, k_centres.shape[2], v_centres.shape[2])
+        packed = [_encode(x, clustering[side][0], ids_wide[side], plan, stored_ids=ids_narrow[side])
+                  for side, x in enumerate((key, value))]
+        if not in_range():
+            raise ValueError("external cluster IDs are out of range")
+        return CompressedKV(*packed)
+
     packed = []
     for side, x in enumerate((key, value)):  # 0 = K, 1 = V
         is_value = side == 1
-        if clustering is not None:
-            centres, ids = clustering[side]
-        elif previous is not None:
+        if previous is not None:
             grown = (previous.key, previous.value)[side].centroids
             centres, ids = _incremental_cluster(x, grown, config, value=is_value)
         else:

@@ -5,6 +5,8 @@
 // table + ids), packing into fresh tensors, six slice copies into the capacity buffers, three slice copies that move
 // the window's remaining tokens to the front.  The device work of all that is ~0.1 ms; issued as ~15 separate tensor
 // operations it costs ~0.45 ms of host time per layer at every batch size.  Here it is two calls.
+#include <initializer_list>
+
 #include "common.cuh"
 
 namespace reskv {
@@ -20,6 +22,28 @@ __global__ void narrow_ids_kernel(const int32_t* k_ids, const int32_t* v_ids, in
     const int unit = i / tokens, t = i % tokens;
     k_dst[static_cast<size_t>(unit) * k_stride + t] = static_cast<int8_t>(k_ids[i]);
     v_dst[static_cast<size_t>(unit) * v_stride + t] = static_cast<int8_t>(v_ids[i]);
+}
+
+// External cluster ids of K and of V (blockIdx.y), contiguous integers of `bytes` bytes each -> int32 and int8 copies;
+// *bad (device or mapped host memory) is set to 1 when an id lies outside [0, clusters).
+__global__ void take_ids_kernel(const void* k_ids, const void* v_ids, int k_bytes, int v_bytes, int k_clusters, int v_clusters,
+                                int32_t* wide, int8_t* k_narrow, int8_t* v_narrow, uint32_t* bad, long long n) {
+    const bool value = blockIdx.y != 0;
+    const void* src = value ? v_ids : k_ids;
+    const int bytes = value ? v_bytes : k_bytes, clusters = value ? v_clusters : k_clusters;
+    int32_t* wide_out = wide + (value ? n : 0);
+    int8_t* narrow_out = value ? v_narrow : k_narrow;
+    bool out = false;
+    for (long long i = static_cast<long long>(blockIdx.x) * kNarrowThreads + threadIdx.x; i < n;
+         i += static_cast<long long>(gridDim.x) * kNarrowThreads) {
+        const long long id = bytes == 4   ? static_cast<const int32_t*>(src)[i]
+                             : bytes == 1 ? static_cast<const int8_t*>(src)[i]
+                             : bytes == 2 ? static_cast<const int16_t*>(src)[i]
+                                          : static_cast<const long long*>(src)[i];
+        out |= id < 0 || id >= clusters;
+        wide_out[i] = static_cast<int32_t>(id), narrow_out[i] = static_cast<int8_t>(id);
+    }
+    if (__syncthreads_or(out) && threadIdx.x == 0) *bad = 1u;
 }
 
 // grid = (units, 3 buffers), 128 threads = 8 tokens x 16 pieces of 16 bytes per pass.  Tokens [src, src + count) of a
@@ -132,6 +156,21 @@ extern "C" int reskv_compress_group(int layout, int bits, int nnz, const void* x
         ids[0], ids[1], static_cast<int8_t*>(k_ids) + seq_len, static_cast<int8_t*>(v_ids) + seq_len, tokens,
         k_tok_stride, v_tok_stride, total);
     return check_cuda(cudaGetLastError(), "compress_group: id rows launch");
+}
+
+extern "C" int reskv_take_ids(const void* k_ids, const void* v_ids, int k_bytes, int v_bytes, int64_t count, int k_clusters,
+                              int v_clusters, int32_t* wide, void* k_narrow, void* v_narrow, uint32_t* bad, void* stream) {
+    if (!k_ids || !v_ids || !wide || !k_narrow || !v_narrow || !bad) return fail(RESKV_ERR_INVALID, "take_ids: null pointer");
+    if (count < 1) return fail(RESKV_ERR_INVALID, "take_ids: no ids");
+    for (int bytes : {k_bytes, v_bytes})
+        if (bytes != 1 && bytes != 2 && bytes != 4 && bytes != 8) return fail(RESKV_ERR_INVALID, "take_ids: ids of %d bytes", bytes);
+    if (int rc = check_device_pointer(k_ids, "take_ids", "k_ids")) return rc;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const long long want = (count + 4 * kNarrowThreads - 1) / (4 * kNarrowThreads), most = 4ll * sm_count();
+    take_ids_kernel<<<dim3(static_cast<unsigned>(want < most ? want : most), 2), kNarrowThreads, 0, s>>>(
+        k_ids, v_ids, k_bytes, v_bytes, k_clusters, v_clusters, wide, static_cast<int8_t*>(k_narrow),
+        static_cast<int8_t*>(v_narrow), bad, count);
+    return check_cuda(cudaGetLastError(), "take_ids launch");
 }
 
 extern "C" int reskv_window_shift(void* window_k, void* window_raw, void* window_v, int batch, int kv_heads,

@@ -47,6 +47,13 @@ __device__ __forceinline__ float half_hi(uint32_t v) {
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 
+// a - fp32(b): one mixed-precision multiply-add (b * -1 + a), rounded once like the subtraction
+__device__ __forceinline__ float sub_f16(float a, unsigned short b) {
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"(b), "h"(static_cast<unsigned short>(0xbc00)), "f"(a));
+    return d;
+}
+
 // r[q] = fp32(x[32 p + q]) - fp32(c[32 p + q]), q = 0..31, from the token's and its centroid's shared-memory rows
 __device__ __forceinline__ void residual_piece(const unsigned char* xrow, const unsigned char* crow, int p,
                                                float (&r)[32]) {
@@ -57,8 +64,8 @@ __device__ __forceinline__ void residual_piece(const unsigned char* xrow, const 
         const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, cs[4] = {cv.x, cv.y, cv.z, cv.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            r[8 * m + 2 * i] = half_lo(xs[i]) - half_lo(cs[i]);
-            r[8 * m + 2 * i + 1] = half_hi(xs[i]) - half_hi(cs[i]);
+            r[8 * m + 2 * i] = sub_f16(half_lo(xs[i]), static_cast<unsigned short>(cs[i] & 0xffffu));
+            r[8 * m + 2 * i + 1] = sub_f16(half_hi(xs[i]), static_cast<unsigned short>(cs[i] >> 16));
         }
     }
 }
@@ -112,49 +119,102 @@ __device__ __forceinline__ void select_topk_thread(const uint32_t (&key)[64], in
     }
 }
 
+// Packed 16-bit keys: larger ones to `a`, smaller ones to `b`, in either half.
+__device__ __forceinline__ void order2(uint32_t& a, uint32_t& b) {
+    const uint32_t hi = __vmaxu2(a, b);
+    b = __vminu2(a, b);
+    a = hi;
+}
+__device__ __forceinline__ void sort4(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {  // descending
+    order2(a, b), order2(c, d), order2(a, c), order2(b, d), order2(b, c);
+}
+// The four largest of two descending quadruples, descending, in `a`.
+__device__ __forceinline__ void top4(uint32_t (&a)[4], const uint32_t (&b)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = __vmaxu2(a[i], b[3 - i]);
+    order2(a[0], a[2]), order2(a[1], a[3]), order2(a[0], a[1]), order2(a[2], a[3]);
+}
+// M-th largest of 16 keys (M = 4 or 8), in either half: sorted runs, then the smallest of the pairwise maxima of one run
+// and the other one reversed.
+template <int M>
+__device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key) {
+    uint32_t a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[i][j] = key[4 * i + j];
+        sort4(a[i][0], a[i][1], a[i][2], a[i][3]);
+    }
+    if constexpr (M == 4) {
+        top4(a[0], a[1]), top4(a[2], a[3]);
+        uint32_t t = __vmaxu2(a[0][0], a[2][3]);
+#pragma unroll
+        for (int i = 1; i < 4; ++i) t = __vminu2(t, __vmaxu2(a[0][i], a[2][3 - i]));
+        return t;
+    } else {
+        uint32_t run[2][8];  // two bitonic merges of a descending and a reversed descending quadruple
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) run[r][i] = a[2 * r][i], run[r][4 + i] = a[2 * r + 1][3 - i];
+#pragma unroll
+            for (int step = 4; step > 0; step >>= 1)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (!(i & step)) order2(run[r][i], run[r][i + step]);
+        }
+        uint32_t t = __vmaxu2(run[0][0], run[1][7]);
+#pragma unroll
+        for (int i = 1; i < 8; ++i) t = __vminu2(t, __vmaxu2(run[0][i], run[1][7 - i]));
+        return t;
+    }
+}
+
 // Keep-mask of the `m` largest keys of every 16-coordinate tile, lower coordinate first among equal keys.
 // key[16 p + j] holds coordinate 32 p + j (tile 2 p) in its LOW and 32 p + 16 + j (tile 2 p + 1) in its HIGH half;
 // keep[p] has coordinate 32 p + q at bit q (the tiled metadata word of the reference, compression.cu:126-139).
+template <int M>
 __device__ __forceinline__ void select_tiles_thread(const uint32_t (&key)[64], int m, uint32_t (&keep)[4]) {
     const __half2 m2 = __float2half2_rn(static_cast<float>(m));
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        // per half: largest v with count(key >= v) >= m; counts up to 16 are exact in FP16
+        // per half: the m-th largest key.  M of the two plans that have this layout: a sorting network (71 and 95 packed
+        // instructions); any other m: bisection, largest v with count(key >= v) >= m (480)
         uint32_t v2 = 0;
-        for (int bit = 14; bit >= 0; --bit) {
-            const uint32_t both = (1u << bit) | (1u << (bit + 16));
-            const __half2 c2 = as_half2(v2 | both);
-            __half2 a0 = __hge2(as_half2(key[16 * p]), c2), a1 = __hge2(as_half2(key[16 * p + 1]), c2);
+        if constexpr (M != 0) {
+            v2 = mth_of_16<M>(key + 16 * p);
+        } else {
+            for (int bit = 14; bit >= 0; --bit) {
+                const uint32_t both = (1u << bit) | (1u << (bit + 16));
+                const __half2 c2 = as_half2(v2 | both);
+                __half2 a0 = __hge2(as_half2(key[16 * p]), c2), a1 = __hge2(as_half2(key[16 * p + 1]), c2);
 #pragma unroll
-            for (int j = 2; j < 16; j += 2) {
-                a0 = __hadd2(a0, __hge2(as_half2(key[16 * p + j]), c2));
-                a1 = __hadd2(a1, __hge2(as_half2(key[16 * p + j + 1]), c2));
+                for (int j = 2; j < 16; j += 2) {
+                    a0 = __hadd2(a0, __hge2(as_half2(key[16 * p + j]), c2));
+                    a1 = __hadd2(a1, __hge2(as_half2(key[16 * p + j + 1]), c2));
+                }
+                v2 |= both & __hge2_mask(__hadd2(a0, a1), m2);  // each half accepts the bit on its own count (exact in FP16)
             }
-            v2 |= both & __hge2_mask(__hadd2(a0, a1), m2);  // each half accepts the bit on its own count
         }
         const __half2 t2 = as_half2(v2);
-        uint32_t ge = 0u, gt = 0u;
+        uint32_t ge = 0u;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const uint32_t place = (1u << j) | (0x10000u << j);
-            ge |= __hge2_mask(as_half2(key[16 * p + j]), t2) & place;
-            gt |= __hgt2_mask(as_half2(key[16 * p + j]), t2) & place;
-        }
-        uint32_t kept = 0u;
+        for (int j = 0; j < 16; ++j) ge |= __hge2_mask(as_half2(key[16 * p + j]), t2) & ((1u << j) | (0x10000u << j));
+        uint32_t kept = ge;
+        if (__popc(ge) != 2 * m) {  // more keys equal to a threshold than places left: the lowest coordinates stay
+            uint32_t gt = 0u;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t g = (ge >> (16 * h)) & 0xffffu, t = (gt >> (16 * h)) & 0xffffu;
-            uint32_t k = g;
-            if (__popc(g) != m) {  // more keys equal to the threshold than places left: the lowest coordinates stay
-                int need = m - __popc(t);
-                uint32_t eq = g ^ t;
-                k = t;
+            for (int j = 0; j < 16; ++j) gt |= __hgt2_mask(as_half2(key[16 * p + j]), t2) & ((1u << j) | (0x10000u << j));
+            kept = gt;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                int need = m - __popc((gt >> (16 * h)) & 0xffffu);
+                uint32_t eq = (ge ^ gt) & (0xffffu << (16 * h));
                 while (eq != 0u && need > 0) {
                     const uint32_t first = eq & (0u - eq);
-                    eq ^= first, k |= first, --need;
+                    eq ^= first, kept |= first, --need;
                 }
             }
-            kept |= k << (16 * h);
         }
         keep[p] = kept;
     }
@@ -271,7 +331,13 @@ __global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const Enco
                 }
             }
             if constexpr (kTiles) {
-                select_tiles_thread(key, p.nnz / 8, keep);
+                const int m = p.nnz / 8;
+                if (MODE == TopkMode::kStructFp16)
+                    select_tiles_thread<4>(key, 4, keep);
+                else if (m == 8)
+                    select_tiles_thread<8>(key, 8, keep);
+                else
+                    select_tiles_thread<0>(key, m, keep);
                 // compact the kept values to the front of the row, ascending coordinates (= tile, then rank)
                 unsigned short* vals = reinterpret_cast<unsigned short*>(xrow);
                 int n = 0;

@@ -11,8 +11,9 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdlib>
-#include <optional>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/reskv_b200.h"
 
@@ -331,6 +332,115 @@ PyObject* py_window_write(PyObject*, PyObject* const* o, Py_ssize_t n) {
     });
 }
 
+// ---- verdicts of take_ids -------------------------------------------------------------------------------------------
+// A word of mapped pinned host memory and an event per call in flight; a few are kept for later calls (any thread, any
+// device: the event is made for the call's device).
+struct Verdict {
+    volatile uint32_t* word;
+    cudaEvent_t event;
+    c10::DeviceIndex device;
+};
+constexpr size_t kKeptVerdicts = 16;
+std::mutex g_verdict_lock;
+std::vector<Verdict*> g_verdicts;
+
+void check_cuda(cudaError_t e, const char* what) {
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    PyErr_Format(PyExc_RuntimeError, "%s: %s", what, cudaGetErrorString(e));
+    throw PyError{};
+}
+
+Verdict* get_verdict(c10::DeviceIndex device) {
+    {
+        const std::lock_guard<std::mutex> lock(g_verdict_lock);
+        for (size_t i = 0; i < g_verdicts.size(); ++i) {
+            if (g_verdicts[i]->device != device) continue;
+            Verdict* v = g_verdicts[i];
+            g_verdicts.erase(g_verdicts.begin() + static_cast<long>(i));
+            return v;
+        }
+    }
+    void* word = nullptr;
+    cudaEvent_t event = nullptr;
+    check_cuda(cudaHostAlloc(&word, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+    check_cuda(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreate");
+    return new Verdict{static_cast<volatile uint32_t*>(word), event, device};
+}
+
+void put_verdict(Verdict* v) {
+    {
+        const std::lock_guard<std::mutex> lock(g_verdict_lock);
+        if (g_verdicts.size() < kKeptVerdicts) {
+            g_verdicts.push_back(v);
+            return;
+        }
+    }
+    cudaEventDestroy(v->event);
+    cudaFreeHost(const_cast<uint32_t*>(v->word));
+    delete v;
+}
+
+void drop_ticket(PyObject* capsule) {  // a call that never asked for its verdict: wait for it, then keep the slot
+    auto* v = static_cast<Verdict*>(PyCapsule_GetPointer(capsule, "reskv verdict"));
+    cudaEventSynchronize(v->event);
+    put_verdict(v);
+}
+
+// take_ids(k_ids, v_ids, k_clusters, v_clusters) -> (int32 ids [2,...], k int8 ids, v int8 ids, ticket)
+PyObject* py_take_ids(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 4);
+        const at::Tensor k = tensor(o[0], "ids").contiguous(), v = tensor(o[1], "ids").contiguous();
+        const c10::DeviceIndex dev = k.get_device();
+        const c10::cuda::CUDAGuard guard(dev);
+        std::vector<int64_t> both(k.sizes().begin(), k.sizes().end());
+        both.insert(both.begin(), 2);
+        const at::Tensor wide = at::empty(both, k.options().dtype(at::kInt));
+        const at::Tensor narrow_k = at::empty(k.sizes(), k.options().dtype(at::kChar)), narrow_v = at::empty_like(narrow_k);
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+        Verdict* verdict = get_verdict(dev);
+        *verdict->word = 0;
+        void* word = nullptr;
+        int rc = RESKV_OK;
+        const cudaError_t mapped = cudaHostGetDevicePointer(&word, const_cast<uint32_t*>(verdict->word), 0);
+        if (mapped == cudaSuccess)
+            rc = reskv_take_ids(k.const_data_ptr(), v.const_data_ptr(), static_cast<int>(k.element_size()), static_cast<int>(v.element_size()),
+                                k.numel(), static_cast<int>(integer(o[2])), static_cast<int>(integer(o[3])),
+                                static_cast<int32_t*>(wide.data_ptr()), narrow_k.data_ptr(), narrow_v.data_ptr(),
+                                static_cast<uint32_t*>(word), stream);
+        cudaEventRecord(verdict->event, stream);
+        PyObject* ticket = PyCapsule_New(verdict, "reskv verdict", drop_ticket);
+        if (!ticket) throw PyError{};
+        if (mapped != cudaSuccess || rc < 0) {
+            Py_DECREF(ticket);
+            check_cuda(mapped, "cudaHostGetDevicePointer");
+            check(rc);
+        }
+        ++g_launches;
+        PyObject* t = PyTuple_New(4);
+        PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(wide));
+        PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(narrow_k));
+        PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(narrow_v));
+        PyTuple_SET_ITEM(t, 3, ticket);
+        return t;
+    });
+}
+
+// ids_in_range(ticket) -> bool; waits until the ids have been looked at
+PyObject* py_ids_in_range(PyObject*, PyObject* ticket) {
+    return guarded([&]() -> PyObject* {
+        auto* v = static_cast<Verdict*>(PyCapsule_GetPointer(ticket, "reskv verdict"));
+        if (!v) throw PyError{};
+        cudaError_t e;
+        Py_BEGIN_ALLOW_THREADS;
+        e = cudaEventSynchronize(v->event);
+        Py_END_ALLOW_THREADS;
+        check_cuda(e, "cudaEventSynchronize");
+        return PyBool_FromLong(*v->word == 0);
+    });
+}
+
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f))
@@ -338,6 +448,8 @@ PyMethodDef g_methods[] = {
     {"decode", FAST(py_decode), METH_FASTCALL, "decode attention on given operands"},
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
     {"window_write", FAST(py_window_write), METH_FASTCALL, "append one token to the dense window"},
+    {"take_ids", FAST(py_take_ids), METH_FASTCALL, "check and convert given cluster ids"},
+    {"ids_in_range", py_ids_in_range, METH_O, "verdict of take_ids"},
     {"launches", py_launches, METH_NOARGS, "kernels launched through this module"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, g_methods};
