@@ -394,6 +394,14 @@ int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, int64_t x_t
                  int iterations, int value, void* workspace, size_t workspace_bytes, void* centroids, int32_t* ids,
                  void* stream);
 
+/* Clustering of K (flavour 0) and of V (flavour 1) of one shape in the same launches, up to 32 centres and at least as
+ * many tokens: what two calls of reskv_kmeans with value = 0 and 1 do.  The workspace is that of 2 * batch sequences.
+ * k_ids8 / v_ids8 (i8 [B*KH,T], or NULL) also receive the ids as int8. */
+int reskv_kmeans_pair(const void* x_k, const void* x_v, int batch, int kv_heads, int tokens, int64_t k_tok_stride,
+                      int64_t v_tok_stride, int clusters, int iterations, void* workspace, size_t workspace_bytes,
+                      void* k_centroids, void* v_centroids, int32_t* k_ids, int32_t* v_ids, void* k_ids8, void* v_ids8,
+                      void* stream);
+
 /* Status word of the kernels of the last reskv_kmeans call on this workspace (RESKV_STATUS_* bits: a bounded
  * wait inside a kernel ran out; 0 = clean).  Copies 4 bytes to the host and synchronises `stream`. */
 int reskv_kmeans_status(const void* workspace, int batch, int kv_heads, int clusters, uint32_t* status, void* stream);

@@ -89,6 +89,7 @@ SIGNATURES = {
     "reskv_window_shift": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     "reskv_kmeans_workspace_bytes": (_Z, [_I, _I, _I]),
     "reskv_kmeans": (_I, [_P, _I, _I, _I, _L, _I, _I, _I, _P, _Z, _P, _P, _P]),
+    "reskv_kmeans_pair": (_I, [_P, _P, _I, _I, _I, _L, _L, _I, _I, _P, _Z] + [_P] * 7),
     "reskv_kmeans_status": (_I, [_P, _I, _I, _I, _P, _P]),
     "reskv_kmeans_incremental": (_I, [_P, _I, _I, _I, _L, _P, _I, _P, _I, _P, _P]),
 }
@@ -288,12 +289,29 @@ class CompressionOps(_Ops):
         ids = torch.empty((b, h, t), dtype=torch.int32, device=x.device)
         flags = int(bool(value)) | (2 if exact else 0) | (4 if warp_mma else 0)
         check(self.lib.reskv_kmeans(x.data_ptr(), b, h, t, xs, count, iterations, flags, ws.data_ptr(), need,
-                                    centroids.data_ptr(), ids.data_ptr(), _stream(x.device)), launches=1 + 2 * iterations)
+                                    centroids.data_ptr(), ids.data_ptr(), _stream(x.device)), launches=1 + 2 * iterations if exact or warp_mma or count > 32 else 1 + iterations)
         if return_status:
             word = ctypes.c_uint32(0xFFFFFFFF)
             check(self.lib.reskv_kmeans_status(ws.data_ptr(), b, h, count, ctypes.addressof(word), _stream(x.device)))
             return centroids, ids, word.value
         return centroids, ids
+
+    def kmeans_pair(self, key, value, count, iterations):
+        """``kmeans`` of K and of V in the same launches -> ``(centroids, int32 ids, int8 ids)`` of each; up to 32 centres,
+        at least as many tokens, 16-byte aligned inputs."""
+        _same_device(self.device.index, key, value)
+        b, h, t, _ = key.shape
+        need = self.lib.reskv_kmeans_workspace_bytes(2 * b, h, count)
+        ws = torch.empty(need, dtype=torch.uint8, device=key.device)
+        sides = [(torch.empty((b, h, count, 128), dtype=torch.float16, device=key.device),
+                  torch.empty((b, h, t), dtype=torch.int32, device=key.device),
+                  torch.empty((b, h, t), dtype=torch.int8, device=key.device)) for _ in range(2)]
+        (kc, ki, k8), (vc, vi, v8) = sides
+        check(self.lib.reskv_kmeans_pair(key.data_ptr(), value.data_ptr(), b, h, t, token_stride_of(key), token_stride_of(value),
+                                         count, iterations, ws.data_ptr(), need, kc.data_ptr(), vc.data_ptr(), ki.data_ptr(),
+                                         vi.data_ptr(), k8.data_ptr(), v8.data_ptr(), _stream(key.device)),
+              launches=1 + iterations)
+        return sides
 
     def kmeans_incremental(self, x, centroids, append):
         """Decode-time step -> (centroids f16 [B,H,C or C+1,128], ids i32 [B,H,T])."""

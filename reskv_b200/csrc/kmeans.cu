@@ -26,6 +26,8 @@
 // V flavour: centres rounded to FP16 after every update, an empty cluster becomes 0.
 #include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
 
+#include <initializer_list>
+
 #include "common.cuh"
 #include "tmem.cuh"
 
@@ -54,6 +56,23 @@ struct KmeansParams {
 
 struct InitIndex {
     int idx[kMaxClusters];
+};
+
+// The tcgen05 form, one launch per Lloyd iteration, over one or two tensors (sides) of the same shape.
+struct UmmaParams {
+    const __half* x[2];   // [units, x_stride, 128]
+    int64_t x_stride[2];
+    int32_t* ids[2];      // [units, tokens]
+    int8_t* ids8[2];      // the same as int8, or null
+    int value[2];         // flavour of a side
+    // State over all sides' units: the centres an iteration used (two generations), the 2^24-scaled sums and the counts
+    // it formed (three generations: the last one is read, this one's added to, the next one's zeroed).
+    float* centres[2];    // [sides * units, C, 128]
+    long long* sums[3];
+    int* counts[3];
+    uint32_t* status;
+    int sides, units, tokens, clusters, iteration, iterations;
+    InitIndex init;       // tokens that are the first centres
 };
 
 __global__ void kmeans_init_kernel(KmeansParams p, InitIndex init, int value) {
@@ -461,6 +480,13 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 // arithmetic on the uniform datapath) and elect one lane per instruction.  The roles run concurrently on
 // different tiles and hand over through mbarriers only (triple-buffered distances and one-hot operands); every
 // wait is bounded.
+//
+// One launch per iteration, over K and V together when both are wanted: a launch costs a set-up, a pipeline fill and a
+// drain (~10 tile times) whatever it covers.  The new centres are formed in the next launch's set-up from the sums of the
+// last one (three generations of them, so nothing has to be cleared in between), and consecutive launches overlap
+// (programmatic stream serialisation): a CTA's set-up and first copies run while the launch before it drains.  Measured,
+// clustering of one layer's K and V, 64 units x 8128 tokens, 10 iterations: 0.79 ms with an update kernel and a launch
+// per side and iteration, 0.58 ms this way.
 constexpr int kUGroups = 3;                    // token-owning groups; group g takes the tiles i = g (mod 3)
 constexpr int kUGroupWarps = 4;                // a group: one warp per 32 token rows (TMEM lane quarter)
 constexpr int kUThreads = (kUGroups * kUGroupWarps + 3) * 32;  // + three issuing warps: distance MMAs, sum MMAs, copies
@@ -523,12 +549,37 @@ constexpr int kUWorkers = kUThreads - 32;  // everyone but the copying warp: the
 
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kUWorkers) : "memory"); }
 
-template <bool HILO>
-__global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const KmeansParams p,
-                                                                           const __grid_constant__ CUtensorMap xmap, int share,
-                                                                           int first, int last) {
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Four coordinates of a centre after iteration `from`: the mean of the tokens assigned then, the old centre (K) or zero
+// (V) where there were none; V's centres are rounded to FP16.
+__device__ __forceinline__ float4 new_centre(const UmmaParams& p, int from, bool value, size_t row, int i4) {
+    const int n = __ldcg(p.counts[from % 3] + row);  // through L2: written by the launch before this one
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n > 0) {
+        const longlong2* s = reinterpret_cast<const longlong2*>(p.sums[from % 3] + row * kHeadDim) + 2 * i4;
+        const longlong2 a = __ldcg(s), b = __ldcg(s + 1);
+        const double scale = 1.0 / 16777216.0 / static_cast<double>(n);
+        c = make_float4(static_cast<float>(static_cast<double>(a.x) * scale), static_cast<float>(static_cast<double>(a.y) * scale),
+                        static_cast<float>(static_cast<double>(b.x) * scale), static_cast<float>(static_cast<double>(b.y) * scale));
+    } else if (!value) {
+        c = __ldcg(reinterpret_cast<const float4*>(p.centres[from & 1] + row * kHeadDim) + i4);
+    }
+    if (value) {
+        const float2 lo = __half22float2(__floats2half2_rn(c.x, c.y)), hi = __half22float2(__floats2half2_rn(c.z, c.w));
+        c = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return c;
+}
+
+__global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap map0,
+                                                                           const __grid_constant__ CUtensorMap map1, int share) {
     extern __shared__ unsigned char smem_u[];
-    constexpr int kN = HILO ? 64 : 32;  // rows of the centre operand: hi halves, then lo halves
+    constexpr int kN = 64;  // rows of the centre operand: hi halves, then lo halves (K's FP32 centres; V's are FP16)
+    const bool first = p.iteration == 0, last = p.iteration + 1 == p.iterations;
+    const int units = p.sides * p.units;
+    let_next_launch_start();
     unsigned char* base = smem_u + ((1024u - (smem_u32(smem_u) & 1023u)) & 1023u);  // swizzled blocks: 1024-byte aligned
     unsigned char* xs = base;                                   // [stages][2 halves][128 tokens][128 B]
     unsigned char* cop = xs + kUStages * kUTileBytes;           // [2 halves][kN rows][128 B]
@@ -551,7 +602,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     // buffer q % 3, sum accumulator q % 4, and every barrier's phase follows from q, so the ring keeps turning across
     // segment boundaries (the copies of the next segment are in flight while this one drains and flushes).
     const int tiles_per_unit = (p.tokens + kUTile - 1) / kUTile;
-    const long long work_total = static_cast<long long>(p.units) * tiles_per_unit;
+    const long long work_total = static_cast<long long>(units) * tiles_per_unit;
     const long long work_begin = static_cast<long long>(blockIdx.x) * share;
     const long long work_end = work_begin + share < work_total ? work_begin + share : work_total;
     struct Segment {
@@ -598,22 +649,31 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                 unsigned char* dst = xs + (q % kUStages) * kUTileBytes;
                 uint64_t* bar = &bar_full[q % kUStages];
                 if (elect_one()) {
+                    const CUtensorMap* xmap = sg.unit < p.units ? &map0 : &map1;
+                    const int unit = sg.unit < p.units ? sg.unit : sg.unit - p.units;
                     mbar_arrive_expect_tx(bar, kUTileBytes);
-                    tma_load_3d(dst, &xmap, 0, (sg.tile0 + i) * kUTile, sg.unit, bar);
-                    tma_load_3d(dst + kUBoxBytes, &xmap, 64, (sg.tile0 + i) * kUTile, sg.unit, bar);
+                    tma_load_3d(dst, xmap, 0, (sg.tile0 + i) * kUTile, unit, bar);
+                    tma_load_3d(dst + kUBoxBytes, xmap, 64, (sg.tile0 + i) * kUTile, unit, bar);
                 }
                 __syncwarp();
             }
             w += sg.tiles;
         }
     } else {
+        // the launches of consecutive iterations overlap: this one's set-up and first copies (the tokens do not change) run
+        // while the last one drains; what that one wrote is touched from here on
+        wait_for_previous_launch();
         int q0 = 0;     // tiles of the earlier segments of this CTA
         int prev = -1;  // byte offset of the element this thread set in its group's one-hot buffer
         for (long long w = work_begin; w < work_end;) {
             const Segment sg = segment_at(w);
             const int unit = sg.unit, n_tiles = sg.tiles;
             const int t_begin = sg.tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
-            const float* cen_g = p.centres + static_cast<size_t>(unit) * p.clusters * kHeadDim;
+            const int side = unit < p.units ? 0 : 1, local = unit - side * p.units;
+            const bool value = p.value[side] != 0;
+            const __half* xu = p.x[side] + static_cast<size_t>(local) * p.x_stride[side] * kHeadDim;
+            const size_t row0 = static_cast<size_t>(unit) * p.clusters;  // first centre of the unit
+            const bool opens_unit = sg.tile0 == 0;  // this CTA also keeps the unit's centres and zeroes its next sums
             // ---- per segment: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 -------------------
             {
                 // four coordinates per thread and step, all loads of a thread in flight together
@@ -622,8 +682,23 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
 #pragma unroll
                 for (int k = 0; k < kSteps; ++k) {
                     const int i4 = tid + k * kUWorkers;
-                    v[k] = (i4 < 32 * kHeadDim / 4 && i4 / (kHeadDim / 4) < p.clusters) ? __ldg(reinterpret_cast<const float4*>(cen_g) + i4)
-                                                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int c = i4 / (kHeadDim / 4), d4 = i4 % (kHeadDim / 4);
+                    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (i4 >= 32 * kHeadDim / 4 || c >= p.clusters) continue;
+                    if (first) {
+                        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(xu + static_cast<size_t>(p.init.idx[c]) * kHeadDim) + d4);
+                        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+                        v[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                    } else {
+                        v[k] = new_centre(p, p.iteration - 1, value, row0 + c, d4);
+                    }
+                    if (opens_unit) {
+                        reinterpret_cast<float4*>(p.centres[p.iteration & 1] + row0 * kHeadDim)[i4] = v[k];
+                        const longlong2 zero = make_longlong2(0, 0);
+                        longlong2* ahead = reinterpret_cast<longlong2*>(p.sums[(p.iteration + 1) % 3] + row0 * kHeadDim) + 2 * i4;
+                        ahead[0] = zero, ahead[1] = zero;
+                        if (d4 == 0) p.counts[(p.iteration + 1) % 3][row0 + c] = 0;
+                    }
                 }
 #pragma unroll
                 for (int k = 0; k < kSteps; ++k) {
@@ -636,7 +711,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     *reinterpret_cast<uint2*>(at + sw128(c, (d & 63) >> 3)) =
                         make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
                     float2 f01 = __half22float2(h01), f23 = __half22float2(h23);  // what the MMA sees: hi (+ lo)
-                    if (HILO) {
+                    if (!value) {
                         const __half2 l01 = __floats2half2_rn(v[k].x - f01.x, v[k].y - f01.y);
                         const __half2 l23 = __floats2half2_rn(v[k].z - f23.x, v[k].w - f23.y);
                         *reinterpret_cast<uint2*>(at + sw128(32 + c, (d & 63) >> 3)) =
@@ -657,7 +732,6 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
             float cmax = lane < p.clusters ? cn_s[lane] : 0.f;  // largest |c|^2, in every thread
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(kFull, cmax, off));
-            const __half* xu = p.x + static_cast<size_t>(unit) * p.x_stride * kHeadDim;
 
             if (warp < kWarpDist) {
                 // ---- ranking: one thread per token; group g takes the tiles with q = g (mod 3), distance buffer g
@@ -667,7 +741,8 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                 // |x|^2 of a token is the same in every Lloyd iteration: the first one forms it and stores it (as FP32
                 // bits) where the token's id goes, the following ones read it from there one tile of the group ahead,
                 // the last one writes the id
-                int32_t* ids_u = p.ids + static_cast<size_t>(unit) * p.tokens;
+                int32_t* ids_u = p.ids[side] + static_cast<size_t>(local) * p.tokens;
+                int8_t* ids8_u = p.ids8[side] ? p.ids8[side] + static_cast<size_t>(local) * p.tokens : nullptr;
                 const int i_first = (g + kUGroups - q0 % kUGroups) % kUGroups;
                 float xn_next = 0.f;
                 if (!first && t_begin + i_first * kUTile + row_in_tile < t_end)
@@ -682,7 +757,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     tc_fence_after();
                     float d[32];
                     tmem_ld32(tmem + lane_base + kUColD + g * 64, d);
-                    if constexpr (HILO) {
+                    if (!value) {
                         float lo[32];
                         tmem_ld32(tmem + lane_base + kUColD + g * 64 + 32, lo);
                         tmem_ld_wait();
@@ -756,6 +831,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     if (live) {
                         if (last) {
                             ids_u[row] = c1;
+                            if (ids8_u) ids8_u[row] = static_cast<int8_t>(c1);
                         } else if (first) {
                             ids_u[row] = __float_as_int(xn);
                         }
@@ -777,6 +853,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                 // ---- distance MMAs (whole warp, one elected lane per tile): tile q goes to buffer q % 3 as soon as
                 // the group has read tile q - 3 out of it ----------------------------------------------------------
                 const uint64_t a0 = umma_desc(smem_u32(xs), 16, 1024), b0 = umma_desc(smem_u32(cop), 16, 1024);
+                const uint32_t idesc = value ? umma_idesc(32, false) : umma_idesc(64, false);  // V's centres have no lo half
                 for (int i = 0; i < n_tiles; ++i) {
                     const int q = q0 + i, buf = q % kUGroups;
                     if (q >= kUGroups) lost |= !mbar_wait(&bar_dist_free[buf], (q / kUGroups - 1) & 1);
@@ -789,7 +866,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                         for (int ks = 0; ks < 8; ++ks) {  // 16 coordinates per step: 32 bytes inside the swizzled 128-byte row
                             const uint64_t ak = a + static_cast<uint64_t>(((ks >> 2) * kUBoxBytes + (ks & 3) * 32) >> 4);
                             const uint64_t bk = b0 + static_cast<uint64_t>(((ks >> 2) * (kN * 128) + (ks & 3) * 32) >> 4);
-                            umma_f16(d, ak, bk, umma_idesc(kN, false), ks > 0);
+                            umma_f16(d, ak, bk, idesc, ks > 0);
                         }
                         umma_commit(&bar_dist[buf]);
                     }
@@ -830,7 +907,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
             if (flusher) {
                 const int half = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
                 const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-                long long* sums_g = p.sums + static_cast<size_t>(unit) * p.clusters * kHeadDim;
+                long long* sums_g = p.sums[p.iteration % 3] + row0 * kHeadDim;
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     float sum[8];  // the accumulators added in the order they were started
@@ -852,7 +929,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     }
                 }
             }
-            if (tid < p.clusters && cnt_s[tid] > 0) atomicAdd(&p.counts[unit * p.clusters + tid], cnt_s[tid]);
+            if (tid < p.clusters && cnt_s[tid] > 0) atomicAdd(&p.counts[p.iteration % 3][row0 + tid], cnt_s[tid]);
             tc_fence_before();
             workers_sync();  // accumulators, counters and the centre tables are free for the next segment
             tc_fence_after();
@@ -864,6 +941,18 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     tc_fence_before();
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kUTmemCols) : "memory");
+}
+
+// FP16 centres after the last iteration of the tcgen05 form; a warp per centre.
+__global__ void __launch_bounds__(256) kmeans_final_kernel(const UmmaParams p, __half* out0, __half* out1) {
+    wait_for_previous_launch();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, rows = p.units * p.clusters;
+    if (row >= p.sides * rows) return;
+    const int side = row < rows ? 0 : 1;
+    const float4 c = new_centre(p, p.iterations - 1, p.value[side] != 0, row, lane);
+    const __half2 lo = __floats2half2_rn(c.x, c.y), hi = __floats2half2_rn(c.z, c.w);
+    reinterpret_cast<uint2*>((side ? out1 : out0) + static_cast<size_t>(row - side * rows) * kHeadDim)[lane] =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 // New centres from the exact sums; clears sums and counts for the next round.
@@ -953,10 +1042,11 @@ void linspace_indices(int t, int count, int* out) {
     }
 }
 
-// sums, centres, counts, then 256 bytes whose first word is the status word
+// 256 bytes whose first word is the status word, then three generations of sums, two of centres, three of counts (the
+// mma.sync form uses the first of each)
 size_t kmeans_ws_bytes(int units, int clusters) {
     const size_t per = static_cast<size_t>(units) * clusters;
-    return per * kHeadDim * (sizeof(float) + sizeof(long long)) + per * sizeof(int) + 256;
+    return 256 + per * kHeadDim * (3 * sizeof(long long) + 2 * sizeof(float)) + 3 * per * sizeof(int);
 }
 
 using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -976,28 +1066,58 @@ TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-template <bool HILO>
-int launch_umma(const KmeansParams& p, int value, int iterations, void* centroids, cudaStream_t s) {
+// x as (coordinate, token, unit): boxes of 64 coordinates x 128 tokens, 128-byte swizzle, zeros beyond the last token of
+// a unit
+int token_map(CUtensorMap* map, const __half* x, int tokens, int units, int64_t x_stride) {
     TensorMapEncodeFn encode = tensor_map_encoder();
     if (!encode) return fail(RESKV_ERR_CUDA, "kmeans: the driver offers no cuTensorMapEncodeTiled");
-    // x as (coordinate, token, unit): boxes of 64 coordinates x 128 tokens, 128-byte swizzle, zeros beyond the
-    // last token of a unit
-    CUtensorMap xmap;
-    const cuuint64_t dims[3] = {kHeadDim, static_cast<cuuint64_t>(p.tokens), static_cast<cuuint64_t>(p.units)};
-    const cuuint64_t strides[2] = {kHeadDim * sizeof(__half), static_cast<cuuint64_t>(p.x_stride) * kHeadDim * sizeof(__half)};
+    const cuuint64_t dims[3] = {kHeadDim, static_cast<cuuint64_t>(tokens), static_cast<cuuint64_t>(units)};
+    const cuuint64_t strides[2] = {kHeadDim * sizeof(__half), static_cast<cuuint64_t>(x_stride) * kHeadDim * sizeof(__half)};
     const cuuint32_t box[3] = {64, kUTile, 1}, elem[3] = {1, 1, 1};
-    const CUresult made = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(p.x), dims, strides, box, elem,
+    const CUresult made = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(x), dims, strides, box, elem,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (made != CUDA_SUCCESS) return fail(RESKV_ERR_CUDA, "kmeans: cuTensorMapEncodeTiled failed with code %d", static_cast<int>(made));
-    constexpr int kN = HILO ? 64 : 32;
+    return RESKV_OK;
+}
+
+// The workspace's arrays for `units` units (all sides together).
+void place_state(UmmaParams& p, void* workspace, size_t per) {
+    unsigned char* at = static_cast<unsigned char*>(workspace) + 256;
+    p.status = static_cast<uint32_t*>(workspace);
+    for (int i = 0; i < 3; ++i, at += per * kHeadDim * sizeof(long long)) p.sums[i] = reinterpret_cast<long long*>(at);
+    for (int i = 0; i < 2; ++i, at += per * kHeadDim * sizeof(float)) p.centres[i] = reinterpret_cast<float*>(at);
+    for (int i = 0; i < 3; ++i, at += per * sizeof(int)) p.counts[i] = reinterpret_cast<int*>(at);
+}
+
+// Launch that may start while the kernel before it in the stream drains (it waits itself before it touches its results).
+template <class Kernel, class... Args>
+cudaError_t launch_overlapped(Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, bool overlapped, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr, cfg.numAttrs = overlapped ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t s) {
+    CUtensorMap maps[2];
+    for (int i = 0; i < 2; ++i)  // one side: the second map repeats the first and is not used
+        if (int rc = token_map(&maps[i], p.x[i < p.sides ? i : 0], p.tokens, p.units, p.x_stride[i < p.sides ? i : 0])) return rc;
+    const size_t per = static_cast<size_t>(p.sides) * p.units * p.clusters;
+    // the first iteration adds to the first generation; every iteration zeroes the next one
+    if (int rc = check_cuda(cudaMemsetAsync(p.status, 0, 256 + per * kHeadDim * sizeof(long long), s), "kmeans: memset")) return rc;
+    if (int rc = check_cuda(cudaMemsetAsync(p.counts[0], 0, per * sizeof(int), s), "kmeans: memset")) return rc;
+    constexpr int kN = 64;
     const size_t smem = 1024 + static_cast<size_t>(kUStages) * kUTileBytes + 2 * kN * 128 + kUGroups * kUOneHotBytes +
                         32 * kHeadDim * sizeof(float) + 32 * (sizeof(float) + sizeof(int));
     static unsigned long long prepared = 0;  // per-device bit: the shared-memory attribute is set
     int dev = 0;
     cudaGetDevice(&dev);
     if (!((prepared >> (dev & 63)) & 1ull)) {
-        if (int rc = check_cuda(cudaFuncSetAttribute(kmeans_assign_umma_kernel<HILO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (int rc = check_cuda(cudaFuncSetAttribute(kmeans_assign_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      static_cast<int>(smem)),
                                 "cudaFuncSetAttribute(kmeans_assign_umma)"))
             return rc;
@@ -1008,10 +1128,11 @@ int launch_umma(const KmeansParams& p, int value, int iterations, void* centroid
     // half as much again - for the shortest slowest CTA: a share that divides the units evenly often beats the
     // smallest one.
     const int tiles_unit = (p.tokens + kUTile - 1) / kUTile, seg_max = kUChunkMax / kUTile;
-    const long long tiles_total = static_cast<long long>(p.units) * tiles_unit;
+    const long long tiles_total = static_cast<long long>(p.sides) * p.units * tiles_unit;
     const long long even = (tiles_total + sm_count() - 1) / sm_count();
     long long share = even < 4 ? 4 : even, best_cost = -1;
-    for (long long cand = share; cand <= share + share / 2 + 1; ++cand) {
+    const long long step = share / 64 + 1;  // at most ~32 candidates: this is host time
+    for (long long cand = share, most = share + share / 2 + 1; cand <= most; cand += step) {
         long long worst = 0;
         for (long long w0 = 0; w0 < tiles_total; w0 += cand) {
             const long long w1 = w0 + cand < tiles_total ? w0 + cand : tiles_total;
@@ -1028,10 +1149,13 @@ int launch_umma(const KmeansParams& p, int value, int iterations, void* centroid
         if (best_cost < 0 || worst < best_cost) best_cost = worst, share = cand;
     }
     const dim3 grid(static_cast<unsigned>((tiles_total + share - 1) / share));
-    for (int it = 0; it < iterations; ++it) {
-        kmeans_assign_umma_kernel<HILO><<<grid, kUThreads, smem, s>>>(p, xmap, static_cast<int>(share), it == 0, it + 1 == iterations);
-        kmeans_update_kernel<<<p.units, 256, 0, s>>>(p, value, it + 1 == iterations ? static_cast<__half*>(centroids) : nullptr);
-    }
+    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration)
+        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, grid, kUThreads, smem, s, p.iteration > 0, p, maps[0], maps[1],
+                                                  static_cast<int>(share)), "kmeans_assign launch"))
+            return rc;
+    if (int rc = check_cuda(launch_overlapped(kmeans_final_kernel, dim3(static_cast<unsigned>((per + 7) / 8)), 256, 0, s, true, p,
+                                              static_cast<__half*>(centroids0), static_cast<__half*>(centroids1)), "kmeans_final launch"))
+        return rc;
     return check_cuda(cudaGetLastError(), "kmeans launch");
 }
 
@@ -1059,13 +1183,11 @@ extern "C" int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, 
         return fail(RESKV_ERR_WORKSPACE, "kmeans: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     if (int rc = check_device_pointer(x, "kmeans", "x")) return rc;
     if (int rc = check_device_pointer(centroids, "kmeans", "centroids")) return rc;
-    const size_t per = static_cast<size_t>(units) * clusters * kHeadDim;
     KmeansParams p{};
     p.x = static_cast<const __half*>(x);
-    p.sums = static_cast<long long*>(workspace);  // 8-byte aligned first
-    p.centres = reinterpret_cast<float*>(p.sums + per);
-    p.counts = reinterpret_cast<int*>(p.centres + per);
-    p.status = reinterpret_cast<uint32_t*>(p.counts + static_cast<size_t>(units) * clusters);
+    UmmaParams u{};
+    place_state(u, workspace, static_cast<size_t>(units) * clusters);
+    p.sums = u.sums[0], p.centres = u.centres[0], p.counts = u.counts[0], p.status = u.status;
     p.ids = ids;
     p.x_stride = x_tok_stride;
     p.units = units, p.tokens = tokens, p.clusters = clusters;
@@ -1081,12 +1203,16 @@ extern "C" int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, 
     const bool exact = (value & 2) != 0, warp_mma = (value & 4) != 0;
     value &= 1;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    kmeans_init_kernel<<<units, 256, 0, s>>>(p, init, value);
     const int padded = (clusters + 7) / 8 * 8;
     // the integer-counter arrays double as the FP32 reduction buffer [32][kRedStride] of the tensor-core form
     size_t counters = static_cast<size_t>(clusters) * kHeadDim * 2 * sizeof(int);
     const bool fast = !exact && padded <= 32 && aligned16(x);  // the row staging copies 16-byte pieces
-    if (fast && !warp_mma && aligned16(workspace)) return value ? launch_umma<false>(p, value, iterations, centroids, s) : launch_umma<true>(p, value, iterations, centroids, s);
+    if (fast && !warp_mma && aligned16(workspace) && aligned16(centroids)) {
+        u.x[0] = p.x, u.x_stride[0] = x_tok_stride, u.ids[0] = ids, u.value[0] = value, u.sides = 1;
+        u.units = units, u.tokens = tokens, u.clusters = clusters, u.iterations = iterations, u.init = init;
+        return launch_umma(u, centroids, nullptr, s);
+    }
+    kmeans_init_kernel<<<units, 256, 0, s>>>(p, init, value);
     if (fast) counters = static_cast<size_t>(kWarps) * 32 * kRedStride * sizeof(float);
     const size_t smem = static_cast<size_t>(clusters) * kHeadDim * sizeof(float) + counters +
                         kMaxClusters * (sizeof(int) + sizeof(float)) +
@@ -1115,13 +1241,40 @@ extern "C" int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, 
     return check_cuda(cudaGetLastError(), "kmeans launch");
 }
 
+extern "C" int reskv_kmeans_pair(const void* x_k, const void* x_v, int batch, int kv_heads, int tokens, int64_t k_tok_stride,
+                                 int64_t v_tok_stride, int clusters, int iterations, void* workspace, size_t workspace_bytes,
+                                 void* k_centroids, void* v_centroids, int32_t* k_ids, int32_t* v_ids, void* k_ids8, void* v_ids8,
+                                 void* stream) {
+    if (!x_k || !x_v || !k_centroids || !v_centroids || !k_ids || !v_ids) return fail(RESKV_ERR_INVALID, "kmeans_pair: null tensor pointer");
+    if (batch < 1 || kv_heads < 1 || tokens < 1) return fail(RESKV_ERR_INVALID, "kmeans_pair: batch, heads and tokens must be positive");
+    if (clusters < 1 || clusters > 32 || clusters > tokens)
+        return fail(RESKV_ERR_INVALID, "kmeans_pair: cluster count must be in [1,32] and at most the token count, got %d", clusters);
+    if (iterations < 1) return fail(RESKV_ERR_INVALID, "kmeans_pair: iterations must be positive");
+    if (k_tok_stride < tokens || v_tok_stride < tokens) return fail(RESKV_ERR_INVALID, "kmeans_pair: token stride smaller than token count");
+    const int units = batch * kv_heads;
+    const size_t need = kmeans_ws_bytes(2 * units, clusters);
+    if (!workspace || workspace_bytes < need)
+        return fail(RESKV_ERR_WORKSPACE, "kmeans_pair: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    for (const void* ptr : {x_k, x_v, static_cast<const void*>(workspace), static_cast<const void*>(k_centroids), static_cast<const void*>(v_centroids)})
+        if (!aligned16(ptr)) return fail(RESKV_ERR_INVALID, "kmeans_pair: x, workspace and centroids must be 16-byte aligned");
+    if (int rc = check_device_pointer(x_k, "kmeans_pair", "x_k")) return rc;
+    if (int rc = check_device_pointer(x_v, "kmeans_pair", "x_v")) return rc;
+    UmmaParams u{};
+    place_state(u, workspace, static_cast<size_t>(2 * units) * clusters);
+    u.x[0] = static_cast<const __half*>(x_k), u.x[1] = static_cast<const __half*>(x_v);
+    u.x_stride[0] = k_tok_stride, u.x_stride[1] = v_tok_stride;
+    u.ids[0] = k_ids, u.ids[1] = v_ids, u.ids8[0] = static_cast<int8_t*>(k_ids8), u.ids8[1] = static_cast<int8_t*>(v_ids8);
+    u.value[0] = 0, u.value[1] = 1;
+    u.sides = 2, u.units = units, u.tokens = tokens, u.clusters = clusters, u.iterations = iterations;
+    linspace_indices(tokens, clusters, u.init.idx);
+    return launch_umma(u, k_centroids, v_centroids, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int reskv_kmeans_status(const void* workspace, int batch, int kv_heads, int clusters, uint32_t* status, void* stream) {
     if (!workspace || !status) return fail(RESKV_ERR_INVALID, "kmeans_status: null pointer");
     if (batch < 1 || kv_heads < 1 || clusters < 1 || clusters > kMaxClusters) return fail(RESKV_ERR_INVALID, "kmeans_status: bad sizes");
-    const size_t per = static_cast<size_t>(batch) * kv_heads * clusters;
-    const size_t at = per * kHeadDim * (sizeof(float) + sizeof(long long)) + per * sizeof(int);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (int rc = check_cuda(cudaMemcpyAsync(status, static_cast<const unsigned char*>(workspace) + at, sizeof(uint32_t),
+    if (int rc = check_cuda(cudaMemcpyAsync(status, workspace, sizeof(uint32_t),
                                             cudaMemcpyDeviceToHost, s),
                             "kmeans_status copy"))
         return rc;
