@@ -105,6 +105,26 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// ---- launches that overlap (programmatic stream serialisation) -----------------------------------------------------
+// A kernel launched with launch_overlapped may start while the kernel before it in the stream still runs, once every
+// block of that one has called let_next_launch_start (or ended).  Before wait_for_previous_launch it touches nothing
+// that an unfinished kernel may write, and writes nothing; data written by others is read through L2 or with plain
+// loads, not with the non-coherent ones.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool overlapped,
+                              const Args&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr, cfg.numAttrs = overlapped ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

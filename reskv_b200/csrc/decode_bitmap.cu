@@ -454,8 +454,7 @@ int launch_partial_mma_beta(const DecodeParams& p, cudaStream_t stream) {
     static unsigned long long done = 0;
     if (int rc = allow_smem(kern, mma::Smem<GQA, ML>::bytes(kMaxClusters), done, "cudaFuncSetAttribute(decode_bitmap_mma)"))
         return rc;
-    kern<<<p.grid, mma::kThreadsM, smem, stream>>>(p);
-    return check_cuda(cudaGetLastError(), "decode_bitmap_mma launch");
+    return check_cuda(launch_overlapped(kern, dim3(p.grid), mma::kThreadsM, smem, stream, true, p), "decode_bitmap_mma launch");
 }
 
 // up to 32 value centroids: the instance with two cluster-mass blocks
@@ -531,15 +530,14 @@ size_t workspace_bytes(int bnh, int splits) {
 struct PartialPlan {
     int slots;     // partial results per query head in the workspace
     int chunk;     // granules (tensor-core kernel) or tiles (warp-per-token kernel) per CTA
+    int n_pad;     // granules a unit is padded to
     int grid;      // CTAs of the tensor-core kernel (the warp-per-token kernel runs slots x units)
-    int balanced;  // 1: equal share of all granules per CTA, 0: one CTA per (unit, split)
+    int balanced;  // 1: partial_schedule, 0: one CTA per (unit, split)
 };
 
-// splits_req > 0 (caller's choice) or the warp-per-token kernel: fixed splits per unit.  Otherwise the balanced
-// schedule: at most one CTA per SM, every CTA streams ceil(all granules / CTAs) consecutive granules, so the per-CTA
-// tables are built once per CTA and no SM idles on a partial last wave.  A unit of n granules is then touched by at
-// most (n - 1) / chunk + 2 CTAs.  With a device-side token count (`dyn`) chunk is recomputed on the device, which keeps
-// that figure below ceil(grid / units) + 1 for any n.
+// splits_req > 0 (caller's choice) or the warp-per-token kernel: fixed splits per unit.  Otherwise partial_schedule for
+// one CTA per SM.  A unit of n granules is then touched by at most (n - 1) / chunk + 2 CTAs; with a device-side token
+// count (`dyn`), where the schedule is made on the device, by at most ceil(grid / units) + 1 for any n.
 PartialPlan plan_partials(int units, int tokens, int splits_req, bool tensor_core, bool dyn, int64_t tok_stride) {
     const int step = tensor_core ? kGranule : kTile, steps = (tokens + step - 1) / step;
     PartialPlan pp{};
@@ -548,21 +546,22 @@ PartialPlan plan_partials(int units, int tokens, int splits_req, bool tensor_cor
         if (splits > steps) splits = steps;
         const int per = (steps + splits - 1) / splits;
         splits = (steps + per - 1) / per;  // drop splits that would get nothing
-        pp.slots = splits, pp.chunk = per, pp.grid = units * splits, pp.balanced = 0;
+        pp.slots = splits, pp.chunk = per, pp.n_pad = per * splits, pp.grid = units * splits, pp.balanced = 0;
         return pp;
     }
-    const long long most = dyn ? (tok_stride + step - 1) / step : steps, all = units * most;
-    long long grid = sm_count();
-    if (grid * kMinChunk > all) grid = (all + kMinChunk - 1) / kMinChunk;
-    const long long chunk = (static_cast<long long>(units) * steps + grid - 1) / grid;
+    const int sms = sm_count();
+    pp.balanced = 1;
     if (dyn) {
-        pp.slots = static_cast<int>((grid + units - 1) / units) + 1;
-    } else {
-        grid = (static_cast<long long>(units) * steps + chunk - 1) / chunk;  // CTAs that get granules
-        const long long s = (steps - 1) / chunk + 2;
-        pp.slots = static_cast<int>(s < steps ? s : steps);
+        const long long most = units * ((tok_stride + step - 1) / step);
+        pp.grid = static_cast<int>(sms * static_cast<long long>(kMinChunk) > most ? (most + kMinChunk - 1) / kMinChunk : sms);
+        pp.slots = (pp.grid + units - 1) / units + 1;
+        return pp;
     }
-    pp.chunk = static_cast<int>(chunk), pp.grid = static_cast<int>(grid), pp.balanced = 1;
+    const PartialSchedule sched = partial_schedule(units, steps, sms);
+    pp.chunk = sched.chunk, pp.n_pad = sched.n_pad;
+    pp.grid = static_cast<int>((static_cast<long long>(units) * pp.n_pad + pp.chunk - 1) / pp.chunk);
+    const int pieces = (steps + pp.chunk - 1) / pp.chunk;
+    pp.slots = pp.n_pad % pp.chunk == 0 ? pieces : (steps - 1) / pp.chunk + 2 < steps ? (steps - 1) / pp.chunk + 2 : steps;
     return pp;
 }
 
@@ -705,7 +704,7 @@ int decode_common(const DecodeArgs& a, LayoutId layout, bool has_meta, bool has_
     p.start_pos = a.start_pos, p.pos_q = a.pos_q, p.splits = splits, p.chunk = per;
     p.theta = a.theta, p.scaling = a.scaling;
     p.dyn = a.dyn;
-    p.units = units, p.balanced = pp.balanced, p.grid = pp.grid;
+    p.units = units, p.balanced = pp.balanced, p.grid = pp.grid, p.n_pad = pp.n_pad;
 
     cudaStream_t s = static_cast<cudaStream_t>(a.stream);
     if (g_ev_start) cudaEventRecord(g_ev_start, s);

@@ -47,10 +47,10 @@ struct DecodeParams {
     // splits = partial slots per query head in the workspace; chunk = granules (tensor-core kernel) or tiles (warp-per-
     // token kernel) per CTA
     int start_pos, pos_q, splits, chunk;
-    // units = batch * kv heads.  balanced != 0: the tensor-core kernel runs a 1-D grid whose CTAs each take an
-    // equal share of all units' granules (a CTA may finish one unit and start the next); balanced == 0: one CTA per
+    // units = batch * kv heads.  n_pad: granules a unit is padded to (see partial_schedule).  balanced != 0: the tensor-
+    // core kernel's own schedule, recomputed on the device when the token count lives there; balanced == 0: one CTA per
     // (unit, split) with `chunk` granules or tiles each.
-    int units, balanced, grid;  // grid = CTAs of the tensor-core kernel
+    int units, balanced, grid, n_pad;  // grid = CTAs of the tensor-core kernel
     float theta, scaling;
     // optional device-resident step state {query position, dense-window tokens, compressed tokens
     // or -1, reserved}: when set it overrides pos_q, the merge kernel's recent-token count and
@@ -101,6 +101,36 @@ __device__ __forceinline__ int split_tiles(const DecodeParams& p, int total_tile
 
 // query position of this launch: from the device step state when one is attached
 __device__ __forceinline__ int query_position(const DecodeParams& p) { return p.dyn ? p.dyn[0] : p.pos_q; }
+
+// How the tensor-core kernel's granules are dealt out to `ctas` CTAs: the granules of all units are laid end to end, every
+// unit padded to n_pad of them, and CTA c takes [c * chunk, (c + 1) * chunk).
+struct PartialSchedule {
+    int chunk, n_pad;
+};
+
+// Either an even share of everything (n_pad = the unit's granules; a CTA may then end one unit and start the next), or
+// ctas / units equal pieces of every unit, whichever has the shorter slowest CTA.  Times in cycles, measured: a pass of
+// 16 rows on each of 4, 8, 12 or 16 warps 4500, 5700, 6800 or 8000; a further segment in a CTA (centroids, query,
+// combining, writing) 5000.
+__host__ __device__ inline long long segment_cycles(long long granules) {
+    constexpr int kPass = 8;  // granules per pass: 256 tokens
+    const long long rest = granules % kPass;
+    return granules / kPass * 8000 + (rest ? 4500 + (rest - 1) / 2 * 1167 : 0);
+}
+__host__ __device__ inline PartialSchedule partial_schedule(int units, int granules, int ctas) {
+    long long even = (static_cast<long long>(units) * granules + ctas - 1) / ctas;
+    if (even < kMinChunk) even = kMinChunk;
+    PartialSchedule s{static_cast<int>(even), granules};
+    if (units <= ctas) {
+        const int pieces = ctas / units;
+        int piece = (granules + pieces - 1) / pieces;
+        if (piece < kMinChunk) piece = kMinChunk;
+        const bool crosses = granules % even != 0;
+        if (segment_cycles(piece) <= segment_cycles(even) + (crosses ? 5000 : 0))
+            s.chunk = piece, s.n_pad = (granules + piece - 1) / piece * piece;
+    }
+    return s;
+}
 
 namespace {
 

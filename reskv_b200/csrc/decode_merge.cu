@@ -43,10 +43,10 @@ __global__ void __launch_bounds__(kMergeThreads, G == 8 ? 1 : 2) decode_merge_ke
     float* stat_s = part_s + kMergeWarps * G * kPart;                                       // [warps][G][4]
     float* prob_s = stat_s + kMergeWarps * G * 4 + warp * kBlock * G;                       // [16][G] of this warp
     float* beta_s = stat_s + kMergeWarps * G * 4 + kMergeWarps * kBlock * G;                // [G][64]
-    const int tr = p.dyn ? max(min(p.dyn[1], recent_max), 0) : p.tr;
-    // a window count beyond the buffers is cut (the newest tokens are then missing from the result): tell the host
-    if (p.dyn && p.status && tid == 0 && unit == 0 && (p.dyn[1] > recent_max || p.dyn[1] < 0))
-        atomicOr(p.status, RESKV_STATUS_STATE_RANGE);
+    // may run while the partial kernel drains: the window, the query and the value centroids are older than that kernel
+    let_next_launch_start();
+    const int counted = p.dyn ? __ldcg(p.dyn + 1) : p.tr;
+    const int tr = p.dyn ? max(min(counted, recent_max), 0) : counted;
     for (int i = tid; i < p.cv * (kHeadDim / 8); i += kMergeThreads)
         cp_async16(vc_s + i * 8, p.vc + static_cast<size_t>(unit) * p.cv * kHeadDim + i * 8);
 
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kMergeThreads, G == 8 ? 1 : 2) decode_merge_ke
             const int t = base + g + 8 * r;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                kf[r][k] = t < tr ? __ldg(reinterpret_cast<const uint4*>(rk_g + static_cast<size_t>(t) * kHeadDim) + piece(k))
+                kf[r][k] = t < tr ? __ldcg(reinterpret_cast<const uint4*>(rk_g + static_cast<size_t>(t) * kHeadDim) + piece(k))
                                   : make_uint4(0u, 0u, 0u, 0u);
         }
     };
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kMergeThreads, G == 8 ? 1 : 2) decode_merge_ke
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (wide) {
-                    qf[k] = __ldg(reinterpret_cast<const uint4*>(qrow) + piece(k));
+                    qf[k] = __ldcg(reinterpret_cast<const uint4*>(qrow) + piece(k));
                 } else {
                     const unsigned short* h = reinterpret_cast<const unsigned short*>(qrow) + 8 * piece(k);
                     qf[k] = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
@@ -89,6 +89,10 @@ __global__ void __launch_bounds__(kMergeThreads, G == 8 ? 1 : 2) decode_merge_ke
         }
         load_values(warp * kBlock);
     }
+
+    wait_for_previous_launch();
+    // a window count beyond the buffers is cut (the newest tokens are then missing from the result): tell the host
+    if (p.dyn && p.status && tid == 0 && unit == 0 && counted != tr) atomicOr(p.status, RESKV_STATUS_STATE_RANGE);
 
     // ---- compressed part: this warp's slots ---------------------------------------------------------------------------
     // per head: running maximum (log2 domain) and sum of the compressed tokens; numerator and cluster masses
@@ -283,8 +287,9 @@ int launch(const MergeParams& mp, int units, int recent_max, cudaStream_t s) {
     }
     MergeParams p = mp;
     p.cv = cv;
-    decode_merge_kernel<G><<<units, kMergeThreads, smem, s>>>(p, recent_max);
-    return check_cuda(cudaGetLastError(), "decode_merge launch");
+    // on its own (no partial kernel of this library in front) it starts when what is in front has ended
+    return check_cuda(launch_overlapped(decode_merge_kernel<G>, dim3(units), kMergeThreads, smem, s, mp.splits > 0, p, recent_max),
+                      "decode_merge launch");
 }
 
 }  // namespace

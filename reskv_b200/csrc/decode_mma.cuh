@@ -135,22 +135,27 @@ __device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
 constexpr int kColTrig = 0, kColAcc = 32, kColBeta = 64, kColsWarp = 80, kTmemCols = 512;
 static_assert(kColsWarp * (kWarpsM / 4) <= kTmemCols, "tensor memory");
 
-// Dynamic shared memory, in this order: the warps' rows (the end of a segment reuses their memory for the warps'
-// results), key centroids, rotated queries (before the first of them: the offset tables), query items, step table, rank
-// bases.
+// A warp's results of one head at the end of a segment: coordinate d at red_pos(d), cluster masses, maximum and sum.  The
+// strides keep the stores of a warp (lanes g, q; one coordinate of the field) in distinct banks.
+constexpr int kRedAcc = 152, kRedBeta = 72;
+__device__ __forceinline__ int red_pos(int d) { return (d & 15) * 9 + (d >> 4); }
+
+// Dynamic shared memory, in this order: the warps' rows and, for the set-up, the offset tables (the end of a segment
+// reuses their memory for the warps' results), key centroids, rotated queries, query items, step table, rank bases.
 template <int GQA, class ML>
 struct Smem {
     static constexpr size_t kRing = sizeof(WarpRows<ML>) * kWarpsM;
-    static constexpr size_t kRed = static_cast<size_t>(kWarpsM) * GQA * (kHeadDim + kMaxClusters + 2) * sizeof(float);
-    static constexpr size_t kRegion = ((kRing > kRed ? kRing : kRed) + 127) / 128 * 128;
+    static constexpr size_t kRed = static_cast<size_t>(kWarpsM) * GQA * (kRedAcc + kRedBeta + 2) * sizeof(float);
+    static constexpr size_t kTrig = (kWarpsM + 8) * 64 * sizeof(float2);
+    static constexpr size_t kRegion = ((kRing + kTrig > kRed ? kRing + kTrig : kRed) + 127) / 128 * 128;
     static constexpr size_t kQuery = 2 * 2 * query_rows<GQA>() * kQStride * sizeof(__half);  // [buffers][hi, lo][rows]
     static constexpr size_t kItems = static_cast<size_t>(2 * GQA) * 32 * 2 * sizeof(float4);  // raw query, angle state
     static constexpr size_t kStep = 64 * (sizeof(float2) + sizeof(float));  // (cos, sin) of a pass's step, frequencies
-    static constexpr size_t kTrig = (kWarpsM + 8) * 64 * sizeof(float2);
     static constexpr size_t kPre = kWarpsM * 32 * sizeof(uint2);
-    static constexpr size_t kQueryOrTrig = kQuery > kTrig ? kQuery : kTrig;
+    static constexpr size_t kFixed = kRegion + kQuery + kItems + kStep + kPre;
+    static_assert(kFixed + kMaxClusters * kCenStride * sizeof(float) <= 227 * 1024 - 256, "shared memory");
     static constexpr size_t bytes(int ck) {
-        return kRegion + static_cast<size_t>(ck) * kCenStride * sizeof(float) + kQueryOrTrig + kItems + kStep + kPre;
+        return kRegion + static_cast<size_t>(ck) * kCenStride * sizeof(float) + kQuery + kItems + kStep + kPre;
     }
 };
 
@@ -481,50 +486,63 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
     constexpr int kQItems = 2 * GQA;  // rows of the rotated query: X's heads, Y's heads
     float* kc_s = reinterpret_cast<float*>(smem_raw + SM::kRegion);
     __half* qf = reinterpret_cast<__half*>(kc_s + static_cast<size_t>(p.ck) * kCenStride);  // [2 bufs][hi, lo][kRows][kQStride]
-    float4* items = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(qf) + SM::kQueryOrTrig);  // [kQItems][32][query, state]
+    float4* items = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(qf) + SM::kQuery);  // [kQItems][32][query, state]
     float2* step_s = reinterpret_cast<float2*>(items + kQItems * 64);                        // [64] (cos, sin) of kTileM f
     float* freq_s = reinterpret_cast<float*>(step_s + 64);                                    // [64]
     uint2* pre = reinterpret_cast<uint2*>(freq_s + 64) + (threadIdx.x >> 5) * 32;             // rank bases: K's 16 rows, V's
     // (cos, sin) of 8 w f and of g f: [pair i][w or g][q], the pair of frequencies 16 q + 2 i, + 1 in 16 bytes
-    float2 *trig_w = reinterpret_cast<float2*>(qf), *trig_g = trig_w + kWarpsM * 64;
+    float2 *trig_w = reinterpret_cast<float2*>(smem_raw + SM::kRing), *trig_g = trig_w + kWarpsM * 64;
+    static_assert(SM::kRing % 16 == 0, "16-byte loads of the tables");
     __shared__ uint64_t query_bar;  // one arrival per warp when its rows of the next rotated query are written
     __shared__ uint32_t tmem_s;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, qd = lane & 3;
     Rows& rows = reinterpret_cast<Rows*>(smem_raw)[warp];
+    // ---- what touches no memory of others: this may run while the kernel before drains -------------------------------
+    if (tid == 0) {
+        mbar_init(&query_bar, kWarpsM);
+        mbar_fence_init();
+    }
+    if (warp == kWarpsM - 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    auto free_tmem = [&] {  // after a barrier that every warp has passed
+        if (warp == kWarpsM - 1)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"(kTmemCols) : "memory");
+    };
+    wait_for_previous_launch();
+    let_next_launch_start();
+
     const float my_freq = rope_freq(p.inv_freq, p.theta, tid & 63);
+    const float q_freq[2] = {rope_freq(p.inv_freq, p.theta, 2 * lane), rope_freq(p.inv_freq, p.theta, 2 * lane + 1)};
     const int tokens = token_count(p);
     const int granules = max((tokens + kGranule - 1) / kGranule, 1);
-    // Work of the launch = the granules of all units laid end to end, every unit padded to n_pad granules.  CTA c takes
-    // the range [c * chunk, (c + 1) * chunk) and walks it unit by unit; the part of one unit inside the range is a
-    // *segment* and produces one partial result (slot = number of CTAs that started earlier on the same unit).
-    // Balanced schedule: n_pad = granules of a unit and chunk = all granules / CTAs; fixed-split schedule: n_pad =
-    // chunk * splits, i.e. exactly one segment per CTA.
-    int n_pad, chunk;
-    if (p.balanced) {
-        n_pad = granules;
-        chunk = p.dyn ? max(static_cast<int>((static_cast<long long>(p.units) * n_pad + gridDim.x - 1) / gridDim.x), kMinChunk)
-                      : p.chunk;
-    } else {
-        chunk = p.dyn ? (granules + p.splits - 1) / p.splits : p.chunk;
-        n_pad = chunk * p.splits;
+    // Work of the launch (see partial_schedule): CTA c takes the granules [c * chunk, (c + 1) * chunk) of all units laid
+    // end to end and walks them unit by unit; the part of one unit inside the range is a *segment* and produces one
+    // partial result (slot = number of CTAs that started earlier on the same unit).
+    int n_pad = p.n_pad, chunk = p.chunk;
+    if (p.dyn) {
+        if (p.balanced) {
+            const PartialSchedule sched = partial_schedule(p.units, granules, gridDim.x);
+            n_pad = sched.n_pad, chunk = sched.chunk;
+        } else {
+            chunk = (granules + p.splits - 1) / p.splits;
+            n_pad = chunk * p.splits;
+        }
     }
     const uint32_t work_total = static_cast<uint32_t>(p.units) * n_pad;  // the host keeps it below 2^31
     uint32_t work = blockIdx.x * static_cast<uint32_t>(chunk);
     const uint32_t work_end = min(work_total, work + chunk);
     // a device-side token count beyond the buffers is cut to the token stride: tell the host
     if (p.dyn && blockIdx.x == 0 && tid == 0 && p.dyn[2] > p.tok_stride) atomicOr(p.status, RESKV_STATUS_STATE_RANGE);
-    if (work >= work_end) return;
+    if (work >= work_end) {
+        __syncthreads();
+        free_tmem();
+        return;
+    }
 
-    if (tid == 0) {
-        mbar_init(&query_bar, kWarpsM);
-        mbar_fence_init();
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     uint32_t query_phase = 0, tmem = 0;
     bool lost = false;
     bool set_up = false;
@@ -549,12 +567,15 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int idx = tid + k * kThreadsM;
-            if (idx < p.ck * (kHeadDim / 8)) cen_raw[k] = __ldg(reinterpret_cast<const uint4*>(p.kc + static_cast<size_t>(unit) * p.ck * kHeadDim) + idx);
+            if (idx < p.ck * (kHeadDim / 8)) cen_raw[k] = reinterpret_cast<const uint4*>(p.kc + static_cast<size_t>(unit) * p.ck * kHeadDim)[idx];
         }
         static_assert(2 * kThreadsM * 8 >= kMaxClusters * kHeadDim, "two steps cover the table");
-        __half q_raw[4] = {};  // query item `warp` (see write_query): coordinates 2 lane, + 1 and their partners
-        if (warp < kQItems) {
-            const __half* qrow = p.q + (static_cast<size_t>(b) * p.nh + hkv * GQA + warp % GQA) * kHeadDim + 2 * lane;
+        // query item of this warp (see write_query): coordinates 2 lane, + 1 and their partners; the upper warps begin,
+        // they have fewer rows of the tables below to fill
+        constexpr int kQFirst = kWarpsM - kQItems;
+        __half q_raw[4] = {};
+        if (warp >= kQFirst) {
+            const __half* qrow = p.q + (static_cast<size_t>(b) * p.nh + hkv * GQA + (warp - kQFirst) % GQA) * kHeadDim + 2 * lane;
             q_raw[0] = qrow[0], q_raw[1] = qrow[1], q_raw[2] = qrow[64], q_raw[3] = qrow[65];
         }
 
@@ -624,10 +645,10 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             if ((lane & 7) < (my_y ? ps.left_y : ps.left_x)) {
                 // volatile: issue the loads here, a whole pass ahead of their use, instead of letting the
                 // compiler sink them next to the consumer
-                asm volatile("ld.global.nc.s8 %0, [%1];" : "=r"(id) : "l"(id_src + off));
+                asm volatile("ld.global.s8 %0, [%1];" : "=r"(id) : "l"(id_src + off));
                 if constexpr (ML::kScale) {
                     unsigned short h;
-                    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(h) : "l"(sc_src + off));
+                    asm volatile("ld.global.u16 %0, [%1];" : "=h"(h) : "l"(sc_src + off));
                     scale = h;
                 }
             }
@@ -656,29 +677,10 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                               : r < kWarpsM + 8 ? trig_g + (pair * 8 + r - kWarpsM) * 8 + at : step_s + i;
                 *dst = make_float2(c, s);
             }
-            tc_fence_before();
-            __syncthreads();  // and the barrier is initialised, tensor memory allocated
-            tc_fence_after();
-            tmem = tmem_s + (static_cast<uint32_t>(warp % 4 * 32) << 16) + warp / 4 * kColsWarp;
-            const float4 *ta = reinterpret_cast<const float4*>(trig_w) + warp * 4 + qd, *tb = reinterpret_cast<const float4*>(trig_g) + lane;
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                float v[8];
-#pragma unroll
-                for (int e2 = 0; e2 < 2; ++e2) {
-                    const float4 a = ta[(2 * ks + e2) * kWarpsM * 4], e = tb[(2 * ks + e2) * 32];
-                    v[2 * e2] = a.x * e.x - a.y * e.y, v[2 * e2 + 1] = a.z * e.z - a.w * e.w;
-                    v[4 + 2 * e2] = a.y * e.x + a.x * e.y, v[5 + 2 * e2] = a.w * e.z + a.z * e.w;
-                }
-                tmem_st8(tmem + kColTrig + 8 * ks, v);
+            if constexpr (GQA == 1) {  // columns without a head: rows 0 and 4 of every buffer have one
+                for (int i = tid; i < static_cast<int>(SM::kQuery / 4); i += kThreadsM)
+                    if (i / (kQStride / 2) % 4 != 0) reinterpret_cast<uint32_t*>(qf)[i] = 0u;
             }
-            tmem_st_wait();
-            __syncthreads();  // the tables' memory takes the rotated queries
-            if constexpr (GQA == 1) {  // columns without a head
-                for (int i = tid; i < static_cast<int>(SM::kQuery / 4); i += kThreadsM) reinterpret_cast<uint32_t*>(qf)[i] = 0u;
-                __syncthreads();
-            }
-            set_up = true;
         }
 
         // ---- per unit: key centroids (FP32, two copies) ----------------------------------------------------------
@@ -699,28 +701,30 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
         // work, two frequencies per lane; the rows move on to other warps from pass to pass.  The angle goes down by
         // kTileM f per pass and is seeded exactly every kReseedTiles passes and where the sub-tile is shorter.
         auto write_query = [&](int it, int sub_len) {
-            for (int r = (warp + it * 4) % kWarpsM; r < kQItems; r += kWarpsM) {
+            for (int r = (warp + kWarpsM - kQFirst + it * 4) % kWarpsM; r < kQItems; r += kWarpsM) {
                 const int sub = r / GQA, h = r % GQA, i2 = 2 * lane;
                 float4* item = items + (r * 32 + lane) * 2;
                 float4 qv, st;
                 if (it == 0) {
-                    const float q_mul = p.scaling * kLog2e;  // here r == warp
+                    const float q_mul = p.scaling * kLog2e;
                     qv = make_float4(__half2float(q_raw[0]) * q_mul, __half2float(q_raw[1]) * q_mul, __half2float(q_raw[2]) * q_mul,
                                      __half2float(q_raw[3]) * q_mul);
                     item[0] = qv;
                 } else {
-                    qv = item[0], st = item[1];
+                    const float4 old = item[1], dn = *reinterpret_cast<const float4*>(step_s + i2);  // angle - kTileM f
+                    qv = item[0];
+                    st = make_float4(old.x * dn.x + old.y * dn.y, old.y * dn.x - old.x * dn.y, old.z * dn.z + old.w * dn.w,
+                                     old.w * dn.z - old.z * dn.w);
                 }
                 if (it % kReseedTiles == 0 || sub_len != kSub) {
                     const float delta = static_cast<float>(query_position(p) - (p.start_pos + t_begin + it * kTileM + sub * sub_len));
-                    sincosf(delta * freq_s[i2], &st.y, &st.x);
-                    sincosf(delta * freq_s[i2 + 1], &st.w, &st.z);
+                    const float f0 = it == 0 ? q_freq[0] : freq_s[i2], f1 = it == 0 ? q_freq[1] : freq_s[i2 + 1];
+                    sincosf(delta * f0, &st.y, &st.x);
+                    sincosf(delta * f1, &st.w, &st.z);
                 }
+                item[1] = st;
                 const float lo0 = qv.x * st.x - qv.z * st.y, hi0 = qv.z * st.x + qv.x * st.y;
                 const float lo1 = qv.y * st.z - qv.w * st.w, hi1 = qv.w * st.z + qv.y * st.w;
-                const float4 dn = *reinterpret_cast<const float4*>(step_s + i2);  // next pass: angle - kTileM f
-                item[1] = make_float4(st.x * dn.x + st.y * dn.y, st.y * dn.x - st.x * dn.y, st.z * dn.z + st.w * dn.w,
-                                      st.w * dn.z - st.z * dn.w);
                 uint32_t lh, ll, hh, hl;
                 split_h2(lo0, lo1, lh, ll);
                 split_h2(hi0, hi1, hh, hl);
@@ -733,6 +737,26 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
         static_assert(kQItems <= kWarpsM, "one query item per warp");
         if (ntiles > 0) write_query(0, next.sub);
 
+        tc_fence_before();
+        __syncthreads();  // tables, centroids and the first rotated query in place (and tensor memory allocated)
+        tc_fence_after();
+        if (!set_up) {
+            tmem = tmem_s + (static_cast<uint32_t>(warp % 4 * 32) << 16) + warp / 4 * kColsWarp;
+            const float4 *ta = reinterpret_cast<const float4*>(trig_w) + warp * 4 + qd, *tb = reinterpret_cast<const float4*>(trig_g) + lane;
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+                float v[8];
+#pragma unroll
+                for (int e2 = 0; e2 < 2; ++e2) {
+                    const float4 a = ta[(2 * ks + e2) * kWarpsM * 4], e = tb[(2 * ks + e2) * 32];
+                    v[2 * e2] = a.x * e.x - a.y * e.y, v[2 * e2 + 1] = a.z * e.z - a.w * e.w;
+                    v[4 + 2 * e2] = a.y * e.x + a.x * e.y, v[5 + 2 * e2] = a.w * e.z + a.z * e.w;
+                }
+                tmem_st8(tmem + kColTrig + 8 * ks, v);
+            }
+            set_up = true;
+        }
+
         // ---- per-warp running state ------------------------------------------------------------------------------------
         // O^T in tensor memory, m-block i -> coordinate 16g + first(i) (c0, c1) and 16g + second(i) (c2, c3), columns 2q,
         // 2q+1; beta[value cluster 16 mb + g (+ 8)][columns 2q, 2q + 1] behind it
@@ -744,8 +768,8 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             tmem_st32(tmem + kColAcc, zero);
             tmem_store_beta<BETA>(tmem + kColBeta, reinterpret_cast<float(&)[4 * BETA]>(zero));
         }
-
-        __syncthreads();  // centroid table and first rotated query ready (and the barrier initialised)
+        tmem_st_wait();
+        const int busy_warps = min(next.sub >> 3, kWarpsM);  // warps that get tokens (all of them unless there is one short pass)
 
         for (int it = 0; it < ntiles; ++it) {
             const int ids_cur = ids_next;
@@ -1001,18 +1025,18 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();  // every warp is done with its rows: their memory takes the warps' results
-        float* red_acc = reinterpret_cast<float*>(smem_raw);             // [warps][GQA][128]
-        float* red_beta = red_acc + kWarpsM * GQA * kHeadDim;            // [warps][GQA][64]
-        float* red_ml = red_beta + kWarpsM * GQA * kMaxClusters;         // [warps][GQA][m, l]
-        if (kDual || qd < 2) {
+        float* red_acc = reinterpret_cast<float*>(smem_raw);             // [warps][GQA][kRedAcc]
+        float* red_beta = red_acc + kWarpsM * GQA * kRedAcc;             // [warps][GQA][kRedBeta]
+        float* red_ml = red_beta + kWarpsM * GQA * kRedBeta;             // [warps][GQA][m, l]
+        if ((kDual || qd < 2) && warp < busy_warps) {
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int h = 2 * qd + u;
                 if (h < GQA) {
-                    float* dst = red_acc + (warp * GQA + h) * kHeadDim + 16 * g;
+                    float* dst = red_acc + (warp * GQA + h) * kRedAcc + g;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) dst[Field::first(i)] = acc[i][u], dst[Field::second(i)] = acc[i][2 + u];
-                    float* bdst = red_beta + (warp * GQA + h) * kMaxClusters + g;
+                    for (int i = 0; i < 8; ++i) dst[9 * Field::first(i)] = acc[i][u], dst[9 * Field::second(i)] = acc[i][2 + u];
+                    float* bdst = red_beta + (warp * GQA + h) * kRedBeta + g;
 #pragma unroll
                     for (int mb = 0; mb < 4; ++mb) {
                         bdst[16 * mb] = mb < BETA ? bacc[mb < BETA ? mb : 0][u] : 0.f;
@@ -1031,18 +1055,19 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             for (int idx = tid; idx < GQA * ((kHeadDim + kMaxClusters) / 2); idx += kThreadsM) {  // two values per step
                 constexpr int kPer = (kHeadDim + kMaxClusters) / 2;
                 const int h = idx / kPer, d = 2 * (idx % kPer);
+                const float* src = d < kHeadDim ? red_acc + h * kRedAcc : red_beta + h * kRedBeta;
+                const int at0 = d < kHeadDim ? red_pos(d) : d - kHeadDim, at1 = d < kHeadDim ? red_pos(d + 1) : at0 + 1;
+                const int stride = d < kHeadDim ? GQA * kRedAcc : GQA * kRedBeta;
                 float fm = kNoMax;
-#pragma unroll
-                for (int w = 0; w < kWarpsM; ++w) fm = fmaxf(fm, red_ml[(w * GQA + h) * 2]);
+#pragma unroll 4
+                for (int w = 0; w < busy_warps; ++w) fm = fmaxf(fm, red_ml[(w * GQA + h) * 2]);
                 float2 sum = make_float2(0.f, 0.f);
                 float fl = 0.f;
-#pragma unroll
-                for (int w = 0; w < kWarpsM; ++w) {
+#pragma unroll 4
+                for (int w = 0; w < busy_warps; ++w) {
                     const float2 ml = *reinterpret_cast<const float2*>(red_ml + (w * GQA + h) * 2);
                     const float weight = fast_exp2(ml.x - fm);
-                    const float2 v = *reinterpret_cast<const float2*>(
-                        d < kHeadDim ? red_acc + (w * GQA + h) * kHeadDim + d : red_beta + (w * GQA + h) * kMaxClusters + d - kHeadDim);
-                    sum.x = fmaf(v.x, weight, sum.x), sum.y = fmaf(v.y, weight, sum.y);
+                    sum.x = fmaf(src[w * stride + at0], weight, sum.x), sum.y = fmaf(src[w * stride + at1], weight, sum.y);
                     fl = fmaf(ml.y, weight, fl);
                 }
                 const size_t row = (part + h) * p.splits + slot;
@@ -1066,8 +1091,7 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
         __syncthreads();  // the next segment's copies go into the memory just read
     }
     if (lost && lane == 0) atomicOr(p.status, RESKV_STATUS_WAIT_TIMEOUT);
-    if (warp == 0)  // every warp is past the last segment's final barrier
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"(kTmemCols) : "memory");
+    free_tmem();  // every warp is past the last segment's final barrier
 }
 
 }  // namespace mma

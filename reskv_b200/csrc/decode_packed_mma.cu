@@ -22,8 +22,7 @@ int launch_beta(const DecodeParams& p, cudaStream_t stream) {
             return rc;
         if (dev >= 0 && dev < 64) done |= 1ull << dev;
     }
-    kern<<<p.grid, mma::kThreadsM, smem, stream>>>(p);
-    return check_cuda(cudaGetLastError(), "decode_mma (packed layout) launch");
+    return check_cuda(launch_overlapped(kern, dim3(p.grid), mma::kThreadsM, smem, stream, true, p), "decode_mma (packed layout) launch");
 }
 
 // up to 32 value centroids: the instance with two cluster-mass blocks

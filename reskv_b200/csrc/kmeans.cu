@@ -549,9 +549,6 @@ constexpr int kUWorkers = kUThreads - 32;  // everyone but the copying warp: the
 
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kUWorkers) : "memory"); }
 
-__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Four coordinates of a centre after iteration `from`: the mean of the tokens assigned then, the old centre (K) or zero
 // (V) where there were none; V's centres are rounded to FP16.
 __device__ __forceinline__ float4 new_centre(const UmmaParams& p, int from, bool value, size_t row, int i4) {
@@ -1088,18 +1085,6 @@ void place_state(UmmaParams& p, void* workspace, size_t per) {
     for (int i = 0; i < 3; ++i, at += per * kHeadDim * sizeof(long long)) p.sums[i] = reinterpret_cast<long long*>(at);
     for (int i = 0; i < 2; ++i, at += per * kHeadDim * sizeof(float)) p.centres[i] = reinterpret_cast<float*>(at);
     for (int i = 0; i < 3; ++i, at += per * sizeof(int)) p.counts[i] = reinterpret_cast<int*>(at);
-}
-
-// Launch that may start while the kernel before it in the stream drains (it waits itself before it touches its results).
-template <class Kernel, class... Args>
-cudaError_t launch_overlapped(Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, bool overlapped, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr, cfg.numAttrs = overlapped ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t s) {

@@ -31,6 +31,8 @@ __global__ void window_write_kernel(__half* win_k, __half* win_raw, __half* win_
     const int unit = blockIdx.x, d = threadIdx.x;
     const size_t dst = (static_cast<size_t>(unit) * capacity + slot) * kHeadDim + d;
     const size_t src = static_cast<size_t>(unit) * kHeadDim + d;
+    let_next_launch_start();
+    wait_for_previous_launch();
     win_k[dst] = k_rot[src];
     win_raw[dst] = k_raw[src];
     win_v[dst] = v[src];
@@ -72,11 +74,11 @@ extern "C" int reskv_window_write(void* window_k, void* window_raw, void* window
     if (slot < 0 || slot >= window_capacity)
         return fail(RESKV_ERR_INVALID, "window_write: slot %d outside the window of %d tokens", slot, window_capacity);
     if (int rc = check_device_pointer(window_k, "window_write", "window_k")) return rc;
-    window_write_kernel<<<batch * kv_heads, kHeadDim, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__half*>(window_k), static_cast<__half*>(window_raw), static_cast<__half*>(window_v),
-        static_cast<const __half*>(k_rot), static_cast<const __half*>(k_raw), static_cast<const __half*>(v),
-        window_capacity, slot);
-    return check_cuda(cudaGetLastError(), "window_write launch");
+    return check_cuda(launch_overlapped(window_write_kernel, dim3(batch * kv_heads), kHeadDim, 0, static_cast<cudaStream_t>(stream), true,
+                                        static_cast<__half*>(window_k), static_cast<__half*>(window_raw), static_cast<__half*>(window_v),
+                                        static_cast<const __half*>(k_rot), static_cast<const __half*>(k_raw),
+                                        static_cast<const __half*>(v), window_capacity, slot),
+                      "window_write launch");
 }
 
 extern "C" int reskv_step_advance(int32_t* step_state, int position_increment, int window_increment, void* stream) {
