@@ -192,6 +192,9 @@ int reskv_window_append(void* window_k, void* window_raw, void* window_v, const 
  * of the reference's cache update (reskv/cache.py:55-60) by one launch. */
 int reskv_window_write(void* window_k, void* window_raw, void* window_v, const void* k_rot, const void* k_raw,
                        const void* v, int batch, int kv_heads, int window_capacity, int slot, void* stream);
+/* The same without the pointer query, for callers that vouch for the pointers being memory of the current device. */
+int reskv_window_put(void* window_k, void* window_raw, void* window_v, const void* k_rot, const void* k_raw,
+                     const void* v, int batch, int kv_heads, int window_capacity, int slot, void* stream);
 
 int reskv_decode_step(int layout, int bits, int nnz, const void* q, const void* k_centroids, const void* k_ids,
                       const void* k_payload, const void* k_meta, const void* k_scale, const void* v_centroids,

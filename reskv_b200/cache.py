@@ -98,7 +98,11 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         elif q_len != 1:
             raise ValueError("ResKV continuation supports one token per step; chunked prefill is unsupported")
         else:
-            self._take_token(key_states, raw, value_states)
+            views = self._take_token(key_states, raw, value_states)
+            self.length += 1
+            if views is not None:
+                return views
+            return self.keys.narrow(2, 0, self.live), self.values.narrow(2, 0, self.live)
         self.length += q_len
         return self.keys.narrow(2, 0, self.live), self.values.narrow(2, 0, self.live)
 
@@ -119,19 +123,22 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
 
     def _take_token(self, key, raw, value):
         """One launch writes the token's rotated key, raw key and value into slot ``live`` of the three
-        buffers; a full window then gives its oldest group to the compressed segment."""
-        from ._extension import host
-
-        cap = self.keys.shape[2]
+        buffers; a full window then gives its oldest group to the compressed segment.  Returns the dense segment's
+        views when they came with the launch."""
+        views = None
         if key.dtype == torch.float16 and key.is_cuda:
-            host().window_write(self.keys, self.raw_keys, self.values, key, raw, value, self.live)
+            from ._extension import host
+
+            views = host().window_append(self.keys, self.raw_keys, self.values, key, raw, value, self.live)
         else:  # other dtypes (a BF16 model before its cast): plain slice copies
             at = self.live
             for buf, src in ((self.keys, key), (self.raw_keys, raw), (self.values, value)):
                 buf[:, :, at : at + 1].copy_(src)
         self.live += 1
-        if self.live == cap:
-            self._compress_oldest_group()
+        if self.live < self.keys.shape[2]:
+            return views
+        self._compress_oldest_group()
+        return None
 
     def _compress_oldest_group(self):
         s, n = self.sink_tokens, self.config.group_size

@@ -6,6 +6,7 @@
 // up to batch 8.  Nothing is kept between calls here: every pointer and size is read from the tensors of the call.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <Python.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -130,6 +131,7 @@ struct Result {
 
 // Outputs and scratch, then the library call.  q: contiguous [B*NH,128].
 Result run_decode(const Decode& d, const at::Tensor& q) {
+    const at::AutoDispatchBelowADInplaceOrView plain;  // nothing here is differentiated
     const c10::DeviceIndex dev = q.get_device();
     for (const Side* s : {d.k, d.v})
         for (const at::Tensor* t : {&s->centroids, &s->ids, &s->payload, &s->meta, &s->scale}) same_device(dev, *t);
@@ -168,11 +170,14 @@ Result run_decode(const Decode& d, const at::Tensor& q) {
     }
     a.device_memory = 1;
     Result r;
-    const auto f32 = q.options().dtype(at::kFloat);
-    r.out = at::empty({rows, 128}, q.options());
-    if (d.stats) r.m = at::empty({rows}, f32), r.l = at::empty({rows}, f32);
+    // straight from the caching allocator (no dispatcher): ~1 us of host time per call
+    const auto empty = [&](at::IntArrayRef size, at::ScalarType type) {
+        return at::detail::empty_cuda(size, type, q.device(), std::nullopt);
+    };
+    r.out = empty({rows, 128}, at::kHalf);
+    if (d.stats) r.m = empty({rows}, at::kFloat), r.l = empty({rows}, at::kFloat);
     const size_t need = reskv_decode_args_workspace_bytes(&a);
-    const at::Tensor ws = at::empty({static_cast<int64_t>(need < 256 ? 256 : need)}, q.options().dtype(at::kByte));
+    const at::Tensor ws = empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::kByte);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
     if (g_check_status) cudaMemsetAsync(ws.data_ptr(), 0, 256, stream);
     a.workspace = ws.data_ptr(), a.workspace_bytes = static_cast<size_t>(ws.numel());
@@ -305,30 +310,38 @@ PyObject* py_attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
         }
         d.splits = integer(o[12]);
         // only the memory order of q matters to the kernels: [B,NH,1,128] dense is [B*NH,128] dense
+        const at::AutoDispatchBelowADInplaceOrView plain;
         const at::Tensor q = (query.is_contiguous() ? query : query.contiguous()).view({b * nh, 128});
         return THPVariable_Wrap(run_decode(d, q).out.view({b, nh, 1, 128}));
     });
 }
 
-// window_write(keys, raw_keys, values, key, raw_key, value, slot): the new token's three rows into slot `slot`.
-PyObject* py_window_write(PyObject*, PyObject* const* o, Py_ssize_t n) {
+// window_append(keys, raw_keys, values, key, raw_key, value, live) -> (keys, values) of the live + 1 tokens: the new
+// token's three rows go to slot `live` of the window buffers [B,H,capacity,128] (this library's own, dense).
+PyObject* py_window_append(PyObject*, PyObject* const* o, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         expect(n, 7);
         const at::Tensor &wk = tensor(o[0], "keys"), &wr = tensor(o[1], "raw keys"), &wv = tensor(o[2], "values");
-        at::Tensor rows[3];
+        const int64_t b = wk.size(0), h = wk.size(1), live = integer(o[6]);
+        const c10::DeviceIndex dev = wk.get_device();
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        at::Tensor dense[3];  // copies of tokens that are not dense, alive until the launch
+        const void* rows[3];
         for (int i = 0; i < 3; ++i) {
-            rows[i] = tensor(o[3 + i], "token").contiguous();
-            same_device(wk.get_device(), rows[i]);
-            if (rows[i].scalar_type() != at::kHalf || rows[i].numel() != wk.size(0) * wk.size(1) * 128)
-                value_error("window_write expects FP16 rows [B,H,1,128]");
+            const at::Tensor& t = tensor(o[3 + i], "token");
+            same_device(dev, t);
+            if (t.scalar_type() != at::kHalf || t.numel() != b * h * 128) value_error("window_append expects FP16 rows [B,H,1,128]");
+            rows[i] = t.is_contiguous() ? t.const_data_ptr() : (dense[i] = t.contiguous()).const_data_ptr();
         }
-        const c10::cuda::CUDAGuard guard(wk.get_device());
-        check(reskv_window_write(wk.data_ptr(), wr.data_ptr(), wv.data_ptr(), rows[0].const_data_ptr(), rows[1].const_data_ptr(),
-                                 rows[2].const_data_ptr(), static_cast<int>(wk.size(0)), static_cast<int>(wk.size(1)),
-                                 static_cast<int>(wk.size(2)), static_cast<int>(integer(o[6])),
-                                 c10::cuda::getCurrentCUDAStream(wk.get_device()).stream()));
+        const c10::cuda::CUDAGuard guard(dev);
+        check(reskv_window_put(wk.data_ptr(), wr.data_ptr(), wv.data_ptr(), rows[0], rows[1], rows[2], static_cast<int>(b),
+                               static_cast<int>(h), static_cast<int>(wk.size(2)), static_cast<int>(live),
+                               c10::cuda::getCurrentCUDAStream(dev).stream()));
         ++g_launches;
-        Py_RETURN_NONE;
+        PyObject* views = PyTuple_New(2);
+        PyTuple_SET_ITEM(views, 0, THPVariable_Wrap(wk.narrow(2, 0, live + 1)));
+        PyTuple_SET_ITEM(views, 1, THPVariable_Wrap(wv.narrow(2, 0, live + 1)));
+        return views;
     });
 }
 
@@ -447,7 +460,7 @@ PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launc
 PyMethodDef g_methods[] = {
     {"decode", FAST(py_decode), METH_FASTCALL, "decode attention on given operands"},
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
-    {"window_write", FAST(py_window_write), METH_FASTCALL, "append one token to the dense window"},
+    {"window_append", FAST(py_window_append), METH_FASTCALL, "append one token to the dense window"},
     {"take_ids", FAST(py_take_ids), METH_FASTCALL, "check and convert given cluster ids"},
     {"ids_in_range", py_ids_in_range, METH_O, "verdict of take_ids"},
     {"launches", py_launches, METH_NOARGS, "kernels launched through this module"},

@@ -74,6 +74,13 @@ extern "C" int reskv_window_write(void* window_k, void* window_raw, void* window
     if (slot < 0 || slot >= window_capacity)
         return fail(RESKV_ERR_INVALID, "window_write: slot %d outside the window of %d tokens", slot, window_capacity);
     if (int rc = check_device_pointer(window_k, "window_write", "window_k")) return rc;
+    return reskv_window_put(window_k, window_raw, window_v, k_rot, k_raw, v, batch, kv_heads, window_capacity, slot, stream);
+}
+
+extern "C" int reskv_window_put(void* window_k, void* window_raw, void* window_v, const void* k_rot, const void* k_raw,
+                                const void* v, int batch, int kv_heads, int window_capacity, int slot, void* stream) {
+    if (slot < 0 || slot >= window_capacity)
+        return fail(RESKV_ERR_INVALID, "window_put: slot %d outside the window of %d tokens", slot, window_capacity);
     return check_cuda(launch_overlapped(window_write_kernel, dim3(batch * kv_heads), kHeadDim, 0, static_cast<cudaStream_t>(stream), true,
                                         static_cast<__half*>(window_k), static_cast<__half*>(window_raw), static_cast<__half*>(window_v),
                                         static_cast<const __half*>(k_rot), static_cast<const __half*>(k_raw),
