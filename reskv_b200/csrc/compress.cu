@@ -1,6 +1,6 @@
 // Residual packers: x - centroid[id] -> top-magnitude selection -> packed layout.
-// This file holds the C entry points of all layouts and the kernel of the compact quantised layout; the
-// layouts of the reference run one thread per token and live in compress_topk.cu.
+// This file holds the C entry points of all layouts and a kernel of the compact quantised layout for inputs that
+// are not 16-byte aligned; everything else runs one thread per token and lives in compress_topk.cu.
 //
 // Compact layout: one warp encodes one token; lane l owns coordinates {l, l+32, l+64, l+96}.
 // With that ownership a warp vote of "lane keeps coordinate l+32i" *is* the
@@ -194,6 +194,7 @@ extern "C" int reskv_encode_compact(const void* x, const void* centroids, const 
                    static_cast<__half*>(scale), x_tok_stride, out_tok_stride, batch * kv_heads, tokens, clusters, nnz};
     const long long rows = static_cast<long long>(p.units) * tokens;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (aligned16(x) && aligned16(centroids) && aligned16(words) && aligned16(bitmap)) return launch_topk_compact(p, bits, s);
     if (bits == 4)
         encode_compact_kernel<4><<<grid_for(rows), kWarpsPerCta * 32, 0, s>>>(p);
     else

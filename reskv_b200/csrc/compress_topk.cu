@@ -1,26 +1,27 @@
 // Residual packers, one THREAD per token: the layouts that keep the globally largest residuals of a token
-// (unstructured FP16 bitmap; unstructured INT4 / INT2), the layouts that keep the largest of every 16-coordinate
-// tile (tiled masks, 4:16 indices) and the 1-of-4 INT4 layout.
+// (unstructured FP16 bitmap; unstructured and compact INT4 / INT2), the layouts that keep the largest of every
+// 16-coordinate tile (tiled masks, 4:16 indices) and the 1-of-4 INT4 layout.
 //
-// The warp-per-token form spends most of its instructions on cross-lane traffic: every round of the
-// threshold bisection ends in a warp reduction, ranks and masks are votes and popcounts.  With a whole
-// token in one thread nothing crosses lanes:
+// With a whole token in one thread nothing crosses lanes (a warp per token spends most of its instructions on warp
+// reductions, votes and popcounts):
 //
 //   * a warp stages the rows of 32 consecutive tokens in shared memory with 16-byte asynchronous copies
 //     (rows 16 bytes apart from dense, so the 16-byte loads of eight lanes fall into distinct banks), the
-//     unit's centroid table is staged once per CTA;
-//   * the thread forms r = fp32(x) - fp32(c) and keeps the 128 selection keys |fp16(r)| as 64 packed pairs;
-//     the pairing is (coordinate a + 16 in the low half, coordinate a in the high half), which makes the
-//     masks of the packed comparisons fall straight onto the MSB-first bitmap words;
+//     unit's centroid table is staged once per CTA; warps meet only when the table changes;
+//   * fp16(r) of two neighbouring coordinates is one packed subtraction: rounding x - c once to FP16 equals rounding it to
+//     FP32 first (24 >= 2 * 11 + 2 bits).  The 128 selection keys |fp16(r)| stay in registers as 64 packed pairs;
 //   * the k-th largest key is found by bisection on its 15 bits: a round is 64 packed comparisons (1.0 / 0.0
 //     per half, integer pipe) summed by packed FP16 additions (floating-point pipe), two instructions per key
 //     pair and round on two different pipes;
 //   * ties at the threshold keep the lower coordinates; the kept FP16 residuals are compacted in place in
-//     the thread's own row and the warp writes the 32 rows out with 16-byte stores.
+//     the thread's own row (one predicated store per coordinate: a loop over the set bits waits for shared memory
+//     at every step) and the warp writes the 32 rows out with 16-byte stores.
 //
-// The tiled layouts run the same bisection per tile, two tiles at a time in the two halves of the packed
-// operations (the accept decision is a packed comparison as well, so nothing is ever unpacked); the 1-of-4 layout
-// compares four keys per group.
+// The tiled layouts take their thresholds from a sorting network, two tiles at a time in the two halves of the packed
+// operations; the 1-of-4 layout compares four keys per group.
+//
+// What bounds it: the integer pipe, then the time a warp waits for its rows.  64 units x 8128 tokens (133 MB of x):
+// @@TIMES@@
 //
 // Rounding points are those of compress.cu (they decide bit-exactness): selection key |fp16(r)|, FP16 layouts
 // store fp16(r), the quantisers divide the FP32 r with the approximate division of the reference's build.
@@ -36,7 +37,7 @@ constexpr int kTopkThreads = kTopkWarps * 32;
 constexpr int kRowBytes = 2 * kHeadDim + 16;  // shared-memory row of one token / one centroid
 constexpr int kChunkTokens = kTopkThreads;    // tokens a CTA takes per pass (32 per warp)
 
-enum class TopkMode { kBitmapFp16, kQuant4, kQuant2, kTiledFp16, kStructFp16, kStructInt4 };
+enum class TopkMode { kBitmapFp16, kQuant4, kQuant2, kCompact4, kCompact2, kTiledFp16, kStructFp16, kStructInt4 };
 
 __device__ __forceinline__ float half_lo(uint32_t v) {
     return __half2float(__ushort_as_half(static_cast<unsigned short>(v & 0xffffu)));
@@ -70,12 +71,25 @@ __device__ __forceinline__ void residual_piece(const unsigned char* xrow, const 
     }
 }
 
+// Even coordinates' bits (high half) and odd ones' (low half) interleaved: bit i of the halves -> bits 2 i + 1 and 2 i.
+__device__ __forceinline__ uint32_t interleave16(uint32_t x) {
+    uint32_t t = (x ^ (x >> 8)) & 0x0000ff00u;
+    x ^= t ^ (t << 8);
+    t = (x ^ (x >> 4)) & 0x00f000f0u;
+    x ^= t ^ (t << 4);
+    t = (x ^ (x >> 2)) & 0x0c0c0c0cu;
+    x ^= t ^ (t << 2);
+    t = (x ^ (x >> 1)) & 0x22222222u;
+    return x ^ t ^ (t << 1);
+}
+
 // Keep-mask of the `k` largest keys, lower coordinate first among equal keys.  key[16 p + j] holds coordinate
-// 32 p + 16 + j in its low and 32 p + j in its high half; keep[p] has coordinate 32 p + q at bit 31 - q.
-__device__ __forceinline__ void select_topk_thread(const uint32_t (&key)[64], int k, uint32_t (&keep)[4]) {
+// 32 p + 2 j in its low and 32 p + 2 j + 1 in its high half; keep[p] has coordinate 32 p + q at bit 31 - q.  True when
+// nothing is above the threshold and not everything at it is kept (the largest key itself is cut).
+__device__ __forceinline__ bool select_topk_thread(const uint32_t (&key)[64], int k, uint32_t (&keep)[4]) {
     // largest v with count(key >= v) >= k
     uint32_t v = 0;
-    int n_ge = kHeadDim;
+#pragma unroll 1
     for (int bit = 14; bit >= 0; --bit) {
         const uint32_t cand = v | (1u << bit);
         const __half2 c2 = as_half2(cand | (cand << 16));
@@ -88,35 +102,40 @@ __device__ __forceinline__ void select_topk_thread(const uint32_t (&key)[64], in
         for (int j = 4; j < 64; ++j) acc[j & 3] = __hadd2(acc[j & 3], __hge2(as_half2(key[j]), c2));
         const __half2 total = __hadd2(__hadd2(acc[0], acc[1]), __hadd2(acc[2], acc[3]));
         const int cnt = __half2int_rn(__hadd(__low2half(total), __high2half(total)));
-        if (cnt >= k) v = cand, n_ge = cnt;
+        if (cnt >= k) v = cand;
     }
     const __half2 v2 = as_half2(v | (v << 16));
-    uint32_t ge[4] = {0u, 0u, 0u, 0u}, gt[4] = {0u, 0u, 0u, 0u};
+    uint32_t ge[4] = {0u, 0u, 0u, 0u};
+    int kept = 0;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const uint32_t place = (0x80000000u >> j) | (0x8000u >> j);
-            ge[p] |= __hge2_mask(as_half2(key[16 * p + j]), v2) & place;
-            gt[p] |= __hgt2_mask(as_half2(key[16 * p + j]), v2) & place;
-        }
+        for (int j = 0; j < 16; ++j) ge[p] |= __hge2_mask(as_half2(key[16 * p + j]), v2) & ((0x80000000u >> j) | (0x8000u >> j));
+        kept += __popc(ge[p]);
+        keep[p] = interleave16(__byte_perm(ge[p], 0u, 0x1032));  // even coordinates to the high half
     }
-    if (n_ge == k) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p) keep[p] = ge[p];
-        return;
-    }
+    if (kept == k) return false;
     // more keys equal to the threshold than places left: the lowest coordinates among them stay
-    int need = k - (__popc(gt[0]) + __popc(gt[1]) + __popc(gt[2]) + __popc(gt[3]));
+    int need = k;
+    uint32_t gt[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        uint32_t eq = ge[p] ^ gt[p], kept = gt[p];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) gt[p] |= __hgt2_mask(as_half2(key[16 * p + j]), v2) & ((0x80000000u >> j) | (0x8000u >> j));
+        need -= __popc(gt[p]);
+        gt[p] = interleave16(__byte_perm(gt[p], 0u, 0x1032));
+    }
+    const bool cut_largest = need == k;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        uint32_t eq = keep[p] ^ gt[p], stay = gt[p];
         while (eq != 0u && need > 0) {
             const uint32_t first = 0x80000000u >> __clz(eq);
-            eq ^= first, kept |= first, --need;
+            eq ^= first, stay |= first, --need;
         }
-        keep[p] = kept;
+        keep[p] = stay;
     }
+    return cut_largest;
 }
 
 // Packed 16-bit keys: larger ones to `a`, smaller ones to `b`, in either half.
@@ -220,9 +239,21 @@ __device__ __forceinline__ void select_tiles_thread(const uint32_t (&key)[64], i
     }
 }
 
+// Code of residual r: the quotient by the FP16 scale s, rounded and clamped.  A scale that underflowed to 0 gives what the
+// reference's (int)lrintf(r / 0) gives: -1 for positive residuals, 0 otherwise (see lrint_low32); every other quotient of
+// a kept residual is small, so the 32-bit conversion equals the 64-bit one.
+template <int QMAX>
+__device__ __forceinline__ int code_of(float r, float s, bool no_scale) {
+    const int q = max(-QMAX, min(QMAX, __float2int_rn(div_fast(r, s))));
+    return no_scale ? (r > 0.f ? -1 : 0) : q;
+}
+
 template <TopkMode MODE>
 __global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const EncodeParams p) {
     extern __shared__ __align__(16) unsigned char topk_smem[];
+    constexpr bool kTiles = MODE == TopkMode::kTiledFp16 || MODE == TopkMode::kStructFp16;
+    constexpr bool kFp16Rows = MODE == TopkMode::kBitmapFp16 || kTiles;  // the row becomes the FP16 payload
+    constexpr bool kCompact = MODE == TopkMode::kCompact4 || MODE == TopkMode::kCompact2;
     unsigned char* cen_s = topk_smem;                                                 // [clusters][kRowBytes]
     unsigned char* rows_s = topk_smem + static_cast<size_t>(p.clusters) * kRowBytes;  // [warps][32][kRowBytes]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -235,98 +266,82 @@ __global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const Enco
         const int unit = static_cast<int>(c / chunks_per_unit);
         const int t0 = static_cast<int>(c % chunks_per_unit) * kChunkTokens + warp * 32;
         const int ntok = max(0, min(32, p.tokens - t0));
-        if (unit != staged_unit) {  // uniform over the CTA
-            __syncthreads();        // nobody still reads the previous table
+        const bool new_table = unit != staged_unit;  // uniform over the CTA
+        if (new_table) {
+            __syncthreads();  // nobody still reads the previous table
             const unsigned char* src = reinterpret_cast<const unsigned char*>(p.cen + static_cast<size_t>(unit) * p.clusters * kHeadDim);
             for (int i = tid; i < p.clusters * 16; i += kTopkThreads) cp_async16(cen_s + (i >> 4) * kRowBytes + (i & 15) * 16, src + i * 16);
             staged_unit = unit;
         }
+        int id = 0;
+        if (lane < ntok) id = min(max(p.ids[static_cast<size_t>(unit) * p.tokens + t0 + lane], 0), p.clusters - 1);
         {
             const unsigned char* src = reinterpret_cast<const unsigned char*>(p.x + (static_cast<size_t>(unit) * p.x_stride + t0) * kHeadDim);
             for (int i = lane; i < ntok * 16; i += 32) cp_async16(my_rows + (i >> 4) * kRowBytes + (i & 15) * 16, src + i * 16);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();  // table and rows in place (uniform: every thread of the CTA gets here every pass)
+        if (new_table) __syncthreads(); else __syncwarp();  // table and this warp's rows in place
 
-        uint32_t keep[4] = {0u, 0u, 0u, 0u};
         const size_t orow = static_cast<size_t>(unit) * p.out_stride + t0 + lane;
-        constexpr bool kTiles = MODE == TopkMode::kTiledFp16 || MODE == TopkMode::kStructFp16;
-        constexpr bool kFp16Rows = MODE == TopkMode::kBitmapFp16 || kTiles;  // the row becomes the FP16 payload
+        const unsigned char* crow = cen_s + id * kRowBytes;
+        // fp16(r) of coordinates 8 m .. 8 m + 7, two per word
+        auto residual8 = [&](int m) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(xrow + 16 * m), cv = *reinterpret_cast<const uint4*>(crow + 16 * m);
+            return make_uint4(as_u32(__hsub2(as_half2(xv.x), as_half2(cv.x))), as_u32(__hsub2(as_half2(xv.y), as_half2(cv.y))),
+                              as_u32(__hsub2(as_half2(xv.z), as_half2(cv.z))), as_u32(__hsub2(as_half2(xv.w), as_half2(cv.w))));
+        };
         if constexpr (MODE == TopkMode::kStructInt4) {
             // one residual of every four consecutive coordinates: the largest |fp16(r)|, lowest index on ties;
             // FP32 scale amax / 7, codes with the approximate division (compression.cu:153-239)
             if (lane < ntok) {
-                int id = p.ids[static_cast<size_t>(unit) * p.tokens + t0 + lane];
-                id = min(max(id, 0), p.clusters - 1);
-                const unsigned char* crow = cen_s + id * kRowBytes;
+                const __half *xh = reinterpret_cast<const __half*>(xrow), *ch = reinterpret_cast<const __half*>(crow);
                 uint32_t which[2] = {0u, 0u};  // 2-bit in-group index of group g at bit 2 (g % 16) of word g / 16
-                float amax = 0.f;
-#pragma unroll 1
-                for (int pc = 0; pc < 4; ++pc) {
-                    float r[32];
-                    residual_piece(xrow, crow, pc, r);
-                    uint32_t w = 0u;
+                float best[32], amax = 0.f;
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        uint32_t bk = __half_as_ushort(__float2half_rn(r[4 * g])) & 0x7fffu, bi = 0u;
-                        float br = r[4 * g];
+                for (int m = 0; m < 16; ++m) {
+                    const uint4 v = residual8(m);
+                    const uint32_t r2[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                        for (int e = 1; e < 4; ++e) {
-                            const uint32_t k = __half_as_ushort(__float2half_rn(r[4 * g + e])) & 0x7fffu;
-                            if (k > bk) bk = k, bi = e, br = r[4 * g + e];
-                        }
-                        amax = fmaxf(amax, fabsf(br));
-                        w |= bi << (2 * g);
+                    for (int h = 0; h < 2; ++h) {
+                        // key and reversed index in one number: equal keys leave the lowest index on top
+                        const uint32_t lo = r2[2 * h] & 0x7fff7fffu, hi = r2[2 * h + 1] & 0x7fff7fffu;
+                        const uint32_t k0 = (lo & 0xffffu) * 4u + 3u, k1 = (lo >> 16) * 4u + 2u, k2 = (hi & 0xffffu) * 4u + 1u, k3 = (hi >> 16) * 4u;
+                        const int g = 2 * m + h, e = static_cast<int>(~max(max(k0, k1), max(k2, k3)) & 3u);
+                        which[g >> 4] |= static_cast<uint32_t>(e) << (2 * (g & 15));
+                        best[g] = __half2float(xh[4 * g + e]) - __half2float(ch[4 * g + e]);
+                        amax = fmaxf(amax, fabsf(best[g]));
                     }
-                    if (pc < 2) which[0] |= w << (16 * pc); else which[1] |= w << (16 * (pc - 2));
                 }
                 const float s = amax > 0.f ? amax * (1.0f / 7.0f) : 1.0f;
-                uint32_t out[4];
-#pragma unroll 1
-                for (int pc = 0; pc < 4; ++pc) {
-                    float r[32];
-                    residual_piece(xrow, crow, pc, r);
-                    const uint32_t w = (pc < 2 ? which[0] >> (16 * pc) : which[1] >> (16 * (pc - 2))) & 0xffffu;
-                    uint32_t word = 0u;
+                uint32_t out[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        const uint32_t bi = (w >> (2 * g)) & 3u;
-                        const float br = bi == 0u ? r[4 * g] : bi == 1u ? r[4 * g + 1] : bi == 2u ? r[4 * g + 2] : r[4 * g + 3];
-                        const int q = max(-7, min(7, __float2int_rn(div_fast(br, s))));
-                        word |= (static_cast<uint32_t>(q) & 15u) << (4 * g);
-                    }
-                    if (pc == 0) out[0] = word; else if (pc == 1) out[1] = word; else if (pc == 2) out[2] = word; else out[3] = word;
+                for (int g = 0; g < 32; ++g) {
+                    const int q = max(-7, min(7, __float2int_rn(div_fast(best[g], s))));
+                    out[g >> 3] |= (static_cast<uint32_t>(q) & 15u) << (4 * (g & 7));
                 }
-                const size_t orow = static_cast<size_t>(unit) * p.out_stride + t0 + lane;
                 static_cast<uint4*>(p.payload)[orow] = make_uint4(out[0], out[1], out[2], out[3]);
                 static_cast<uint2*>(p.meta)[orow] = make_uint2(which[0], which[1]);
                 p.scale[orow] = __float2half_rn(s);
             }
-            __syncthreads();  // rows are rewritten by the next pass
-            continue;
-        }
-        if (lane < ntok) {
-            int id = p.ids[static_cast<size_t>(unit) * p.tokens + t0 + lane];
-            id = min(max(id, 0), p.clusters - 1);
-            const unsigned char* crow = cen_s + id * kRowBytes;
-            uint32_t key[64];
+        } else if (lane < ntok) {
+            uint32_t keep[4], key[64];
+            bool cut_largest = false;
 #pragma unroll
             for (int pc = 0; pc < 4; ++pc) {
-                float r[32];
-                residual_piece(xrow, crow, pc, r);
+                uint32_t r2[16];  // fp16(r) of coordinates 32 pc + 2 j (low half), + 1
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    key[16 * pc + j] = as_u32(kTiles ? __floats2half2_rn(r[j], r[16 + j]) : __floats2half2_rn(r[16 + j], r[j])) & 0x7fff7fffu;
-                if constexpr (kFp16Rows) {
-                    // fp16(r) in coordinate order replaces the (fully consumed) x values of this piece
+                for (int m = 0; m < 4; ++m) {
+                    const uint4 v = residual8(4 * pc + m);
+                    r2[4 * m] = v.x, r2[4 * m + 1] = v.y, r2[4 * m + 2] = v.z, r2[4 * m + 3] = v.w;
+                    if constexpr (kFp16Rows) *reinterpret_cast<uint4*>(xrow + 64 * pc + 16 * m) = v;  // replaces the consumed x
+                }
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        uint4 o;
-                        o.x = as_u32(__floats2half2_rn(r[8 * m], r[8 * m + 1]));
-                        o.y = as_u32(__floats2half2_rn(r[8 * m + 2], r[8 * m + 3]));
-                        o.z = as_u32(__floats2half2_rn(r[8 * m + 4], r[8 * m + 5]));
-                        o.w = as_u32(__floats2half2_rn(r[8 * m + 6], r[8 * m + 7]));
-                        *reinterpret_cast<uint4*>(xrow + 64 * pc + 16 * m) = o;
+                for (int j = 0; j < 8; ++j) {
+                    if constexpr (kTiles) {  // coordinate j' of tile 2 pc in the low, of tile 2 pc + 1 in the high half
+                        key[16 * pc + 2 * j] = __byte_perm(r2[j], r2[8 + j], 0x5410) & 0x7fff7fffu;
+                        key[16 * pc + 2 * j + 1] = __byte_perm(r2[j], r2[8 + j], 0x7632) & 0x7fff7fffu;
+                    } else {
+                        key[16 * pc + 2 * j] = r2[2 * j] & 0x7fff7fffu, key[16 * pc + 2 * j + 1] = r2[2 * j + 1] & 0x7fff7fffu;
                     }
                 }
             }
@@ -338,107 +353,146 @@ __global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const Enco
                     select_tiles_thread<8>(key, 8, keep);
                 else
                     select_tiles_thread<0>(key, m, keep);
-                // compact the kept values to the front of the row, ascending coordinates (= tile, then rank)
-                unsigned short* vals = reinterpret_cast<unsigned short*>(xrow);
-                int n = 0;
-                uint32_t code[4] = {0u, 0u, 0u, 0u};  // 4:16 form: four 4-bit in-tile indices per tile, rank r at bit 4 r
+            } else {
+                cut_largest = select_topk_thread(key, p.nnz, keep);
+            }
+
+            if constexpr (kFp16Rows) {
+                // kept values to the front of the row, ascending coordinates (write position <= read position throughout)
+                uint32_t to = smem_u32(xrow);
 #pragma unroll
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t w = keep[pc];
-                    int rank = 0;
-                    while (w != 0u) {
-                        const int q = __ffs(w) - 1;
-                        w &= w - 1u;
-                        vals[n++] = vals[32 * pc + q];
-                        if constexpr (MODE == TopkMode::kStructFp16) {
-                            // ranks restart at the second tile of the word (bit 16): four values per tile
-                            code[pc] |= static_cast<uint32_t>(q & 15) << (4 * (rank & 3) + (q & 16));
-                            ++rank;
+                for (int m = 0; m < 16; ++m) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(xrow + 16 * m);
+                    const uint32_t r2[4] = {v.x, v.y, v.z, v.w}, w = keep[m >> 2];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int q = 8 * (m & 3) + i;
+                        const bool kept = kTiles ? (w >> q) & 1u : w & (0x80000000u >> q);
+                        if (kept) {
+                            asm volatile("st.shared.u16 [%0], %1;" ::"r"(to), "h"(static_cast<unsigned short>(i & 1 ? r2[i >> 1] >> 16 : r2[i >> 1])) : "memory");
+                            to += 2;
                         }
                     }
                 }
-                if constexpr (MODE == TopkMode::kStructFp16)
-                    static_cast<uint4*>(p.meta)[orow] = make_uint4(code[0], code[1], code[2], code[3]);
-                else
-                    static_cast<uint4*>(p.meta)[orow] = make_uint4(keep[0], keep[1], keep[2], keep[3]);
-            } else {
-                select_topk_thread(key, p.nnz, keep);
             }
-
-            if constexpr (kTiles) {
-            } else if constexpr (MODE == TopkMode::kBitmapFp16) {
-                // compact the kept values to the front of the row (write index <= read index throughout)
-                unsigned short* vals = reinterpret_cast<unsigned short*>(xrow);
-                int n = 0;
-#pragma unroll
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t w = keep[pc];
-                    while (w != 0u) {
-                        const int q = __clz(w);
-                        w ^= 0x80000000u >> q;
-                        vals[n++] = vals[32 * pc + q];
-                    }
-                }
+            if constexpr (MODE == TopkMode::kBitmapFp16) {
                 // bitmap words: coordinate d at bit 63 - d % 64 of word d / 64
                 static_cast<uint4*>(p.meta)[orow] = make_uint4(keep[1], keep[0], keep[3], keep[2]);
+            } else if constexpr (MODE == TopkMode::kTiledFp16) {
+                static_cast<uint4*>(p.meta)[orow] = make_uint4(keep[0], keep[1], keep[2], keep[3]);
+            } else if constexpr (MODE == TopkMode::kStructFp16) {
+                uint32_t code[4];  // four 4-bit in-tile indices per tile, rank r at bit 4 r
+#pragma unroll
+                for (int pc = 0; pc < 4; ++pc) {
+                    uint32_t lo = keep[pc] & 0xffffu, hi = keep[pc] >> 16, word = 0u;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {  // exactly four bits set in either half
+                        word |= (static_cast<uint32_t>(__ffs(lo) - 1) << (4 * r)) | (static_cast<uint32_t>(__ffs(hi) - 1) << (16 + 4 * r));
+                        lo &= lo - 1u, hi &= hi - 1u;
+                    }
+                    code[pc] = word;
+                }
+                static_cast<uint4*>(p.meta)[orow] = make_uint4(code[0], code[1], code[2], code[3]);
             } else {
-                constexpr int kBits = MODE == TopkMode::kQuant4 ? 4 : 2;
+                constexpr int kBits = MODE == TopkMode::kQuant4 || MODE == TopkMode::kCompact4 ? 4 : 2;
                 constexpr int kQmax = (1 << (kBits - 1)) - 1;
                 constexpr int kPer = 32 / kBits;  // codes per word
                 // Two more passes over the residuals (largest kept magnitude, then the codes); the pieces are
-                // taken one at a time (no unrolling over pc) so that only 32 residuals are live at once.
+                // taken one at a time (no unrolling over pc) so that only 32 residuals are live at once.  The largest
+                // magnitude of all is a kept one unless the largest keys themselves were cut.
                 float amax = 0.f;
 #pragma unroll 1
                 for (int pc = 0; pc < 4; ++pc) {
-                    const uint32_t kw = pc == 0 ? keep[0] : pc == 1 ? keep[1] : pc == 2 ? keep[2] : keep[3];
                     float r[32];
                     residual_piece(xrow, crow, pc, r);
+                    if (cut_largest) {
+                        const uint32_t kw = pc == 0 ? keep[0] : pc == 1 ? keep[1] : pc == 2 ? keep[2] : keep[3];
 #pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        if (kw & (0x80000000u >> q)) amax = fmaxf(amax, fabsf(r[q]));
+                        for (int q = 0; q < 32; ++q)
+                            if (kw & (0x80000000u >> q)) amax = fmaxf(amax, fabsf(r[q]));
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) amax = fmaxf(amax, fabsf(r[q]));
+                    }
                 }
                 const __half hs = quant_scale<kQmax>(amax);
                 const float s = __half2float(hs);
-                uint32_t* words = reinterpret_cast<uint32_t*>(p.payload) + orow * (4 * kBits);
+                const bool no_scale = s == 0.f;
+                uint32_t* words = reinterpret_cast<uint32_t*>(p.payload) + orow * (kCompact ? p.nnz / kPer : 4 * kBits);
+                uint32_t to = smem_u32(xrow);
 #pragma unroll 1
                 for (int pc = 0; pc < 4; ++pc) {
                     const uint32_t kw = pc == 0 ? keep[0] : pc == 1 ? keep[1] : pc == 2 ? keep[2] : keep[3];
                     float r[32];
                     residual_piece(xrow, crow, pc, r);
-                    uint32_t out[32 / kPer];
+                    if constexpr (kCompact) {
+                        // one byte per kept code to the front of the row (behind the read position throughout)
 #pragma unroll
-                    for (int w = 0; w < 32 / kPer; ++w) {
-                        uint32_t word = 0u;
-#pragma unroll
-                        for (int i = 0; i < kPer; ++i) {
-                            const int q = w * kPer + i;
-                            if (kw & (0x80000000u >> q))
-                                word |= (static_cast<uint32_t>(quant_code<kQmax>(r[q], s)) & ((1u << kBits) - 1u)) << (i * kBits);
+                        for (int q = 0; q < 32; ++q) {
+                            if (kw & (0x80000000u >> q)) {
+                                asm volatile("st.shared.u8 [%0], %1;" ::"r"(to), "r"(code_of<kQmax>(r[q], s, no_scale)) : "memory");
+                                ++to;
+                            }
                         }
-                        out[w] = word;
-                    }
-                    // coordinates 32 pc .. 32 pc + 31 = words (32 / kPer) pc ...
-                    if constexpr (kBits == 4) {
-                        *reinterpret_cast<uint4*>(words + 4 * pc) = make_uint4(out[0], out[1], out[2], out[3]);
                     } else {
-                        *reinterpret_cast<uint2*>(words + 2 * pc) = make_uint2(out[0], out[1]);
+                        uint32_t out[32 / kPer];
+#pragma unroll
+                        for (int w = 0; w < 32 / kPer; ++w) {
+                            uint32_t word = 0u;
+#pragma unroll
+                            for (int i = 0; i < kPer; ++i) {
+                                const int q = w * kPer + i;
+                                const int code = code_of<kQmax>(r[q], s, no_scale);
+                                if (kw & (0x80000000u >> q)) word |= (static_cast<uint32_t>(code) & ((1u << kBits) - 1u)) << (i * kBits);
+                            }
+                            out[w] = word;
+                        }
+                        // coordinates 32 pc .. 32 pc + 31 = words (32 / kPer) pc ...
+                        if constexpr (kBits == 4) {
+                            *reinterpret_cast<uint4*>(words + 4 * pc) = make_uint4(out[0], out[1], out[2], out[3]);
+                        } else {
+                            *reinterpret_cast<uint2*>(words + 2 * pc) = make_uint2(out[0], out[1]);
+                        }
                     }
+                }
+                if constexpr (kCompact) {
+                    // the bytes' low bits side by side, 16 bytes of codes at a time
+                    for (int w4 = 0; w4 < p.nnz / (4 * kPer); ++w4) {
+                        uint32_t out[4];
+#pragma unroll
+                        for (int w = 0; w < 4; ++w) {
+                            uint32_t word = 0u;
+#pragma unroll
+                            for (int i = 0; i < kPer / 4; ++i) {
+                                uint32_t four = *reinterpret_cast<const uint32_t*>(xrow + (4 * w4 + w) * kPer + 4 * i);
+                                if constexpr (kBits == 4) {
+                                    four &= 0x0f0f0f0fu;
+                                    four |= four >> 4;
+                                    word |= __byte_perm(four, 0u, 0x4420) << (16 * i);
+                                } else {
+                                    four &= 0x03030303u;
+                                    four |= four >> 6;
+                                    word |= ((four & 15u) | ((four >> 12) & 0xf0u)) << (8 * i);
+                                }
+                            }
+                            out[w] = word;
+                        }
+                        reinterpret_cast<uint4*>(words)[w4] = make_uint4(out[0], out[1], out[2], out[3]);
+                    }
+                    static_cast<uint4*>(p.meta)[orow] = make_uint4(keep[1], keep[0], keep[3], keep[2]);
                 }
                 p.scale[orow] = hs;
             }
         }
+        __syncwarp();
         if constexpr (kFp16Rows) {
-            __syncwarp();
             // the warp's rows are consecutive in the output: 16-byte pieces when the row length allows it
             unsigned char* dst = reinterpret_cast<unsigned char*>(static_cast<__half*>(p.payload) +
                                                                   (static_cast<size_t>(unit) * p.out_stride + t0) * p.nnz);
-            if (p.nnz % 8 == 0) {
-                const int pieces = p.nnz / 8;
-                for (int i = lane; i < ntok * pieces; i += 32) {
-                    const int row = i / pieces, piece = i % pieces;
-                    *reinterpret_cast<uint4*>(dst + static_cast<size_t>(row) * p.nnz * 2 + piece * 16) =
-                        *reinterpret_cast<const uint4*>(my_rows + row * kRowBytes + piece * 16);
-                }
+            if (p.nnz == 32 || p.nnz == 64) {
+                const int shift = p.nnz == 32 ? 2 : 3, mask = (1 << shift) - 1;
+                for (int i = lane; i < ntok << shift; i += 32)
+                    reinterpret_cast<uint4*>(dst)[i] = *reinterpret_cast<const uint4*>(my_rows + (i >> shift) * kRowBytes + (i & mask) * 16);
             } else {
                 for (int i = lane; i < ntok * p.nnz; i += 32) {
                     const int row = i / p.nnz, e = i % p.nnz;
@@ -446,8 +500,8 @@ __global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const Enco
                         *reinterpret_cast<const unsigned short*>(my_rows + row * kRowBytes + e * 2);
                 }
             }
+            __syncwarp();  // rows are rewritten by the next pass
         }
-        __syncthreads();  // rows are rewritten by the next pass
     }
 }
 
@@ -488,6 +542,11 @@ int launch_topk_tiled_fp16(const EncodeParams& p, bool indexed, cudaStream_t str
 
 int launch_topk_structured_int4(const EncodeParams& p, cudaStream_t stream) {
     return launch_topk<TopkMode::kStructInt4>(p, stream, "encode_structured_int4 launch");
+}
+
+int launch_topk_compact(const EncodeParams& p, int bits, cudaStream_t stream) {
+    return bits == 4 ? launch_topk<TopkMode::kCompact4>(p, stream, "encode_compact launch")
+                     : launch_topk<TopkMode::kCompact2>(p, stream, "encode_compact launch");
 }
 
 int launch_topk_quantized(const EncodeParams& p, int bits, cudaStream_t stream) {
