@@ -249,7 +249,7 @@ __device__ __forceinline__ int code_of(float r, float s, bool no_scale) {
 }
 
 template <TopkMode MODE>
-__global__ void __launch_bounds__(kTopkThreads, 4) encode_topk_kernel(const EncodeParams p) {
+__global__ void __launch_bounds__(kTopkThreads, 5) encode_topk_kernel(const EncodeParams p) {
     extern __shared__ __align__(16) unsigned char topk_smem[];
     constexpr bool kTiles = MODE == TopkMode::kTiledFp16 || MODE == TopkMode::kStructFp16;
     constexpr bool kFp16Rows = MODE == TopkMode::kBitmapFp16 || kTiles;  // the row becomes the FP16 payload
@@ -523,7 +523,7 @@ int launch_topk(const EncodeParams& p, cudaStream_t stream, const char* what) {
         if (dev >= 0 && dev < 64) allowed |= 1ull << dev;
     }
     const long long chunks = static_cast<long long>(p.units) * ((p.tokens + kChunkTokens - 1) / kChunkTokens);
-    const long long cap = static_cast<long long>(sm_count()) * 4;
+    const long long cap = static_cast<long long>(sm_count()) * 5;
     const int grid = static_cast<int>(chunks < cap ? chunks : cap);
     kern<<<grid, kTopkThreads, topk_smem_bytes(p.clusters), stream>>>(p);
     return check_cuda(cudaGetLastError(), what);
