@@ -1115,7 +1115,7 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     const int tiles_unit = (p.tokens + kUTile - 1) / kUTile, seg_max = kUChunkMax / kUTile;
     const long long tiles_total = static_cast<long long>(p.sides) * p.units * tiles_unit;
     const long long even = (tiles_total + sm_count() - 1) / sm_count();
-    long long share = even < 4 ? 4 : even, best_cost = -1;
+    long long share = even < 1 ? 1 : even, best_cost = -1;
     const long long step = share / 64 + 1;  // at most ~32 candidates: this is host time
     for (long long cand = share, most = share + share / 2 + 1; cand <= most; cand += step) {
         long long worst = 0;
