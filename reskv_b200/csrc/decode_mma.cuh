@@ -425,23 +425,24 @@ struct LayoutMmaCompact {
 struct StructInt4Field : GroupBlock<StructInt4Field> {
     static constexpr bool kSlotwise = false;
     uint32_t c02, c13;  // the field's four group codes as FP16: groups (0, 2) and (1, 3)
-    uint32_t sel;       // four 2-bit in-group positions
+    uint32_t sel;       // four 2-bit in-group positions, times 16 (shift amounts)
     __device__ __forceinline__ uint32_t code(int ks) const {  // in the low half
         const uint32_t p = (ks & 1) ? c13 : c02;
         return (ks & 2) ? p >> 16 : p & 0xffffu;
     }
-    __device__ __forceinline__ void add4(int ks, float (&k)[4], unsigned short scale) const {
-        const uint32_t pos = (sel >> (2 * ks)) & 3u;
-        const unsigned short c = static_cast<unsigned short>(code(ks));
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (pos == static_cast<uint32_t>(e)) k[e] = fma_f16_f16_f32(c, scale, k[e]);
-    }
-    // coordinates 2 i and 2 i + 1: half a group, at most one of them set
+    // coordinates 2 i and 2 i + 1, half a group: the code shifted to its place; shifts beyond the word leave zero
     __device__ __forceinline__ uint32_t pair(int i) const {
-        const uint32_t pos = (sel >> (2 * (i >> 1))) & 3u, c = code(i >> 1);
-        const uint32_t at = pos - 2u * (i & 1);
-        return at == 0u ? c : at == 1u ? c << 16 : 0u;
+        const uint32_t at = ((sel >> (2 * (i >> 1))) & 0x30u) - 32u * (i & 1);
+        uint32_t v;
+        asm("shl.b32 %0, %1, %2;" : "=r"(v) : "r"(code(i >> 1)), "r"(at));
+        return v;
+    }
+    __device__ __forceinline__ void add4(int ks, float (&k)[4], unsigned short scale) const {
+        const uint32_t lo = pair(2 * ks), hi = pair(2 * ks + 1);
+        k[0] = fma_f16_f16_f32(static_cast<unsigned short>(lo & 0xffffu), scale, k[0]);
+        k[1] = fma_f16_f16_f32(static_cast<unsigned short>(lo >> 16), scale, k[1]);
+        k[2] = fma_f16_f16_f32(static_cast<unsigned short>(hi & 0xffffu), scale, k[2]);
+        k[3] = fma_f16_f16_f32(static_cast<unsigned short>(hi >> 16), scale, k[3]);
     }
 };
 
@@ -457,7 +458,7 @@ struct LayoutMmaStructInt4 {
             const uint32_t nib = *reinterpret_cast<const unsigned short*>(pay + 2 * f);
             const uint32_t two = nib | (nib << 8);  // nibbles 0, 1 at bits 0, 4 and nibbles 2, 3 at bits 16, 20
             fd.c02 = codes_to_h2<4, 0>(two), fd.c13 = codes_to_h2<4, 4>(two);
-            fd.sel = meta[f];
+            fd.sel = static_cast<uint32_t>(meta[f]) << 4;
         }
         return fd;
     }
