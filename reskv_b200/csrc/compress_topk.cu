@@ -357,7 +357,31 @@ __global__ void __launch_bounds__(kTopkThreads, 5) encode_topk_kernel(const Enco
                 cut_largest = select_topk_thread(key, p.nnz, keep);
             }
 
-            if constexpr (kFp16Rows) {
+            uint32_t code[4] = {0u, 0u, 0u, 0u};  // 4:16 form: four 4-bit in-tile indices per tile, rank r at bit 4 r
+            const bool whole_tiles = MODE == TopkMode::kStructFp16 || (MODE == TopkMode::kTiledFp16 && p.nnz == 64);
+            if (kTiles && whole_tiles) {
+                // a fixed number per tile: the kept values are fetched by index and packed in registers, two tiles at a time
+                constexpr int kPerTile = MODE == TopkMode::kStructFp16 ? 4 : 8;
+#pragma unroll
+                for (int pc = 0; pc < 4; ++pc) {
+                    uint32_t left[2] = {keep[pc] & 0xffffu, keep[pc] >> 16}, out[kPerTile];
+#pragma unroll
+                    for (int r = 0; r < kPerTile; ++r) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int q = __ffs(left[h]) - 1;
+                            left[h] &= left[h] - 1u;
+                            const uint32_t v = *reinterpret_cast<const unsigned short*>(xrow + 64 * pc + 32 * h + 2 * q);
+                            uint32_t& w = out[h * (kPerTile / 2) + (r >> 1)];
+                            w = r & 1 ? __byte_perm(w, v, 0x5410) : v;
+                            if constexpr (MODE == TopkMode::kStructFp16) code[pc] |= static_cast<uint32_t>(q) << (4 * r + 16 * h);
+                        }
+                    }
+#pragma unroll
+                    for (int w = 0; w < kPerTile; w += 4)  // behind the read position throughout
+                        *reinterpret_cast<uint4*>(xrow + 4 * kPerTile * pc + 4 * w) = make_uint4(out[w], out[w + 1], out[w + 2], out[w + 3]);
+                }
+            } else if constexpr (kFp16Rows && MODE != TopkMode::kStructFp16) {
                 // kept values to the front of the row, ascending coordinates (write position <= read position throughout)
                 uint32_t to = smem_u32(xrow);
 #pragma unroll
@@ -381,17 +405,6 @@ __global__ void __launch_bounds__(kTopkThreads, 5) encode_topk_kernel(const Enco
             } else if constexpr (MODE == TopkMode::kTiledFp16) {
                 static_cast<uint4*>(p.meta)[orow] = make_uint4(keep[0], keep[1], keep[2], keep[3]);
             } else if constexpr (MODE == TopkMode::kStructFp16) {
-                uint32_t code[4];  // four 4-bit in-tile indices per tile, rank r at bit 4 r
-#pragma unroll
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t lo = keep[pc] & 0xffffu, hi = keep[pc] >> 16, word = 0u;
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {  // exactly four bits set in either half
-                        word |= (static_cast<uint32_t>(__ffs(lo) - 1) << (4 * r)) | (static_cast<uint32_t>(__ffs(hi) - 1) << (16 + 4 * r));
-                        lo &= lo - 1u, hi &= hi - 1u;
-                    }
-                    code[pc] = word;
-                }
                 static_cast<uint4*>(p.meta)[orow] = make_uint4(code[0], code[1], code[2], code[3]);
             } else {
                 constexpr int kBits = MODE == TopkMode::kQuant4 || MODE == TopkMode::kCompact4 ? 4 : 2;
