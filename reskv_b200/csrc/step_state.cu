@@ -39,6 +39,8 @@ __global__ void window_write_kernel(__half* win_k, __half* win_raw, __half* win_
 }
 
 __global__ void step_advance_kernel(int32_t* step_state, int pos_inc, int live_inc) {
+    let_next_launch_start();
+    wait_for_previous_launch();
     if (threadIdx.x == 0) {
         step_state[0] += pos_inc;
         step_state[1] += live_inc;
@@ -90,7 +92,7 @@ extern "C" int reskv_window_put(void* window_k, void* window_raw, void* window_v
 
 extern "C" int reskv_step_advance(int32_t* step_state, int position_increment, int window_increment, void* stream) {
     if (!step_state) return fail(RESKV_ERR_INVALID, "step_advance: null step state");
-    step_advance_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(step_state, position_increment,
-                                                                        window_increment);
-    return check_cuda(cudaGetLastError(), "step_advance launch");
+    return check_cuda(launch_overlapped(step_advance_kernel, dim3(1), 32, 0, static_cast<cudaStream_t>(stream), true, step_state,
+                                        position_increment, window_increment),
+                      "step_advance launch");
 }

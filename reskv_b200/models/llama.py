@@ -312,13 +312,12 @@ class ResKVLlama:
         def project(x, inp, weight):
             """x + inp @ weight^T, summed over the tensor-parallel group."""
             if self.tp == 1:
-                return torch.addmm(x, inp, weight.t())
+                return x.addmm_(inp, weight.t())  # in place: no copy of x in front of the product
             return x + self._all_reduce(F.linear(inp, weight))
 
-        if reskv:
-            # count the new token into the window first: it goes to slot count - 1 and the
-            # attention of this step already includes it
-            check(lib.reskv_step_advance(state, 0, 1, stream))
+        # one step on: the new token's position, and (compressed cache) its place in the window -- it goes to slot
+        # count - 1 and the attention of this step already includes it
+        check(lib.reskv_step_advance(state, 1, 1 if reskv else 0, stream))
         x = self.embed[tok]
         for index, (layer, cache) in enumerate(zip(self.layers, self.caches)):
             qkv = F.linear(norm(x, layer["norm1"]), layer["wqkv"])
@@ -362,7 +361,6 @@ class ResKVLlama:
             act = half(b, self.ffn)
             check(lib.reskv_silu_mul(gate_up.data_ptr(), act.data_ptr(), b, self.ffn, stream))
             x = project(x, act, layer["w_down"])
-        check(lib.reskv_step_advance(state, 1, 0, stream))
         if not reskv:
             self._seqlens += 1
         return F.linear(norm(x, self.final_norm), self.lm_head).float()
@@ -389,7 +387,7 @@ class ResKVLlama:
         else:
             if _flash_kvcache is None:
                 raise RuntimeError("graph decode of the dense baseline needs flash_attn")
-            self._state = torch.tensor([self.length, 0], dtype=torch.int32, device=self.device)
+            self._state = torch.tensor([self.length - 1, 0], dtype=torch.int32, device=self.device)
             self._seqlens = torch.full((batch,), self.length, dtype=torch.int32, device=self.device)
             for c in self.caches:  # flash_attn_with_kvcache wants [B, T, H, D]
                 c.k = c.k.transpose(1, 2).contiguous()
@@ -399,7 +397,7 @@ class ResKVLlama:
         """Refresh what a captured step reads: counts in the step state, centroid tables, and the
         addresses of the compressed buffers (a buffer that had to grow invalidates the graph)."""
         comp = self.caches[0].compressed
-        self._state.copy_(torch.tensor([self.length, self.caches[0].live, comp.seq_len if comp is not None else -1, 0],
+        self._state.copy_(torch.tensor([self.length - 1, self.caches[0].live, comp.seq_len if comp is not None else -1, 0],
                                        dtype=torch.int32))
         addresses = []
         for cache, (kc, vc) in zip(self.caches, self._centroids):
