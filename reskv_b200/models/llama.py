@@ -20,6 +20,7 @@ compressed cache goes through ``reskv_b200.compress`` / ``attention``.
 
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -60,6 +61,20 @@ def _rope(x, cos, sin):
     """Half-split RoPE; x [B, H, T, 128], cos/sin [T, 64] (FP32)."""
     a, b = x.float()[..., :64], x.float()[..., 64:]
     return torch.cat((a * cos - b * sin, b * cos + a * sin), dim=-1).to(x.dtype)
+
+
+_streams = threading.local()
+
+
+def _capture_stream(device) -> torch.cuda.Stream:
+    """The calling thread's stream for captures on ``device``: one for all models, so that a new model finds the
+    library workspaces and cached blocks of that stream instead of allocating them again."""
+    by_device = _streams.__dict__.setdefault("by_device", {})
+    index = torch.device(device).index
+    index = torch.cuda.current_device() if index is None else index
+    if index not in by_device:
+        by_device[index] = torch.cuda.Stream(device=index)
+    return by_device[index]
 
 
 class _DenseLayerCache:
@@ -138,9 +153,8 @@ class ResKVLlama:
         self.caches = None
         self.length = 0
         self._lib = None
-        # graph decode: stream of the captures, the last captured graph (owner of their memory pool), batch sizes whose
-        # step has run once
-        self._capture_stream = self._last_graph = None
+        # graph decode: the last captured graph (owner of the captures' memory pool), batch sizes whose step has run once
+        self._last_graph = None
         self._warm = set()
 
     # -- helpers -----------------------------------------------------------------------------
@@ -372,8 +386,6 @@ class ResKVLlama:
 
         self._tok_in = torch.zeros(batch, dtype=torch.long, device=self.device)
         self._graph = self._logits_out = None
-        if self._capture_stream is None:
-            self._capture_stream = torch.cuda.Stream(device=self.device)
         if self.cache_kind == "reskv":
             self._state = torch.zeros(4, dtype=torch.int32, device=self.device)
             # centroid tables at their final shape (zero rows beyond the live count), one pair per layer
@@ -418,7 +430,7 @@ class ResKVLlama:
         allocates next would go back to ``cudaMalloc`` (72 of 114 ms for a prompt of 4 x 1024 tokens and 72 steps).  The
         step's temporaries come from one pool per model: the graph captured last stays alive, and with it the pool,
         until the next capture has taken the pool over."""
-        side, main = self._capture_stream, torch.cuda.current_stream(self.device)
+        side, main = _capture_stream(self.device), torch.cuda.current_stream(self.device)
         side.wait_stream(main)
         with torch.cuda.stream(side):
             if self._tok_in.shape[0] not in self._warm:
