@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from ._extension import load_extension, token_stride_of
+from ._extension import LAYOUT_IDS, host, load_extension, require_device, token_stride_of
 from .config import KernelPlan, ResKVKernelConfig
 from .tensors import CompressedKV, CompressedTensor
 
@@ -80,22 +80,12 @@ def _encode(x, centers, ids, plan: KernelPlan, *, value=False, stored_ids=None):
     """Residuals of ``x`` to its centres in the layout of ``plan``
     (reference compression.py:72-101).  ``value`` is accepted for signature
     compatibility: K and V use the same selection rule here.  ``stored_ids``: the ids as int8, when there."""
-    ids = ids.int().contiguous()
-    centers = centers.half().contiguous()
-    x = _dense_or_slice(x)
-    ops = _ops(x)
-    metadata = scale = None
-    if plan.layout == "compact":
-        payload, metadata, scale = ops.compress_compact(x, centers, ids, plan.nnz, plan.bits)
-    elif plan.bits == 16 and plan.layout == "unstructured":
-        payload, metadata = ops.compress_bitmap_fp16(x, centers, ids, plan.nnz)
-    elif plan.bits == 16:
-        payload, metadata = ops.compress_fp16(x, centers, ids, plan.nnz, plan.layout == "structured")
-    elif plan.layout == "structured":
-        payload, metadata, scale = ops.compress_structured_int4(x, centers, ids)
-    else:
-        payload, scale = ops.compress_quantized(x, centers, ids, plan.nnz, plan.bits)
-    return CompressedTensor(centers, ids if stored_ids is None else stored_ids, payload, metadata, scale, plan)
+    require_device(x.get_device())
+    ids, centers = ids.int().contiguous(), centers.half().contiguous()
+    stored = ids.to(torch.int8) if stored_ids is None else stored_ids
+    payload, metadata, scale, native = host().encode(LAYOUT_IDS[plan.layout], plan.bits, plan.nnz, _dense_or_slice(x), centers,
+                                                     ids, stored)
+    return CompressedTensor._packed(centers, stored, payload, metadata, scale, plan, native)
 
 
 def _plan_for(config: ResKVKernelConfig, previous, plan, batch: int) -> KernelPlan:

@@ -345,6 +345,64 @@ PyObject* py_window_append(PyObject*, PyObject* const* o, Py_ssize_t n) {
     });
 }
 
+// encode(layout, bits, nnz, x, centroids, ids32, ids8) -> (payload, metadata, scale, native): one side packed, and the
+// views the decode kernels take: (centroids [U,C,128], ids [U,T], payload [U,T,w], metadata [U,T,m], scale [U,T]).
+PyObject* py_encode(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 7);
+        const int layout = static_cast<int>(integer(o[0])), bits = static_cast<int>(integer(o[1])), nnz = static_cast<int>(integer(o[2]));
+        const at::Tensor &x = tensor(o[3], "x"), &cen = tensor(o[4], "centroids"), &ids = tensor(o[5], "ids"), &ids8 = tensor(o[6], "ids");
+        if (x.scalar_type() != at::kHalf || cen.scalar_type() != at::kHalf || ids.scalar_type() != at::kInt)
+            value_error("compression ops expect FP16 x/centroids and int32 ids");
+        if (x.dim() != 4 || cen.dim() != 4 || ids.dim() != 3 || x.size(3) != 128 || cen.size(3) != 128)
+            value_error("compression ops expect x[B,H,T,128], centroids[B,H,C,128], ids[B,H,T]");
+        const int64_t stride = token_stride_of(x);
+        if (stride < 0 || !cen.is_contiguous() || !ids.is_contiguous() || !ids8.is_contiguous())
+            value_error("compression ops expect contiguous tensors (x may be a token slice of a dense buffer)");
+        const c10::DeviceIndex dev = x.get_device();
+        for (const at::Tensor* t : {&cen, &ids, &ids8}) same_device(dev, *t);
+        const c10::cuda::CUDAGuard guard(dev);
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        const int64_t b = x.size(0), h = x.size(1), t = x.size(2), c = cen.size(2);
+        const auto empty = [&](at::IntArrayRef size, at::ScalarType type) {
+            return at::detail::empty_cuda(size, type, x.device(), std::nullopt);
+        };
+        const bool compact = layout == RESKV_LAYOUT_COMPACT, structured = layout == RESKV_LAYOUT_STRUCTURED;
+        const int64_t width = bits == 16 ? nnz : compact ? static_cast<int64_t>(nnz) * bits / 32 : structured ? 4 : 4 * bits;
+        at::Tensor payload = empty({b, h, t, width}, bits == 16 ? at::kHalf : at::kInt), meta, scale;
+        if (compact || (layout == RESKV_LAYOUT_UNSTRUCTURED && bits == 16))
+            meta = empty({b, h, t, 2}, at::kLong);
+        else if (bits == 16 || structured)
+            meta = empty({b, h, t, bits == 4 ? 2 : 4}, at::kInt);
+        if (bits != 16) scale = empty({b, h, t}, at::kHalf);
+        const int bi = static_cast<int>(b), hi = static_cast<int>(h), ti = static_cast<int>(t), ci = static_cast<int>(c);
+        const auto* id = static_cast<const int32_t*>(ids.const_data_ptr());
+        const void *xp = x.const_data_ptr(), *cp = cen.const_data_ptr();
+        void *pp = payload.data_ptr(), *mp = meta.defined() ? meta.data_ptr() : nullptr, *sp = scale.defined() ? scale.data_ptr() : nullptr;
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+        check(compact ? reskv_encode_compact(xp, cp, id, bi, hi, ti, stride, ci, nnz, bits, pp, mp, sp, t, stream)
+              : bits == 16 && layout == RESKV_LAYOUT_UNSTRUCTURED ? reskv_encode_bitmap_fp16(xp, cp, id, bi, hi, ti, stride, ci, nnz, pp, mp, t, stream)
+              : bits == 16 ? reskv_encode_tiled_fp16(xp, cp, id, bi, hi, ti, stride, ci, nnz, structured, pp, mp, t, stream)
+              : structured ? reskv_encode_structured_int4(xp, cp, id, bi, hi, ti, stride, ci, pp, mp, sp, t, stream)
+                           : reskv_encode_quantized(xp, cp, id, bi, hi, ti, stride, ci, nnz, bits, pp, sp, t, stream));
+        ++g_launches;
+        const auto none = [] { return Py_NewRef(Py_None); };
+        const auto units = [&](const at::Tensor& v) {
+            if (!v.defined()) return none();
+            return THPVariable_Wrap(v.dim() == 4 ? v.view({b * h, v.size(2), v.size(3)}) : v.view({b * h, t}));
+        };
+        PyObject* native = PyTuple_New(5);
+        const at::Tensor* parts[5] = {&cen, &ids8, &payload, &meta, &scale};
+        for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(native, i, units(*parts[i]));
+        PyObject* r = PyTuple_New(4);
+        PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(payload));
+        PyTuple_SET_ITEM(r, 1, meta.defined() ? THPVariable_Wrap(meta) : none());
+        PyTuple_SET_ITEM(r, 2, scale.defined() ? THPVariable_Wrap(scale) : none());
+        PyTuple_SET_ITEM(r, 3, native);
+        return r;
+    });
+}
+
 // ---- verdicts of take_ids -------------------------------------------------------------------------------------------
 // A word of mapped pinned host memory and an event per call in flight; a few are kept for later calls (any thread, any
 // device: the event is made for the call's device).
@@ -461,6 +519,7 @@ PyMethodDef g_methods[] = {
     {"decode", FAST(py_decode), METH_FASTCALL, "decode attention on given operands"},
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
     {"window_append", FAST(py_window_append), METH_FASTCALL, "append one token to the dense window"},
+    {"encode", FAST(py_encode), METH_FASTCALL, "pack one side"},
     {"take_ids", FAST(py_take_ids), METH_FASTCALL, "check and convert given cluster ids"},
     {"ids_in_range", py_ids_in_range, METH_O, "verdict of take_ids"},
     {"launches", py_launches, METH_NOARGS, "kernels launched through this module"},

@@ -149,6 +149,15 @@ class CompressedTensor:
         return new
 
     @classmethod
+    def _packed(cls, centroids, cluster_ids, payload, metadata, scale, plan, native) -> "CompressedTensor":
+        """Tensor over what a packer has just written: dense tensors (ids int8) and their kernel views."""
+        self = cls.__new__(cls)
+        self.centroids, self.cluster_ids, self.payload, self.metadata, self.scale = centroids, cluster_ids, payload, metadata, scale
+        self.plan, self._buffers = plan, (cluster_ids, payload, metadata, scale)
+        self._live, self._native, self._flat = [cluster_ids.shape[2]], native, native[1:]
+        return self
+
+    @classmethod
     def _window(cls, centroids, buffers, length, plan, live=None) -> "CompressedTensor":
         """Tensor over the first ``length`` tokens of capacity ``buffers``; ``live`` is the written-length
         marker of those buffers (a fresh one when they are new)."""
