@@ -76,10 +76,15 @@ def _incremental_cluster(x, centers, config, *, value=False):
 
 
 @torch.no_grad()
-def _encode(x, centers, ids, plan: KernelPlan, *, value=False, stored_ids=None):
+def _encode(x, centers, ids, plan: KernelPlan, *, value=False):
     """Residuals of ``x`` to its centres in the layout of ``plan``
     (reference compression.py:72-101).  ``value`` is accepted for signature
-    compatibility: K and V use the same selection rule here.  ``stored_ids``: the ids as int8, when there."""
+    compatibility: K and V use the same selection rule here."""
+    return _pack(x, centers, ids, plan)
+
+
+def _pack(x, centers, ids, plan: KernelPlan, stored_ids=None):
+    """``_encode`` with autograd off already; ``stored_ids``: the ids as int8, when there."""
     require_device(x.get_device())
     ids, centers = ids.int().contiguous(), centers.half().contiguous()
     stored = ids.to(torch.int8) if stored_ids is None else stored_ids
@@ -206,7 +211,7 @@ def compress(
         # been launched behind it, so the device does not wait for the host
         (k_centres, k_ids), (v_centres, v_ids) = clustering
         ids_wide, ids_narrow, in_range = _ops(key).take_ids(k_ids, v_ids, k_centres.shape[2], v_centres.shape[2])
-        packed = [_encode(x, clustering[side][0], ids_wide[side], plan, stored_ids=ids_narrow[side])
+        packed = [_pack(x, clustering[side][0], ids_wide[side], plan, ids_narrow[side])
                   for side, x in enumerate((key, value))]
         if not in_range():
             raise ValueError("external cluster IDs are out of range")
@@ -216,7 +221,7 @@ def compress(
     if previous is None and config.num_clusters <= min(32, key.shape[2]) and (key.data_ptr() | value.data_ptr()) % 16 == 0:
         # K and V in the same launches: an iteration's fixed costs are paid once
         sides = _ops(key).kmeans_pair(key, value, config.num_clusters, config.kmeans_iterations)
-        return CompressedKV(*(_encode(x, centres, ids, plan, stored_ids=stored)
+        return CompressedKV(*(_pack(x, centres, ids, plan, stored)
                               for x, (centres, ids, stored) in zip((key, value), sides)))
 
     packed = []
@@ -227,6 +232,6 @@ def compress(
             centres, ids = _incremental_cluster(x, grown, config, value=is_value)
         else:
             centres, ids = cluster(x, config.num_clusters, config.kmeans_iterations, value=is_value)
-        new = _encode(x, centres, ids, plan, value=is_value)
+        new = _pack(x, centres, ids, plan)
         packed.append(new if previous is None else (previous.key, previous.value)[side].append(new))
     return CompressedKV(*packed)

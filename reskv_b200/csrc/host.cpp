@@ -465,10 +465,13 @@ PyObject* py_take_ids(PyObject*, PyObject* const* o, Py_ssize_t n) {
         const at::Tensor k = tensor(o[0], "ids").contiguous(), v = tensor(o[1], "ids").contiguous();
         const c10::DeviceIndex dev = k.get_device();
         const c10::cuda::CUDAGuard guard(dev);
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        const auto empty = [&](at::IntArrayRef size, at::ScalarType type) {
+            return at::detail::empty_cuda(size, type, k.device(), std::nullopt);
+        };
         std::vector<int64_t> both(k.sizes().begin(), k.sizes().end());
         both.insert(both.begin(), 2);
-        const at::Tensor wide = at::empty(both, k.options().dtype(at::kInt));
-        const at::Tensor narrow_k = at::empty(k.sizes(), k.options().dtype(at::kChar)), narrow_v = at::empty_like(narrow_k);
+        const at::Tensor wide = empty(both, at::kInt), narrow_k = empty(k.sizes(), at::kChar), narrow_v = empty(k.sizes(), at::kChar);
         const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
         Verdict* verdict = get_verdict(dev);
         *verdict->word = 0;
