@@ -65,7 +65,6 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         self.length = 0  # tokens seen
         self.live = 0    # tokens in the dense segment (sinks included)
         self.plan = None
-        self._lib = None
 
     @property
     def start_position(self) -> int:
@@ -73,15 +72,12 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         return min(self.sink_tokens, self.length)
 
     def lazy_initialization(self, key_states, value_states=None):
-        from ._extension import bound_library
-
         b, h, _, d = key_states.shape
         slots = self.sink_tokens + self.config.recent_size + self.config.group_size
         # one allocation for the three window buffers
         window = torch.empty((3, b, h, slots, d), device=key_states.device, dtype=key_states.dtype)
         self.keys, self.raw_keys, self.values = window[0], window[1], window[2]
         self.plan = self.config.resolve(b)
-        self._lib = bound_library(key_states.device)
         self.is_initialized = True
 
     def update(self, key_states, value_states, cache_kwargs=None, *args, **kwargs):
@@ -146,11 +142,9 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
                                    previous=self.compressed, plan=self.plan)
         remain = self.live - s - n
         if self.keys.dtype == torch.float16 and self.keys.is_cuda:
-            from ._extension import _stream, check
+            from ._extension import host
 
-            b, h, cap, _ = self.keys.shape
-            check(self._lib.reskv_window_shift(self.keys.data_ptr(), self.raw_keys.data_ptr(), self.values.data_ptr(),
-                                               b, h, cap, s, s + n, remain, _stream(self.keys.device)))
+            host().window_shift(self.keys, self.raw_keys, self.values, s, s + n, remain)
         else:
             for buf in (self.keys, self.raw_keys, self.values):
                 tail = buf[:, :, s + n : self.live]

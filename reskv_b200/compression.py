@@ -144,26 +144,18 @@ def _append_group_in_place(key, value, previous: CompressedKV, config, plan: Ker
     n, t = previous.seq_len, key.shape[2]
     if previous.key._live[0] != n or previous.value._live[0] != n:
         return None
-    if min(previous.key.token_stride, previous.value.token_stride) < n + t:  # full: twice the needed length
-        previous = CompressedKV(*(side.reserve(max(2 * (n + t), 256)) for side in (previous.key, previous.value)))
-    if token_stride_of(key) is None or token_stride_of(key) != token_stride_of(value):
-        key, value = key.contiguous(), value.contiguous()
-    b, h = key.shape[:2]
-    sides = []
-    for side in (previous.key, previous.value):
-        old = side._native[0]
-        count = old.shape[1]
-        new = side.centroids
-        if count < config.max_clusters:
-            new = torch.empty((b, h, count + 1, 128), dtype=torch.float16, device=key.device)
-        elif not new.is_contiguous():
-            new = old.view(b, h, count, 128)
-        sides.append((old, new, side._buffers))
-    _ops(key).compress_group(plan, key, value, sides, n)
+    require_device(key.get_device())
+    sides = previous.key, previous.value
+    held = [(side._buffers, side._flat) for side in sides]
+    lives = [side._live for side in sides]
+    if min(side.token_stride for side in sides) < n + t:  # full: twice the needed length
+        held, lives = host().regrow(held[0][0], held[1][0], n, max(2 * (n + t), 256)), [[n], [n]]
+    grown = host().append_group(LAYOUT_IDS[plan.layout], plan.bits, plan.nnz, config.max_clusters, n, key, value,
+                                sides[0].centroids, sides[0]._native[0], *held[0], sides[1].centroids, sides[1]._native[0], *held[1])
     windows = []
-    for side, (_, new, _) in zip((previous.key, previous.value), sides):
-        side._live[0] = n + t
-        windows.append(side._grown(new, n + t))
+    for side, live, (buffers, flat), (centroids, views, native) in zip(sides, lives, held, grown):
+        live[0] = n + t
+        windows.append(side._grown(centroids, views, buffers, flat, native, live))
     return CompressedKV(*windows)
 
 

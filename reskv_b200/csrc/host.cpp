@@ -34,6 +34,13 @@ void check(int rc) {
     throw PyError{};
 }
 
+void check_cuda(cudaError_t e, const char* what) {
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    PyErr_Format(PyExc_RuntimeError, "%s: %s", what, cudaGetErrorString(e));
+    throw PyError{};
+}
+
 long long g_launches = 0;  // kernels launched through this module (the interpreter lock serialises the calls)
 bool g_check_status = false;
 
@@ -403,6 +410,150 @@ PyObject* py_encode(PyObject*, PyObject* const* o, Py_ssize_t n) {
     });
 }
 
+// ---- a decode group behind the live tokens of a cache ------------------------------------------------------------------
+PyObject* wrap(const at::Tensor& t) { return t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None); }
+
+// The buffers [B,H,capacity,...] of one side: ids, payload, metadata or None, scale or None.
+struct Buffers {
+    at::Tensor part[4];
+    explicit Buffers(PyObject* tuple) {
+        for (int i = 0; i < 4; ++i) part[i] = i < 2 ? tensor(item(tuple, i), "buffer") : optional_tensor(item(tuple, i), "buffer");
+    }
+};
+
+// regrow(k_buffers, v_buffers, tokens, capacity) -> ((buffers, merged views) of K, the same of V): the first `tokens` tokens
+// in fresh buffers of `capacity` tokens, all carved from one allocation (every buffer starts on a 256-byte boundary); the
+// merged views are the buffers as [B*H, capacity, ...].
+PyObject* py_regrow(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 4);
+        const Buffers sides[2] = {Buffers(o[0]), Buffers(o[1])};
+        const int64_t tokens = integer(o[2]), capacity = integer(o[3]);
+        const at::Tensor& first = sides[0].part[0];
+        const c10::DeviceIndex dev = first.get_device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        const int64_t units = first.size(0) * first.size(1);
+        int64_t row[2][4] = {}, total = 0;  // bytes of a token
+        for (int i = 0; i < 8; ++i) {
+            const at::Tensor& t = sides[i / 4].part[i % 4];
+            if (!t.defined()) continue;
+            same_device(dev, t);
+            if (!t.is_contiguous() || t.dim() < 3 || t.size(0) * t.size(1) != units || t.size(2) < tokens || capacity < tokens)
+                value_error("regrow expects dense buffers [B,H,capacity,...] that hold the tokens");
+            row[i / 4][i % 4] = t.element_size() * (t.dim() == 4 ? t.size(3) : 1);
+            total += (units * capacity * row[i / 4][i % 4] + 255) / 256 * 256;
+        }
+        const at::Tensor arena = at::detail::empty_cuda({total}, at::kByte, first.device(), std::nullopt);
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+        PyObject* both = PyTuple_New(2);
+        int64_t at = 0;
+        for (int side = 0; side < 2; ++side) {
+            PyObject *grown = PyTuple_New(4), *flat = PyTuple_New(4);
+            for (int i = 0; i < 4; ++i) {
+                const at::Tensor& t = sides[side].part[i];
+                at::Tensor whole, merged;
+                if (t.defined()) {
+                    const int64_t bytes = row[side][i], used = units * capacity * bytes;
+                    const at::Tensor typed = arena.narrow(0, at, used).view(t.scalar_type());
+                    const bool wide = t.dim() == 4;
+                    whole = wide ? typed.view({t.size(0), t.size(1), capacity, t.size(3)}) : typed.view({t.size(0), t.size(1), capacity});
+                    merged = wide ? typed.view({units, capacity, t.size(3)}) : typed.view({units, capacity});
+                    const cudaError_t e = cudaMemcpy2DAsync(typed.data_ptr(), capacity * bytes, t.const_data_ptr(), t.size(2) * bytes,
+                                                            tokens * bytes, units, cudaMemcpyDeviceToDevice, stream);
+                    if (e != cudaSuccess) {
+                        Py_DECREF(grown), Py_DECREF(flat), Py_DECREF(both);
+                        check_cuda(e, "regrow");
+                    }
+                    at += (used + 255) / 256 * 256;
+                }
+                PyTuple_SET_ITEM(grown, i, wrap(whole));
+                PyTuple_SET_ITEM(flat, i, wrap(merged));
+            }
+            PyTuple_SET_ITEM(both, side, PyTuple_Pack(2, grown, flat));
+            Py_DECREF(grown), Py_DECREF(flat);
+        }
+        return both;
+    });
+}
+
+// append_group(layout, bits, nnz, limit, seq_len, x_k, x_v, then for K and for V: centroids, centroids [B*H,C,128], buffers,
+// merged views) -> for K and V (centroids, the views of seq_len + T tokens, the views the decode kernels take): clusters
+// the group, packs it and writes it behind token seq_len of the buffers.
+PyObject* py_append_group(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 15);
+        const int layout = static_cast<int>(integer(o[0])), bits = static_cast<int>(integer(o[1])), nnz = static_cast<int>(integer(o[2]));
+        const int64_t limit = integer(o[3]), seq = integer(o[4]);
+        at::Tensor x[2] = {tensor(o[5], "key"), tensor(o[6], "value")};
+        const c10::DeviceIndex dev = x[0].get_device();
+        const c10::cuda::CUDAGuard guard(dev);
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        if (token_stride_of(x[0]) < 0 || token_stride_of(x[0]) != token_stride_of(x[1]))
+            x[0] = x[0].contiguous(), x[1] = x[1].contiguous();
+        const int64_t b = x[0].size(0), h = x[0].size(1), t = x[0].size(2);
+        at::Tensor old[2], next[2];
+        const Buffers sides[2] = {Buffers(o[9]), Buffers(o[13])};
+        for (int i = 0; i < 2; ++i) {
+            const at::Tensor& given = tensor(o[7 + 4 * i], "centroids");
+            old[i] = tensor(o[8 + 4 * i], "centroids");
+            const int64_t c = old[i].size(1);
+            same_device(dev, old[i]);
+            if (x[i].scalar_type() != at::kHalf || old[i].scalar_type() != at::kHalf || !old[i].is_contiguous())
+                value_error("append_group expects FP16 keys, values and dense FP16 centroids");
+            if (c < limit)
+                next[i] = at::detail::empty_cuda({b, h, c + 1, 128}, at::kHalf, x[0].device(), std::nullopt);
+            else
+                next[i] = given.is_contiguous() ? given : old[i].view({b, h, c, 128});
+            for (const at::Tensor& part : sides[i].part)
+                if (part.defined()) {
+                    same_device(dev, part);
+                    if (!part.is_contiguous()) value_error("append_group expects dense capacity buffers");
+                }
+            if (sides[i].part[0].scalar_type() != at::kChar) value_error("append_group expects int8 ids");
+        }
+        const at::Tensor scratch = at::detail::empty_cuda({2, b * h, t}, at::kInt, x[0].device(), std::nullopt);
+        const auto at_part = [&](int i, int k) { return sides[i].part[k].defined() ? sides[i].part[k].data_ptr() : nullptr; };
+        check(reskv_compress_group(
+            layout, bits, nnz, x[0].const_data_ptr(), x[1].const_data_ptr(), static_cast<int>(b), static_cast<int>(h), static_cast<int>(t),
+            token_stride_of(x[0]), old[0].const_data_ptr(), static_cast<int>(old[0].size(1)), next[0].data_ptr(),
+            static_cast<int>(next[0].size(2)), at_part(0, 0), at_part(0, 1), at_part(0, 2), at_part(0, 3), sides[0].part[0].size(2),
+            old[1].const_data_ptr(), static_cast<int>(old[1].size(1)), next[1].data_ptr(), static_cast<int>(next[1].size(2)),
+            at_part(1, 0), at_part(1, 1), at_part(1, 2), at_part(1, 3), sides[1].part[0].size(2), static_cast<int>(seq),
+            static_cast<int32_t*>(scratch.data_ptr()), c10::cuda::getCurrentCUDAStream(dev).stream()));
+        g_launches += 5;
+        PyObject* both = PyTuple_New(2);
+        for (int i = 0; i < 2; ++i) {
+            PyObject *views = PyTuple_New(4), *native = PyTuple_New(5);
+            PyTuple_SET_ITEM(native, 0, THPVariable_Wrap(next[i].view({b * h, next[i].size(2), 128})));
+            for (int k = 0; k < 4; ++k) {
+                const at::Tensor merged = optional_tensor(item(o[10 + 4 * i], k), "buffer");
+                PyTuple_SET_ITEM(views, k, wrap(merged.defined() ? sides[i].part[k].narrow(2, 0, seq + t) : merged));
+                PyTuple_SET_ITEM(native, k + 1, wrap(merged.defined() ? merged.narrow(1, 0, seq + t) : merged));
+            }
+            PyObject* centroids = THPVariable_Wrap(next[i]);
+            PyTuple_SET_ITEM(both, i, PyTuple_Pack(3, centroids, views, native));
+            Py_DECREF(centroids), Py_DECREF(views), Py_DECREF(native);
+        }
+        return both;
+    });
+}
+
+// window_shift(keys, raw_keys, values, dst, src, count): moves `count` tokens of the window buffers [B,H,capacity,128]
+PyObject* py_window_shift(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 6);
+        const at::Tensor &wk = tensor(o[0], "keys"), &wr = tensor(o[1], "raw keys"), &wv = tensor(o[2], "values");
+        const c10::DeviceIndex dev = wk.get_device();
+        const c10::cuda::CUDAGuard guard(dev);
+        check(reskv_window_shift(wk.data_ptr(), wr.data_ptr(), wv.data_ptr(), static_cast<int>(wk.size(0)), static_cast<int>(wk.size(1)),
+                                 static_cast<int>(wk.size(2)), static_cast<int>(integer(o[3])), static_cast<int>(integer(o[4])),
+                                 static_cast<int>(integer(o[5])), c10::cuda::getCurrentCUDAStream(dev).stream()));
+        ++g_launches;
+        return Py_NewRef(Py_None);
+    });
+}
+
 // ---- verdicts of take_ids -------------------------------------------------------------------------------------------
 // A word of mapped pinned host memory and an event per call in flight; a few are kept for later calls (any thread, any
 // device: the event is made for the call's device).
@@ -414,13 +565,6 @@ struct Verdict {
 constexpr size_t kKeptVerdicts = 16;
 std::mutex g_verdict_lock;
 std::vector<Verdict*> g_verdicts;
-
-void check_cuda(cudaError_t e, const char* what) {
-    if (e == cudaSuccess) return;
-    cudaGetLastError();
-    PyErr_Format(PyExc_RuntimeError, "%s: %s", what, cudaGetErrorString(e));
-    throw PyError{};
-}
 
 Verdict* get_verdict(c10::DeviceIndex device) {
     {
@@ -523,6 +667,9 @@ PyMethodDef g_methods[] = {
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
     {"window_append", FAST(py_window_append), METH_FASTCALL, "append one token to the dense window"},
     {"encode", FAST(py_encode), METH_FASTCALL, "pack one side"},
+    {"regrow", FAST(py_regrow), METH_FASTCALL, "larger buffers for a cache"},
+    {"append_group", FAST(py_append_group), METH_FASTCALL, "cluster, pack and append one decode group"},
+    {"window_shift", FAST(py_window_shift), METH_FASTCALL, "move tokens of the dense window"},
     {"take_ids", FAST(py_take_ids), METH_FASTCALL, "check and convert given cluster ids"},
     {"ids_in_range", py_ids_in_range, METH_O, "verdict of take_ids"},
     {"launches", py_launches, METH_NOARGS, "kernels launched through this module"},

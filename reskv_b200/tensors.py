@@ -136,16 +136,12 @@ class CompressedTensor:
         return (centroids.reshape(b * h, -1, 128).contiguous(),
                 *(None if flat is None else flat.narrow(1, 0, n) for flat in self._flat))
 
-    def _grown(self, centroids, length: int) -> "CompressedTensor":
-        """Window over the first ``length`` tokens of this tensor's own buffers with a newer centroid table, for
-        library calls that have just written tokens ``[seq_len, length)`` there: same plan, same buffers, same
-        written-length marker, nothing to validate again."""
+    def _grown(self, centroids, views, buffers, flat, native, live) -> "CompressedTensor":
+        """Window of the same plan over ``buffers``, for library calls that have just written tokens there: the views are
+        given, nothing to validate again."""
         new = CompressedTensor.__new__(CompressedTensor)
-        new.centroids, new.plan, new._buffers, new._live = centroids, self.plan, self._buffers, self._live
-        new._flat = self._flat
-        new.cluster_ids, new.payload, new.metadata, new.scale = (
-            None if buf is None else buf.narrow(2, 0, length) for buf in self._buffers)
-        new._native = new._native_views(centroids, length)
+        new.centroids, new.plan, new._buffers, new._flat, new._native, new._live = centroids, self.plan, buffers, flat, native, live
+        new.cluster_ids, new.payload, new.metadata, new.scale = views
         return new
 
     @classmethod
