@@ -593,15 +593,16 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     __shared__ uint32_t tmem_base_s;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // Work of the launch = the tiles of all units laid end to end; CTA c takes [c * share, (c + 1) * share) and walks
-    // it segment by segment (consecutive tiles of one unit, at most kUChunkMax tokens: one set of FP32 partial sums).
+    // Work of the launch = the tiles of all units laid end to end, or of each side's units (gridDim.y ranges); CTA c of a
+    // range takes [c * share, (c + 1) * share) of it and walks that segment by segment (consecutive tiles of one unit, at
+    // most kUChunkMax tokens: one set of FP32 partial sums).
     // Tiles are numbered q = 0, 1, ... through the CTA's whole range: stage q % 5, group / distance buffer / one-hot
     // buffer q % 3, sum accumulator q % 4, and every barrier's phase follows from q, so the ring keeps turning across
     // segment boundaries (the copies of the next segment are in flight while this one drains and flushes).
     const int tiles_per_unit = (p.tokens + kUTile - 1) / kUTile;
-    const long long work_total = static_cast<long long>(units) * tiles_per_unit;
-    const long long work_begin = static_cast<long long>(blockIdx.x) * share;
-    const long long work_end = work_begin + share < work_total ? work_begin + share : work_total;
+    const long long range = static_cast<long long>(units) * tiles_per_unit / gridDim.y;
+    const long long range_end = range * (blockIdx.y + 1), work_begin = range * blockIdx.y + static_cast<long long>(blockIdx.x) * share;
+    const long long work_end = work_begin + share < range_end ? work_begin + share : range_end;
     struct Segment {
         int unit, tile0, tiles;
     };
@@ -1087,6 +1088,35 @@ void place_state(UmmaParams& p, void* workspace, size_t per) {
     for (int i = 0; i < 3; ++i, at += per * sizeof(int)) p.counts[i] = reinterpret_cast<int*>(at);
 }
 
+// Tiles per CTA of the assignment kernel.  One CTA per SM, every CTA an equal share of all units' tiles.  A CTA pays about
+// ten tile times per segment (pipeline drain, flush, new centre tables, refill), so the share is chosen - between the even
+// split and half as much again - for the shortest slowest CTA: a share that divides the units evenly often beats the
+// smallest one.  About `tries` of the shares in between are looked at (this is host time).
+long long cta_share(long long tiles_total, int tiles_unit, int least, int tries) {
+    const int seg_max = kUChunkMax / kUTile;
+    const long long even = (tiles_total + sm_count() - 1) / sm_count();
+    const long long low = even < least ? least : even, most = low + low / 2 + 1, step = low / (2 * tries) + 1;
+    long long share = low, best_cost = -1;
+    for (long long cand = low; cand <= most; cand += step) {
+        long long worst = 0;
+        int in_unit = tiles_unit;  // tiles left in the unit
+        for (long long left = tiles_total; left > 0;) {
+            const int work = static_cast<int>(cand < left ? cand : left);
+            int segments = 0;
+            for (int rest = work; rest > 0; ++segments) {  // same walk as the kernel's
+                int n = in_unit < rest ? in_unit : rest;
+                if (n > seg_max) n = seg_max;
+                rest -= n, in_unit -= n;
+                if (in_unit == 0) in_unit = tiles_unit;
+            }
+            if (work + 10 * segments > worst) worst = work + 10 * segments;
+            left -= work;
+        }
+        if (best_cost < 0 || worst < best_cost) best_cost = worst, share = cand;
+    }
+    return share;
+}
+
 int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t s) {
     CUtensorMap maps[2];
     for (int i = 0; i < 2; ++i)  // one side: the second map repeats the first and is not used
@@ -1108,36 +1138,25 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
             return rc;
         prepared |= 1ull << (dev & 63);
     }
-    // One CTA per SM, every CTA an equal share of all units' tiles.  A CTA pays about ten tile times per segment
-    // (pipeline drain, flush, new centre tables, refill), so the share is chosen - between the even split and
-    // half as much again - for the shortest slowest CTA: a share that divides the units evenly often beats the
-    // smallest one.
-    const int tiles_unit = (p.tokens + kUTile - 1) / kUTile, seg_max = kUChunkMax / kUTile;
-    const long long tiles_total = static_cast<long long>(p.sides) * p.units * tiles_unit;
-    const long long even = (tiles_total + sm_count() - 1) / sm_count();
-    long long share = even < 1 ? 1 : even, best_cost = -1;
-    const long long step = share / 64 + 1;  // at most ~32 candidates: this is host time
-    for (long long cand = share, most = share + share / 2 + 1; cand <= most; cand += step) {
-        long long worst = 0;
-        for (long long w0 = 0; w0 < tiles_total; w0 += cand) {
-            const long long w1 = w0 + cand < tiles_total ? w0 + cand : tiles_total;
-            long long segments = 0;
-            for (long long w = w0; w < w1;) {  // same walk as the kernel's
-                const long long in_unit = tiles_unit - w % tiles_unit;
-                long long n = in_unit < w1 - w ? in_unit : w1 - w;
-                if (n > seg_max) n = seg_max;
-                w += n, ++segments;
-            }
-            const long long cost = (w1 - w0) + 10 * segments;
-            if (cost > worst) worst = cost;
+    // A call for one side takes at least four tiles per CTA in every iteration.  K and V together take smaller shares, which
+    // are faster for short contexts (16.4 -> 9 us per iteration at 8 units x 1024 tokens), except in the last iteration: it
+    // is cut side by side as the call for one side is.  The centres that are returned are then sums of the same pieces
+    // whether the sides share launches or not; FP32 sums of other pieces differ in their last bits, enough to round some of
+    // a million FP16 coordinates differently and with them the choice between nearly equal residuals.
+    const int tiles_unit = (p.tokens + kUTile - 1) / kUTile;
+    const long long tiles_side = static_cast<long long>(p.units) * tiles_unit;
+    const bool pair = p.sides == 2;
+    long long share = pair ? cta_share(p.sides * tiles_side, tiles_unit, 1, 32) : cta_share(tiles_side, tiles_unit, 4, 1 << 30);
+    unsigned per_range = static_cast<unsigned>((p.sides * tiles_side + share - 1) / share), ranges = 1;
+    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration) {
+        if (pair && p.iteration + 1 == p.iterations) {
+            share = cta_share(tiles_side, tiles_unit, 4, 1 << 30);
+            per_range = static_cast<unsigned>((tiles_side + share - 1) / share), ranges = 2;
         }
-        if (best_cost < 0 || worst < best_cost) best_cost = worst, share = cand;
-    }
-    const dim3 grid(static_cast<unsigned>((tiles_total + share - 1) / share));
-    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration)
-        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, grid, kUThreads, smem, s, p.iteration > 0, p, maps[0], maps[1],
-                                                  static_cast<int>(share)), "kmeans_assign launch"))
+        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, dim3(per_range, ranges), kUThreads, smem, s, p.iteration > 0, p,
+                                                  maps[0], maps[1], static_cast<int>(share)), "kmeans_assign launch"))
             return rc;
+    }
     if (int rc = check_cuda(launch_overlapped(kmeans_final_kernel, dim3(static_cast<unsigned>((per + 7) / 8)), 256, 0, s, true, p,
                                               static_cast<__half*>(centroids0), static_cast<__half*>(centroids1)), "kmeans_final launch"))
         return rc;
