@@ -33,7 +33,7 @@
 //  * Rotations are packed FP32 pairs (fma.rn.f32x2), quantised codes are decoded two at a time by one AND-XOR and one
 //    HFMA2.
 //
-// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.232 ms, 71 % of the issue slots, 73 % of the
+// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.222 ms, 71 % of the issue slots, 73 % of the
 // shared-memory pipe, 55 % of the integer pipe; 82 instructions and 22 shared-memory wavefronts per token and KV head.
 // Before (two CTAs of four warps, sin/cos and accumulators in registers): 0.280 ms.  INT4, batch 8, 16320 tokens: 0.128
 // -> 0.102 ms.  A 128-token call costs ~9 us, most of it the set-up (tables, centroids, first query) and one pass.
