@@ -155,7 +155,7 @@ def _append_group_in_place(key, value, previous: CompressedKV, config, plan: Ker
     windows = []
     for side, live, (buffers, flat), (centroids, views, native) in zip(sides, lives, held, grown):
         live[0] = n + t
-        windows.append(side._grown(centroids, views, buffers, flat, native, live))
+        windows.append(side._grown(centroids, n + t, (buffers, flat, live), (views, native)))
     return CompressedKV(*windows)
 
 

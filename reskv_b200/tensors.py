@@ -136,12 +136,18 @@ class CompressedTensor:
         return (centroids.reshape(b * h, -1, 128).contiguous(),
                 *(None if flat is None else flat.narrow(1, 0, n) for flat in self._flat))
 
-    def _grown(self, centroids, views, buffers, flat, native, live) -> "CompressedTensor":
-        """Window of the same plan over ``buffers``, for library calls that have just written tokens there: the views are
-        given, nothing to validate again."""
+    def _grown(self, centroids, length: int, held=None, views=None) -> "CompressedTensor":
+        """Window over the first ``length`` tokens of this tensor's buffers with a newer centroid table, for library calls
+        that have just written tokens ``[seq_len, length)`` there: same plan and written-length marker, nothing to
+        validate again.  ``held = (buffers, merged views, marker)``: over these instead; ``views = (the public fields, the
+        kernels' views)``: already made."""
         new = CompressedTensor.__new__(CompressedTensor)
-        new.centroids, new.plan, new._buffers, new._flat, new._native, new._live = centroids, self.plan, buffers, flat, native, live
-        new.cluster_ids, new.payload, new.metadata, new.scale = views
+        new.centroids, new.plan = centroids, self.plan
+        new._buffers, new._flat, new._live = held or (self._buffers, self._flat, self._live)
+        if views is None:
+            views = (tuple(None if buf is None else buf.narrow(2, 0, length) for buf in new._buffers),
+                     new._native_views(centroids, length))
+        (new.cluster_ids, new.payload, new.metadata, new.scale), new._native = views
         return new
 
     @classmethod
