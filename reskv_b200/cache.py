@@ -114,8 +114,9 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         if self.live > self.keys.shape[2]:
             raise ValueError("prefill leaves more dense tokens than the window holds")
         for buf, src in ((self.keys, keys), (self.raw_keys, raw), (self.values, values)):
-            buf[:, :, :s].copy_(src[:, :, :s])
-            buf[:, :, s : self.live].copy_(src[:, :, s + n :])
+            if s:
+                buf[:, :, :s].copy_(src[:, :, :s])
+            buf.narrow(2, s, t - n - s).copy_(src.narrow(2, s + n, t - n - s))
 
     def _take_token(self, key, raw, value):
         """One launch writes the token's rotated key, raw key and value into slot ``live`` of the three
