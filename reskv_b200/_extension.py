@@ -301,18 +301,7 @@ class CompressionOps(_Ops):
         """``kmeans`` of K and of V in the same launches -> ``(centroids, int32 ids, int8 ids)`` of each; up to 32 centres,
         at least as many tokens, 16-byte aligned inputs."""
         _same_device(self.device.index, key, value)
-        b, h, t, _ = key.shape
-        need = self.lib.reskv_kmeans_workspace_bytes(2 * b, h, count)
-        ws = torch.empty(need, dtype=torch.uint8, device=key.device)
-        sides = [(torch.empty((b, h, count, 128), dtype=torch.float16, device=key.device),
-                  torch.empty((b, h, t), dtype=torch.int32, device=key.device),
-                  torch.empty((b, h, t), dtype=torch.int8, device=key.device)) for _ in range(2)]
-        (kc, ki, k8), (vc, vi, v8) = sides
-        check(self.lib.reskv_kmeans_pair(key.data_ptr(), value.data_ptr(), b, h, t, token_stride_of(key), token_stride_of(value),
-                                         count, iterations, ws.data_ptr(), need, kc.data_ptr(), vc.data_ptr(), ki.data_ptr(),
-                                         vi.data_ptr(), k8.data_ptr(), v8.data_ptr(), _stream(key.device)),
-              launches=1 + iterations)
-        return sides
+        return host().kmeans_pair(key, value, count, iterations)
 
     def kmeans_incremental(self, x, centroids, append):
         """Decode-time step -> (centroids f16 [B,H,C or C+1,128], ids i32 [B,H,T])."""

@@ -410,6 +410,44 @@ PyObject* py_encode(PyObject*, PyObject* const* o, Py_ssize_t n) {
     });
 }
 
+// kmeans_pair(key, value, clusters, iterations) -> for K and V (centroids [B,H,C,128], int32 ids [B,H,T], int8 ids)
+PyObject* py_kmeans_pair(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 4);
+        const at::Tensor &k = tensor(o[0], "key"), &v = tensor(o[1], "value");
+        const int64_t count = integer(o[2]), iterations = integer(o[3]);
+        const c10::DeviceIndex dev = k.get_device();
+        same_device(dev, v);
+        if (k.scalar_type() != at::kHalf || v.scalar_type() != at::kHalf || k.dim() != 4 || k.sizes() != v.sizes() ||
+            token_stride_of(k) < 0 || token_stride_of(v) < 0)
+            value_error("kmeans_pair expects FP16 K and V [B,H,T,128], dense or token slices of dense buffers");
+        const c10::cuda::CUDAGuard guard(dev);
+        const at::AutoDispatchBelowADInplaceOrView plain;
+        const auto empty = [&](at::IntArrayRef size, at::ScalarType type) {
+            return at::detail::empty_cuda(size, type, k.device(), std::nullopt);
+        };
+        const int64_t b = k.size(0), h = k.size(1), t = k.size(2);
+        const int bi = static_cast<int>(b), hi = static_cast<int>(h), ci = static_cast<int>(count);
+        if (count < 1 || count > 64) value_error("kmeans_pair: cluster count must be in [1,32] and at most the token count");
+        const size_t need = reskv_kmeans_workspace_bytes(2 * bi, hi, ci);
+        const at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte);
+        at::Tensor part[2][3];
+        for (auto& side : part) side[0] = empty({b, h, count, 128}, at::kHalf), side[1] = empty({b, h, t}, at::kInt), side[2] = empty({b, h, t}, at::kChar);
+        check(reskv_kmeans_pair(k.const_data_ptr(), v.const_data_ptr(), bi, hi, static_cast<int>(t), token_stride_of(k), token_stride_of(v), ci,
+                                static_cast<int>(iterations), ws.data_ptr(), need, part[0][0].data_ptr(), part[1][0].data_ptr(),
+                                static_cast<int32_t*>(part[0][1].data_ptr()), static_cast<int32_t*>(part[1][1].data_ptr()),
+                                part[0][2].data_ptr(), part[1][2].data_ptr(), c10::cuda::getCurrentCUDAStream(dev).stream()));
+        g_launches += 1 + iterations;
+        PyObject* both = PyTuple_New(2);
+        for (int i = 0; i < 2; ++i) {
+            PyObject* side = PyTuple_New(3);
+            for (int j = 0; j < 3; ++j) PyTuple_SET_ITEM(side, j, THPVariable_Wrap(part[i][j]));
+            PyTuple_SET_ITEM(both, i, side);
+        }
+        return both;
+    });
+}
+
 // ---- a decode group behind the live tokens of a cache ------------------------------------------------------------------
 PyObject* wrap(const at::Tensor& t) { return t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None); }
 
@@ -667,6 +705,7 @@ PyMethodDef g_methods[] = {
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
     {"window_append", FAST(py_window_append), METH_FASTCALL, "append one token to the dense window"},
     {"encode", FAST(py_encode), METH_FASTCALL, "pack one side"},
+    {"kmeans_pair", FAST(py_kmeans_pair), METH_FASTCALL, "cluster K and V in the same launches"},
     {"regrow", FAST(py_regrow), METH_FASTCALL, "larger buffers for a cache"},
     {"append_group", FAST(py_append_group), METH_FASTCALL, "cluster, pack and append one decode group"},
     {"window_shift", FAST(py_window_shift), METH_FASTCALL, "move tokens of the dense window"},
