@@ -156,9 +156,10 @@ __device__ __forceinline__ void top4(uint32_t (&a)[4], const uint32_t (&b)[4]) {
     order2(a[0], a[2]), order2(a[1], a[3]), order2(a[0], a[1]), order2(a[2], a[3]);
 }
 // M-th largest of 16 keys (M = 4 or 8), in either half: sorted runs, then the smallest of the pairwise maxima of one run
-// and the other one reversed.
+// and the other one reversed.  Bit patterns are ordered: a NaN key comes out above every number, and `largest` turns NaN then
+// (one FP16 operation on the largest keys of both halves; infinity times zero does so too, which costs time only).
 template <int M>
-__device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key) {
+__device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key, __half2& largest) {
     uint32_t a[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -168,6 +169,7 @@ __device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key) {
     }
     if constexpr (M == 4) {
         top4(a[0], a[1]), top4(a[2], a[3]);
+        largest = __hfma2(as_half2(a[0][0]), as_half2(a[2][0]), largest);
         uint32_t t = __vmaxu2(a[0][0], a[2][3]);
 #pragma unroll
         for (int i = 1; i < 4; ++i) t = __vminu2(t, __vmaxu2(a[0][i], a[2][3 - i]));
@@ -184,6 +186,7 @@ __device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key) {
                 for (int i = 0; i < 8; ++i)
                     if (!(i & step)) order2(run[r][i], run[r][i + step]);
         }
+        largest = __hfma2(as_half2(run[0][0]), as_half2(run[1][0]), largest);
         uint32_t t = __vmaxu2(run[0][0], run[1][7]);
 #pragma unroll
         for (int i = 1; i < 8; ++i) t = __vminu2(t, __vmaxu2(run[0][i], run[1][7 - i]));
@@ -191,54 +194,78 @@ __device__ __forceinline__ uint32_t mth_of_16(const uint32_t* key) {
     }
 }
 
-// Keep-mask of the `m` largest keys of every 16-coordinate tile, lower coordinate first among equal keys.
+// Per half, of 16 packed keys: the largest v with count(key >= v) >= m, 0 when there are fewer than m numbers.
+__device__ __forceinline__ uint32_t mth_by_bisection(const uint32_t* key, int m) {
+    const __half2 m2 = __float2half2_rn(static_cast<float>(m));
+    uint32_t v2 = 0;
+#pragma unroll 1
+    for (int bit = 14; bit >= 0; --bit) {
+        const uint32_t both = (1u << bit) | (1u << (bit + 16));
+        const __half2 c2 = as_half2(v2 | both);
+        __half2 a0 = __hge2(as_half2(key[0]), c2), a1 = __hge2(as_half2(key[1]), c2);
+#pragma unroll
+        for (int j = 2; j < 16; j += 2) {
+            a0 = __hadd2(a0, __hge2(as_half2(key[j]), c2));
+            a1 = __hadd2(a1, __hge2(as_half2(key[j + 1]), c2));
+        }
+        v2 |= both & __hge2_mask(__hadd2(a0, a1), m2);  // each half accepts the bit on its own count (exact in FP16)
+    }
+    return v2;
+}
+
+// Keys of two tiles from fp16(r) of their 32 coordinates (two a word): coordinate j of the first tile in the low, of the
+// second one in the high half.
+__device__ __forceinline__ void tile_keys(const uint32_t (&r2)[16], uint32_t* key) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        key[2 * j] = __byte_perm(r2[j], r2[8 + j], 0x5410) & 0x7fff7fffu;
+        key[2 * j + 1] = __byte_perm(r2[j], r2[8 + j], 0x7632) & 0x7fff7fffu;
+    }
+}
+
+// Keep-mask of the `m` largest keys of every 16-coordinate tile, lower coordinate first among equal keys; NaN keys come
+// behind all numbers, so a tile always keeps exactly m.
 // key[16 p + j] holds coordinate 32 p + j (tile 2 p) in its LOW and 32 p + 16 + j (tile 2 p + 1) in its HIGH half;
 // keep[p] has coordinate 32 p + q at bit q (the tiled metadata word of the reference, compression.cu:126-139).
+// M of the two plans that have this layout: thresholds from a sorting network (71 and 95 packed instructions per pair of
+// tiles), false when the token has a NaN key and `keep` is not to be used; M = 0, any m: bisection (480).
 template <int M>
-__device__ __forceinline__ void select_tiles_thread(const uint32_t (&key)[64], int m, uint32_t (&keep)[4]) {
-    const __half2 m2 = __float2half2_rn(static_cast<float>(m));
+__device__ __forceinline__ bool select_tiles_thread(const uint32_t (&key)[64], int m, uint32_t (&keep)[4]) {
+    __half2 largest = __float2half2_rn(0.f);
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        // per half: the m-th largest key.  M of the two plans that have this layout: a sorting network (71 and 95 packed
-        // instructions); any other m: bisection, largest v with count(key >= v) >= m (480)
-        uint32_t v2 = 0;
-        if constexpr (M != 0) {
-            v2 = mth_of_16<M>(key + 16 * p);
-        } else {
-            for (int bit = 14; bit >= 0; --bit) {
-                const uint32_t both = (1u << bit) | (1u << (bit + 16));
-                const __half2 c2 = as_half2(v2 | both);
-                __half2 a0 = __hge2(as_half2(key[16 * p]), c2), a1 = __hge2(as_half2(key[16 * p + 1]), c2);
-#pragma unroll
-                for (int j = 2; j < 16; j += 2) {
-                    a0 = __hadd2(a0, __hge2(as_half2(key[16 * p + j]), c2));
-                    a1 = __hadd2(a1, __hge2(as_half2(key[16 * p + j + 1]), c2));
-                }
-                v2 |= both & __hge2_mask(__hadd2(a0, a1), m2);  // each half accepts the bit on its own count (exact in FP16)
-            }
-        }
-        const __half2 t2 = as_half2(v2);
+        const uint32_t* k16 = key + 16 * p;
+        uint32_t v2;  // per half: the m-th largest key
+        if constexpr (M != 0) v2 = mth_of_16<M>(k16, largest); else v2 = mth_by_bisection(k16, m);
         uint32_t ge = 0u;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) ge |= __hge2_mask(as_half2(key[16 * p + j]), t2) & ((1u << j) | (0x10000u << j));
+        for (int j = 0; j < 16; ++j) ge |= __hge2_mask(as_half2(k16[j]), as_half2(v2)) & ((1u << j) | (0x10000u << j));
         uint32_t kept = ge;
-        if (__popc(ge) != 2 * m) {  // more keys equal to a threshold than places left: the lowest coordinates stay
+        // in all, as each tile has at least m unless there are NaNs
+        if (M != 0 ? __popc(ge) != 2 * m : __popc(ge & 0xffffu) != m || __popc(ge >> 16) != m) {
             uint32_t gt = 0u;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) gt |= __hgt2_mask(as_half2(key[16 * p + j]), t2) & ((1u << j) | (0x10000u << j));
+            for (int j = 0; j < 16; ++j) gt |= __hgt2_mask(as_half2(k16[j]), as_half2(v2)) & ((1u << j) | (0x10000u << j));
             kept = gt;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                int need = m - __popc((gt >> (16 * h)) & 0xffffu);
-                uint32_t eq = (ge ^ gt) & (0xffffu << (16 * h));
-                while (eq != 0u && need > 0) {
-                    const uint32_t first = eq & (0u - eq);
-                    eq ^= first, kept |= first, --need;
+                const uint32_t half = 0xffffu << (16 * h);
+                int need = m - __popc(gt & half);
+                // more keys equal to the threshold than places left: the lowest coordinates stay; fewer than m numbers:
+                // the lowest of the NaNs as well
+#pragma unroll
+                for (int fill = 0; fill < (M != 0 ? 1 : 2); ++fill) {
+                    uint32_t from = (fill ? ~ge : ge ^ gt) & half;
+                    while (from != 0u && need > 0) {
+                        const uint32_t first = from & (0u - from);
+                        from ^= first, kept |= first, --need;
+                    }
                 }
             }
         }
         keep[p] = kept;
     }
+    return M == 0 || !(__hisnan(__low2half(largest)) || __hisnan(__high2half(largest)));
 }
 
 // Code of residual r: the quotient by the FP16 scale s, rounded and clamped.  A scale that underflowed to 0 gives what the
@@ -337,24 +364,31 @@ __global__ void __launch_bounds__(kTopkThreads, 5) encode_topk_kernel(const Enco
                     r2[4 * m] = v.x, r2[4 * m + 1] = v.y, r2[4 * m + 2] = v.z, r2[4 * m + 3] = v.w;
                     if constexpr (kFp16Rows) *reinterpret_cast<uint4*>(xrow + 64 * pc + 16 * m) = v;  // replaces the consumed x
                 }
+                if constexpr (kTiles) {
+                    tile_keys(r2, key + 16 * pc);
+                } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if constexpr (kTiles) {  // coordinate j' of tile 2 pc in the low, of tile 2 pc + 1 in the high half
-                        key[16 * pc + 2 * j] = __byte_perm(r2[j], r2[8 + j], 0x5410) & 0x7fff7fffu;
-                        key[16 * pc + 2 * j + 1] = __byte_perm(r2[j], r2[8 + j], 0x7632) & 0x7fff7fffu;
-                    } else {
-                        key[16 * pc + 2 * j] = r2[2 * j] & 0x7fff7fffu, key[16 * pc + 2 * j + 1] = r2[2 * j + 1] & 0x7fff7fffu;
-                    }
+                    for (int j = 0; j < 16; ++j) key[16 * pc + j] = r2[j] & 0x7fff7fffu;
                 }
             }
             if constexpr (kTiles) {
                 const int m = p.nnz / 8;
+                bool done = false;
                 if (MODE == TopkMode::kStructFp16)
-                    select_tiles_thread<4>(key, 4, keep);
+                    done = select_tiles_thread<4>(key, 4, keep);
                 else if (m == 8)
-                    select_tiles_thread<8>(key, 8, keep);
-                else
+                    done = select_tiles_thread<8>(key, 8, keep);
+                if (!done) {
+                    // another count, or NaNs; the keys once more from the row, so that they are not held until here
+#pragma unroll
+                    for (int pc = 0; pc < 4; ++pc) {
+                        uint32_t r2[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r2[j] = reinterpret_cast<const uint32_t*>(xrow)[16 * pc + j];
+                        tile_keys(r2, key + 16 * pc);
+                    }
                     select_tiles_thread<0>(key, m, keep);
+                }
             } else {
                 cut_largest = select_topk_thread(key, p.nnz, keep);
             }
