@@ -570,12 +570,39 @@ __device__ __forceinline__ float4 new_centre(const UmmaParams& p, int from, bool
     return c;
 }
 
+// Where the tiles of a launch are cut.  The tiles of a side's units lie end to end; they are cut where a unit ends and at
+// every multiple of `piece` tiles of the side, and a piece longer than kUChunkMax tokens into segments of that many.  A
+// segment is one set of FP32 partial sums, so the centres depend on the cuts and on nothing else: not on which CTA takes a
+// piece, and not on whether K and V share a launch.
+struct Cuts {
+    int tiles_unit, tiles_side, tiles, piece;  // tiles: of all sides
+};
+struct Segment {
+    int unit, tile0, tiles;
+};
+// First cut at or behind tile w (the end of all tiles if there is none).
+__host__ __device__ inline int cut_from(const Cuts& c, int w) {
+    if (w >= c.tiles) return c.tiles;
+    const int side = w / c.tiles_side * c.tiles_side, in_side = w - side;
+    const int by_piece = (in_side + c.piece - 1) / c.piece * c.piece, by_unit = (in_side + c.tiles_unit - 1) / c.tiles_unit * c.tiles_unit;
+    return side + (by_piece < by_unit ? by_piece : by_unit);
+}
+// The segment that starts at tile w.
+__host__ __device__ inline Segment segment_at(const Cuts& c, int w) {
+    Segment sg;
+    sg.unit = w / c.tiles_unit, sg.tile0 = w - sg.unit * c.tiles_unit;
+    const int in_unit = c.tiles_unit - sg.tile0, in_piece = c.piece - w % c.tiles_side % c.piece;
+    const int n = in_unit < in_piece ? in_unit : in_piece;
+    sg.tiles = n < kUChunkMax / kUTile ? n : kUChunkMax / kUTile;
+    return sg;
+}
+
 __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap map0,
-                                                                           const __grid_constant__ CUtensorMap map1, int share) {
+                                                                           const __grid_constant__ CUtensorMap map1, const Cuts cuts,
+                                                                           int share) {
     extern __shared__ unsigned char smem_u[];
     constexpr int kN = 64;  // rows of the centre operand: hi halves, then lo halves (K's FP32 centres; V's are FP16)
     const bool first = p.iteration == 0, last = p.iteration + 1 == p.iterations;
-    const int units = p.sides * p.units;
     let_next_launch_start();
     unsigned char* base = smem_u + ((1024u - (smem_u32(smem_u) & 1023u)) & 1023u);  // swizzled blocks: 1024-byte aligned
     unsigned char* xs = base;                                   // [stages][2 halves][128 tokens][128 B]
@@ -593,27 +620,11 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     __shared__ uint32_t tmem_base_s;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // Work of the launch = the tiles of all units laid end to end, or of each side's units (gridDim.y ranges); CTA c of a
-    // range takes [c * share, (c + 1) * share) of it and walks that segment by segment (consecutive tiles of one unit, at
-    // most kUChunkMax tokens: one set of FP32 partial sums).
+    // CTA c takes the pieces that start in [c * share, (c + 1) * share) of all tiles and walks them segment by segment.
     // Tiles are numbered q = 0, 1, ... through the CTA's whole range: stage q % 5, group / distance buffer / one-hot
     // buffer q % 3, sum accumulator q % 4, and every barrier's phase follows from q, so the ring keeps turning across
     // segment boundaries (the copies of the next segment are in flight while this one drains and flushes).
-    const int tiles_per_unit = (p.tokens + kUTile - 1) / kUTile;
-    const long long range = static_cast<long long>(units) * tiles_per_unit / gridDim.y;
-    const long long range_end = range * (blockIdx.y + 1), work_begin = range * blockIdx.y + static_cast<long long>(blockIdx.x) * share;
-    const long long work_end = work_begin + share < range_end ? work_begin + share : range_end;
-    struct Segment {
-        int unit, tile0, tiles;
-    };
-    auto segment_at = [&](long long w) {
-        Segment sg;
-        sg.unit = static_cast<int>(w / tiles_per_unit);
-        sg.tile0 = static_cast<int>(w - static_cast<long long>(sg.unit) * tiles_per_unit);
-        const long long left = work_end - w;
-        sg.tiles = min(min(tiles_per_unit - sg.tile0, kUChunkMax / kUTile), static_cast<int>(left < 1 << 20 ? left : 1 << 20));
-        return sg;
-    };
+    const int work_begin = cut_from(cuts, static_cast<int>(blockIdx.x) * share), work_end = cut_from(cuts, (static_cast<int>(blockIdx.x) + 1) * share);
     bool lost = false;
 
     if (tid == 0) {
@@ -640,8 +651,8 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
         // ---- copies, through all segments without a stop: the stage of tile q is free once the sums of tile
         // q - 5 have run (whole warp, one elected lane per tile) --------------------------------------------------
         int q = 0;
-        for (long long w = work_begin; w < work_end;) {
-            const Segment sg = segment_at(w);
+        for (int w = work_begin; w < work_end;) {
+            const Segment sg = segment_at(cuts, w);
             for (int i = 0; i < sg.tiles; ++i, ++q) {
                 if (q >= kUStages) lost |= !mbar_wait(&bar_empty[q % kUStages], (q / kUStages - 1) & 1);
                 unsigned char* dst = xs + (q % kUStages) * kUTileBytes;
@@ -663,8 +674,9 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
         wait_for_previous_launch();
         int q0 = 0;     // tiles of the earlier segments of this CTA
         int prev = -1;  // byte offset of the element this thread set in its group's one-hot buffer
-        for (long long w = work_begin; w < work_end;) {
-            const Segment sg = segment_at(w);
+        int unit_in_tables = -1;
+        for (int w = work_begin; w < work_end;) {
+            const Segment sg = segment_at(cuts, w);
             const int unit = sg.unit, n_tiles = sg.tiles;
             const int t_begin = sg.tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
             const int side = unit < p.units ? 0 : 1, local = unit - side * p.units;
@@ -672,8 +684,9 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
             const __half* xu = p.x[side] + static_cast<size_t>(local) * p.x_stride[side] * kHeadDim;
             const size_t row0 = static_cast<size_t>(unit) * p.clusters;  // first centre of the unit
             const bool opens_unit = sg.tile0 == 0;  // this CTA also keeps the unit's centres and zeroes its next sums
-            // ---- per segment: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 -------------------
-            {
+            // ---- per unit: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 ----------------------
+            if (unit != unit_in_tables) {
+                unit_in_tables = unit;
                 // four coordinates per thread and step, all loads of a thread in flight together
                 constexpr int kSteps = (32 * kHeadDim / 4 + kUWorkers - 1) / kUWorkers;
                 float4 v[kSteps];
@@ -1088,20 +1101,20 @@ void place_state(UmmaParams& p, void* workspace, size_t per) {
     for (int i = 0; i < 3; ++i, at += per * sizeof(int)) p.counts[i] = reinterpret_cast<int*>(at);
 }
 
-// Tiles per CTA of the assignment kernel.  One CTA per SM, every CTA an equal share of all units' tiles.  A CTA pays about
-// ten tile times per segment (pipeline drain, flush, new centre tables, refill), so the share is chosen - between the even
-// split and half as much again - for the shortest slowest CTA: a share that divides the units evenly often beats the
-// smallest one.  About `tries` of the shares in between are looked at (this is host time).
-long long cta_share(long long tiles_total, int tiles_unit, int least, int tries) {
-    const int seg_max = kUChunkMax / kUTile;
-    const long long even = (tiles_total + sm_count() - 1) / sm_count();
-    const long long low = even < least ? least : even, most = low + low / 2 + 1, step = low / (2 * tries) + 1;
-    long long share = low, best_cost = -1;
-    for (long long cand = low; cand <= most; cand += step) {
-        long long worst = 0;
+// Tiles per CTA of a call for one side, which is also where its tiles are cut.  One CTA per SM, every CTA an equal share of
+// all units' tiles, at least four.  A CTA pays about ten tile times per segment (pipeline drain, flush, new centre tables,
+// refill), so the share is chosen - between the even split and half as much again - for the shortest slowest CTA: a share
+// that divides the units evenly often beats the smallest one.
+int side_share(int tiles_side, int tiles_unit) {
+    constexpr int kLeast = 4, seg_max = kUChunkMax / kUTile;
+    const int even = (tiles_side + sm_count() - 1) / sm_count();
+    const int low = even < kLeast ? kLeast : even;
+    int share = low, best_cost = -1;
+    for (int cand = low; cand <= low + low / 2 + 1; ++cand) {
+        int worst = 0;
         int in_unit = tiles_unit;  // tiles left in the unit
-        for (long long left = tiles_total; left > 0;) {
-            const int work = static_cast<int>(cand < left ? cand : left);
+        for (int left = tiles_side; left > 0;) {
+            const int work = cand < left ? cand : left;
             int segments = 0;
             for (int rest = work; rest > 0; ++segments) {  // same walk as the kernel's
                 int n = in_unit < rest ? in_unit : rest;
@@ -1111,6 +1124,37 @@ long long cta_share(long long tiles_total, int tiles_unit, int least, int tries)
             }
             if (work + 10 * segments > worst) worst = work + 10 * segments;
             left -= work;
+        }
+        if (best_cost < 0 || worst < best_cost) best_cost = worst, share = cand;
+    }
+    return share;
+}
+
+// Tiles per CTA when K and V share the launches.  They are cut as a call for one side cuts them, so that ids and centres
+// are those of two such calls bit for bit; only how many of the pieces a CTA takes is chosen here, again for the shortest
+// slowest CTA.  A segment of the unit whose tables a CTA already has costs about four tile times (drain and flush: 55.2 ->
+// 57.8 us per iteration at 64 units x 8128 tokens with one per CTA).  About `kTries` shares are looked at (host time).
+int pair_share(const Cuts& c) {
+    constexpr int kNewUnit = 10, kSameUnit = 4, kTries = 16, seg_max = kUChunkMax / kUTile;
+    const int low = (c.tiles + sm_count() - 1) / sm_count();
+    int share = low, best_cost = -1;
+    for (int cand = low; cand <= low + low / 2 + 1; cand += low / (2 * kTries) + 1) {
+        int worst = 0, cost = 0, unit_of_cta = -1;
+        int unit = 0, in_unit = c.tiles_unit, in_side = c.tiles_side, in_piece = c.piece;  // tiles left
+        long long next_cta = cand;
+        for (int w = 0; w < c.tiles;) {
+            if (w >= next_cta) {
+                do next_cta += cand; while (w >= next_cta);
+                cost = 0, unit_of_cta = -1;
+            }
+            const int n = in_unit < in_piece ? in_unit : in_piece;
+            cost += n + (unit == unit_of_cta ? kSameUnit : kNewUnit) + (n - 1) / seg_max * kSameUnit;
+            unit_of_cta = unit;
+            if (cost > worst) worst = cost;
+            w += n, in_unit -= n, in_side -= n, in_piece -= n;
+            if (in_unit == 0) in_unit = c.tiles_unit, ++unit;
+            if (in_side == 0) in_side = c.tiles_side, in_piece = c.piece;
+            if (in_piece == 0) in_piece = c.piece;
         }
         if (best_cost < 0 || worst < best_cost) best_cost = worst, share = cand;
     }
@@ -1138,25 +1182,16 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
             return rc;
         prepared |= 1ull << (dev & 63);
     }
-    // A call for one side takes at least four tiles per CTA in every iteration.  K and V together take smaller shares, which
-    // are faster for short contexts (16.4 -> 9 us per iteration at 8 units x 1024 tokens), except in the last iteration: it
-    // is cut side by side as the call for one side is.  The centres that are returned are then sums of the same pieces
-    // whether the sides share launches or not; FP32 sums of other pieces differ in their last bits, enough to round some of
-    // a million FP16 coordinates differently and with them the choice between nearly equal residuals.
-    const int tiles_unit = (p.tokens + kUTile - 1) / kUTile;
-    const long long tiles_side = static_cast<long long>(p.units) * tiles_unit;
-    const bool pair = p.sides == 2;
-    long long share = pair ? cta_share(p.sides * tiles_side, tiles_unit, 1, 32) : cta_share(tiles_side, tiles_unit, 4, 1 << 30);
-    unsigned per_range = static_cast<unsigned>((p.sides * tiles_side + share - 1) / share), ranges = 1;
-    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration) {
-        if (pair && p.iteration + 1 == p.iterations) {
-            share = cta_share(tiles_side, tiles_unit, 4, 1 << 30);
-            per_range = static_cast<unsigned>((tiles_side + share - 1) / share), ranges = 2;
-        }
-        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, dim3(per_range, ranges), kUThreads, smem, s, p.iteration > 0, p,
-                                                  maps[0], maps[1], static_cast<int>(share)), "kmeans_assign launch"))
+    Cuts cuts{};
+    cuts.tiles_unit = (p.tokens + kUTile - 1) / kUTile;
+    cuts.tiles_side = p.units * cuts.tiles_unit, cuts.tiles = p.sides * cuts.tiles_side;
+    cuts.piece = side_share(cuts.tiles_side, cuts.tiles_unit);
+    const int share = p.sides == 2 ? pair_share(cuts) : cuts.piece;
+    const dim3 grid(static_cast<unsigned>((cuts.tiles + share - 1) / share));
+    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration)
+        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, grid, kUThreads, smem, s, p.iteration > 0, p, maps[0], maps[1],
+                                                  cuts, share), "kmeans_assign launch"))
             return rc;
-    }
     if (int rc = check_cuda(launch_overlapped(kmeans_final_kernel, dim3(static_cast<unsigned>((per + 7) / 8)), 256, 0, s, true, p,
                                               static_cast<__half*>(centroids0), static_cast<__half*>(centroids1)), "kmeans_final launch"))
         return rc;
