@@ -43,7 +43,7 @@ int check_device_pointer(const void* ptr, const char* who, const char* what) {
 }
 
 int sm_count() {
-    static int cached[64] = {0};
+    static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
     if (cached[dev] == 0) {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -30,6 +31,20 @@ int check_device_pointer(const void* ptr, const char* who, const char* what);
 
 // Number of SMs of the current device (cached per device).
 int sm_count();
+
+// cudaFuncSetAttribute(max dynamic shared memory) once per kernel instance and device, not per call.  `done` is a bit mask
+// over device ordinals (< 64), one per instance; two host threads at once only repeat the idempotent call.
+template <class Kernel>
+int allow_smem(Kernel kern, size_t smem, std::atomic<unsigned long long>& done, const char* what) {
+    int dev = 0;
+    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
+    const bool tracked = dev >= 0 && dev < 64;
+    if (tracked && (done.load() >> dev & 1ull)) return RESKV_OK;
+    if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), what))
+        return rc;
+    if (tracked) done.fetch_or(1ull << dev);
+    return RESKV_OK;
+}
 
 // ---- device side: async bulk copies (TMA, 1-D) and mbarriers -------------------
 // All waits are bounded: a wait that runs out records RESKV_STATUS_WAIT_TIMEOUT in

@@ -561,16 +561,9 @@ size_t topk_smem_bytes(int clusters) {
 template <TopkMode MODE>
 int launch_topk(const EncodeParams& p, cudaStream_t stream, const char* what) {
     auto kern = encode_topk_kernel<MODE>;
-    // the kernel's shared memory grows with the centroid count: allow the maximum once per device
-    static unsigned long long allowed = 0;
-    int dev = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
-    if (dev < 0 || dev >= 64 || !(allowed >> dev & 1ull)) {
-        if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(topk_smem_bytes(kMaxClusters))), what))
-            return rc;
-        if (dev >= 0 && dev < 64) allowed |= 1ull << dev;
-    }
+    static std::atomic<unsigned long long> done{0};
+    // for the largest centroid table
+    if (int rc = allow_smem(kern, topk_smem_bytes(kMaxClusters), done, what)) return rc;
     const long long chunks = static_cast<long long>(p.units) * ((p.tokens + kChunkTokens - 1) / kChunkTokens);
     const long long cap = static_cast<long long>(sm_count()) * 5;
     const int grid = static_cast<int>(chunks < cap ? chunks : cap);

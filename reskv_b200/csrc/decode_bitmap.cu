@@ -433,7 +433,7 @@ int launch_simt_cvs(const DecodeParams& p, int units, cudaStream_t stream) {
     if (smem < red_bytes) smem = red_bytes;
     auto kern = decode_simt_partial_kernel<GQA, L, CVS>;
     // the kernel's shared memory grows with the key centroid count: allow the maximum once
-    static unsigned long long done = 0;
+    static std::atomic<unsigned long long> done{0};
     const size_t smem_max = sizeof(Stage<L>) * kStages + static_cast<size_t>(kMaxClusters) * kHeadDim * sizeof(__half);
     if (int rc = allow_smem(kern, smem_max > red_bytes ? smem_max : red_bytes, done, "cudaFuncSetAttribute(decode_simt_partial)"))
         return rc;
@@ -451,7 +451,7 @@ int launch_partial_mma_beta(const DecodeParams& p, cudaStream_t stream) {
     using ML = mma::LayoutMmaBitmap<NNZ>;
     const size_t smem = mma::Smem<GQA, ML>::bytes(p.ck);
     auto kern = mma::decode_mma_kernel<GQA, ML, BETA>;
-    static unsigned long long done = 0;
+    static std::atomic<unsigned long long> done{0};
     if (int rc = allow_smem(kern, mma::Smem<GQA, ML>::bytes(kMaxClusters), done, "cudaFuncSetAttribute(decode_bitmap_mma)"))
         return rc;
     return check_cuda(launch_overlapped(kern, dim3(p.grid), mma::kThreadsM, smem, stream, true, p), "decode_bitmap_mma launch");
@@ -888,11 +888,11 @@ namespace {
 // Device address of g_noalloc_scratch on the current device.  In host code the
 // array's name is only a handle for the runtime, not something a kernel can
 // dereference, so the address is looked up once per device (with that device
-// current) and remembered.  The remembered value is written without a lock: two
+// current) and remembered.  No lock: two
 // host threads that make their first call on a device together both look the
 // address up and store the same value.
 int noalloc_scratch_address(void** out) {
-    static void* cached[64] = {nullptr};
+    static std::atomic<void*> cached[64];
     int dev = 0;
     if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
     if (dev < 0 || dev >= 64) return fail(RESKV_ERR_LIMIT, "decode_bitmap_fp16_noalloc: device index %d not supported", dev);

@@ -146,20 +146,5 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// cudaFuncSetAttribute(max dynamic shared memory) once per kernel instance and device, not per call.
-// `done` is a per-instantiation bit mask over device ordinals (< 64); a race between host threads only
-// repeats the idempotent call.
-template <class Kernel>
-int allow_smem(Kernel kern, size_t smem, unsigned long long& done, const char* what) {
-    int dev = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
-    const bool tracked = dev >= 0 && dev < 64;
-    if (tracked && (done >> dev & 1ull)) return RESKV_OK;
-    if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), what))
-        return rc;
-    if (tracked) done |= 1ull << dev;
-    return RESKV_OK;
-}
-
 }  // namespace
 }  // namespace reskv

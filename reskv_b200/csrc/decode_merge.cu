@@ -292,7 +292,7 @@ int launch(const MergeParams& mp, int units, int heads, int recent_max, cudaStre
     const int cv = mp.splits > 0 ? mp.cv : 0;
     const size_t smem = merge_smem_bytes<G>(cv);
     if (smem > 48 * 1024) {
-        static unsigned long long done = 0;
+        static std::atomic<unsigned long long> done{0};
         if (int rc = allow_smem(decode_merge_kernel<G>, merge_smem_bytes<G>(kMaxClusters), done, "cudaFuncSetAttribute(decode_merge)"))
             return rc;
     }

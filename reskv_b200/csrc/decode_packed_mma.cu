@@ -11,17 +11,9 @@ template <int GQA, class ML, int BETA>
 int launch_beta(const DecodeParams& p, cudaStream_t stream) {
     const size_t smem = mma::Smem<GQA, ML>::bytes(p.ck);
     auto kern = mma::decode_mma_kernel<GQA, ML, BETA>;
-    // allowed once per kernel instance and device (bit mask over device ordinals), for the largest centroid table
-    static unsigned long long done = 0;
-    int dev = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return rc;
-    if (dev < 0 || dev >= 64 || !(done >> dev & 1ull)) {
-        if (int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(mma::Smem<GQA, ML>::bytes(kMaxClusters))),
-                                "cudaFuncSetAttribute(decode_mma packed)"))
-            return rc;
-        if (dev >= 0 && dev < 64) done |= 1ull << dev;
-    }
+    static std::atomic<unsigned long long> done{0};
+    // for the largest centroid table
+    if (int rc = allow_smem(kern, mma::Smem<GQA, ML>::bytes(kMaxClusters), done, "cudaFuncSetAttribute(decode_mma packed)")) return rc;
     return check_cuda(launch_overlapped(kern, dim3(p.grid), mma::kThreadsM, smem, stream, true, p), "decode_mma (packed layout) launch");
 }
 

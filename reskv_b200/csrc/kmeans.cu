@@ -1172,16 +1172,8 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     constexpr int kN = 64;
     const size_t smem = 1024 + static_cast<size_t>(kUStages) * kUTileBytes + 2 * kN * 128 + kUGroups * kUOneHotBytes +
                         32 * kHeadDim * sizeof(float) + 32 * (sizeof(float) + sizeof(int));
-    static unsigned long long prepared = 0;  // per-device bit: the shared-memory attribute is set
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!((prepared >> (dev & 63)) & 1ull)) {
-        if (int rc = check_cuda(cudaFuncSetAttribute(kmeans_assign_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(smem)),
-                                "cudaFuncSetAttribute(kmeans_assign_umma)"))
-            return rc;
-        prepared |= 1ull << (dev & 63);
-    }
+    static std::atomic<unsigned long long> done{0};
+    if (int rc = allow_smem(kmeans_assign_umma_kernel, smem, done, "cudaFuncSetAttribute(kmeans_assign_umma)")) return rc;
     Cuts cuts{};
     cuts.tiles_unit = (p.tokens + kUTile - 1) / kUTile;
     cuts.tiles_side = p.units * cuts.tiles_unit, cuts.tiles = p.sides * cuts.tiles_side;
