@@ -1,0 +1,75 @@
+"""The native host calls let other Python threads run: a launch that waits because the stream's queue is full, and a verdict
+that is dropped while its kernel is still queued, hold no interpreter lock."""
+
+import threading
+import time
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BUSY_CYCLES = 1_500_000_000  # 0.8 s of a spinning kernel at 1.9 GHz
+
+
+class Pulse(threading.Thread):
+    """Longest time between two turns of a thread that only sleeps."""
+
+    def __init__(self):
+        super().__init__()
+        self.done, self.gap = threading.Event(), 0.0
+
+    def run(self):
+        last = time.perf_counter()
+        while not self.done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            self.gap, last = max(self.gap, now - last), now
+
+
+def _longest_gap(work):
+    """(longest gap of another thread, duration) while ``work`` runs behind a busy stream."""
+    torch.cuda.synchronize()
+    pulse = Pulse()
+    pulse.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(BUSY_CYCLES)
+    try:
+        work()
+        took = time.perf_counter() - start
+    finally:
+        pulse.done.set()
+        pulse.join()
+        torch.cuda.synchronize()
+    return pulse.gap, took
+
+
+def test_a_launch_that_waits_lets_other_threads_run():
+    from reskv_b200 import ResKVKernelConfig, attention, compress
+    from reskv_b200.synthetic import gaussian, mixture
+
+    cache = compress(mixture(1, 2, 200, seed=1, device=DEV), mixture(1, 2, 200, seed=2, device=DEV),
+                     ResKVKernelConfig(num_clusters=8, kmeans_iterations=2))
+    q = gaussian(1, 8, 1, 128, seed=3, device=DEV)
+    attention(q, cache, position=200)
+    gap, took = _longest_gap(lambda: [attention(q, cache, position=200) for _ in range(2000)])  # 4000 launches
+    assert took > 0.3, "the queue never filled"
+    assert gap < 0.2
+
+
+def test_a_dropped_verdict_lets_other_threads_run():
+    from reskv_b200._extension import load_extension
+
+    ids = torch.zeros((1, 2, 64), dtype=torch.int32, device=DEV)
+    ops = load_extension("compression")
+
+    def drop_twice():
+        for _ in range(2):
+            ticket = ops.take_ids(ids, ids, 4, 4)
+            del ticket
+
+    drop_twice()
+    gap, _ = _longest_gap(drop_twice)
+    assert gap < 0.2
+    assert ops.take_ids(ids, ids, 4, 4)[2]()
+    assert not ops.take_ids(ids + 4, ids, 4, 4)[2]()
