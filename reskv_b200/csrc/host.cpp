@@ -641,54 +641,69 @@ PyObject* py_window_shift(PyObject*, PyObject* const* o, Py_ssize_t n) {
 }
 
 // ---- verdicts of take_ids -------------------------------------------------------------------------------------------
-// A word of mapped pinned host memory and an event per call in flight; a few are kept for later calls (any thread, any
-// device: the event is made for the call's device).
+// A word of mapped pinned host memory and an event per call in flight (the event is made for the call's device).  They are
+// kept for later calls of any thread, about kKeptVerdicts of them.  A ticket may be dropped by a finaliser, at any time and
+// inside a stream capture too, so dropping one makes no CUDA call: the slot goes back as it is, is taken again only once its
+// event is over, and surplus slots are freed by the calls that take one.
 struct Verdict {
     volatile uint32_t* word;
     cudaEvent_t event;
     c10::DeviceIndex device;
+    std::atomic<bool> seen{false};  // the event of its last call is known to be over
 };
 constexpr size_t kKeptVerdicts = 16;
 std::mutex g_verdict_lock;
 std::vector<Verdict*> g_verdicts;
 
+bool is_over(Verdict* v) {
+    if (v->seen) return true;
+    const cudaError_t e = cudaEventQuery(v->event);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+
 Verdict* get_verdict(c10::DeviceIndex device) {
+    Verdict* found = nullptr;
+    std::vector<Verdict*> surplus;
     {
         const std::lock_guard<std::mutex> lock(g_verdict_lock);
-        for (size_t i = 0; i < g_verdicts.size(); ++i) {
-            if (g_verdicts[i]->device != device) continue;
+        for (size_t i = 0; i < g_verdicts.size();) {
             Verdict* v = g_verdicts[i];
-            g_verdicts.erase(g_verdicts.begin() + static_cast<long>(i));
-            return v;
+            const bool take = !found && v->device == device, free = g_verdicts.size() > kKeptVerdicts;
+            if ((take || free) && is_over(v)) {
+                if (take) found = v; else surplus.push_back(v);
+                g_verdicts[i] = g_verdicts.back();
+                g_verdicts.pop_back();
+            } else {
+                ++i;
+            }
         }
     }
-    void* word = nullptr;
-    cudaEvent_t event = nullptr;
-    check_cuda(cudaHostAlloc(&word, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
-    check_cuda(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreate");
-    return new Verdict{static_cast<volatile uint32_t*>(word), event, device};
+    for (Verdict* v : surplus) {
+        cudaEventDestroy(v->event);
+        cudaFreeHost(const_cast<uint32_t*>(v->word));
+        delete v;
+    }
+    if (!found) {
+        void* word = nullptr;
+        cudaEvent_t event = nullptr;
+        check_cuda(cudaHostAlloc(&word, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+        check_cuda(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreate");
+        found = new Verdict{static_cast<volatile uint32_t*>(word), event, device};
+    }
+    found->seen = false;
+    return found;
 }
 
-void put_verdict(Verdict* v) {
-    {
+void put_verdict(Verdict* v) noexcept {
+    try {
         const std::lock_guard<std::mutex> lock(g_verdict_lock);
-        if (g_verdicts.size() < kKeptVerdicts) {
-            g_verdicts.push_back(v);
-            return;
-        }
+        g_verdicts.push_back(v);
+    } catch (...) {  // no memory for the list: the slot is lost
     }
-    cudaEventDestroy(v->event);
-    cudaFreeHost(const_cast<uint32_t*>(v->word));
-    delete v;
 }
 
-void drop_ticket(PyObject* capsule) {  // a call that never asked for its verdict: wait for it, then keep the slot
-    auto* v = static_cast<Verdict*>(PyCapsule_GetPointer(capsule, "reskv verdict"));
-    Py_BEGIN_ALLOW_THREADS;
-    cudaEventSynchronize(v->event);
-    put_verdict(v);
-    Py_END_ALLOW_THREADS;
-}
+void drop_ticket(PyObject* capsule) { put_verdict(static_cast<Verdict*>(PyCapsule_GetPointer(capsule, "reskv verdict"))); }
 
 // take_ids(k_ids, v_ids, k_clusters, v_clusters) -> (int32 ids [2,...], k int8 ids, v int8 ids, ticket)
 PyObject* py_take_ids(PyObject*, PyObject* const* o, Py_ssize_t n) {
@@ -719,17 +734,21 @@ PyObject* py_take_ids(PyObject*, PyObject* const* o, Py_ssize_t n) {
                 rc = reskv_take_ids(k.const_data_ptr(), v.const_data_ptr(), static_cast<int>(k.element_size()), static_cast<int>(v.element_size()),
                                     k.numel(), clusters_k, clusters_v, static_cast<int32_t*>(wide.data_ptr()), narrow_k.data_ptr(),
                                     narrow_v.data_ptr(), static_cast<uint32_t*>(word), stream);
-            cudaEventRecord(verdict->event, stream);
-            if (mapped != cudaSuccess || rc < 0) {
-                cudaEventSynchronize(verdict->event);
+            const cudaError_t recorded = cudaEventRecord(verdict->event, stream);
+            if (recorded != cudaSuccess) cudaStreamSynchronize(stream);  // nothing else tells when the word is written
+            if (mapped != cudaSuccess || rc < 0 || recorded != cudaSuccess) {
                 put_verdict(verdict);
                 check_cuda(mapped, "cudaHostGetDevicePointer");
                 check(rc);
+                check_cuda(recorded, "cudaEventRecord");
             }
             ++g_launches;
         }
         PyObject* ticket = PyCapsule_New(verdict, "reskv verdict", drop_ticket);
-        if (!ticket) throw PyError{};
+        if (!ticket) {
+            put_verdict(verdict);
+            throw PyError{};
+        }
         PyObject* t = PyTuple_New(4);
         PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(wide));
         PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(narrow_k));
@@ -749,6 +768,7 @@ PyObject* py_ids_in_range(PyObject*, PyObject* ticket) {
         e = cudaEventSynchronize(v->event);
         Py_END_ALLOW_THREADS;
         check_cuda(e, "cudaEventSynchronize");
+        v->seen = true;
         return PyBool_FromLong(*v->word == 0);
     });
 }
