@@ -20,6 +20,8 @@ compressed cache goes through ``reskv_b200.compress`` / ``attention``.
 
 from __future__ import annotations
 
+import contextlib
+import gc
 import threading
 from dataclasses import dataclass
 
@@ -63,6 +65,31 @@ def _rope(x, cos, sin):
     return torch.cat((a * cos - b * sin, b * cos + a * sin), dim=-1).to(x.dtype)
 
 
+class _CollectorHold:
+    """Keeps Python's cyclic collector from running while any thread is inside: a finaliser that it ran in a stream capture
+    (of another graph, an event, a device buffer) could call CUDA there and spoil the capture.  A collection before the
+    capture would not rule that out and takes longer than the capture."""
+
+    def __init__(self):
+        self._lock, self._inside, self._was_on = threading.Lock(), 0, False
+
+    @contextlib.contextmanager
+    def __call__(self):
+        with self._lock:
+            if self._inside == 0:
+                self._was_on = gc.isenabled()
+                gc.disable()
+            self._inside += 1
+        try:
+            yield
+        finally:
+            with self._lock:
+                self._inside -= 1
+                if self._inside == 0 and self._was_on:
+                    gc.enable()
+
+
+_collector_held = _CollectorHold()
 _streams = threading.local()
 
 
@@ -444,11 +471,12 @@ class ResKVLlama:
                     counts.copy_(saved)
                 self._warm.add(self._tok_in.shape[0])
             graph = torch.cuda.CUDAGraph()
-            graph.capture_begin(pool=None if self._last_graph is None else self._last_graph.pool())
-            try:
-                self._logits_out = self._step_body(self._tok_in)
-            finally:
-                graph.capture_end()
+            with _collector_held():
+                graph.capture_begin(pool=None if self._last_graph is None else self._last_graph.pool())
+                try:
+                    self._logits_out = self._step_body(self._tok_in)
+                finally:
+                    graph.capture_end()
         main.wait_stream(side)
         self._graph = self._last_graph = graph
 
