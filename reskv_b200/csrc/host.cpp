@@ -459,7 +459,7 @@ PyObject* py_kmeans_pair(PyObject*, PyObject* const* o, Py_ssize_t n) {
             value_error("kmeans_pair expects FP16 K and V [B,H,T,128], dense or token slices of dense buffers");
         const int64_t b = k.size(0), h = k.size(1), t = k.size(2);
         const int bi = static_cast<int>(b), hi = static_cast<int>(h), ci = static_cast<int>(count);
-        if (count < 1 || count > 64) value_error("kmeans_pair: cluster count must be in [1,32] and at most the token count");
+        if (count < 1 || count > 32 || count > t) value_error("kmeans_pair: cluster count must be in [1,32] and at most the token count");
         at::Tensor part[2][3];
         {
             const Unlocked free;
