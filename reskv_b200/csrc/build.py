@@ -71,15 +71,33 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objs = [objdir / (s.stem + ".o") for s in sources()]
     if force or jobs or _stale(LIB, objs):
         run([nvcc, *ARCH_FLAGS, "-shared", "-Xlinker=-soname=libreskv_b200.so", "-o", str(LIB), *map(str, objs), "-lcudart"])
-    if force or _stale(HOST, [HERE / "host.cpp", headers[-1]]):
-        run(_host_command(nvcc))
+    command, record = _host_command(nvcc), objdir / "_host.txt"
+    if force or _host_stale([HERE / "host.cpp", headers[-1]], command, record):
+        run(command)
+        record.write_text(_host_record(command))
     return LIB
 
 
+def _host_record(command: list[str]) -> str:
+    """What ``_host.so`` depends on besides its sources: the command line (interpreter and torch by path) and torch's
+    version, whose internal headers it compiles against."""
+    version = _torch_dir() / "version.py"
+    return " ".join(command) + "\n" + (version.read_text() if version.exists() else "")
+
+
+def _host_stale(deps: list[Path], command: list[str], record: Path) -> bool:
+    return _stale(HOST, deps) or not record.exists() or record.read_text() != _host_record(command)
+
+
+def _torch_dir() -> Path:
+    """torch is only located, not imported: its headers and libraries sit in the package, and at run time they are already
+    loaded."""
+    return Path(importlib.util.find_spec("torch").origin).parent
+
+
 def _host_command(nvcc: str) -> list[str]:
-    """g++ for the tensor-facing module.  torch is only located, not imported: its headers and libraries sit in the
-    package, and at run time they are already loaded."""
-    torch = Path(importlib.util.find_spec("torch").origin).parent
+    """g++ for the tensor-facing module."""
+    torch = _torch_dir()
     cuda = Path(nvcc).resolve().parent.parent
     includes = [torch / "include", torch / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
     libs = ["c10", "c10_cuda", "torch_cpu", "torch_cuda", "torch_python"]
