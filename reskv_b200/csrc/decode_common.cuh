@@ -109,9 +109,15 @@ struct PartialSchedule {
 };
 
 // Either an even share of everything (n_pad = the unit's granules; a CTA may then end one unit and start the next), or
-// ctas / units equal pieces of every unit, whichever has the shorter slowest CTA.  Times in cycles, measured: a pass of
-// 16 rows on each of 4, 8, 12 or 16 warps 4500, 5700, 6800 or 8000; a further segment in a CTA (centroids, query,
-// combining, writing) 5000.
+// ctas / units equal pieces of every unit, whichever has the shorter slowest CTA.  In cycles: a pass of 16 rows on each of
+// 4, 8, 12 or 16 warps 4500, 5700, 6800 or 8000, a further segment in a CTA 11500 (centroids, query, combining, writing,
+// and that two segments leave two passes unfilled).
+//
+// Measured with 144 units, one CTA each, up to 32 granules: a full pass takes 6200 (INT2), 6400 (INT4), 7500 (32 of 128 in
+// a bitmap), 8100 (4:16), 8800 (64 of 128) with four query heads per KV head, 8100 and 7700 (32 of 128, 1-of-4 INT4) with
+// eight; a last pass on 4 or 8 warps 3200 to 5000 and 2000 to 3600 less.  One set of figures serves all: with five of these
+// forms, batch 1 to 16 and 192 to 16320 tokens, what it picks is within 1.5 % of the better of both (mean 0.05 %; with 5000
+// for a further segment up to 15 %, batch 16 at 1100 tokens 32.2 instead of 28.5 us).
 __host__ __device__ inline long long segment_cycles(long long granules) {
     constexpr int kPass = 8;  // granules per pass: 256 tokens
     const long long rest = granules % kPass;
@@ -126,7 +132,7 @@ __host__ __device__ inline PartialSchedule partial_schedule(int units, int granu
         int piece = (granules + pieces - 1) / pieces;
         if (piece < kMinChunk) piece = kMinChunk;
         const bool crosses = granules % even != 0;
-        if (segment_cycles(piece) <= segment_cycles(even) + (crosses ? 5000 : 0))
+        if (segment_cycles(piece) <= segment_cycles(even) + (crosses ? 11500 : 0))
             s.chunk = piece, s.n_pad = (granules + piece - 1) / piece * piece;
     }
     return s;
