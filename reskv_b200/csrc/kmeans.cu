@@ -908,14 +908,14 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                 }
             }
             // ---- end of the segment: its sums go out (the commit of the last sum MMAs covers all of them) -----------
+            // The wait stands behind the barrier: a parity tells two neighbouring phases apart, and only once the last tile's
+            // group has come this far is the phase before the awaited one over for sure.
             const bool flusher = warp < 2 * kUGroupWarps;  // groups 0 and 1: coordinate row_in_tile, sixteen clusters each
+            workers_sync();
             if (flusher) {
                 const int q_last = q0 + n_tiles - 1;
                 lost |= !mbar_wait(&bar_sums[q_last % kUGroups], (q_last / kUGroups) & 1);
                 tc_fence_after();
-            }
-            workers_sync();
-            if (flusher) {
                 const int half = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
                 const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
                 long long* sums_g = p.sums[p.iteration % 3] + row0 * kHeadDim;
