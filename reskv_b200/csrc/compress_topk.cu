@@ -18,11 +18,11 @@
 //     at every step) and the warp writes the 32 rows out with 16-byte stores.
 //
 // The tiled layouts take their thresholds from a sorting network, two tiles at a time in the two halves of the packed
-// operations; the 1-of-4 layout compares four keys per group.
+// operations, and look for NaNs beside it (1 % of the time); the 1-of-4 layout compares four keys per group.
 //
 // What bounds it: the integer pipe, then the time a warp waits for its rows.  Microseconds per side of 64 units x 8128
 // tokens (133 MB of x), and what the same layouts took with FP32 keys, a bisection of both halves apart and a compaction
-// loop: bitmap 87 for 32 and 90 for 64 of 128 values (112, 126), INT4 110 (128), INT2 110 (126), tiled 67 (91), 4:16 53
+// loop: bitmap 87 for 32 and 90 for 64 of 128 values (112, 126), INT4 110 (128), INT2 110 (126), tiled 67 (91), 4:16 52
 // (73), 1-of-4 INT4 48 (79), compact INT4 127 to 138 (320).
 //
 // Rounding points are those of compress.cu (they decide bit-exactness): selection key |fp16(r)|, FP16 layouts

@@ -33,8 +33,9 @@
 //  * Rotations are packed FP32 pairs (fma.rn.f32x2), quantised codes are decoded two at a time by one AND-XOR and one
 //    HFMA2.
 //
-// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.222 ms, 71 % of the issue slots, 73 % of the
-// shared-memory pipe, 55 % of the integer pipe; 82 instructions and 22 shared-memory wavefronts per token and KV head.
+// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.222 ms; of active cycles 72 % of the issue slots,
+// 76 % of the shared-memory pipe, 53 % of the integer pipe; 83 instructions and 21 shared-memory wavefronts per token and
+// KV head (64 kept: 91 and 29, INT4: 68 and 11.5).
 // Before (two CTAs of four warps, sin/cos and accumulators in registers): 0.280 ms.  INT4, batch 8, 16320 tokens: 0.128
 // -> 0.102 ms.  A 128-token call costs ~9 us, most of it the set-up (tables, centroids, first query) and one pass.
 //
