@@ -74,3 +74,40 @@ def test_a_dropped_verdict_lets_other_threads_run_and_does_not_wait():
     for _ in range(20):
         assert ops.take_ids(ids, ids, 4, 4)[2]()
     assert not ops.take_ids(ids + 4, ids, 4, 4)[2]()
+
+
+def test_calls_of_several_threads_give_the_bits_of_calls_in_turn():
+    from reskv_b200 import ResKVKernelConfig, attention, compress
+    from reskv_b200.cache import ResKVLayerCache
+    from reskv_b200.compression import cluster
+    from reskv_b200.synthetic import gaussian, mixture
+
+    cfg = ResKVKernelConfig(sparsity=0.75, num_clusters=8, kmeans_iterations=2, max_clusters=16)
+
+    def request(seed):
+        key, value = (mixture(1, 2, 300, seed=seed + i, device=DEV) for i in (0, 1))
+        given = compress(key, value, cfg, clustering=(cluster(key, 8, 2), cluster(value, 8, 2, value=True)))
+        layer, out = ResKVLayerCache(cfg, 0), []
+        layer.update(key, value, {"raw_keys": key})
+        for step in range(80):  # a decode group is compressed on the way
+            token, q = gaussian(1, 2, 1, 128, seed=seed + step, device=DEV), gaussian(1, 8, 1, 128, seed=step, device=DEV)
+            position = layer.length
+            keys, values = layer.update(token, token, {"raw_keys": token})
+            out.append(attention(q, layer.compressed, position=position, recent=(q, keys, values)))
+        return torch.cat([*out, attention(q, given, position=300)])
+
+    want = [request(100 * i) for i in range(6)]
+    got = [None] * 6
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[i] = request(100 * i)
+            torch.cuda.current_stream().synchronize()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(g is not None and torch.equal(g, w) for g, w in zip(got, want))
