@@ -1113,7 +1113,7 @@ int side_share(int tiles_side, int tiles_unit) {
     for (int cand = low; cand <= low + low / 2 + 1; ++cand) {
         int worst = 0;
         int in_unit = tiles_unit;  // tiles left in the unit
-        for (int left = tiles_side; left > 0;) {
+        for (int left = tiles_side; left > 0 && (best_cost < 0 || worst < best_cost);) {
             const int work = cand < left ? cand : left;
             int segments = 0;
             for (int rest = work; rest > 0; ++segments) {  // same walk as the kernel's
@@ -1142,7 +1142,7 @@ int pair_share(const Cuts& c) {
         int worst = 0, cost = 0, unit_of_cta = -1;
         int unit = 0, in_unit = c.tiles_unit, in_side = c.tiles_side, in_piece = c.piece;  // tiles left
         long long next_cta = cand;
-        for (int w = 0; w < c.tiles;) {
+        for (int w = 0; w < c.tiles && (best_cost < 0 || worst < best_cost);) {
             if (w >= next_cta) {
                 do next_cta += cand; while (w >= next_cta);
                 cost = 0, unit_of_cta = -1;
