@@ -11,6 +11,15 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&r)[4]) {
+    uint32_t u[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = __uint_as_float(u[i]);
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&r)[8]) {
     uint32_t u[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -79,6 +88,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&r)[16]) {
 }
 
 // The same, tying the loaded registers to the wait (nothing that reads them can move in front of it).
+__device__ __forceinline__ void tmem_ld_wait(float (&r)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3])::"memory");
+}
 __device__ __forceinline__ void tmem_ld_wait(float (&r)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]),
                  "+f"(r[5]), "+f"(r[6]), "+f"(r[7])::"memory");
