@@ -17,7 +17,7 @@
 //    registers kept two per scheduler and issued on 58 % of the cycles.)
 //  * What makes 128 registers enough: the accumulators and the 32 sin/cos values of a lane live in tensor memory, whose
 //    loads and stores do not touch the shared-memory pipe (the other busy unit): a k-step's eight sin/cos values are
-//    loaded while its residuals are walked, the accumulators for the value phase only.  And the two tokens of a lane have
+//    loaded while its residuals are walked, the accumulators for the value phase only, half of them at a time.  And the two tokens of a lane have
 //    the *same* offset j = 8 warp + g inside two sub-tiles X and Y of (up to) 128 tokens, so one set of 16 (cos, sin)
 //    values rotates both.  RoPE: a token at offset j of a sub-tile starting at position P0 scores < R(pos_q) q, R(P0 + j) k > = < R(pos_q - P0) q, R(j) k >; the query is
 //    rotated once per sub-tile, and the eight columns of the score MMA hold X's heads (0..3) next to Y's (4..7).  Rows
@@ -33,11 +33,17 @@
 //  * Rotations are packed FP32 pairs (fma.rn.f32x2), quantised codes are decoded two at a time by one AND-XOR and one
 //    HFMA2.
 //
-// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.222 ms; of active cycles 72 % of the issue slots,
-// 76 % of the shared-memory pipe, 53 % of the integer pipe; 83 instructions and 21 shared-memory wavefronts per token and
-// KV head (64 kept: 91 and 29, INT4: 68 and 11.5).
+// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.219 ms; of active cycles 69 % of the issue slots,
+// 76 % of the shared-memory pipe, 47 % of the integer pipe; 78 instructions and 21 shared-memory wavefronts per token and
+// KV head.  Neither unit is full: four warps per scheduler do not cover the latencies of a pass, so a shorter instruction
+// stream alone gives little.  The fields' walks in groups of four, half of the accumulators in registers at a time and the
+// maximum taken across lanes only where it grows: 83 -> 78 instructions, calls with their merge, us: batch 32 228 -> 224.6,
+// batch 8, 16320 tokens INT4 105.5 -> 102, batch 16, 8128 tokens INT2 105 -> 100, 64 of 128 kept 139.6 -> 136.4.
+// Tried and slower (same call, from 224): the rotated query in tensor memory, 19 wavefronts fewer per pass and 47
+// instructions more, 232; 20 warps at 96 registers 239; a fused multiply-add for the rotation's subtraction 228; the
+// k-steps or the halves as loops 226 to 232.
 // Before (two CTAs of four warps, sin/cos and accumulators in registers): 0.280 ms.  INT4, batch 8, 16320 tokens: 0.128
-// -> 0.102 ms.  A 128-token call costs ~9 us, most of it the set-up (tables, centroids, first query) and one pass.
+// -> 0.100 ms.  A 128-token call costs ~9 us, most of it the set-up (tables, centroids, first query) and one pass.
 //
 // Softmax keeps a lazily updated running maximum per column (rescale only when it grows by more than 2^8), P is rounded
 // to FP16 once and that rounded value is used for the sum, the cluster masses and the PV product alike.  The cluster
@@ -201,15 +207,15 @@ __device__ __forceinline__ uint32_t high_halves(uint32_t a, uint32_t b) { return
 // ---- fields: the 16 coordinates [16 f, 16 f + 16) of one token, as a lane consumes them --------
 // keys:   order(i) = which four coordinates [4 ks, 4 ks + 4) come i-th; add4(ks, k, scale): k[e] += residual of
 //         coordinate 4 ks + e (k holds the FP32 centroid), called in that order.
-// values: block(i, f0..f3, a): A operand of value MMA i for the tokens of f0, f1 (k columns 2q, 2q + 1) and f2, f3
-//         (2q + 8, 2q + 9): coordinate first(i) in the rows g (a[0], a[2]), coordinate second(i) in the rows g + 8
-//         (a[1], a[3]); called for i = 0..7 in order.
+// values: half_block(half, f0..f3, a): A operands of the value MMAs i = 4 half .. 4 half + 3 for the tokens of f0, f1
+//         (k columns 2q, 2q + 1) and f2, f3 (2q + 8, 2q + 9): coordinate first(i) in the rows g (a[0], a[2]), coordinate
+//         second(i) in the rows g + 8 (a[1], a[3]); called for half = 0, then 1.
 // `meta` and `pay` point at the token's own rows, `pre` at its eight rank bases.
 
 // Sparse FP16 layouts: a 16-bit keep mask (bit 15 = first coordinate) and a pointer to the
 // field's first retained value; retained values are consecutive in the payload row.
 struct WalkField {
-    static constexpr bool kSlotwise = true;  // offers add1: callers interleave the walks of several fields
+    static constexpr bool kSlotwise = true;  // offers add1, a single coordinate
     uint32_t mask;
     const __half* ptr;
     __device__ static constexpr int order(int i) { return i; }
@@ -221,22 +227,38 @@ struct WalkField {
             ++ptr;
         }
     }
-    // the coordinate's FP16 bits, 0 when it was dropped, of two tokens
-    __device__ static __forceinline__ uint32_t pair(WalkField& lo, WalkField& hi, int slot) {
-        uint32_t v = 0;
-        if (lo.mask & (0x8000u >> slot)) {
-            v = *reinterpret_cast<const unsigned short*>(lo.ptr);
-            ++lo.ptr;
+    // FP16 bits of the coordinates [s0, s0 + 4) of two tokens (low and high half), 0 where dropped.  One field's four steps
+    // follow one another, so that the compiler tests its mask bits together: 3.2 instructions per coordinate instead of
+    // 3.8 with the two fields in turn (eight at a time: fewer still, but slower, the registers are short).
+    __device__ static __forceinline__ void pairs(WalkField& lo, WalkField& hi, int s0, uint32_t (&v)[4]) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            v[e] = 0;
+            if (lo.mask & (0x8000u >> (s0 + e))) {
+                v[e] = *reinterpret_cast<const unsigned short*>(lo.ptr);
+                ++lo.ptr;
+            }
         }
-        if (hi.mask & (0x8000u >> slot)) {
-            v = low_halves(v, *reinterpret_cast<const unsigned short*>(hi.ptr));
-            ++hi.ptr;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (hi.mask & (0x8000u >> (s0 + e))) {
+                v[e] = low_halves(v[e], *reinterpret_cast<const unsigned short*>(hi.ptr));
+                ++hi.ptr;
+            }
         }
-        return v;
     }
-    __device__ static __forceinline__ void block(int i, WalkField& f0, WalkField& f1, WalkField& f2, WalkField& f3, uint32_t (&a)[4]) {
-        a[0] = pair(f0, f1, 2 * i), a[2] = pair(f2, f3, 2 * i);
-        a[1] = pair(f0, f1, 2 * i + 1), a[3] = pair(f2, f3, 2 * i + 1);
+    __device__ static __forceinline__ void half_block(int half, WalkField& f0, WalkField& f1, WalkField& f2, WalkField& f3, uint32_t (&a)[4][4]) {
+#pragma unroll
+        for (int s0 = 0; s0 < 8; s0 += 4) {
+            uint32_t x[4], y[4];
+            pairs(f0, f1, 8 * half + s0, x);
+            pairs(f2, f3, 8 * half + s0, y);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint32_t (&to)[4] = a[s0 / 2 + j];
+                to[0] = x[2 * j], to[1] = x[2 * j + 1], to[2] = y[2 * j], to[3] = y[2 * j + 1];
+            }
+        }
     }
 };
 
@@ -335,6 +357,10 @@ struct QuantField {
                    : i == 4 ? pair<4>(w0) : i == 5 ? pair<5>(w0) : i == 6 ? pair<6>(w0) : pair<7>(w0);
         }
     }
+    __device__ static __forceinline__ void half_block(int half, QuantField& f0, QuantField& f1, QuantField& f2, QuantField& f3, uint32_t (&a)[4][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) block(4 * half + i, f0, f1, f2, f3, a[i]);
+    }
     __device__ static __forceinline__ void block(int i, QuantField& f0, QuantField& f1, QuantField& f2, QuantField& f3, uint32_t (&a)[4]) {
         const uint32_t v0 = f0.value(i), v1 = f1.value(i), v2 = f2.value(i), v3 = f3.value(i);
         a[0] = low_halves(v0, v1), a[1] = high_halves(v0, v1), a[2] = low_halves(v2, v3), a[3] = high_halves(v2, v3);
@@ -367,6 +393,10 @@ struct GroupBlock {
     __device__ static constexpr int order(int i) { return i; }
     __device__ static constexpr int first(int i) { return 2 * i; }
     __device__ static constexpr int second(int i) { return 2 * i + 1; }
+    __device__ static __forceinline__ void half_block(int half, F& f0, F& f1, F& f2, F& f3, uint32_t (&a)[4][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) block(4 * half + i, f0, f1, f2, f3, a[i]);
+    }
     __device__ static __forceinline__ void block(int i, F& f0, F& f1, F& f2, F& f3, uint32_t (&a)[4]) {
         const uint32_t v0 = f0.pair(i), v1 = f1.pair(i), v2 = f2.pair(i), v3 = f3.pair(i);
         a[0] = low_halves(v0, v1), a[1] = high_halves(v0, v1), a[2] = low_halves(v2, v3), a[3] = high_halves(v2, v3);
@@ -760,16 +790,18 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
         if (!set_up) {
             tmem = tmem_s + (static_cast<uint32_t>(warp % 4 * 32) << 16) + warp / 4 * kColsWarp;
             const float4 *ta = reinterpret_cast<const float4*>(trig_w) + warp * 4 + qd, *tb = reinterpret_cast<const float4*>(trig_g) + lane;
+            if (8 * warp < next.sub || ntiles > 1 || work < work_end) {  // else the warp gets no tokens in this call
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                float v[8];
+                for (int ks = 0; ks < 4; ++ks) {
+                    float v[8];
 #pragma unroll
-                for (int e2 = 0; e2 < 2; ++e2) {
-                    const float4 a = ta[(2 * ks + e2) * kWarpsM * 4], e = tb[(2 * ks + e2) * 32];
-                    v[2 * e2] = a.x * e.x - a.y * e.y, v[2 * e2 + 1] = a.z * e.z - a.w * e.w;
-                    v[4 + 2 * e2] = a.y * e.x + a.x * e.y, v[5 + 2 * e2] = a.w * e.z + a.z * e.w;
+                    for (int e2 = 0; e2 < 2; ++e2) {
+                        const float4 a = ta[(2 * ks + e2) * kWarpsM * 4], e = tb[(2 * ks + e2) * 32];
+                        v[2 * e2] = a.x * e.x - a.y * e.y, v[2 * e2 + 1] = a.z * e.z - a.w * e.w;
+                        v[4 + 2 * e2] = a.y * e.x + a.x * e.y, v[5 + 2 * e2] = a.w * e.z + a.z * e.w;
+                    }
+                    tmem_st8(tmem + kColTrig + 8 * ks, v);
                 }
-                tmem_st8(tmem + kColTrig + 8 * ks, v);
             }
             set_up = true;
         }
@@ -838,14 +870,15 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     float kAl[4] = {al.x, al.y, al.z, al.w}, kAh[4] = {ah.x, ah.y, ah.z, ah.w};
                     float kBl[4] = {bl.x, bl.y, bl.z, bl.w}, kBh[4] = {bh.x, bh.y, bh.z, bh.w};
                     if constexpr (Field::kSlotwise) {
-                        // the four walks advance together, one coordinate each at a time
+                        // one field after the other, four coordinates each: their mask bits are tested together
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            fAl.add1(4 * ks + e, kAl[e]);
-                            fAh.add1(4 * ks + e, kAh[e]);
-                            fBl.add1(4 * ks + e, kBl[e]);
-                            fBh.add1(4 * ks + e, kBh[e]);
-                        }
+                        for (int e = 0; e < 4; ++e) fAl.add1(4 * ks + e, kAl[e]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) fAh.add1(4 * ks + e, kAh[e]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) fBl.add1(4 * ks + e, kBl[e]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) fBh.add1(4 * ks + e, kBh[e]);
                     } else {
                         fAl.add4(ks, kAl, kscA);
                         fAh.add4(ks, kAh, kscA);
@@ -907,11 +940,7 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();  // the values have landed
             if (any) {
-                // accumulators into registers for this phase
-                float flat[32], beta[4 * BETA];
-                tmem_st_wait();
-                tmem_ld32(tmem + kColAcc, flat);
-                tmem_load_beta<BETA>(tmem + kColBeta, beta);
+                tmem_st_wait();  // last pass's accumulators are in place
                 // value fields of rows 2q, 2q+1 (X), 2q+8, 2q+9 (Y), coordinates [16g, 16g+16)
                 const unsigned char* pv = reinterpret_cast<const unsigned char*>(pre + 16 + 2 * qd);
                 const unsigned char *pay = rows.vp + 2 * qd * kRow, *met = vm + 2 * qd * kMeta;
@@ -920,18 +949,14 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                 Field f2 = ML::field(pay + 8 * kRow, met + 8 * kMeta, pv + 64, g, 2 * qd < now.left_y);
                 Field f3 = ML::field(pay + 9 * kRow, met + 9 * kMeta, pv + 72, g, 2 * qd + 1 < now.left_y);
                 // ================= softmax (lazy running maximum per column), log2 domain =================
-                float mt[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
-#pragma unroll
-                for (int off = 4; off < 32; off <<= 1) {
-                    mt[0] = fmaxf(mt[0], __shfl_xor_sync(0xffffffffu, mt[0], off));
-                    mt[1] = fmaxf(mt[1], __shfl_xor_sync(0xffffffffu, mt[1], off));
-                }
-                tmem_ld_wait(flat);
-                tmem_ld_wait(beta);
-                float (&acc)[8][4] = reinterpret_cast<float(&)[8][4]>(flat);
-                float (&bacc)[BETA][4] = reinterpret_cast<float(&)[BETA][4]>(beta);
+                float mt[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};  // of this lane's tokens
                 const bool grow = mt[0] > m_used[0] + kRescaleThreshold || mt[1] > m_used[1] + kRescaleThreshold;
-                if (__any_sync(0xffffffffu, grow)) {
+                if (__any_sync(0xffffffffu, grow)) {  // rare: the columns' maxima, and everything summed so far scaled down
+#pragma unroll
+                    for (int off = 4; off < 32; off <<= 1) {
+                        mt[0] = fmaxf(mt[0], __shfl_xor_sync(0xffffffffu, mt[0], off));
+                        mt[1] = fmaxf(mt[1], __shfl_xor_sync(0xffffffffu, mt[1], off));
+                    }
                     float alpha[2];
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
@@ -940,17 +965,23 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                         m_used[u] = m_new;
                         l_part[u] *= alpha[u];
                     }
+                    if (it > 0) {  // nothing is summed yet in a segment's first pass
+                        float flat[32], beta[4 * BETA];
+                        tmem_ld32(tmem + kColAcc, flat);
+                        tmem_load_beta<BETA>(tmem + kColBeta, beta);
+                        tmem_ld_wait(flat);
+                        tmem_ld_wait(beta);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        acc[i][0] *= alpha[0], acc[i][2] *= alpha[0];
-                        acc[i][1] *= alpha[1], acc[i][3] *= alpha[1];
-                    }
+                        for (int i = 0; i < 32; ++i) flat[i] *= alpha[i & 1];
 #pragma unroll
-                    for (int mb = 0; mb < BETA; ++mb) {
-                        bacc[mb][0] *= alpha[0], bacc[mb][2] *= alpha[0];
-                        bacc[mb][1] *= alpha[1], bacc[mb][3] *= alpha[1];
+                        for (int i = 0; i < 4 * BETA; ++i) beta[i] *= alpha[i & 1];
+                        tmem_st32(tmem + kColAcc, flat);
+                        tmem_store_beta<BETA>(tmem + kColBeta, beta);
+                        tmem_st_wait();
                     }
                 }
+                float beta[4 * BETA];
+                tmem_load_beta<BETA>(tmem + kColBeta, beta);
                 __half2 p01, p23;
                 if constexpr (kDual) {
                     p01 = __floats2half2_rn(fast_exp2(sc[0] - m_used[0]), fast_exp2(sc[1] - m_used[1]));
@@ -973,8 +1004,10 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     const int w0 = __shfl_sync(0xffffffffu, ids_cur, at), w1 = __shfl_sync(0xffffffffu, ids_cur, at + 1);
                     const int w2 = __shfl_sync(0xffffffffu, ids_cur, at + 8), w3 = __shfl_sync(0xffffffffu, ids_cur, at + 9);
                     const __half2 gg = __half2half2(__int2half_rn(g));
+                    float (&bacc)[BETA][4] = reinterpret_cast<float(&)[BETA][4]>(beta);
                     const __half2 d01 = __hsub2(__halves2half2(__int2half_rn(w0), __int2half_rn(w1)), gg);
                     const __half2 d23 = __hsub2(__halves2half2(__int2half_rn(w2), __int2half_rn(w3)), gg);
+                    tmem_ld_wait(beta);
 #pragma unroll
                     for (int mb = 0; mb < BETA; ++mb) {
                         if (16 * mb < p.cv) {
@@ -983,6 +1016,7 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                                       as_bits(__heq2(d23, hi)), pb0, pb1);
                         }
                     }
+                    tmem_store_beta<BETA>(tmem + kColBeta, beta);
                 }
                 if constexpr (ML::kScale) {
                     // quantised values enter the MMA as integer codes: their per-token scale rides on P
@@ -991,15 +1025,19 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     pb0 = movmatrix_trans(as_bits(__floats2half2_rn(p01f.x * vsA, p01f.y * vsA)));
                     pb1 = movmatrix_trans(as_bits(__floats2half2_rn(p23f.x * vsB, p23f.y * vsB)));
                 }
-                // O^T += Vres^T . P, two coordinates per MMA
+                // O^T += Vres^T . P, two coordinates per MMA; half of the accumulators in registers at a time
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    uint32_t a[4];
-                    Field::block(i, f0, f1, f2, f3, a);
-                    mma_16816(acc[i], a[0], a[1], a[2], a[3], pb0, pb1);
+                for (int half = 0; half < 2; ++half) {
+                    float flat[16];
+                    tmem_ld16(tmem + kColAcc + 16 * half, flat);
+                    uint32_t a[4][4];
+                    Field::half_block(half, f0, f1, f2, f3, a);
+                    tmem_ld_wait(flat);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        mma_16816(reinterpret_cast<float(&)[4][4]>(flat)[i], a[i][0], a[i][1], a[i][2], a[i][3], pb0, pb1);
+                    tmem_st16(tmem + kColAcc + 16 * half, flat);
                 }
-                tmem_st32(tmem + kColAcc, flat);
-                tmem_store_beta<BETA>(tmem + kColBeta, beta);
             }
             __syncwarp();  // the value rows and rank bases may be rewritten
             issue_values(next);
@@ -1065,22 +1103,26 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             const int quarter = warp % 4, mine = warp / 4;
             const uint32_t quarter_cols = tmem - mine * kColsWarp;
             float acc[8] = {}, bacc[4] = {};  // m-blocks 2 mine, 2 mine + 1; cluster block `mine`
+            // two source warps at a time; one without tokens has weight zero and is not read
 #pragma unroll 1
-            for (int from_warp = quarter; from_warp < busy_warps; from_warp += 4) {
+            for (int from_warp = quarter; from_warp < busy_warps; from_warp += 8) {
+                const bool two = from_warp + 4 < busy_warps;
                 const uint32_t at = quarter_cols + from_warp / 4 * kColsWarp;
-                float v[8], vb[4];
-                tmem_ld8(at + kColAcc + 8 * mine, v);
-                if (mine < BETA) tmem_ld4(at + kColBeta + 4 * mine, vb);
-                const float2 ms2 = *reinterpret_cast<const float2*>(all_stats + from_warp * kStatsWarp + 2 * qd);
-                const float w[2] = {fast_exp2(ms2.x - m_head[0]), fast_exp2(ms2.y - m_head[1])};
-                tmem_ld_wait(v);
+                float v0[8], v1[8], b0[4], b1[4];
+                tmem_ld8(at + kColAcc + 8 * mine, v0);
+                tmem_ld4(at + kColBeta + 4 * (mine < BETA ? mine : 0), b0);
+                const uint32_t at1 = two ? at + kColsWarp : at;
+                tmem_ld8(at1 + kColAcc + 8 * mine, v1);
+                tmem_ld4(at1 + kColBeta + 4 * (mine < BETA ? mine : 0), b1);
+                const float* st = all_stats + from_warp * kStatsWarp + 2 * qd;
+                const float2 s0 = *reinterpret_cast<const float2*>(st), s1 = *reinterpret_cast<const float2*>(two ? st + 4 * kStatsWarp : st);
+                const float w0[2] = {fast_exp2(s0.x - m_head[0]), fast_exp2(s0.y - m_head[1])};
+                const float w1[2] = {two ? fast_exp2(s1.x - m_head[0]) : 0.f, two ? fast_exp2(s1.y - m_head[1]) : 0.f};
+                tmem_ld_wait(v0), tmem_ld_wait(v1), tmem_ld_wait(b0), tmem_ld_wait(b1);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] = fmaf(v[e], w[e & 1], acc[e]);
-                if (mine < BETA) {
-                    tmem_ld_wait(vb);
+                for (int e = 0; e < 8; ++e) acc[e] = fmaf(v1[e], w1[e & 1], fmaf(v0[e], w0[e & 1], acc[e]));
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) bacc[e] = fmaf(vb[e], w[e & 1], bacc[e]);
-                }
+                for (int e = 0; e < 4; ++e) bacc[e] = fmaf(b1[e], w1[e & 1], fmaf(b0[e], w0[e & 1], bacc[e]));
             }
             if constexpr (!kDual) {  // X's columns and Y's
 #pragma unroll
@@ -1098,7 +1140,7 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                         for (int i = 0; i < 2; ++i)
                             dst[9 * Field::first(2 * mine + i)] = acc[4 * i + u], dst[9 * Field::second(2 * mine + i)] = acc[4 * i + 2 + u];
                         float* bdst = red_beta + (quarter * GQA + h) * kRedBeta + 16 * mine + g;
-                        bdst[0] = bacc[u], bdst[8] = bacc[2 + u];
+                        bdst[0] = mine < BETA ? bacc[u] : 0.f, bdst[8] = mine < BETA ? bacc[2 + u] : 0.f;
                     }
                 }
             }
