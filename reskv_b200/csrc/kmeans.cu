@@ -58,7 +58,7 @@ struct InitIndex {
     int idx[kMaxClusters];
 };
 
-// The tcgen05 form, one launch per Lloyd iteration, over one or two tensors (sides) of the same shape.
+// The tcgen05 form, one launch for all Lloyd iterations, over one or two tensors (sides) of the same shape.
 struct UmmaParams {
     const __half* x[2];   // [units, x_stride, 128]
     int64_t x_stride[2];
@@ -70,8 +70,10 @@ struct UmmaParams {
     float* centres[2];    // [sides * units, C, 128]
     long long* sums[3];
     int* counts[3];
+    int* arrived;         // [sides * units] segments flushed so far, zero on entry
     uint32_t* status;
-    int sides, units, tokens, clusters, iteration, iterations;
+    __half* out[2];       // [units, C, 128] the centres after the last iteration
+    int sides, units, tokens, clusters, iterations;
     InitIndex init;       // tokens that are the first centres
 };
 
@@ -481,12 +483,17 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 // different tiles and hand over through mbarriers only (triple-buffered distances and one-hot operands); every
 // wait is bounded.
 //
-// One launch per iteration, over K and V together when both are wanted: a launch costs a set-up, a pipeline fill and a
-// drain (~10 tile times) whatever it covers.  The new centres are formed in the next launch's set-up from the sums of the
-// last one (three generations of them, so nothing has to be cleared in between), and consecutive launches overlap
-// (programmatic stream serialisation): a CTA's set-up and first copies run while the launch before it drains.  Measured,
-// clustering of one layer's K and V, 64 units x 8128 tokens, 10 iterations: 0.79 ms with an update kernel and a launch
-// per side and iteration, 0.58 ms this way (0.63 ms in two calls).
+// One cooperative launch for all iterations, over K and V together when both are wanted.  A CTA keeps its segments; between
+// iterations it waits for the other CTAs of its units only (a counter of flushed segments per unit), and not at all for a
+// unit that is its own, whose sums it writes without atomic additions.  The new centres are formed at the start of the next
+// iteration from the sums of the last one (three generations of them, so nothing has to be cleared in between).  The ring of
+// copies runs on across iterations, and every second iteration takes the tiles backwards: what the last one read at its end
+// is still in L2.  Where a unit's iteration begins, the loads of all sums are in flight together, and the next segment is
+// worked out by a thread that waits anyway.
+//
+// Measured, clustering of one layer's K and V, 10 iterations, us, one launch per iteration -> now: 64 units x 8128 tokens
+// 578 -> 508, 128 x 3000 517 -> 422, 64 x 2000 221 -> 192, 8 x 1152 105 -> 98, 8 x 8128 (many CTAs per unit) 164 -> 165.
+// Of that the single launch by itself gives 2 %, the order of the tiles 3 to 5, stores in place of atomics 4 to 6.
 constexpr int kUGroups = 3;                    // token-owning groups; group g takes the tiles i = g (mod 3)
 constexpr int kUGroupWarps = 4;                // a group: one warp per 32 token rows (TMEM lane quarter)
 constexpr int kUThreads = (kUGroups * kUGroupWarps + 3) * 32;  // + three issuing warps: distance MMAs, sum MMAs, copies
@@ -550,16 +557,22 @@ constexpr int kUWorkers = kUThreads - 32;  // everyone but the copying warp: the
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kUWorkers) : "memory"); }
 
 // Four coordinates of a centre after iteration `from`: the mean of the tokens assigned then, the old centre (K) or zero
-// (V) where there were none; V's centres are rounded to FP16.
-__device__ __forceinline__ float4 new_centre(const UmmaParams& p, int from, bool value, size_t row, int i4) {
-    const int n = __ldcg(p.counts[from % 3] + row);  // through L2: written by the launch before this one
+// (V) where there were none; V's centres are rounded to FP16.  In two parts, so that a thread has all its loads in flight
+// together (the sums requested behind the count: two trips to L2 per centre, 7000 instead of 2500 cycles for the tables).
+struct CentreSums {
+    int n;
+    longlong2 a, b;
+};
+__device__ __forceinline__ CentreSums load_sums(const UmmaParams& p, int from, size_t row, int i4) {
+    const longlong2* s = reinterpret_cast<const longlong2*>(p.sums[from % 3] + row * kHeadDim) + 2 * i4;
+    return {__ldcg(p.counts[from % 3] + row), __ldcg(s), __ldcg(s + 1)};  // through L2: written by other CTAs
+}
+__device__ __forceinline__ float4 new_centre(const UmmaParams& p, const CentreSums& cs, int from, bool value, size_t row, int i4) {
     float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n > 0) {
-        const longlong2* s = reinterpret_cast<const longlong2*>(p.sums[from % 3] + row * kHeadDim) + 2 * i4;
-        const longlong2 a = __ldcg(s), b = __ldcg(s + 1);
-        const double scale = 1.0 / 16777216.0 / static_cast<double>(n);
-        c = make_float4(static_cast<float>(static_cast<double>(a.x) * scale), static_cast<float>(static_cast<double>(a.y) * scale),
-                        static_cast<float>(static_cast<double>(b.x) * scale), static_cast<float>(static_cast<double>(b.y) * scale));
+    if (cs.n > 0) {
+        const double scale = __drcp_rn(static_cast<double>(cs.n)) * (1.0 / 16777216.0);
+        c = make_float4(static_cast<float>(static_cast<double>(cs.a.x) * scale), static_cast<float>(static_cast<double>(cs.a.y) * scale),
+                        static_cast<float>(static_cast<double>(cs.b.x) * scale), static_cast<float>(static_cast<double>(cs.b.y) * scale));
     } else if (!value) {
         c = __ldcg(reinterpret_cast<const float4*>(p.centres[from & 1] + row * kHeadDim) + i4);
     }
@@ -597,13 +610,40 @@ __host__ __device__ inline Segment segment_at(const Cuts& c, int w) {
     return sg;
 }
 
+// The segment that ends in front of tile w (w > 0, a cut or the end of a segment).
+__host__ __device__ inline Segment segment_before(const Cuts& c, int w) {
+    constexpr int kMost = kUChunkMax / kUTile;
+    const int last = w - 1, unit = last / c.tiles_unit, side = last / c.tiles_side * c.tiles_side;
+    const int by_piece = side + (last - side) / c.piece * c.piece, by_unit = unit * c.tiles_unit;
+    const int from = by_piece > by_unit ? by_piece : by_unit;  // the cut in front
+    const int start = from + (last - from) / kMost * kMost;
+    return Segment{unit, start - by_unit, w - start};
+}
+// Segments of a unit.
+__host__ __device__ inline int segments_of(const Cuts& c, int unit) {
+    const int begin = unit * c.tiles_unit, in_side = begin % c.tiles_side;
+    if (c.piece <= kUChunkMax / kUTile) return 1 + (in_side + c.tiles_unit - 1) / c.piece - in_side / c.piece;
+    int n = 0;
+    for (int w = begin; w < begin + c.tiles_unit; ++n) w += segment_at(c, w).tiles;
+    return n;
+}
+
+// Waits until `count` segments of a unit have been flushed, by one thread.  Every CTA of the launch is resident and takes
+// its segments iteration by iteration, so the wait ends; it gives up after 2^22 looks (seconds) all the same.
+__device__ __forceinline__ bool wait_for_segments(const int* arrived, int count) {
+    for (uint32_t spin = 0; spin < (1u << 22); ++spin) {
+        int n;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
+        if (n >= count) return true;
+    }
+    return false;
+}
+
 __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap map0,
                                                                            const __grid_constant__ CUtensorMap map1, const Cuts cuts,
                                                                            int share) {
     extern __shared__ unsigned char smem_u[];
     constexpr int kN = 64;  // rows of the centre operand: hi halves, then lo halves (K's FP32 centres; V's are FP16)
-    const bool first = p.iteration == 0, last = p.iteration + 1 == p.iterations;
-    let_next_launch_start();
     unsigned char* base = smem_u + ((1024u - (smem_u32(smem_u) & 1023u)) & 1023u);  // swizzled blocks: 1024-byte aligned
     unsigned char* xs = base;                                   // [stages][2 halves][128 tokens][128 B]
     unsigned char* cop = xs + kUStages * kUTileBytes;           // [2 halves][kN rows][128 B]
@@ -618,6 +658,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     __shared__ uint64_t bar_full[kUStages], bar_empty[kUStages], bar_dist[kUGroups], bar_dist_free[kUGroups], bar_onehot[kUGroups],
         bar_sums[kUGroups];
     __shared__ uint32_t tmem_base_s;
+    __shared__ Segment next_s;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // CTA c takes the pieces that start in [c * share, (c + 1) * share) of all tiles and walks them segment by segment.
@@ -651,319 +692,370 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
         // ---- copies, through all segments without a stop: the stage of tile q is free once the sums of tile
         // q - 5 have run (whole warp, one elected lane per tile) --------------------------------------------------
         int q = 0;
-        for (int w = work_begin; w < work_end;) {
-            const Segment sg = segment_at(cuts, w);
-            for (int i = 0; i < sg.tiles; ++i, ++q) {
-                if (q >= kUStages) lost |= !mbar_wait(&bar_empty[q % kUStages], (q / kUStages - 1) & 1);
-                unsigned char* dst = xs + (q % kUStages) * kUTileBytes;
-                uint64_t* bar = &bar_full[q % kUStages];
-                if (elect_one()) {
-                    const CUtensorMap* xmap = sg.unit < p.units ? &map0 : &map1;
-                    const int unit = sg.unit < p.units ? sg.unit : sg.unit - p.units;
-                    mbar_arrive_expect_tx(bar, kUTileBytes);
-                    tma_load_3d(dst, xmap, 0, (sg.tile0 + i) * kUTile, unit, bar);
-                    tma_load_3d(dst + kUBoxBytes, xmap, 64, (sg.tile0 + i) * kUTile, unit, bar);
+        for (int it = 0; it < p.iterations; ++it) {
+            const bool back = it & 1;
+            for (int w = back ? work_end : work_begin; back ? w > work_begin : w < work_end;) {
+                const Segment sg = back ? segment_before(cuts, w) : segment_at(cuts, w);
+                for (int i = 0; i < sg.tiles; ++i, ++q) {
+                    const int row = (sg.tile0 + (back ? sg.tiles - 1 - i : i)) * kUTile;
+                    if (q >= kUStages) lost |= !mbar_wait(&bar_empty[q % kUStages], (q / kUStages - 1) & 1);
+                    unsigned char* dst = xs + (q % kUStages) * kUTileBytes;
+                    uint64_t* bar = &bar_full[q % kUStages];
+                    if (elect_one()) {
+                        const CUtensorMap* xmap = sg.unit < p.units ? &map0 : &map1;
+                        const int unit = sg.unit < p.units ? sg.unit : sg.unit - p.units;
+                        mbar_arrive_expect_tx(bar, kUTileBytes);
+                        tma_load_3d(dst, xmap, 0, row, unit, bar);
+                        tma_load_3d(dst + kUBoxBytes, xmap, 64, row, unit, bar);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
+                w += back ? -sg.tiles : sg.tiles;
             }
-            w += sg.tiles;
         }
     } else {
-        // the launches of consecutive iterations overlap: this one's set-up and first copies (the tokens do not change) run
-        // while the last one drains; what that one wrote is touched from here on
-        wait_for_previous_launch();
         int q0 = 0;     // tiles of the earlier segments of this CTA
         int prev = -1;  // byte offset of the element this thread set in its group's one-hot buffer
-        int unit_in_tables = -1;
-        for (int w = work_begin; w < work_end;) {
-            const Segment sg = segment_at(cuts, w);
-            const int unit = sg.unit, n_tiles = sg.tiles;
-            const int t_begin = sg.tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
-            const int side = unit < p.units ? 0 : 1, local = unit - side * p.units;
-            const bool value = p.value[side] != 0;
-            const __half* xu = p.x[side] + static_cast<size_t>(local) * p.x_stride[side] * kHeadDim;
-            const size_t row0 = static_cast<size_t>(unit) * p.clusters;  // first centre of the unit
-            const bool opens_unit = sg.tile0 == 0;  // this CTA also keeps the unit's centres and zeroes its next sums
-            // ---- per unit: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 ----------------------
-            if (unit != unit_in_tables) {
-                unit_in_tables = unit;
-                // four coordinates per thread and step, all loads of a thread in flight together
-                constexpr int kSteps = (32 * kHeadDim / 4 + kUWorkers - 1) / kUWorkers;
-                float4 v[kSteps];
-#pragma unroll
-                for (int k = 0; k < kSteps; ++k) {
-                    const int i4 = tid + k * kUWorkers;
-                    const int c = i4 / (kHeadDim / 4), d4 = i4 % (kHeadDim / 4);
-                    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (i4 >= 32 * kHeadDim / 4 || c >= p.clusters) continue;
-                    if (first) {
-                        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(xu + static_cast<size_t>(p.init.idx[c]) * kHeadDim) + d4);
-                        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                        v[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
-                    } else {
-                        v[k] = new_centre(p, p.iteration - 1, value, row0 + c, d4);
+        int unit_in_tables = -1, segments = 0;  // unit of the tables, its segments
+        // an iteration ends where the next one begins: its last segment is the next one's first
+        Segment sg = work_begin < work_end ? segment_at(cuts, work_begin) : Segment{};
+        for (int it = 0; it < p.iterations; ++it) {
+            const bool first = it == 0, last = it + 1 == p.iterations, back = it & 1;
+            bool stale = true;  // the tables are those of the iteration before
+            for (int w = back ? work_end : work_begin; back ? w > work_begin : w < work_end;) {
+                const int unit = sg.unit, n_tiles = sg.tiles, w_next = back ? w - n_tiles : w + n_tiles;
+                const int t_begin = sg.tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
+                const int side = unit < p.units ? 0 : 1, local = unit - side * p.units;
+                const bool value = p.value[side] != 0;
+                const __half* xu = p.x[side] + static_cast<size_t>(local) * p.x_stride[side] * kHeadDim;
+                const size_t row0 = static_cast<size_t>(unit) * p.clusters;  // first centre of the unit
+                const bool opens_unit = unit * cuts.tiles_unit >= work_begin;  // this CTA also keeps the unit's centres and zeroes its next sums
+                // the whole unit is this CTA's: its first segment writes the sums instead of adding to zeros (a 64-bit atomic
+                // addition costs eight times a store: 2300 cycles a segment), and no other CTA is waited for
+                const bool owned = opens_unit && (unit + 1) * cuts.tiles_unit <= work_end;
+                const bool writes = owned && (back ? sg.tile0 + n_tiles == cuts.tiles_unit : sg.tile0 == 0);
+                // ---- per unit: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 ----------------------
+                if (stale || unit != unit_in_tables) {
+                    if (unit != unit_in_tables && !owned) segments = segments_of(cuts, unit);
+                    stale = false, unit_in_tables = unit;
+                    // the sums of the iteration before are complete (a unit of one segment: this CTA has made them)
+                    if (!first && !owned) {
+                        if (tid == 0) lost |= !wait_for_segments(p.arrived + unit, it * segments);
+                        workers_sync();
                     }
-                    if (opens_unit) {
-                        reinterpret_cast<float4*>(p.centres[p.iteration & 1] + row0 * kHeadDim)[i4] = v[k];
-                        const longlong2 zero = make_longlong2(0, 0);
-                        longlong2* ahead = reinterpret_cast<longlong2*>(p.sums[(p.iteration + 1) % 3] + row0 * kHeadDim) + 2 * i4;
-                        ahead[0] = zero, ahead[1] = zero;
-                        if (d4 == 0) p.counts[(p.iteration + 1) % 3][row0 + c] = 0;
+                    // four coordinates per thread and step, all loads of a thread in flight together
+                    constexpr int kMakers = kUWorkers - 32;  // not the last worker warp, which may still announce the segment before
+                    constexpr int kSteps = (32 * kHeadDim / 4 + kMakers - 1) / kMakers;
+                    if (tid < kMakers) {
+                    float4 v[kSteps];
+                    CentreSums sums[kSteps];
+                    if (!first) {
+#pragma unroll
+                        for (int k = 0; k < kSteps; ++k) {
+                            const int i4 = min(tid + k * kMakers, p.clusters * (kHeadDim / 4) - 1);
+                            sums[k] = load_sums(p, it - 1, row0 + i4 / (kHeadDim / 4), i4 % (kHeadDim / 4));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kSteps; ++k) {
+                        const int i4 = tid + k * kMakers;
+                        const int c = i4 / (kHeadDim / 4), d4 = i4 % (kHeadDim / 4);
+                        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (i4 >= 32 * kHeadDim / 4 || c >= p.clusters) continue;
+                        if (first) {
+                            const uint2 raw = __ldg(reinterpret_cast<const uint2*>(xu + static_cast<size_t>(p.init.idx[c]) * kHeadDim) + d4);
+                            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+                            v[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                        } else {
+                            v[k] = new_centre(p, sums[k], it - 1, value, row0 + c, d4);
+                        }
+                        if (opens_unit) {
+                            reinterpret_cast<float4*>(p.centres[it & 1] + row0 * kHeadDim)[i4] = v[k];
+                            if (owned) continue;
+                            const longlong2 zero = make_longlong2(0, 0);
+                            longlong2* ahead = reinterpret_cast<longlong2*>(p.sums[(it + 1) % 3] + row0 * kHeadDim) + 2 * i4;
+                            ahead[0] = zero, ahead[1] = zero;
+                            if (d4 == 0) p.counts[(it + 1) % 3][row0 + c] = 0;
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kSteps; ++k) {
+                        const int i4 = tid + k * kMakers;
+                        if (i4 >= 32 * kHeadDim / 4) break;
+                        const int c = i4 / (kHeadDim / 4), d = (i4 % (kHeadDim / 4)) * 4;
+                        reinterpret_cast<float4*>(cen_s)[i4] = v[k];
+                        const __half2 h01 = __floats2half2_rn(v[k].x, v[k].y), h23 = __floats2half2_rn(v[k].z, v[k].w);
+                        unsigned char* at = cop + (d >> 6) * (kN * 128) + ((d & 7) << 1);
+                        *reinterpret_cast<uint2*>(at + sw128(c, (d & 63) >> 3)) =
+                            make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+                        float2 f01 = __half22float2(h01), f23 = __half22float2(h23);  // what the MMA sees: hi (+ lo)
+                        if (!value) {
+                            const __half2 l01 = __floats2half2_rn(v[k].x - f01.x, v[k].y - f01.y);
+                            const __half2 l23 = __floats2half2_rn(v[k].z - f23.x, v[k].w - f23.y);
+                            *reinterpret_cast<uint2*>(at + sw128(32 + c, (d & 63) >> 3)) =
+                                make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
+                            const float2 g01 = __half22float2(l01), g23 = __half22float2(l23);
+                            f01.x += g01.x, f01.y += g01.y, f23.x += g23.x, f23.y += g23.y;
+                        }
+                        // |c|^2: the 32 threads of a warp hold one centre (the worker count is a multiple of 32)
+                        float sq = fmaf(f01.x, f01.x, fmaf(f01.y, f01.y, fmaf(f23.x, f23.x, f23.y * f23.y)));
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(kFull, sq, off);
+                        if (lane == 0) cn_s[c] = c < p.clusters ? sq : INFINITY;
+                    }
                     }
                 }
+                if (tid < 32) cnt_s[tid] = 0;
+                proxy_fence();  // the operands written above are read by the tensor core (async proxy)
+                workers_sync();
+                // the next segment, by a thread that has to wait for its first tile anyway (four divisions)
+                if (tid == 2 * kUGroupWarps * 32 && (back ? w_next > work_begin : w_next < work_end))
+                    next_s = back ? segment_before(cuts, w_next) : segment_at(cuts, w_next);
+                float cmax = lane < p.clusters ? cn_s[lane] : 0.f;  // largest |c|^2, in every thread
 #pragma unroll
-                for (int k = 0; k < kSteps; ++k) {
-                    const int i4 = tid + k * kUWorkers;
-                    if (i4 >= 32 * kHeadDim / 4) break;
-                    const int c = i4 / (kHeadDim / 4), d = (i4 % (kHeadDim / 4)) * 4;
-                    reinterpret_cast<float4*>(cen_s)[i4] = v[k];
-                    const __half2 h01 = __floats2half2_rn(v[k].x, v[k].y), h23 = __floats2half2_rn(v[k].z, v[k].w);
-                    unsigned char* at = cop + (d >> 6) * (kN * 128) + ((d & 7) << 1);
-                    *reinterpret_cast<uint2*>(at + sw128(c, (d & 63) >> 3)) =
-                        make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
-                    float2 f01 = __half22float2(h01), f23 = __half22float2(h23);  // what the MMA sees: hi (+ lo)
-                    if (!value) {
-                        const __half2 l01 = __floats2half2_rn(v[k].x - f01.x, v[k].y - f01.y);
-                        const __half2 l23 = __floats2half2_rn(v[k].z - f23.x, v[k].w - f23.y);
-                        *reinterpret_cast<uint2*>(at + sw128(32 + c, (d & 63) >> 3)) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
-                        const float2 g01 = __half22float2(l01), g23 = __half22float2(l23);
-                        f01.x += g01.x, f01.y += g01.y, f23.x += g23.x, f23.y += g23.y;
-                    }
-                    // |c|^2: the 32 threads of a warp hold one centre (the worker count is a multiple of 32)
-                    float sq = fmaf(f01.x, f01.x, fmaf(f01.y, f01.y, fmaf(f23.x, f23.x, f23.y * f23.y)));
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(kFull, sq, off);
-                    if (lane == 0) cn_s[c] = c < p.clusters ? sq : INFINITY;
-                }
-            }
-            if (tid < 32) cnt_s[tid] = 0;
-            proxy_fence();  // the operands written above are read by the tensor core (async proxy)
-            workers_sync();
-            float cmax = lane < p.clusters ? cn_s[lane] : 0.f;  // largest |c|^2, in every thread
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(kFull, cmax, off));
+                for (int off = 16; off > 0; off >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(kFull, cmax, off));
 
-            if (warp < kWarpDist) {
-                // ---- ranking: one thread per token; group g takes the tiles with q = g (mod 3), distance buffer g
-                // and one-hot buffer g ---------------------------------------------------------------------------
-                const int g = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
-                const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-                // |x|^2 of a token is the same in every Lloyd iteration: the first one forms it and stores it (as FP32
-                // bits) where the token's id goes, the following ones read it from there one tile of the group ahead,
-                // the last one writes the id
-                int32_t* ids_u = p.ids[side] + static_cast<size_t>(local) * p.tokens;
-                int8_t* ids8_u = p.ids8[side] ? p.ids8[side] + static_cast<size_t>(local) * p.tokens : nullptr;
-                const int i_first = (g + kUGroups - q0 % kUGroups) % kUGroups;
-                float xn_next = 0.f;
-                if (!first && t_begin + i_first * kUTile + row_in_tile < t_end)
-                    xn_next = __int_as_float(ids_u[t_begin + i_first * kUTile + row_in_tile]);
-                for (int i = i_first; i < n_tiles; i += kUGroups) {
-                    const int q = q0 + i, use = q / kUGroups, st = q % kUStages;
-                    const int row = t_begin + i * kUTile + row_in_tile;
-                    const bool live = row < t_end;
-                    float xn = xn_next;
-                    if (!first && row + kUGroups * kUTile < t_end) xn_next = __int_as_float(ids_u[row + kUGroups * kUTile]);
-                    lost |= !mbar_wait(&bar_dist[g], use & 1);
-                    tc_fence_after();
-                    float d[32];
-                    tmem_ld32(tmem + lane_base + kUColD + g * 64, d);
-                    if (!value) {
-                        float lo[32];
-                        tmem_ld32(tmem + lane_base + kUColD + g * 64 + 32, lo);
-                        tmem_ld_wait();
+                if (warp < kWarpDist) {
+                    // ---- ranking: one thread per token; group g takes the tiles with q = g (mod 3), distance buffer g
+                    // and one-hot buffer g ---------------------------------------------------------------------------
+                    const int g = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
+                    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+                    // |x|^2 of a token is the same in every Lloyd iteration: the first one forms it and stores it (as FP32
+                    // bits) where the token's id goes, the following ones read it from there one tile of the group ahead,
+                    // the last one writes the id
+                    int32_t* ids_u = p.ids[side] + static_cast<size_t>(local) * p.tokens;
+                    int8_t* ids8_u = p.ids8[side] ? p.ids8[side] + static_cast<size_t>(local) * p.tokens : nullptr;
+                    const int i_first = (g + kUGroups - q0 % kUGroups) % kUGroups;
+                    const auto row_of = [&](int i) { return t_begin + (back ? n_tiles - 1 - i : i) * kUTile + row_in_tile; };
+                    float xn_next = 0.f;
+                    if (!first && i_first < n_tiles && row_of(i_first) < t_end) xn_next = __int_as_float(ids_u[row_of(i_first)]);
+                    for (int i = i_first; i < n_tiles; i += kUGroups) {
+                        const int q = q0 + i, use = q / kUGroups, st = q % kUStages;
+                        const int row = row_of(i), tile_row = row - row_in_tile;
+                        const bool live = row < t_end;
+                        float xn = xn_next;
+                        if (!first && i + kUGroups < n_tiles && row_of(i + kUGroups) < t_end) xn_next = __int_as_float(ids_u[row_of(i + kUGroups)]);
+                        lost |= !mbar_wait(&bar_dist[g], use & 1);
+                        tc_fence_after();
+                        float d[32];
+                        tmem_ld32(tmem + lane_base + kUColD + g * 64, d);
+                        if (!value) {
+                            float lo[32];
+                            tmem_ld32(tmem + lane_base + kUColD + g * 64 + 32, lo);
+                            tmem_ld_wait();
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) d[c] += lo[c];
-                    } else {
-                        tmem_ld_wait();
-                    }
-                    tc_fence_before();
-                    mbar_arrive(&bar_dist_free[g]);  // the next distances of this group may be issued
-                    float d1 = INFINITY, d2 = INFINITY;
-                    int c1 = 0;
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) {  // branch-free: best, second best, index of the best
-                        d[c] = fmaf(-2.f, d[c], cn_s[c]);
-                        d2 = fminf(d2, fmaxf(d[c], d1));
-                        c1 = d[c] < d1 ? c : c1;  // a strict comparison keeps the lower index on ties
-                        d1 = fminf(d1, d[c]);
-                    }
-                    if (first) {
-                        // |x|^2 for the near-tie bound: packed FP16 products, eight at a time (an overflow gives +inf:
-                        // re-rank)
-                        lost |= !mbar_wait(&bar_full[st], (q / kUStages) & 1);
-                        const unsigned char* xt = xs + st * kUTileBytes;
-                        xn = 0.f;
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const uint4 v = *reinterpret_cast<const uint4*>(xt + (j >> 3) * kUBoxBytes + sw128(row_in_tile, j & 7));
-                            const __half2* h = reinterpret_cast<const __half2*>(&v);
-                            __half2 s = __hmul2(h[0], h[0]);
-                            s = __hfma2(h[1], h[1], s), s = __hfma2(h[2], h[2], s), s = __hfma2(h[3], h[3], s);
-                            const float2 f = __half22float2(s);
-                            xn += f.x + f.y;
+                            for (int c = 0; c < 32; ++c) d[c] += lo[c];
+                        } else {
+                            tmem_ld_wait();
                         }
-                    }
-                    // near-ties: only a centre whose distance lies inside the bound can win; the warp forms the exact
-                    // FP32 sums of those few (same arithmetic, same order as `nearest`), one tied token at a time
-                    const float bound = kTieBound * (1.01f * xn + cmax);
-                    uint32_t inside = 0u;
-                    if (live && !((d2 - d1) > bound)) {
+                        tc_fence_before();
+                        mbar_arrive(&bar_dist_free[g]);  // the next distances of this group may be issued
+                        float d1 = INFINITY, d2 = INFINITY;
+                        int c1 = 0;
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) inside |= !((d[c] - d1) > bound) ? 1u << c : 0u;
-                    }
-                    uint32_t redo = __ballot_sync(kFull, inside != 0u);
-                    while (redo) {
-                        const int src = __ffs(redo) - 1;
-                        redo &= redo - 1;
-                        uint32_t cands = __shfl_sync(kFull, inside, src) & (p.clusters >= 32 ? 0xffffffffu : (1u << p.clusters) - 1u);
-                        const __half* xr = xu + static_cast<size_t>(t_begin + i * kUTile + quarter * 32 + src) * kHeadDim;
-                        float xv[4];
+                        for (int c = 0; c < 32; ++c) {  // branch-free: best, second best, index of the best
+                            d[c] = fmaf(-2.f, d[c], cn_s[c]);
+                            d2 = fminf(d2, fmaxf(d[c], d1));
+                            c1 = d[c] < d1 ? c : c1;  // a strict comparison keeps the lower index on ties
+                            d1 = fminf(d1, d[c]);
+                        }
+                        if (first) {
+                            // |x|^2 for the near-tie bound: packed FP16 products, eight at a time (an overflow gives +inf:
+                            // re-rank)
+                            lost |= !mbar_wait(&bar_full[st], (q / kUStages) & 1);
+                            const unsigned char* xt = xs + st * kUTileBytes;
+                            xn = 0.f;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) xv[k] = __half2float(xr[lane + 32 * k]);
-                        float best = INFINITY;
-                        int bc = 0;
-                        while (cands) {  // ascending centre index: the lower one wins ties
-                            const int c = __ffs(cands) - 1;
-                            cands &= cands - 1;
-                            const float* crow = cen_s + c * kHeadDim;
-                            float acc = 0.f;
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float df = xv[e] - crow[lane + 32 * e];
-                                acc = fmaf(df, df, acc);
+                            for (int j = 0; j < 16; ++j) {
+                                const uint4 v = *reinterpret_cast<const uint4*>(xt + (j >> 3) * kUBoxBytes + sw128(row_in_tile, j & 7));
+                                const __half2* h = reinterpret_cast<const __half2*>(&v);
+                                __half2 s = __hmul2(h[0], h[0]);
+                                s = __hfma2(h[1], h[1], s), s = __hfma2(h[2], h[2], s), s = __hfma2(h[3], h[3], s);
+                                const float2 f = __half22float2(s);
+                                xn += f.x + f.y;
                             }
+                        }
+                        // near-ties: only a centre whose distance lies inside the bound can win; the warp forms the exact
+                        // FP32 sums of those few (same arithmetic, same order as `nearest`), one tied token at a time
+                        const float bound = kTieBound * (1.01f * xn + cmax);
+                        uint32_t inside = 0u;
+                        if (live && !((d2 - d1) > bound)) {
 #pragma unroll
-                            for (int off = 16; off > 0; off >>= 1) acc = acc + __shfl_xor_sync(kFull, acc, off);
-                            if (acc < best) best = acc, bc = c;
+                            for (int c = 0; c < 32; ++c) inside |= !((d[c] - d1) > bound) ? 1u << c : 0u;
                         }
-                        if (lane == src) c1 = bc;
-                    }
-                    if (live) {
-                        if (last) {
-                            ids_u[row] = c1;
-                            if (ids8_u) ids8_u[row] = static_cast<int8_t>(c1);
-                        } else if (first) {
-                            ids_u[row] = __float_as_int(xn);
+                        uint32_t redo = __ballot_sync(kFull, inside != 0u);
+                        while (redo) {
+                            const int src = __ffs(redo) - 1;
+                            redo &= redo - 1;
+                            uint32_t cands = __shfl_sync(kFull, inside, src) & (p.clusters >= 32 ? 0xffffffffu : (1u << p.clusters) - 1u);
+                            const __half* xr = xu + static_cast<size_t>(tile_row + quarter * 32 + src) * kHeadDim;
+                            float xv[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) xv[k] = __half2float(xr[lane + 32 * k]);
+                            float best = INFINITY;
+                            int bc = 0;
+                            while (cands) {  // ascending centre index: the lower one wins ties
+                                const int c = __ffs(cands) - 1;
+                                cands &= cands - 1;
+                                const float* crow = cen_s + c * kHeadDim;
+                                float acc = 0.f;
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float df = xv[e] - crow[lane + 32 * e];
+                                    acc = fmaf(df, df, acc);
+                                }
+#pragma unroll
+                                for (int off = 16; off > 0; off >>= 1) acc = acc + __shfl_xor_sync(kFull, acc, off);
+                                if (acc < best) best = acc, bc = c;
+                            }
+                            if (lane == src) c1 = bc;
                         }
-                        atomicAdd(&cnt_s[c1], 1);
+                        if (live) {
+                            if (last) {
+                                ids_u[row] = c1;
+                                if (ids8_u) ids8_u[row] = static_cast<int8_t>(c1);
+                            } else if (first) {
+                                ids_u[row] = __float_as_int(xn);
+                            }
+                            atomicAdd(&cnt_s[c1], 1);
+                        }
+                        // one-hot buffer g was last read by the sums of tile q - 3
+                        if (q >= kUGroups) lost |= !mbar_wait(&bar_sums[g], (use - 1) & 1);
+                        unsigned char* ob = oh + g * kUOneHotBytes;
+                        if (prev >= 0) *reinterpret_cast<unsigned short*>(ob + prev) = 0;
+                        prev = -1;
+                        if (live) {
+                            prev = (row_in_tile >> 6) * (32 * 128) + sw128(c1, (row_in_tile & 63) >> 3) + ((row_in_tile & 7) << 1);
+                            *reinterpret_cast<unsigned short*>(ob + prev) = 0x3C00;  // 1.0
+                        }
+                        proxy_fence();  // the tensor core (async proxy) reads what this thread wrote
+                        mbar_arrive(&bar_onehot[g]);
                     }
-                    // one-hot buffer g was last read by the sums of tile q - 3
-                    if (q >= kUGroups) lost |= !mbar_wait(&bar_sums[g], (use - 1) & 1);
-                    unsigned char* ob = oh + g * kUOneHotBytes;
-                    if (prev >= 0) *reinterpret_cast<unsigned short*>(ob + prev) = 0;
-                    prev = -1;
-                    if (live) {
-                        prev = (row_in_tile >> 6) * (32 * 128) + sw128(c1, (row_in_tile & 63) >> 3) + ((row_in_tile & 7) << 1);
-                        *reinterpret_cast<unsigned short*>(ob + prev) = 0x3C00;  // 1.0
+                } else if (warp == kWarpDist) {
+                    // ---- distance MMAs (whole warp, one elected lane per tile): tile q goes to buffer q % 3 as soon as
+                    // the group has read tile q - 3 out of it ----------------------------------------------------------
+                    const uint64_t a0 = umma_desc(smem_u32(xs), 16, 1024), b0 = umma_desc(smem_u32(cop), 16, 1024);
+                    const uint32_t idesc = value ? umma_idesc(32, false) : umma_idesc(64, false);  // V's centres have no lo half
+                    for (int i = 0; i < n_tiles; ++i) {
+                        const int q = q0 + i, buf = q % kUGroups;
+                        if (q >= kUGroups) lost |= !mbar_wait(&bar_dist_free[buf], (q / kUGroups - 1) & 1);
+                        lost |= !mbar_wait(&bar_full[q % kUStages], (q / kUStages) & 1);
+                        tc_fence_after();
+                        const uint64_t a = a0 + static_cast<uint64_t>(((q % kUStages) * kUTileBytes) >> 4);
+                        const uint32_t d = tmem + kUColD + buf * 64;
+                        if (elect_one()) {  // the eight MMAs and their commit in one elected stretch
+#pragma unroll
+                            for (int ks = 0; ks < 8; ++ks) {  // 16 coordinates per step: 32 bytes inside the swizzled 128-byte row
+                                const uint64_t ak = a + static_cast<uint64_t>(((ks >> 2) * kUBoxBytes + (ks & 3) * 32) >> 4);
+                                const uint64_t bk = b0 + static_cast<uint64_t>(((ks >> 2) * (kN * 128) + (ks & 3) * 32) >> 4);
+                                umma_f16(d, ak, bk, idesc, ks > 0);
+                            }
+                            umma_commit(&bar_dist[buf]);
+                        }
+                        __syncwarp();
                     }
-                    proxy_fence();  // the tensor core (async proxy) reads what this thread wrote
-                    mbar_arrive(&bar_onehot[g]);
+                } else {
+                    // ---- sum MMAs: the first four tiles of a segment start the four accumulators ----------------------
+                    const uint64_t a0 = umma_desc(smem_u32(xs), kUBoxBytes, 1024);  // MN-major: other half of the coordinates at LBO
+                    const uint64_t b0 = umma_desc(smem_u32(oh), 16, 1024);
+                    for (int i = 0; i < n_tiles; ++i) {
+                        const int q = q0 + i, buf = q % kUGroups;
+                        const uint64_t a = a0 + static_cast<uint64_t>(((q % kUStages) * kUTileBytes) >> 4);
+                        const uint64_t o = b0 + static_cast<uint64_t>((buf * kUOneHotBytes) >> 4);
+                        const uint32_t d = tmem + kUColS + (q % kUSumBuffers) * 32;
+                        lost |= !mbar_wait(&bar_onehot[buf], (q / kUGroups) & 1);
+                        tc_fence_after();
+                        if (elect_one()) {
+#pragma unroll
+                            for (int ks = 0; ks < 8; ++ks) {  // 16 tokens per step: two 8-row groups of the tile = 2048 bytes
+                                const uint64_t ak = a + static_cast<uint64_t>((ks * 2048) >> 4);
+                                const uint64_t bk = o + static_cast<uint64_t>(((ks >> 2) * (32 * 128) + (ks & 3) * 32) >> 4);
+                                umma_f16(d, ak, bk, umma_idesc(32, true), (i >= kUSumBuffers || ks > 0) ? 1u : 0u);
+                            }
+                            umma_commit(&bar_sums[buf]);
+                            umma_commit(&bar_empty[q % kUStages]);
+                        }
+                        __syncwarp();
+                    }
                 }
-            } else if (warp == kWarpDist) {
-                // ---- distance MMAs (whole warp, one elected lane per tile): tile q goes to buffer q % 3 as soon as
-                // the group has read tile q - 3 out of it ----------------------------------------------------------
-                const uint64_t a0 = umma_desc(smem_u32(xs), 16, 1024), b0 = umma_desc(smem_u32(cop), 16, 1024);
-                const uint32_t idesc = value ? umma_idesc(32, false) : umma_idesc(64, false);  // V's centres have no lo half
-                for (int i = 0; i < n_tiles; ++i) {
-                    const int q = q0 + i, buf = q % kUGroups;
-                    if (q >= kUGroups) lost |= !mbar_wait(&bar_dist_free[buf], (q / kUGroups - 1) & 1);
-                    lost |= !mbar_wait(&bar_full[q % kUStages], (q / kUStages) & 1);
+                // ---- end of the segment: its sums go out (the commit of the last sum MMAs covers all of them) -----------
+                // The wait stands behind the barrier: a parity tells two neighbouring phases apart, and only once the last tile's
+                // group has come this far is the phase before the awaited one over for sure.
+                const bool flusher = warp < 2 * kUGroupWarps;  // groups 0 and 1: coordinate row_in_tile, sixteen clusters each
+                workers_sync();
+                if (flusher) {
+                    const int q_last = q0 + n_tiles - 1;
+                    lost |= !mbar_wait(&bar_sums[q_last % kUGroups], (q_last / kUGroups) & 1);
                     tc_fence_after();
-                    const uint64_t a = a0 + static_cast<uint64_t>(((q % kUStages) * kUTileBytes) >> 4);
-                    const uint32_t d = tmem + kUColD + buf * 64;
-                    if (elect_one()) {  // the eight MMAs and their commit in one elected stretch
+                    const int half = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
+                    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+                    long long* sums_g = p.sums[it % 3] + row0 * kHeadDim;
+                    float acc[kUSumBuffers][16];  // all requested together
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {  // 16 coordinates per step: 32 bytes inside the swizzled 128-byte row
-                            const uint64_t ak = a + static_cast<uint64_t>(((ks >> 2) * kUBoxBytes + (ks & 3) * 32) >> 4);
-                            const uint64_t bk = b0 + static_cast<uint64_t>(((ks >> 2) * (kN * 128) + (ks & 3) * 32) >> 4);
-                            umma_f16(d, ak, bk, idesc, ks > 0);
-                        }
-                        umma_commit(&bar_dist[buf]);
-                    }
-                    __syncwarp();
-                }
-            } else {
-                // ---- sum MMAs: the first four tiles of a segment start the four accumulators ----------------------
-                const uint64_t a0 = umma_desc(smem_u32(xs), kUBoxBytes, 1024);  // MN-major: other half of the coordinates at LBO
-                const uint64_t b0 = umma_desc(smem_u32(oh), 16, 1024);
-                for (int i = 0; i < n_tiles; ++i) {
-                    const int q = q0 + i, buf = q % kUGroups;
-                    const uint64_t a = a0 + static_cast<uint64_t>(((q % kUStages) * kUTileBytes) >> 4);
-                    const uint64_t o = b0 + static_cast<uint64_t>((buf * kUOneHotBytes) >> 4);
-                    const uint32_t d = tmem + kUColS + (q % kUSumBuffers) * 32;
-                    lost |= !mbar_wait(&bar_onehot[buf], (q / kUGroups) & 1);
-                    tc_fence_after();
-                    if (elect_one()) {
+                    for (int a = 0; a < kUSumBuffers; ++a)  // one that no tile has used is read and not added
+                        tmem_ld16(tmem + lane_base + kUColS + ((q0 + a) % kUSumBuffers) * 32 + 16 * half, acc[a]);
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {  // 16 tokens per step: two 8-row groups of the tile = 2048 bytes
-                            const uint64_t ak = a + static_cast<uint64_t>((ks * 2048) >> 4);
-                            const uint64_t bk = o + static_cast<uint64_t>(((ks >> 2) * (32 * 128) + (ks & 3) * 32) >> 4);
-                            umma_f16(d, ak, bk, umma_idesc(32, true), (i >= kUSumBuffers || ks > 0) ? 1u : 0u);
+                    for (int a = 0; a < kUSumBuffers; ++a) tmem_ld_wait(acc[a]);
+#pragma unroll
+                    for (int a = 1; a < kUSumBuffers; ++a)  // added in the order they were started
+                        if (a < n_tiles) {
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) acc[0][k] += acc[a][k];
                         }
-                        umma_commit(&bar_sums[buf]);
-                        umma_commit(&bar_empty[q % kUStages]);
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        const int c = 16 * half + k;
+                        if (c >= p.clusters || (cnt_s[c] == 0 && !writes)) continue;
+                        const long long sum = cnt_s[c] > 0 ? __float2ll_rn(acc[0][k] * kFix) : 0;
+                        long long* at = sums_g + c * kHeadDim + row_in_tile;
+                        if (writes)
+                            *at = sum;
+                        else
+                            atomicAdd(reinterpret_cast<unsigned long long*>(at), static_cast<unsigned long long>(sum));
                     }
-                    __syncwarp();
                 }
-            }
-            // ---- end of the segment: its sums go out (the commit of the last sum MMAs covers all of them) -----------
-            // The wait stands behind the barrier: a parity tells two neighbouring phases apart, and only once the last tile's
-            // group has come this far is the phase before the awaited one over for sure.
-            const bool flusher = warp < 2 * kUGroupWarps;  // groups 0 and 1: coordinate row_in_tile, sixteen clusters each
-            workers_sync();
-            if (flusher) {
-                const int q_last = q0 + n_tiles - 1;
-                lost |= !mbar_wait(&bar_sums[q_last % kUGroups], (q_last / kUGroups) & 1);
+                if (tid < p.clusters) {
+                    int* at = &p.counts[it % 3][row0 + tid];
+                    if (writes)
+                        *at = cnt_s[tid];
+                    else if (cnt_s[tid] > 0)
+                        atomicAdd(at, cnt_s[tid]);
+                }
+                tc_fence_before();
+                workers_sync();  // accumulators, counters and the centre tables are free for the next segment
                 tc_fence_after();
-                const int half = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
-                const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-                long long* sums_g = p.sums[p.iteration % 3] + row0 * kHeadDim;
-#pragma unroll
-                for (int part = 0; part < 2; ++part) {
-                    float sum[8];  // the accumulators added in the order they were started
-                    tmem_ld8(tmem + lane_base + kUColS + (q0 % kUSumBuffers) * 32 + 16 * half + 8 * part, sum);
-                    tmem_ld_wait();
-                    for (int a = 1; a < kUSumBuffers && a < n_tiles; ++a) {
-                        float more[8];
-                        tmem_ld8(tmem + lane_base + kUColS + ((q0 + a) % kUSumBuffers) * 32 + 16 * half + 8 * part, more);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) sum[k] += more[k];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int c = 16 * half + 8 * part + k;
-                        if (c < p.clusters && cnt_s[c] > 0)
-                            atomicAdd(reinterpret_cast<unsigned long long*>(sums_g + c * kHeadDim + row_in_tile),
-                                      static_cast<unsigned long long>(__float2ll_rn(sum[k] * kFix)));
-                    }
+                if (warp == kWarpDist + 1 && lane == 0 && !owned) {  // (the warp whose next step is the farthest)
+                    __threadfence();
+                    atomicAdd(p.arrived + unit, 1);
                 }
+                q0 += n_tiles;
+                w = w_next;
+                if (back ? w > work_begin : w < work_end) sg = next_s;
             }
-            if (tid < p.clusters && cnt_s[tid] > 0) atomicAdd(&p.counts[p.iteration % 3][row0 + tid], cnt_s[tid]);
-            tc_fence_before();
-            workers_sync();  // accumulators, counters and the centre tables are free for the next segment
-            tc_fence_after();
-            q0 += n_tiles;
-            w += n_tiles;
+        }
+        // ---- FP16 centres of the units that begin here; a warp per centre --------------------------------------------
+        for (int w = work_begin; w < work_end;) {
+            const int unit = w / cuts.tiles_unit, begin = unit * cuts.tiles_unit;
+            w = begin + cuts.tiles_unit;
+            if (begin < work_begin) continue;  // the CTA that has its first tile writes them
+            if (w > work_end) {
+                if (tid == 0) lost |= !wait_for_segments(p.arrived + unit, p.iterations * segments_of(cuts, unit));
+                workers_sync();
+            }
+            const int side = unit < p.units ? 0 : 1;
+            for (int c = warp; c < p.clusters; c += kUWorkers / 32) {
+                const size_t row = static_cast<size_t>(unit) * p.clusters + c;
+                const float4 v = new_centre(p, load_sums(p, p.iterations - 1, row, lane), p.iterations - 1, p.value[side] != 0, row, lane);
+                const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+                reinterpret_cast<uint2*>(p.out[side] + (row - static_cast<size_t>(side) * p.units * p.clusters) * kHeadDim)[lane] =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
         }
     }
     if (lost) atomicOr(p.status, RESKV_STATUS_WAIT_TIMEOUT);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kUTmemCols) : "memory");
-}
-
-// FP16 centres after the last iteration of the tcgen05 form; a warp per centre.
-__global__ void __launch_bounds__(256) kmeans_final_kernel(const UmmaParams p, __half* out0, __half* out1) {
-    wait_for_previous_launch();
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, rows = p.units * p.clusters;
-    if (row >= p.sides * rows) return;
-    const int side = row < rows ? 0 : 1;
-    const float4 c = new_centre(p, p.iterations - 1, p.value[side] != 0, row, lane);
-    const __half2 lo = __floats2half2_rn(c.x, c.y), hi = __floats2half2_rn(c.z, c.w);
-    reinterpret_cast<uint2*>((side ? out1 : out0) + static_cast<size_t>(row - side * rows) * kHeadDim)[lane] =
-        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 // New centres from the exact sums; clears sums and counts for the next round.
@@ -1053,11 +1145,12 @@ void linspace_indices(int t, int count, int* out) {
     }
 }
 
-// 256 bytes whose first word is the status word, then three generations of sums, two of centres, three of counts (the
-// mma.sync form uses the first of each)
+// 256 bytes whose first word is the status word, flushed segments per unit, then three generations of counts, three of sums,
+// two of centres (the mma.sync form uses the first of each).  What a call starts from as zeros lies in front.
+constexpr size_t round16(size_t bytes) { return (bytes + 15) / 16 * 16; }
 size_t kmeans_ws_bytes(int units, int clusters) {
     const size_t per = static_cast<size_t>(units) * clusters;
-    return 256 + per * kHeadDim * (3 * sizeof(long long) + 2 * sizeof(float)) + 3 * per * sizeof(int);
+    return 256 + round16(units * sizeof(int)) + 3 * round16(per * sizeof(int)) + per * kHeadDim * (3 * sizeof(long long) + 2 * sizeof(float));
 }
 
 using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -1093,12 +1186,15 @@ int token_map(CUtensorMap* map, const __half* x, int tokens, int units, int64_t 
 }
 
 // The workspace's arrays for `units` units (all sides together).
-void place_state(UmmaParams& p, void* workspace, size_t per) {
+void place_state(UmmaParams& p, void* workspace, int units, int clusters) {
+    const size_t per = static_cast<size_t>(units) * clusters;
     unsigned char* at = static_cast<unsigned char*>(workspace) + 256;
     p.status = static_cast<uint32_t*>(workspace);
+    p.arrived = reinterpret_cast<int*>(at), at += round16(units * sizeof(int));
+    p.counts[0] = reinterpret_cast<int*>(at), at += round16(per * sizeof(int));
     for (int i = 0; i < 3; ++i, at += per * kHeadDim * sizeof(long long)) p.sums[i] = reinterpret_cast<long long*>(at);
     for (int i = 0; i < 2; ++i, at += per * kHeadDim * sizeof(float)) p.centres[i] = reinterpret_cast<float*>(at);
-    for (int i = 0; i < 3; ++i, at += per * sizeof(int)) p.counts[i] = reinterpret_cast<int*>(at);
+    for (int i = 1; i < 3; ++i, at += round16(per * sizeof(int))) p.counts[i] = reinterpret_cast<int*>(at);
 }
 
 // Tiles per CTA of a call for one side, which is also where its tiles are cut.  One CTA per SM, every CTA an equal share of
@@ -1165,10 +1261,11 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     CUtensorMap maps[2];
     for (int i = 0; i < 2; ++i)  // one side: the second map repeats the first and is not used
         if (int rc = token_map(&maps[i], p.x[i < p.sides ? i : 0], p.tokens, p.units, p.x_stride[i < p.sides ? i : 0])) return rc;
+    p.out[0] = static_cast<__half*>(centroids0), p.out[1] = static_cast<__half*>(centroids1);
+    // status, flushed segments, and what the first iteration adds to; every iteration zeroes the next one's
     const size_t per = static_cast<size_t>(p.sides) * p.units * p.clusters;
-    // the first iteration adds to the first generation; every iteration zeroes the next one
-    if (int rc = check_cuda(cudaMemsetAsync(p.status, 0, 256 + per * kHeadDim * sizeof(long long), s), "kmeans: memset")) return rc;
-    if (int rc = check_cuda(cudaMemsetAsync(p.counts[0], 0, per * sizeof(int), s), "kmeans: memset")) return rc;
+    const size_t zeros = reinterpret_cast<unsigned char*>(p.sums[0] + per * kHeadDim) - reinterpret_cast<unsigned char*>(p.status);
+    if (int rc = check_cuda(cudaMemsetAsync(p.status, 0, zeros, s), "kmeans: memset")) return rc;
     constexpr int kN = 64;
     const size_t smem = 1024 + static_cast<size_t>(kUStages) * kUTileBytes + 2 * kN * 128 + kUGroups * kUOneHotBytes +
                         32 * kHeadDim * sizeof(float) + 32 * (sizeof(float) + sizeof(int));
@@ -1180,14 +1277,14 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     cuts.piece = side_share(cuts.tiles_side, cuts.tiles_unit);
     const int share = p.sides == 2 ? pair_share(cuts) : cuts.piece;
     const dim3 grid(static_cast<unsigned>((cuts.tiles + share - 1) / share));
-    for (p.iteration = 0; p.iteration < p.iterations; ++p.iteration)
-        if (int rc = check_cuda(launch_overlapped(kmeans_assign_umma_kernel, grid, kUThreads, smem, s, p.iteration > 0, p, maps[0], maps[1],
-                                                  cuts, share), "kmeans_assign launch"))
-            return rc;
-    if (int rc = check_cuda(launch_overlapped(kmeans_final_kernel, dim3(static_cast<unsigned>((per + 7) / 8)), 256, 0, s, true, p,
-                                              static_cast<__half*>(centroids0), static_cast<__half*>(centroids1)), "kmeans_final launch"))
-        return rc;
-    return check_cuda(cudaGetLastError(), "kmeans launch");
+    // cooperative: CTAs wait for one another between iterations, so all of them have to be resident
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = dim3(kUThreads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr, cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kmeans_assign_umma_kernel, p, maps[0], maps[1], cuts, share), "kmeans launch");
 }
 
 }  // namespace
@@ -1217,7 +1314,7 @@ extern "C" int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, 
     KmeansParams p{};
     p.x = static_cast<const __half*>(x);
     UmmaParams u{};
-    place_state(u, workspace, static_cast<size_t>(units) * clusters);
+    place_state(u, workspace, units, clusters);
     p.sums = u.sums[0], p.centres = u.centres[0], p.counts = u.counts[0], p.status = u.status;
     p.ids = ids;
     p.x_stride = x_tok_stride;
@@ -1291,7 +1388,7 @@ extern "C" int reskv_kmeans_pair(const void* x_k, const void* x_v, int batch, in
     if (int rc = check_device_pointer(x_k, "kmeans_pair", "x_k")) return rc;
     if (int rc = check_device_pointer(x_v, "kmeans_pair", "x_v")) return rc;
     UmmaParams u{};
-    place_state(u, workspace, static_cast<size_t>(2 * units) * clusters);
+    place_state(u, workspace, 2 * units, clusters);
     u.x[0] = static_cast<const __half*>(x_k), u.x[1] = static_cast<const __half*>(x_v);
     u.x_stride[0] = k_tok_stride, u.x_stride[1] = v_tok_stride;
     u.ids[0] = k_ids, u.ids[1] = v_ids, u.ids8[0] = static_cast<int8_t*>(k_ids8), u.ids8[1] = static_cast<int8_t*>(v_ids8);
