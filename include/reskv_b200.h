@@ -234,6 +234,20 @@ int reskv_rope_prompt(const void* qkv, int batch, int tokens, int q_heads, int k
 
 int reskv_silu_mul(const void* gate_up, void* out, int rows, int ffn, void* stream);
 
+/* ---- linear layers of a decode step ------------------------------------------------------
+ * out = x . weight^T for 1 to 8 rows of x [rows, k] and weight [n, k] (f16, row-major, FP32 sums, one rounding).
+ * norm_weight [k] or NULL: x is replaced by its RMS norm first (as reskv_rms_norm).
+ * mode 0: out f16 [rows, n].  1: out += product (out f16 holds the residual).  2: weight [2 n, k] holds gate and
+ * up rows, out f16 [rows, n] = silu(gate) * up (as reskv_silu_mul).  3: out f32 [rows, n], rounded to f16 before.
+ * k % 512 == 0, n % 16 == 0 (mode 2: n % 8), x within shared memory: reskv_skinny_linear_fits tells (1 or 0), and
+ * other sizes return RESKV_ERR_LIMIT.  Pointers 16-byte aligned.  The launch may read `weight` while the kernel in
+ * front of it in the stream is still running: that kernel must not write it unless it is an ordinary launch.
+ * reskv_skinny_linear_status: RESKV_STATUS_* bits of all calls on the device so far (synchronises the stream). */
+int reskv_skinny_linear_fits(int rows, int n, int k, int mode);
+int reskv_skinny_linear(const void* x, const void* norm_weight, float eps, const void* weight, void* out, int rows, int n,
+                        int k, int mode, void* stream);
+int reskv_skinny_linear_status(uint32_t* status, void* stream);
+
 /* ---- decode attention for callers that cannot provide scratch memory -------------------
  * No counterpart in the reference (its ops allocate their partial buffers with
  * torch::empty on every call, cluster_mass.cu:1222-1232).

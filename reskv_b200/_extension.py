@@ -72,6 +72,9 @@ SIGNATURES = {
     "reskv_rope_split": (_I, [_P, _I, _I, _I, _P, _P] + [_P] * 7 + [_I, _P]),
     "reskv_rope_prompt": (_I, [_P, _I, _I, _I, _I] + [_P] * 7),
     "reskv_silu_mul": (_I, [_P, _P, _I, _I, _P]),
+    "reskv_skinny_linear_fits": (_I, [_I, _I, _I, _I]),
+    "reskv_skinny_linear": (_I, [_P, _P, _F, _P, _P, _I, _I, _I, _I, _P]),
+    "reskv_skinny_linear_status": (_I, [_P, _P]),
     "reskv_decode_auto_splits": (_I, [_I, _I, _I]),
     "reskv_decode_noalloc_status": (_I, [_P, _P]),
     "reskv_decode_set_variant": (_I, [_I]),

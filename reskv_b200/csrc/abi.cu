@@ -1,7 +1,7 @@
 // Error reporting and device queries shared by every entry point.
 #include <cstring>
 
-#include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace reskv {
 namespace {
@@ -52,6 +52,37 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+namespace {
+using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                       const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                       CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's tensor-map encoder, looked up once through the runtime (no link against libcuda).
+TensorMapEncodeFn tensor_map_encoder() {
+    static const TensorMapEncodeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<TensorMapEncodeFn>(f);
+    }();
+    return fn;
+}
+}  // namespace
+
+int encode_tensor_map(CUtensorMap* map, const void* x, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                      CUtensorMapSwizzle swizzle, const char* who) {
+    TensorMapEncodeFn encode = tensor_map_encoder();
+    if (!encode) return fail(RESKV_ERR_CUDA, "%s: the driver offers no cuTensorMapEncodeTiled", who);
+    const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    const CUresult made = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(x), dims, strides,
+                                 box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (made != CUDA_SUCCESS) return fail(RESKV_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed with code %d", who, static_cast<int>(made));
+    return RESKV_OK;
 }
 }  // namespace reskv
 

@@ -24,11 +24,11 @@
 //
 // K flavour: FP32 centres, an empty cluster keeps its centre.
 // V flavour: centres rounded to FP16 after every update, an empty cluster becomes 0.
-#include <cuda.h>  // CUtensorMap and its enums; the encoder itself is looked up at run time
 
 #include <initializer_list>
 
 #include "common.cuh"
+#include "tensor_map.cuh"
 #include "tmem.cuh"
 
 namespace reskv {
@@ -532,15 +532,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// One box of a rank-3 tensor map (coordinate, token, unit) -> shared memory, completion counted on `bar`.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
 
 // Byte offset of 16-byte piece `piece` (0..7) of row `row` in a [rows][128 B] block with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t sw128(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
@@ -1153,36 +1144,13 @@ size_t kmeans_ws_bytes(int units, int clusters) {
     return 256 + round16(units * sizeof(int)) + 3 * round16(per * sizeof(int)) + per * kHeadDim * (3 * sizeof(long long) + 2 * sizeof(float));
 }
 
-using TensorMapEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                       const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                       CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver's tensor-map encoder, looked up once through the runtime (no link against libcuda).
-TensorMapEncodeFn tensor_map_encoder() {
-    static const TensorMapEncodeFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess ||
-            found != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<TensorMapEncodeFn>(f);
-    }();
-    return fn;
-}
-
 // x as (coordinate, token, unit): boxes of 64 coordinates x 128 tokens, 128-byte swizzle, zeros beyond the last token of
 // a unit
 int token_map(CUtensorMap* map, const __half* x, int tokens, int units, int64_t x_stride) {
-    TensorMapEncodeFn encode = tensor_map_encoder();
-    if (!encode) return fail(RESKV_ERR_CUDA, "kmeans: the driver offers no cuTensorMapEncodeTiled");
     const cuuint64_t dims[3] = {kHeadDim, static_cast<cuuint64_t>(tokens), static_cast<cuuint64_t>(units)};
     const cuuint64_t strides[2] = {kHeadDim * sizeof(__half), static_cast<cuuint64_t>(x_stride) * kHeadDim * sizeof(__half)};
-    const cuuint32_t box[3] = {64, kUTile, 1}, elem[3] = {1, 1, 1};
-    const CUresult made = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(x), dims, strides, box, elem,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (made != CUDA_SUCCESS) return fail(RESKV_ERR_CUDA, "kmeans: cuTensorMapEncodeTiled failed with code %d", static_cast<int>(made));
-    return RESKV_OK;
+    const cuuint32_t box[3] = {64, kUTile, 1};
+    return encode_tensor_map(map, x, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "kmeans");
 }
 
 // The workspace's arrays for `units` units (all sides together).

@@ -350,9 +350,24 @@ class ResKVLlama:
         def ptr(t):
             return None if t is None else t.data_ptr()
 
+        def streamed(x, weight, n, mode, out, norm_weight=None):
+            """The library's own weight stream, for few rows; False where it does not take the sizes."""
+            if not lib.reskv_skinny_linear_fits(b, n, x.shape[-1], mode):
+                return False
+            check(lib.reskv_skinny_linear(x.data_ptr(), ptr(norm_weight), float(self.shape.rms_eps), weight.data_ptr(),
+                                          out.data_ptr(), b, n, x.shape[-1], mode, stream))
+            return True
+
+        def linear(x, weight, norm_weight):
+            """norm(x) @ weight^T"""
+            out = half(b, weight.shape[0])
+            return out if streamed(x, weight, weight.shape[0], 0, out, norm_weight) else F.linear(norm(x, norm_weight), weight)
+
         def project(x, inp, weight):
             """x + inp @ weight^T, summed over the tensor-parallel group."""
             if self.tp == 1:
+                if streamed(inp, weight, d, 1, x):
+                    return x
                 return x.addmm_(inp, weight.t())  # in place: no copy of x in front of the product
             return x + self._all_reduce(F.linear(inp, weight))
 
@@ -361,7 +376,7 @@ class ResKVLlama:
         check(lib.reskv_step_advance(state, 1, 1 if reskv else 0, stream))
         x = self.embed[tok]
         for index, (layer, cache) in enumerate(zip(self.layers, self.caches)):
-            qkv = F.linear(norm(x, layer["norm1"]), layer["wqkv"])
+            qkv = linear(x, layer["wqkv"], layer["norm1"])
             q_rot = half(b * self.h_q, 128)
             if reskv:
                 cap = cache.keys.shape[2]
@@ -398,12 +413,16 @@ class ResKVLlama:
             else:
                 raise RuntimeError("graph decode of the dense baseline needs flash_attn")
             x = project(x, att, layer["wo"])
-            gate_up = F.linear(norm(x, layer["norm2"]), layer["w_gate_up"])
             act = half(b, self.ffn)
-            check(lib.reskv_silu_mul(gate_up.data_ptr(), act.data_ptr(), b, self.ffn, stream))
+            if not streamed(x, layer["w_gate_up"], self.ffn, 2, act, layer["norm2"]):
+                gate_up = F.linear(norm(x, layer["norm2"]), layer["w_gate_up"])
+                check(lib.reskv_silu_mul(gate_up.data_ptr(), act.data_ptr(), b, self.ffn, stream))
             x = project(x, act, layer["w_down"])
         if not reskv:
             self._seqlens += 1
+        logits = torch.empty((b, self.lm_head.shape[0]), dtype=torch.float32, device=self.device)
+        if streamed(x, self.lm_head, self.lm_head.shape[0], 3, logits, self.final_norm):
+            return logits
         return F.linear(norm(x, self.final_norm), self.lm_head).float()
 
     @torch.no_grad()
