@@ -491,9 +491,12 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 // is still in L2.  Where a unit's iteration begins, the loads of all sums are in flight together, and the next segment is
 // worked out by a thread that waits anyway.
 //
+// Two segments of a unit in a row are taken without a stop, with accumulators of their own, and flushed together.
+//
 // Measured, clustering of one layer's K and V, 10 iterations, us, one launch per iteration -> now: 64 units x 8128 tokens
-// 578 -> 508, 128 x 3000 517 -> 422, 64 x 2000 221 -> 192, 8 x 1152 105 -> 98, 8 x 8128 (many CTAs per unit) 164 -> 165.
-// Of that the single launch by itself gives 2 %, the order of the tiles 3 to 5, stores in place of atomics 4 to 6.
+// 578 -> 486, 128 x 3000 517 -> 417, 64 x 2000 221 -> 162, 8 x 1152 105 -> 97, 8 x 8128 164 -> 133, 24 x 4870 262 -> 229.
+// Of that at 64 x 8128 the single launch by itself gives 2 %, the order of the tiles 3, the loads together 1, stores in place
+// of atomics and the next segment worked out ahead 6, two segments without a stop 4 (at 8 x 8128 20).
 constexpr int kUGroups = 3;                    // token-owning groups; group g takes the tiles i = g (mod 3)
 constexpr int kUGroupWarps = 4;                // a group: one warp per 32 token rows (TMEM lane quarter)
 constexpr int kUThreads = (kUGroups * kUGroupWarps + 3) * 32;  // + three issuing warps: distance MMAs, sum MMAs, copies
@@ -502,9 +505,10 @@ constexpr int kUStages = 5;
 constexpr int kUBoxBytes = kUTile * 128;       // 128 rows x 64 coordinates
 constexpr int kUTileBytes = 2 * kUBoxBytes;
 constexpr int kUOneHotBytes = 2 * 32 * 128;    // [2 token halves][32 clusters][64 tokens] FP16
-constexpr uint32_t kUTmemCols = 512;           // distances 3 x 64 columns, sums 4 x 32 columns; a power of two
+constexpr uint32_t kUTmemCols = 512;           // distances 3 x 64 columns, sums 2 x 4 x 32 columns; a power of two
 constexpr uint32_t kUColD = 0, kUColS = 192;
-constexpr int kUSumBuffers = 4;                // tile i adds to accumulator i % 4: shorter FP32 chains, no MMA-to-MMA dependency
+constexpr int kUSumBuffers = 4;                // tile i of a segment adds to accumulator i % 4: shorter FP32 chains, no MMA-to-MMA dependency
+constexpr int kURun = 2;                       // segments of a unit that a CTA takes without a stop, accumulators of their own
 constexpr int kUChunkMax = 8192;               // most tokens per CTA (2048 per accumulator)
 
 // Shared-memory matrix descriptor, 128-byte swizzle, address bits [4, 18), leading / stride byte offsets.
@@ -610,6 +614,22 @@ __host__ __device__ inline Segment segment_before(const Cuts& c, int w) {
     const int start = from + (last - from) / kMost * kMost;
     return Segment{unit, start - by_unit, w - start};
 }
+// What a CTA takes without a stop: the segment that comes at tile w in its order of the iteration and, if it belongs to the
+// same unit, the one behind it.  Their sums are kept apart and meet as integers, so the cuts decide them as before.
+struct Run {
+    int unit, tile0, tiles, first_tiles;  // first_tiles: of the segment taken first
+};
+template <bool PAIRS>
+__device__ inline Run run_at(const Cuts& c, int w, bool back, int work_begin, int work_end) {
+    const Segment a = back ? segment_before(c, w) : segment_at(c, w);
+    Run r{a.unit, a.tile0, a.tiles, a.tiles};
+    const int next = back ? w - a.tiles : w + a.tiles, unit0 = a.unit * c.tiles_unit;
+    if (PAIRS && (back ? next > work_begin && next > unit0 : next < work_end && next < unit0 + c.tiles_unit)) {
+        const Segment b = back ? segment_before(c, next) : segment_at(c, next);
+        r.tile0 = back ? b.tile0 : a.tile0, r.tiles += b.tiles;
+    }
+    return r;
+}
 // Segments of a unit.
 __host__ __device__ inline int segments_of(const Cuts& c, int unit) {
     const int begin = unit * c.tiles_unit, in_side = begin % c.tiles_side;
@@ -630,6 +650,8 @@ __device__ __forceinline__ bool wait_for_segments(const int* arrived, int count)
     return false;
 }
 
+// PAIRS: CTAs may have two segments of a unit in a row (a launch that has none is 5 % faster without).
+template <bool PAIRS>
 __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap map0,
                                                                            const __grid_constant__ CUtensorMap map1, const Cuts cuts,
                                                                            int share) {
@@ -641,7 +663,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     unsigned char* oh = cop + 2 * kN * 128;                     // [groups][2 token halves][32 clusters][128 B]
     float* cen_s = reinterpret_cast<float*>(oh + kUGroups * kUOneHotBytes);  // [32][128] FP32 centres (exact re-ranking)
     float* cn_s = cen_s + 32 * kHeadDim;                        // [32] |c|^2, +inf for padding
-    int* cnt_s = reinterpret_cast<int*>(cn_s + 32);             // [32]
+    int* cnt_s = reinterpret_cast<int*>(cn_s + 32);             // [kURun][32]
     // full: tile landed (TMA bytes).  dist / sums: MMAs complete (tcgen05.commit); empty: the same event as sums,
     // counted per stage for the copying warp (a barrier of its own: no later completion can overtake its wait).
     // dist_free: the 128 threads of a group have read their distance buffer.  onehot: they have written their one-hot
@@ -649,7 +671,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
     __shared__ uint64_t bar_full[kUStages], bar_empty[kUStages], bar_dist[kUGroups], bar_dist_free[kUGroups], bar_onehot[kUGroups],
         bar_sums[kUGroups];
     __shared__ uint32_t tmem_base_s;
-    __shared__ Segment next_s;
+    __shared__ Run runs_s[2];  // the run in work and the next one, in turn
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // CTA c takes the pieces that start in [c * share, (c + 1) * share) of all tiles and walks them segment by segment.
@@ -708,14 +730,17 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
         int q0 = 0;     // tiles of the earlier segments of this CTA
         int prev = -1;  // byte offset of the element this thread set in its group's one-hot buffer
         int unit_in_tables = -1, segments = 0;  // unit of the tables, its segments
-        // an iteration ends where the next one begins: its last segment is the next one's first
-        Segment sg = work_begin < work_end ? segment_at(cuts, work_begin) : Segment{};
+        int turn = 0;
+        if (tid == (kWarpDist + 1) * 32 && work_begin < work_end) runs_s[0] = run_at<PAIRS>(cuts, work_begin, false, work_begin, work_end);
+        workers_sync();
         for (int it = 0; it < p.iterations; ++it) {
             const bool first = it == 0, last = it + 1 == p.iterations, back = it & 1;
             bool stale = true;  // the tables are those of the iteration before
             for (int w = back ? work_end : work_begin; back ? w > work_begin : w < work_end;) {
-                const int unit = sg.unit, n_tiles = sg.tiles, w_next = back ? w - n_tiles : w + n_tiles;
-                const int t_begin = sg.tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
+                const int unit = runs_s[turn].unit, n_tiles = runs_s[turn].tiles, tile0 = runs_s[turn].tile0;
+                const int first_tiles = PAIRS ? runs_s[turn].first_tiles : n_tiles, w_next = back ? w - n_tiles : w + n_tiles;
+                const bool two = PAIRS && first_tiles < n_tiles;  // segments
+                const int t_begin = tile0 * kUTile, t_end = min(p.tokens, t_begin + n_tiles * kUTile);
                 const int side = unit < p.units ? 0 : 1, local = unit - side * p.units;
                 const bool value = p.value[side] != 0;
                 const __half* xu = p.x[side] + static_cast<size_t>(local) * p.x_stride[side] * kHeadDim;
@@ -724,7 +749,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                 // the whole unit is this CTA's: its first segment writes the sums instead of adding to zeros (a 64-bit atomic
                 // addition costs eight times a store: 2300 cycles a segment), and no other CTA is waited for
                 const bool owned = opens_unit && (unit + 1) * cuts.tiles_unit <= work_end;
-                const bool writes = owned && (back ? sg.tile0 + n_tiles == cuts.tiles_unit : sg.tile0 == 0);
+                const bool writes = owned && (back ? tile0 + n_tiles == cuts.tiles_unit : tile0 == 0);
                 // ---- per unit: centre operand (FP16 hi | lo rows, swizzled), FP32 centres, |c|^2 ----------------------
                 if (stale || unit != unit_in_tables) {
                     if (unit != unit_in_tables && !owned) segments = segments_of(cuts, unit);
@@ -796,12 +821,19 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     }
                     }
                 }
-                if (tid < 32) cnt_s[tid] = 0;
+                if (tid < (PAIRS ? 64 : 32)) cnt_s[tid] = 0;
                 proxy_fence();  // the operands written above are read by the tensor core (async proxy)
                 workers_sync();
-                // the next segment, by a thread that has to wait for its first tile anyway (four divisions)
-                if (tid == 2 * kUGroupWarps * 32 && (back ? w_next > work_begin : w_next < work_end))
-                    next_s = back ? segment_before(cuts, w_next) : segment_at(cuts, w_next);
+                // the next run, by a thread whose first tile is the farthest; a handful of divisions, unless the CTA has only
+                // this one, which it then takes the other way round
+                if (tid == (kWarpDist + 1) * 32) {
+                    const bool more = back ? w_next > work_begin : w_next < work_end;
+                    if (!more && n_tiles == work_end - work_begin)
+                        runs_s[turn ^ 1] = Run{unit, tile0, n_tiles, two ? n_tiles - first_tiles : n_tiles};
+                    else if (more || !last)
+                        runs_s[turn ^ 1] = more ? run_at<PAIRS>(cuts, w_next, back, work_begin, work_end)
+                                                : run_at<PAIRS>(cuts, back ? work_begin : work_end, !back, work_begin, work_end);
+                }
                 float cmax = lane < p.clusters ? cn_s[lane] : 0.f;  // largest |c|^2, in every thread
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(kFull, cmax, off));
@@ -908,7 +940,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                             } else if (first) {
                                 ids_u[row] = __float_as_int(xn);
                             }
-                            atomicAdd(&cnt_s[c1], 1);
+                            atomicAdd(&cnt_s[(!PAIRS || i < first_tiles ? 0 : 32) + c1], 1);
                         }
                         // one-hot buffer g was last read by the sums of tile q - 3
                         if (q >= kUGroups) lost |= !mbar_wait(&bar_sums[g], (use - 1) & 1);
@@ -953,7 +985,8 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                         const int q = q0 + i, buf = q % kUGroups;
                         const uint64_t a = a0 + static_cast<uint64_t>(((q % kUStages) * kUTileBytes) >> 4);
                         const uint64_t o = b0 + static_cast<uint64_t>((buf * kUOneHotBytes) >> 4);
-                        const uint32_t d = tmem + kUColS + (q % kUSumBuffers) * 32;
+                        const int in_segment = !PAIRS || i < first_tiles ? i : i - first_tiles;
+                        const uint32_t d = tmem + kUColS + ((!PAIRS || i < first_tiles ? 0 : kUSumBuffers) + in_segment % kUSumBuffers) * 32;
                         lost |= !mbar_wait(&bar_onehot[buf], (q / kUGroups) & 1);
                         tc_fence_after();
                         if (elect_one()) {
@@ -961,7 +994,7 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                             for (int ks = 0; ks < 8; ++ks) {  // 16 tokens per step: two 8-row groups of the tile = 2048 bytes
                                 const uint64_t ak = a + static_cast<uint64_t>((ks * 2048) >> 4);
                                 const uint64_t bk = o + static_cast<uint64_t>(((ks >> 2) * (32 * 128) + (ks & 3) * 32) >> 4);
-                                umma_f16(d, ak, bk, umma_idesc(32, true), (i >= kUSumBuffers || ks > 0) ? 1u : 0u);
+                                umma_f16(d, ak, bk, umma_idesc(32, true), (in_segment >= kUSumBuffers || ks > 0) ? 1u : 0u);
                             }
                             umma_commit(&bar_sums[buf]);
                             umma_commit(&bar_empty[q % kUStages]);
@@ -981,47 +1014,76 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     const int half = warp / kUGroupWarps, quarter = warp % kUGroupWarps, row_in_tile = quarter * 32 + lane;
                     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
                     long long* sums_g = p.sums[it % 3] + row0 * kHeadDim;
-                    float acc[kUSumBuffers][16];  // all requested together
-#pragma unroll
-                    for (int a = 0; a < kUSumBuffers; ++a)  // one that no tile has used is read and not added
-                        tmem_ld16(tmem + lane_base + kUColS + ((q0 + a) % kUSumBuffers) * 32 + 16 * half, acc[a]);
-#pragma unroll
-                    for (int a = 0; a < kUSumBuffers; ++a) tmem_ld_wait(acc[a]);
-#pragma unroll
-                    for (int a = 1; a < kUSumBuffers; ++a)  // added in the order they were started
-                        if (a < n_tiles) {
-#pragma unroll
-                            for (int k = 0; k < 16; ++k) acc[0][k] += acc[a][k];
-                        }
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        const int c = 16 * half + k;
-                        if (c >= p.clusters || (cnt_s[c] == 0 && !writes)) continue;
-                        const long long sum = cnt_s[c] > 0 ? __float2ll_rn(acc[0][k] * kFix) : 0;
+                    const auto put = [&](int c, long long sum) {
                         long long* at = sums_g + c * kHeadDim + row_in_tile;
                         if (writes)
                             *at = sum;
                         else
                             atomicAdd(reinterpret_cast<unsigned long long*>(at), static_cast<unsigned long long>(sum));
+                    };
+                    if (two) {
+#pragma unroll
+                        for (int part = 0; part < 2; ++part) {  // eight clusters at a time
+                            const int c0 = 16 * half + 8 * part;
+                            float acc[2 * kUSumBuffers][8];
+#pragma unroll
+                            for (int a = 0; a < 2 * kUSumBuffers; ++a) tmem_ld8(tmem + lane_base + kUColS + a * 32 + c0, acc[a]);
+#pragma unroll
+                            for (int a = 0; a < 2 * kUSumBuffers; ++a) tmem_ld_wait(acc[a]);
+#pragma unroll
+                            for (int a = 1; a < kUSumBuffers; ++a) {  // added in the order they were started
+#pragma unroll
+                                for (int k = 0; k < 8; ++k) {
+                                    if (a < first_tiles) acc[0][k] += acc[a][k];
+                                    if (a < n_tiles - first_tiles) acc[kUSumBuffers][k] += acc[kUSumBuffers + a][k];
+                                }
+                            }
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                const int c = c0 + k, n0 = cnt_s[c], n1 = cnt_s[32 + c];
+                                if (c >= p.clusters || (!writes && n0 + n1 == 0)) continue;
+                                put(c, (n0 > 0 ? __float2ll_rn(acc[0][k] * kFix) : 0) + (n1 > 0 ? __float2ll_rn(acc[kUSumBuffers][k] * kFix) : 0));
+                            }
+                        }
+                    } else {
+                        float acc[kUSumBuffers][16];  // all requested together
+#pragma unroll
+                        for (int a = 0; a < kUSumBuffers; ++a)  // one that no tile has used is read and not added
+                            tmem_ld16(tmem + lane_base + kUColS + a * 32 + 16 * half, acc[a]);
+#pragma unroll
+                        for (int a = 0; a < kUSumBuffers; ++a) tmem_ld_wait(acc[a]);
+#pragma unroll
+                        for (int a = 1; a < kUSumBuffers; ++a)  // added in the order they were started
+                            if (a < n_tiles) {
+#pragma unroll
+                                for (int k = 0; k < 16; ++k) acc[0][k] += acc[a][k];
+                            }
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) {
+                            const int c = 16 * half + k, n = cnt_s[c];
+                            if (c >= p.clusters || (!writes && n == 0)) continue;
+                            put(c, n > 0 ? __float2ll_rn(acc[0][k] * kFix) : 0);
+                        }
                     }
                 }
                 if (tid < p.clusters) {
                     int* at = &p.counts[it % 3][row0 + tid];
+                    const int n = cnt_s[tid] + (PAIRS ? cnt_s[32 + tid] : 0);
                     if (writes)
-                        *at = cnt_s[tid];
-                    else if (cnt_s[tid] > 0)
-                        atomicAdd(at, cnt_s[tid]);
+                        *at = n;
+                    else if (n > 0)
+                        atomicAdd(at, n);
                 }
                 tc_fence_before();
                 workers_sync();  // accumulators, counters and the centre tables are free for the next segment
                 tc_fence_after();
                 if (warp == kWarpDist + 1 && lane == 0 && !owned) {  // (the warp whose next step is the farthest)
                     __threadfence();
-                    atomicAdd(p.arrived + unit, 1);
+                    atomicAdd(p.arrived + unit, two ? 2 : 1);
                 }
                 q0 += n_tiles;
                 w = w_next;
-                if (back ? w > work_begin : w < work_end) sg = next_s;
+                turn ^= 1;
             }
         }
         // ---- FP16 centres of the units that begin here; a warp per centre --------------------------------------------
@@ -1236,15 +1298,17 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     if (int rc = check_cuda(cudaMemsetAsync(p.status, 0, zeros, s), "kmeans: memset")) return rc;
     constexpr int kN = 64;
     const size_t smem = 1024 + static_cast<size_t>(kUStages) * kUTileBytes + 2 * kN * 128 + kUGroups * kUOneHotBytes +
-                        32 * kHeadDim * sizeof(float) + 32 * (sizeof(float) + sizeof(int));
-    static std::atomic<unsigned long long> done{0};
-    if (int rc = allow_smem(kmeans_assign_umma_kernel, smem, done, "cudaFuncSetAttribute(kmeans_assign_umma)")) return rc;
+                        32 * kHeadDim * sizeof(float) + 32 * (sizeof(float) + kURun * sizeof(int));
     Cuts cuts{};
     cuts.tiles_unit = (p.tokens + kUTile - 1) / kUTile;
     cuts.tiles_side = p.units * cuts.tiles_unit, cuts.tiles = p.sides * cuts.tiles_side;
     cuts.piece = side_share(cuts.tiles_side, cuts.tiles_unit);
     const int share = p.sides == 2 ? pair_share(cuts) : cuts.piece;
     const dim3 grid(static_cast<unsigned>((cuts.tiles + share - 1) / share));
+    const bool pairs = share > cuts.piece && cuts.piece % cuts.tiles_unit != 0;
+    const auto kern = pairs ? kmeans_assign_umma_kernel<true> : kmeans_assign_umma_kernel<false>;
+    static std::atomic<unsigned long long> done[2];
+    if (int rc = allow_smem(kern, smem, done[pairs], "cudaFuncSetAttribute(kmeans_assign_umma)")) return rc;
     // cooperative: CTAs wait for one another between iterations, so all of them have to be resident
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = dim3(kUThreads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
@@ -1252,7 +1316,7 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
     cfg.attrs = &attr, cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kmeans_assign_umma_kernel, p, maps[0], maps[1], cuts, share), "kmeans launch");
+    return check_cuda(cudaLaunchKernelEx(&cfg, kern, p, maps[0], maps[1], cuts, share), "kmeans launch");
 }
 
 }  // namespace
