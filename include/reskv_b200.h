@@ -204,6 +204,12 @@ int reskv_decode_step(int layout, int bits, int nnz, const void* q, const void* 
                       const void* recent_q, const void* window_k, const void* window_v, int window_capacity,
                       const int32_t* step_state, void* workspace, size_t workspace_bytes, void* out, void* stream);
 
+/* Tokens [first, first + count) of a prompt's k_rot, k_raw and v ([batch, kv_heads, T, 128] f16, *_stride tokens between
+ * (sequence, head) units) into the window's slots [slot, slot + count), one launch; all pointers 16-byte aligned. */
+int reskv_window_fill(void* window_k, void* window_raw, void* window_v, const void* k_rot, const void* k_raw, const void* v,
+                      int batch, int kv_heads, int window_capacity, int slot, int64_t k_rot_stride, int64_t k_raw_stride,
+                      int64_t v_stride, int first, int count, void* stream);
+
 int reskv_step_advance(int32_t* step_state, int position_increment, int window_increment, void* stream);
 
 /* ---- the rest of a decoder layer's decode step, fused -----------------------------------

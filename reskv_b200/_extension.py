@@ -63,6 +63,7 @@ SIGNATURES = {
     "reskv_window_append": (_I, [_P] * 6 + [_I, _I, _I, _P, _P]),
     "reskv_window_write": (_I, [_P] * 6 + [_I, _I, _I, _I, _P]),
     "reskv_window_put": (_I, [_P] * 6 + [_I, _I, _I, _I, _P]),
+    "reskv_window_fill": (_I, [_P] * 6 + [_I, _I, _I, _I, _L, _L, _L, _I, _I, _P]),
     "reskv_decode_step": (
         _I,
         [_I, _I, _I] + [_P] * 11 + [_I, _I, _I, _I, _L, _I, _I, _I, _F, _P, _F, _I, _P, _P, _P, _I, _P, _P, _Z, _P, _P],

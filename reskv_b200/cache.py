@@ -113,10 +113,19 @@ class ResKVLayerCache(_HFLayer or _LayerBase):
         self.live = t - n
         if self.live > self.keys.shape[2]:
             raise ValueError("prefill leaves more dense tokens than the window holds")
+        for slot, first, count in ((0, 0, s), (s, s + n, t - n - s)):
+            if count:
+                self._fill(keys, raw, values, slot, first, count)
+
+    def _fill(self, keys, raw, values, slot, first, count):
+        """Tokens [first, first + count) of the prompt into the window from ``slot`` on."""
+        if keys.is_cuda and keys.dtype == torch.float16:
+            from ._extension import host
+
+            if host().window_fill(self.keys, self.raw_keys, self.values, keys, raw, values, slot, first, count):
+                return
         for buf, src in ((self.keys, keys), (self.raw_keys, raw), (self.values, values)):
-            if s:
-                buf[:, :, :s].copy_(src[:, :, :s])
-            buf.narrow(2, s, t - n - s).copy_(src.narrow(2, s + n, t - n - s))
+            buf.narrow(2, slot, count).copy_(src.narrow(2, first, count))
 
     def _take_token(self, key, raw, value):
         """One launch writes the token's rotated key, raw key and value into slot ``live`` of the three

@@ -8,6 +8,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <Python.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -640,6 +641,40 @@ PyObject* py_window_shift(PyObject*, PyObject* const* o, Py_ssize_t n) {
     });
 }
 
+// window_fill(keys, raw_keys, values, key, raw_key, value, slot, first, count) -> bool: tokens [first, first + count) of a
+// prompt's [B,H,T,128] tensors into the window buffers from `slot` on, in one launch; False (nothing done) for tensors that
+// the kernel does not take as they are.
+PyObject* py_window_fill(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        expect(n, 9);
+        const at::Tensor window[3] = {tensor(o[0], "keys"), tensor(o[1], "raw keys"), tensor(o[2], "values")};
+        const at::Tensor src[3] = {tensor(o[3], "key"), tensor(o[4], "raw key"), tensor(o[5], "value")};
+        const int64_t slot = integer(o[6]), first = integer(o[7]), count = integer(o[8]);
+        const c10::DeviceIndex dev = window[0].get_device();
+        const bool grad = c10::GradMode::is_enabled();
+        int64_t stride[3];
+        for (int i = 0; i < 3; ++i) {
+            const at::Tensor& x = src[i];
+            if (!x.is_cuda() || x.get_device() != dev || x.scalar_type() != at::kHalf || window[i].scalar_type() != at::kHalf || x.dim() != 4 ||
+                x.size(0) != window[i].size(0) || x.size(1) != window[i].size(1) || x.size(2) < first + count || !window[i].is_contiguous() ||
+                (grad && x.requires_grad()) || x.is_conj() || x.is_neg())
+                return Py_NewRef(Py_False);
+            stride[i] = token_stride_of(x);
+            if (stride[i] < x.size(2) || !aligned16(x.const_data_ptr()) || !aligned16(window[i].const_data_ptr())) return Py_NewRef(Py_False);
+        }
+        {
+            const Unlocked free;
+            const c10::cuda::CUDAGuard guard(dev);
+            check(reskv_window_fill(window[0].data_ptr(), window[1].data_ptr(), window[2].data_ptr(), src[0].const_data_ptr(), src[1].const_data_ptr(),
+                                    src[2].const_data_ptr(), static_cast<int>(window[0].size(0)), static_cast<int>(window[0].size(1)),
+                                    static_cast<int>(window[0].size(2)), static_cast<int>(slot), stride[0], stride[1], stride[2],
+                                    static_cast<int>(first), static_cast<int>(count), c10::cuda::getCurrentCUDAStream(dev).stream()));
+            ++g_launches;
+        }
+        return Py_NewRef(Py_True);
+    });
+}
+
 // ---- verdicts of take_ids -------------------------------------------------------------------------------------------
 // A word of mapped pinned host memory and an event per call in flight (the event is made for the call's device).  They are
 // kept for later calls of any thread, about kKeptVerdicts of them.  A ticket may be dropped by a finaliser, at any time and
@@ -784,6 +819,7 @@ PyMethodDef g_methods[] = {
     {"kmeans_pair", FAST(py_kmeans_pair), METH_FASTCALL, "cluster K and V in the same launches"},
     {"regrow", FAST(py_regrow), METH_FASTCALL, "larger buffers for a cache"},
     {"append_group", FAST(py_append_group), METH_FASTCALL, "cluster, pack and append one decode group"},
+    {"window_fill", FAST(py_window_fill), METH_FASTCALL, "a prompt's dense tail into the window"},
     {"window_shift", FAST(py_window_shift), METH_FASTCALL, "move tokens of the dense window"},
     {"take_ids", FAST(py_take_ids), METH_FASTCALL, "check and convert given cluster ids"},
     {"ids_in_range", py_ids_in_range, METH_O, "verdict of take_ids"},
