@@ -142,7 +142,7 @@ __device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
 constexpr int kColTrig = 0, kColAcc = 32, kColBeta = 64, kColsWarp = 80, kTmemCols = 512;
 static_assert(kColsWarp * (kWarpsM / 4) <= kTmemCols, "tensor memory");
 
-// A lane quarter's results of one head at the end of a segment: coordinate d at red_pos(d), cluster masses.  The
+// A lane quarter's (one head per KV head: a warp's) results of one head at the end of a segment: coordinate d at red_pos(d), cluster masses.  The
 // strides keep the stores of a warp (lanes g, q; one coordinate of the field) in distinct banks.
 constexpr int kRedAcc = 152, kRedBeta = 72;
 constexpr int kStatsWarp = 64;  // floats between the warps' column maxima and sums (one warp's rank bases)
@@ -153,7 +153,8 @@ __device__ __forceinline__ int red_pos(int d) { return (d & 15) * 9 + (d >> 4); 
 template <int GQA, class ML>
 struct Smem {
     static constexpr size_t kRing = sizeof(WarpRows<ML>) * kWarpsM;
-    static constexpr size_t kRed = static_cast<size_t>(4) * GQA * (kRedAcc + kRedBeta) * sizeof(float);
+    static constexpr size_t kRed =  // warps' or quarters' results
+        (GQA == 1 ? kWarpsM * (kRedAcc + kRedBeta + 2) : 4 * GQA * (kRedAcc + kRedBeta)) * sizeof(float);
     static constexpr size_t kTrig = (kWarpsM + 8) * 64 * sizeof(float2);
     static constexpr size_t kRegion = ((kRing + kTrig > kRed ? kRing + kTrig : kRed) + 127) / 128 * 128;
     static constexpr size_t kQuery = 2 * 2 * query_rows<GQA>() * kQStride * sizeof(__half);  // [buffers][hi, lo][rows]
@@ -246,6 +247,19 @@ struct WalkField {
                 ++hi.ptr;
             }
         }
+    }
+    // The same of one coordinate, the two walks in turn: more instructions, less waiting.
+    __device__ static __forceinline__ uint32_t pair(WalkField& lo, WalkField& hi, int slot) {
+        uint32_t v = 0;
+        if (lo.mask & (0x8000u >> slot)) {
+            v = *reinterpret_cast<const unsigned short*>(lo.ptr);
+            ++lo.ptr;
+        }
+        if (hi.mask & (0x8000u >> slot)) {
+            v = low_halves(v, *reinterpret_cast<const unsigned short*>(hi.ptr));
+            ++hi.ptr;
+        }
+        return v;
     }
     __device__ static __forceinline__ void half_block(int half, WalkField& f0, WalkField& f1, WalkField& f2, WalkField& f3, uint32_t (&a)[4][4]) {
 #pragma unroll
@@ -524,6 +538,9 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
     using Field = typename ML::Field;
     constexpr int kRows = query_rows<GQA>(), kRow = Rows::kRow, kMeta = ML::kMetaBytes;
     constexpr bool kDual = GQA == 8;  // X and Y need all eight columns each: MMAs of their own
+    // One head per KV head, walked layouts: the walks in turn and all accumulators in registers (8 units x 30000 tokens, 64 of
+    // 128 kept: 40.1 us, in groups and halves 41.3; with four heads the groups are faster, see above).
+    constexpr bool kWhole = GQA == 1 && Field::kSlotwise;
     constexpr int kQItems = 2 * GQA;  // rows of the rotated query: X's heads, Y's heads
     float* kc_s = reinterpret_cast<float*>(smem_raw + SM::kRegion);
     __half* qf = reinterpret_cast<__half*>(kc_s + static_cast<size_t>(p.ck) * kCenStride);  // [2 bufs][hi, lo][kRows][kQStride]
@@ -871,15 +888,25 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     float kAl[4] = {al.x, al.y, al.z, al.w}, kAh[4] = {ah.x, ah.y, ah.z, ah.w};
                     float kBl[4] = {bl.x, bl.y, bl.z, bl.w}, kBh[4] = {bh.x, bh.y, bh.z, bh.w};
                     if constexpr (Field::kSlotwise) {
-                        // one field after the other, four coordinates each: their mask bits are tested together
+                        if constexpr (kWhole) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) fAl.add1(4 * ks + e, kAl[e]);
+                            for (int e = 0; e < 4; ++e) {
+                                fAl.add1(4 * ks + e, kAl[e]);
+                                fAh.add1(4 * ks + e, kAh[e]);
+                                fBl.add1(4 * ks + e, kBl[e]);
+                                fBh.add1(4 * ks + e, kBh[e]);
+                            }
+                        } else {
+                            // one field after the other, four coordinates each: their mask bits are tested together
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) fAh.add1(4 * ks + e, kAh[e]);
+                            for (int e = 0; e < 4; ++e) fAl.add1(4 * ks + e, kAl[e]);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) fBl.add1(4 * ks + e, kBl[e]);
+                            for (int e = 0; e < 4; ++e) fAh.add1(4 * ks + e, kAh[e]);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) fBh.add1(4 * ks + e, kBh[e]);
+                            for (int e = 0; e < 4; ++e) fBl.add1(4 * ks + e, kBl[e]);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) fBh.add1(4 * ks + e, kBh[e]);
+                        }
                     } else {
                         fAl.add4(ks, kAl, kscA);
                         fAh.add4(ks, kAh, kscA);
@@ -942,6 +969,8 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             __syncwarp();  // the values have landed
             if (any) {
                 tmem_st_wait();  // last pass's accumulators are in place
+                float whole[kWhole ? 32 : 1];
+                if constexpr (kWhole) tmem_ld32(tmem + kColAcc, whole);
                 // value fields of rows 2q, 2q+1 (X), 2q+8, 2q+9 (Y), coordinates [16g, 16g+16)
                 const unsigned char* pv = reinterpret_cast<const unsigned char*>(pre + 16 + 2 * qd);
                 const unsigned char *pay = rows.vp + 2 * qd * kRow, *met = vm + 2 * qd * kMeta;
@@ -967,16 +996,23 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                         l_part[u] *= alpha[u];
                     }
                     if (it > 0) {  // nothing is summed yet in a segment's first pass
-                        float flat[32], beta[4 * BETA];
-                        tmem_ld32(tmem + kColAcc, flat);
+                        float beta[4 * BETA];
                         tmem_load_beta<BETA>(tmem + kColBeta, beta);
-                        tmem_ld_wait(flat);
+                        if constexpr (kWhole) {
+                            tmem_ld_wait(whole);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) whole[i] *= alpha[i & 1];
+                        } else {
+                            float flat[32];
+                            tmem_ld32(tmem + kColAcc, flat);
+                            tmem_ld_wait(flat);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) flat[i] *= alpha[i & 1];
+                            tmem_st32(tmem + kColAcc, flat);
+                        }
                         tmem_ld_wait(beta);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) flat[i] *= alpha[i & 1];
-#pragma unroll
                         for (int i = 0; i < 4 * BETA; ++i) beta[i] *= alpha[i & 1];
-                        tmem_st32(tmem + kColAcc, flat);
                         tmem_store_beta<BETA>(tmem + kColBeta, beta);
                         tmem_st_wait();
                     }
@@ -1026,18 +1062,29 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     pb0 = movmatrix_trans(as_bits(__floats2half2_rn(p01f.x * vsA, p01f.y * vsA)));
                     pb1 = movmatrix_trans(as_bits(__floats2half2_rn(p23f.x * vsB, p23f.y * vsB)));
                 }
-                // O^T += Vres^T . P, two coordinates per MMA; half of the accumulators in registers at a time
+                if constexpr (kWhole) {
+                    tmem_ld_wait(whole);
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float flat[16];
-                    tmem_ld16(tmem + kColAcc + 16 * half, flat);
-                    uint32_t a[4][4];
-                    Field::half_block(half, f0, f1, f2, f3, a);
-                    tmem_ld_wait(flat);
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t a0 = Field::pair(f0, f1, 2 * i), a2 = Field::pair(f2, f3, 2 * i);
+                        const uint32_t a1 = Field::pair(f0, f1, 2 * i + 1), a3 = Field::pair(f2, f3, 2 * i + 1);
+                        mma_16816(reinterpret_cast<float(&)[8][4]>(whole)[i], a0, a1, a2, a3, pb0, pb1);
+                    }
+                    tmem_st32(tmem + kColAcc, whole);
+                } else {
+                    // O^T += Vres^T . P, two coordinates per MMA; half of the accumulators in registers at a time
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        mma_16816(reinterpret_cast<float(&)[4][4]>(flat)[i], a[i][0], a[i][1], a[i][2], a[i][3], pb0, pb1);
-                    tmem_st16(tmem + kColAcc + 16 * half, flat);
+                    for (int half = 0; half < 2; ++half) {
+                        float flat[16];
+                        tmem_ld16(tmem + kColAcc + 16 * half, flat);
+                        uint32_t a[4][4];
+                        Field::half_block(half, f0, f1, f2, f3, a);
+                        tmem_ld_wait(flat);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            mma_16816(reinterpret_cast<float(&)[4][4]>(flat)[i], a[i][0], a[i][1], a[i][2], a[i][3], pb0, pb1);
+                        tmem_st16(tmem + kColAcc + 16 * half, flat);
+                    }
                 }
             }
             __syncwarp();  // the value rows and rank bases may be rewritten
@@ -1054,115 +1101,190 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
             l_part[0] += __shfl_xor_sync(0xffffffffu, l_part[0], off);
             l_part[1] += __shfl_xor_sync(0xffffffffu, l_part[1], off);
         }
-        // per warp, in its rank bases' place: maximum and sum of the eight columns
-        float* stats = reinterpret_cast<float*>(pre);
-        const float* all_stats = stats - warp * kStatsWarp;
-        if (g == 0) {
-            *reinterpret_cast<float2*>(stats + 2 * qd) = make_float2(m_used[0], m_used[1]);
-            *reinterpret_cast<float2*>(stats + 8 + 2 * qd) = make_float2(l_part[0], l_part[1]);
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();  // every warp is done with its rows: their memory takes the quarters' results
-        tc_fence_after();
-        float* red_acc = reinterpret_cast<float*>(smem_raw);  // [quarters][GQA][kRedAcc]
-        float* red_beta = red_acc + 4 * GQA * kRedAcc;        // [quarters][GQA][kRedBeta]
         const size_t part = static_cast<size_t>(b) * p.nh + hkv * GQA;
         const bool in_range = slot >= 0 && slot < p.splits;
-        {
-            // lane -> warp lane % 16, four columns (X's or Y's heads, or a half of the eight heads)
-            const int from = lane & 15, four = lane >> 4 << 2;
-            const float4 ms = from < busy_warps ? *reinterpret_cast<const float4*>(all_stats + from * kStatsWarp + four)
-                                                : make_float4(kNoMax, kNoMax, kNoMax, kNoMax);
-            float mx[4] = {ms.x, ms.y, ms.z, ms.w};
+        if constexpr (GQA == 1) {
+            // one head: sixteen sets are little to write and to read (8 units x 8000 tokens: 17.5 us, as quarters 18.1)
+            float flat[32], beta[4 * BETA];
+            tmem_ld32(tmem + kColAcc, flat);
+            tmem_load_beta<BETA>(tmem + kColBeta, beta);
+            tmem_ld_wait(flat);
+            tmem_ld_wait(beta);
+            const float m = fmaxf(m_used[0], __shfl_xor_sync(0xffffffffu, m_used[0], 2)), mine = fast_exp2(m_used[0] - m);
+            l_part[0] *= mine;
+            l_part[0] += __shfl_xor_sync(0xffffffffu, l_part[0], 2);
 #pragma unroll
-            for (int off = kDual ? 8 : 16; off > 0; off >>= 1)
+            for (int i = 0; i < 32; i += 2) {  // columns 0 and 4: X's and Y's head
+                flat[i] *= mine;
+                flat[i] += __shfl_xor_sync(0xffffffffu, flat[i], 2);
+            }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], off));
-            if (warp == kWarpsM - 1) {  // the heads' maxima and sums
-                const float4 ls = from < busy_warps ? *reinterpret_cast<const float4*>(all_stats + from * kStatsWarp + 8 + four)
-                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-                float sum[4] = {ls.x * fast_exp2(ms.x - mx[0]), ls.y * fast_exp2(ms.y - mx[1]), ls.z * fast_exp2(ms.z - mx[2]),
-                                ls.w * fast_exp2(ms.w - mx[3])};
+            for (int i = 0; i < 4 * BETA; i += 2) {
+                beta[i] *= mine;
+                beta[i] += __shfl_xor_sync(0xffffffffu, beta[i], 2);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();  // every warp is done with its rows: their memory takes the warps' results
+            float* red_acc = reinterpret_cast<float*>(smem_raw);    // [warps][kRedAcc]
+            float* red_beta = red_acc + kWarpsM * kRedAcc;          // [warps][kRedBeta]
+            float* red_ml = red_beta + kWarpsM * kRedBeta;          // [warps][m, l]
+            if (qd == 0 && warp < busy_warps) {
+                float *dst = red_acc + warp * kRedAcc + g, *bdst = red_beta + warp * kRedBeta + g;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dst[9 * Field::first(i)] = flat[4 * i], dst[9 * Field::second(i)] = flat[4 * i + 2];
+#pragma unroll
+                for (int mb = 0; mb < 4; ++mb) {
+                    bdst[16 * mb] = mb < BETA ? beta[mb < BETA ? 4 * mb : 0] : 0.f;
+                    bdst[16 * mb + 8] = mb < BETA ? beta[mb < BETA ? 4 * mb + 2 : 0] : 0.f;
+                }
+                if (g == 0) red_ml[2 * warp] = m, red_ml[2 * warp + 1] = l_part[0];
+            }
+            __syncthreads();
+            if (in_range && tid < 4 * ((kHeadDim + kMaxClusters) / 2)) {  // two values per four threads, four warps' sets each
+                const int d = 2 * (tid >> 2), sub = tid & 3;
+                const float* src = d < kHeadDim ? red_acc : red_beta;
+                const int at0 = d < kHeadDim ? red_pos(d) : d - kHeadDim, at1 = d < kHeadDim ? red_pos(d + 1) : at0 + 1;
+                const int stride = d < kHeadDim ? kRedAcc : kRedBeta;
+                float2 ml[4];
+                float fm = kNoMax, fl = 0.f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int w = sub + 4 * k;
+                    ml[k] = w < busy_warps ? *reinterpret_cast<const float2*>(red_ml + 2 * w) : make_float2(kNoMax, 0.f);
+                    fm = fmaxf(fm, ml[k].x);
+                }
+                fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, 1)), fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, 2));
+                float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int w = sub + 4 * k;
+                    if (w < busy_warps) {
+                        const float weight = fast_exp2(ml[k].x - fm);
+                        sum.x = fmaf(src[w * stride + at0], weight, sum.x), sum.y = fmaf(src[w * stride + at1], weight, sum.y);
+                        fl = fmaf(ml[k].y, weight, fl);
+                    }
+                }
+#pragma unroll
+                for (int off = 1; off < 4; off <<= 1) {
+                    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, off), sum.y += __shfl_xor_sync(0xffffffffu, sum.y, off);
+                    fl += __shfl_xor_sync(0xffffffffu, fl, off);
+                }
+                const size_t row = part * p.splits + slot;
+                if (sub == 0)
+                    *reinterpret_cast<float2*>(d < kHeadDim ? p.ws_delta + row * kHeadDim + d : p.ws_beta + row * kMaxClusters + d - kHeadDim) = sum;
+                if (tid == 0) p.ws_m[row] = ntiles > 0 ? fm : -INFINITY, p.ws_l[row] = fl;
+            }
+        } else {
+            // per warp, in its rank bases' place: maximum and sum of the eight columns
+            float* stats = reinterpret_cast<float*>(pre);
+            const float* all_stats = stats - warp * kStatsWarp;
+            if (g == 0) {
+                *reinterpret_cast<float2*>(stats + 2 * qd) = make_float2(m_used[0], m_used[1]);
+                *reinterpret_cast<float2*>(stats + 8 + 2 * qd) = make_float2(l_part[0], l_part[1]);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            tc_fence_before();
+            __syncthreads();  // every warp is done with its rows: their memory takes the quarters' results
+            tc_fence_after();
+            float* red_acc = reinterpret_cast<float*>(smem_raw);  // [quarters][GQA][kRedAcc]
+            float* red_beta = red_acc + 4 * GQA * kRedAcc;        // [quarters][GQA][kRedBeta]
+            {
+                // lane -> warp lane % 16, four columns (X's or Y's heads, or a half of the eight heads)
+                const int from = lane & 15, four = lane >> 4 << 2;
+                const float4 ms = from < busy_warps ? *reinterpret_cast<const float4*>(all_stats + from * kStatsWarp + four)
+                                                    : make_float4(kNoMax, kNoMax, kNoMax, kNoMax);
+                float mx[4] = {ms.x, ms.y, ms.z, ms.w};
 #pragma unroll
                 for (int off = kDual ? 8 : 16; off > 0; off >>= 1)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], off);
-                if (in_range && from == 0 && (kDual || lane == 0)) {
+                    for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], off));
+                if (warp == kWarpsM - 1) {  // the heads' maxima and sums
+                    const float4 ls = from < busy_warps ? *reinterpret_cast<const float4*>(all_stats + from * kStatsWarp + 8 + four)
+                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+                    float sum[4] = {ls.x * fast_exp2(ms.x - mx[0]), ls.y * fast_exp2(ms.y - mx[1]), ls.z * fast_exp2(ms.z - mx[2]),
+                                    ls.w * fast_exp2(ms.w - mx[3])};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const size_t row = (part + four + e) * p.splits + slot;
-                        if (four + e < GQA) p.ws_m[row] = ntiles > 0 ? mx[e] : -INFINITY, p.ws_l[row] = sum[e];
+                    for (int off = kDual ? 8 : 16; off > 0; off >>= 1)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], off);
+                    if (in_range && from == 0 && (kDual || lane == 0)) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const size_t row = (part + four + e) * p.splits + slot;
+                            if (four + e < GQA) p.ws_m[row] = ntiles > 0 ? mx[e] : -INFINITY, p.ws_l[row] = sum[e];
+                        }
+                    }
+                }
+                if constexpr (kDual) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) mx[e] = __shfl_sync(0xffffffffu, mx[e], qd >> 1 << 4);
+                }
+                const float m_head[2] = {qd & 1 ? mx[2] : mx[0], qd & 1 ? mx[3] : mx[1]};  // of this lane's columns
+                const int quarter = warp % 4, mine = warp / 4;
+                const uint32_t quarter_cols = tmem - mine * kColsWarp;
+                float acc[8] = {}, bacc[4] = {};  // m-blocks 2 mine, 2 mine + 1; cluster block `mine`
+                // two source warps at a time; one without tokens has weight zero and is not read
+#pragma unroll 1
+                for (int from_warp = quarter; from_warp < busy_warps; from_warp += 8) {
+                    const bool two = from_warp + 4 < busy_warps;
+                    const uint32_t at = quarter_cols + from_warp / 4 * kColsWarp;
+                    float v0[8], v1[8], b0[4], b1[4];
+                    tmem_ld8(at + kColAcc + 8 * mine, v0);
+                    tmem_ld4(at + kColBeta + 4 * (mine < BETA ? mine : 0), b0);
+                    const uint32_t at1 = two ? at + kColsWarp : at;
+                    tmem_ld8(at1 + kColAcc + 8 * mine, v1);
+                    tmem_ld4(at1 + kColBeta + 4 * (mine < BETA ? mine : 0), b1);
+                    const float* st = all_stats + from_warp * kStatsWarp + 2 * qd;
+                    const float2 s0 = *reinterpret_cast<const float2*>(st), s1 = *reinterpret_cast<const float2*>(two ? st + 4 * kStatsWarp : st);
+                    const float w0[2] = {fast_exp2(s0.x - m_head[0]), fast_exp2(s0.y - m_head[1])};
+                    const float w1[2] = {two ? fast_exp2(s1.x - m_head[0]) : 0.f, two ? fast_exp2(s1.y - m_head[1]) : 0.f};
+                    tmem_ld_wait(v0), tmem_ld_wait(v1), tmem_ld_wait(b0), tmem_ld_wait(b1);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] = fmaf(v1[e], w1[e & 1], fmaf(v0[e], w0[e & 1], acc[e]));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) bacc[e] = fmaf(b1[e], w1[e & 1], fmaf(b0[e], w0[e & 1], bacc[e]));
+                }
+                if constexpr (!kDual) {  // X's columns and Y's
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 2);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) bacc[e] += __shfl_xor_sync(0xffffffffu, bacc[e], 2);
+                }
+                if (kDual || qd < 2) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int h = 2 * qd + u;
+                        if (h < GQA) {
+                            float* dst = red_acc + (quarter * GQA + h) * kRedAcc + g;
+#pragma unroll
+                            for (int i = 0; i < 2; ++i)
+                                dst[9 * Field::first(2 * mine + i)] = acc[4 * i + u], dst[9 * Field::second(2 * mine + i)] = acc[4 * i + 2 + u];
+                            float* bdst = red_beta + (quarter * GQA + h) * kRedBeta + 16 * mine + g;
+                            bdst[0] = mine < BETA ? bacc[u] : 0.f, bdst[8] = mine < BETA ? bacc[2 + u] : 0.f;
+                        }
                     }
                 }
             }
-            if constexpr (kDual) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) mx[e] = __shfl_sync(0xffffffffu, mx[e], qd >> 1 << 4);
-            }
-            const float m_head[2] = {qd & 1 ? mx[2] : mx[0], qd & 1 ? mx[3] : mx[1]};  // of this lane's columns
-            const int quarter = warp % 4, mine = warp / 4;
-            const uint32_t quarter_cols = tmem - mine * kColsWarp;
-            float acc[8] = {}, bacc[4] = {};  // m-blocks 2 mine, 2 mine + 1; cluster block `mine`
-            // two source warps at a time; one without tokens has weight zero and is not read
+            tc_fence_before();
+            __syncthreads();
+            tc_fence_after();
+            if (in_range) {
 #pragma unroll 1
-            for (int from_warp = quarter; from_warp < busy_warps; from_warp += 8) {
-                const bool two = from_warp + 4 < busy_warps;
-                const uint32_t at = quarter_cols + from_warp / 4 * kColsWarp;
-                float v0[8], v1[8], b0[4], b1[4];
-                tmem_ld8(at + kColAcc + 8 * mine, v0);
-                tmem_ld4(at + kColBeta + 4 * (mine < BETA ? mine : 0), b0);
-                const uint32_t at1 = two ? at + kColsWarp : at;
-                tmem_ld8(at1 + kColAcc + 8 * mine, v1);
-                tmem_ld4(at1 + kColBeta + 4 * (mine < BETA ? mine : 0), b1);
-                const float* st = all_stats + from_warp * kStatsWarp + 2 * qd;
-                const float2 s0 = *reinterpret_cast<const float2*>(st), s1 = *reinterpret_cast<const float2*>(two ? st + 4 * kStatsWarp : st);
-                const float w0[2] = {fast_exp2(s0.x - m_head[0]), fast_exp2(s0.y - m_head[1])};
-                const float w1[2] = {two ? fast_exp2(s1.x - m_head[0]) : 0.f, two ? fast_exp2(s1.y - m_head[1]) : 0.f};
-                tmem_ld_wait(v0), tmem_ld_wait(v1), tmem_ld_wait(b0), tmem_ld_wait(b1);
+                for (int idx = tid; idx < GQA * ((kHeadDim + kMaxClusters) / 2); idx += kThreadsM) {  // two values per step
+                    constexpr int kPer = (kHeadDim + kMaxClusters) / 2;
+                    const int h = idx / kPer, d = 2 * (idx % kPer);
+                    const float* src = d < kHeadDim ? red_acc + h * kRedAcc : red_beta + h * kRedBeta;
+                    const int at0 = d < kHeadDim ? red_pos(d) : d - kHeadDim, at1 = d < kHeadDim ? red_pos(d + 1) : at0 + 1;
+                    const int stride = d < kHeadDim ? GQA * kRedAcc : GQA * kRedBeta;
+                    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] = fmaf(v1[e], w1[e & 1], fmaf(v0[e], w0[e & 1], acc[e]));
-#pragma unroll
-                for (int e = 0; e < 4; ++e) bacc[e] = fmaf(b1[e], w1[e & 1], fmaf(b0[e], w0[e & 1], bacc[e]));
-            }
-            if constexpr (!kDual) {  // X's columns and Y's
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 2);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) bacc[e] += __shfl_xor_sync(0xffffffffu, bacc[e], 2);
-            }
-            if (kDual || qd < 2) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int h = 2 * qd + u;
-                    if (h < GQA) {
-                        float* dst = red_acc + (quarter * GQA + h) * kRedAcc + g;
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            dst[9 * Field::first(2 * mine + i)] = acc[4 * i + u], dst[9 * Field::second(2 * mine + i)] = acc[4 * i + 2 + u];
-                        float* bdst = red_beta + (quarter * GQA + h) * kRedBeta + 16 * mine + g;
-                        bdst[0] = mine < BETA ? bacc[u] : 0.f, bdst[8] = mine < BETA ? bacc[2 + u] : 0.f;
-                    }
+                    for (int w = 0; w < 4; ++w) sum.x += src[w * stride + at0], sum.y += src[w * stride + at1];
+                    const size_t row = (part + h) * p.splits + slot;
+                    *reinterpret_cast<float2*>(d < kHeadDim ? p.ws_delta + row * kHeadDim + d : p.ws_beta + row * kMaxClusters + d - kHeadDim) = sum;
                 }
             }
         }
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
         if (in_range) {
-#pragma unroll 1
-            for (int idx = tid; idx < GQA * ((kHeadDim + kMaxClusters) / 2); idx += kThreadsM) {  // two values per step
-                constexpr int kPer = (kHeadDim + kMaxClusters) / 2;
-                const int h = idx / kPer, d = 2 * (idx % kPer);
-                const float* src = d < kHeadDim ? red_acc + h * kRedAcc : red_beta + h * kRedBeta;
-                const int at0 = d < kHeadDim ? red_pos(d) : d - kHeadDim, at1 = d < kHeadDim ? red_pos(d + 1) : at0 + 1;
-                const int stride = d < kHeadDim ? GQA * kRedAcc : GQA * kRedBeta;
-                float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int w = 0; w < 4; ++w) sum.x += src[w * stride + at0], sum.y += src[w * stride + at1];
-                const size_t row = (part + h) * p.splits + slot;
-                *reinterpret_cast<float2*>(d < kHeadDim ? p.ws_delta + row * kHeadDim + d : p.ws_beta + row * kMaxClusters + d - kHeadDim) = sum;
-            }
             // the segment that ends its unit marks the unit's unused slots as empty
             if (closes_unit) {
                 for (int idx = tid; idx < GQA * (p.splits - slot - 1); idx += kThreadsM) {
