@@ -17,10 +17,10 @@
 //    registers kept two per scheduler and issued on 58 % of the cycles.)
 //  * What makes 128 registers enough: the accumulators and the 32 sin/cos values of a lane live in tensor memory, whose
 //    loads and stores do not touch the shared-memory pipe (the other busy unit): a k-step's eight sin/cos values are
-//    loaded while its residuals are walked, the accumulators for the value phase only, half of them at a time.  And the two tokens of a lane have
-//    the *same* offset j = 8 warp + g inside two sub-tiles X and Y of (up to) 128 tokens, so one set of 16 (cos, sin)
-//    values rotates both.  RoPE: a token at offset j of a sub-tile starting at position P0 scores < R(pos_q) q, R(P0 + j) k > = < R(pos_q - P0) q, R(j) k >; the query is
-//    rotated once per sub-tile, and the eight columns of the score MMA hold X's heads (0..3) next to Y's (4..7).  Rows
+//    loaded while its residuals are walked, the accumulators for the value phase only, half of them at a time.  And the
+//    two tokens of a lane have the *same* offset j = 8 warp + g inside two sub-tiles X and Y of (up to) 128 tokens, so one
+//    set of 16 (cos, sin) values rotates both.  RoPE: a token at offset j of a sub-tile starting at position P0 scores
+//    < R(pos_q) q, R(P0 + j) k > = < R(pos_q - P0) q, R(j) k >; the query is rotated once per sub-tile, and the eight columns of the score MMA hold X's heads (0..3) next to Y's (4..7).  Rows
 //    of X use the one half of the columns, rows of Y the other; the columns stay apart to the end of the segment
 //    (running maxima, sums, cluster masses and numerators are per column), where they are added.  With eight query heads
 //    per KV head X and Y get MMAs of their own.
@@ -33,12 +33,13 @@
 //  * Rotations are packed FP32 pairs (fma.rn.f32x2), quantised codes are decoded two at a time by one AND-XOR and one
 //    HFMA2.
 //
-// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.219 ms; of active cycles 69 % of the issue slots,
-// 76 % of the shared-memory pipe, 47 % of the integer pipe; 78 instructions and 21 shared-memory wavefronts per token and
+// Measured (batch 32, 8 KV heads, 8128 tokens, 32 of 128 values kept): 0.219 ms; of active cycles 67 % of the issue slots,
+// 76 % of the shared-memory pipe, 46 % of the integer pipe; 75 instructions and 21 shared-memory wavefronts per token and
 // KV head.  Neither unit is full: four warps per scheduler do not cover the latencies of a pass, so a shorter instruction
-// stream alone gives little.  The fields' walks in groups of four, half of the accumulators in registers at a time and the
-// maximum taken across lanes only where it grows: 83 -> 78 instructions, calls with their merge, us: batch 32 228 -> 224.6,
-// batch 8, 16320 tokens INT4 105.5 -> 102, batch 16, 8128 tokens INT2 105 -> 100, 64 of 128 kept 139.6 -> 136.4.
+// stream alone gives little.  The fields' walks in groups of four, half of the accumulators in registers at a time, two
+// score accumulators and the maximum taken across lanes only where it grows: 83 -> 75 instructions, calls with their merge,
+// us: batch 32 228 -> 225, batch 8, 16320 tokens INT4 105.4 -> 100.5, batch 16, 8128 tokens INT2 105 -> 100, batch 8, 65536
+// tokens 426 -> 420.
 // Tried and slower (same call, from 224): the rotated query in tensor memory, 19 wavefronts fewer per pass and 47
 // instructions more, 232; 20 warps at 96 registers 239; a fused multiply-add for the rotation's subtraction 228; the
 // k-steps or the halves as loops 226 to 232.

@@ -1258,8 +1258,8 @@ int side_share(int tiles_side, int tiles_unit) {
 
 // Tiles per CTA when K and V share the launches.  They are cut as a call for one side cuts them, so that ids and centres
 // are those of two such calls bit for bit; only how many of the pieces a CTA takes is chosen here, again for the shortest
-// slowest CTA.  A segment of the unit whose tables a CTA already has costs about four tile times (drain and flush: 55.2 ->
-// 57.8 us per iteration at 64 units x 8128 tokens with one per CTA).  About `kTries` shares are looked at (host time).
+// slowest CTA.  A segment of the unit whose tables a CTA already has is counted as four tile times, one of another unit as
+// ten; 7 and 1, 7 and 3, 14 and 2 choose shares of the same time, 8 units x 1152 to 64 x 8128 tokens.  About `kTries` shares are looked at (host time).
 int pair_share(const Cuts& c) {
     constexpr int kNewUnit = 10, kSameUnit = 4, kTries = 16, seg_max = kUChunkMax / kUTile;
     const int low = (c.tiles + sm_count() - 1) / sm_count();
