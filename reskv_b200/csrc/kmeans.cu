@@ -1259,7 +1259,8 @@ int side_share(int tiles_side, int tiles_unit) {
 // Tiles per CTA when K and V share the launches.  They are cut as a call for one side cuts them, so that ids and centres
 // are those of two such calls bit for bit; only how many of the pieces a CTA takes is chosen here, again for the shortest
 // slowest CTA.  A segment of the unit whose tables a CTA already has is counted as four tile times, one of another unit as
-// ten; 7 and 1, 7 and 3, 14 and 2 choose shares of the same time, 8 units x 1152 to 64 x 8128 tokens.  About `kTries` shares are looked at (host time).
+// ten; 7 and 1, 7 and 3, 14 and 2 choose shares of the same time, 8 units x 1152 to 64 x 8128 tokens.  About `kTries` shares
+// are looked at (host time).
 int pair_share(const Cuts& c) {
     constexpr int kNewUnit = 10, kSameUnit = 4, kTries = 16, seg_max = kUChunkMax / kUTile;
     const int low = (c.tiles + sm_count() - 1) / sm_count();
@@ -1303,20 +1304,25 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     cuts.tiles_unit = (p.tokens + kUTile - 1) / kUTile;
     cuts.tiles_side = p.units * cuts.tiles_unit, cuts.tiles = p.sides * cuts.tiles_side;
     cuts.piece = side_share(cuts.tiles_side, cuts.tiles_unit);
-    const int share = p.sides == 2 ? pair_share(cuts) : cuts.piece;
-    const dim3 grid(static_cast<unsigned>((cuts.tiles + share - 1) / share));
+    int share = p.sides == 2 ? pair_share(cuts) : cuts.piece;
     const bool pairs = share > cuts.piece && cuts.piece % cuts.tiles_unit != 0;
     const auto kern = pairs ? kmeans_assign_umma_kernel<true> : kmeans_assign_umma_kernel<false>;
     static std::atomic<unsigned long long> done[2];
     if (int rc = allow_smem(kern, smem, done[pairs], "cudaFuncSetAttribute(kmeans_assign_umma)")) return rc;
-    // cooperative: CTAs wait for one another between iterations, so all of them have to be resident
+    // cooperative: CTAs wait for one another between iterations, so all of them have to be resident.  A stream that has only
+    // a part of the SMs takes fewer CTAs with more pieces each; the cuts, and with them the results, stay.
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid, cfg.blockDim = dim3(kUThreads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cfg.blockDim = dim3(kUThreads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
     cfg.attrs = &attr, cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kern, p, maps[0], maps[1], cuts, share), "kmeans launch");
+    for (;; share *= 2) {
+        cfg.gridDim = dim3(static_cast<unsigned>((cuts.tiles + share - 1) / share));
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, maps[0], maps[1], cuts, share);
+        if (e != cudaErrorCooperativeLaunchTooLarge || cfg.gridDim.x == 1) return check_cuda(e, "kmeans launch");
+        cudaGetLastError();  // the refused launch must not poison later calls
+    }
 }
 
 }  // namespace
