@@ -65,6 +65,15 @@ def _rope(x, cos, sin):
     return torch.cat((a * cos - b * sin, b * cos + a * sin), dim=-1).to(x.dtype)
 
 
+def _dense_half(tensor, shape, device) -> bool:
+    """Whether a kernel may read ``tensor`` by its address alone: FP16 of this shape on ``device``, row-major without gaps, on
+    a 16-byte boundary.  Everything else that a caller may assign to the model (transposed views, slices of a fused matrix,
+    expanded or misaligned tensors, other types, subclasses with a product of their own) is left to tensor operations."""
+    return (type(tensor) in (torch.Tensor, torch.nn.Parameter) and tensor.layout == torch.strided
+            and tensor.dtype == torch.float16 and tensor.device == device and tensor.shape == shape
+            and tensor.is_contiguous() and not tensor.is_neg() and tensor.data_ptr() % 16 == 0)
+
+
 class _CollectorHold:
     """Keeps Python's cyclic collector from running while any thread is inside: a finaliser that it ran in a stream capture
     (of another graph, an event, a device buffer) could call CUDA there and spoil the capture.  A collection before the
@@ -343,6 +352,8 @@ class ResKVLlama:
             return torch.empty(shape, dtype=torch.float16, device=self.device)
 
         def norm(x, weight):
+            if not (_dense_half(x, (b, d), x.device) and _dense_half(weight, (d,), x.device)):
+                return self._norm(x, weight)
             out = half(b, d)
             check(lib.reskv_rms_norm(x.data_ptr(), weight.data_ptr(), out.data_ptr(), b, d, float(self.shape.rms_eps), stream))
             return out
@@ -351,11 +362,15 @@ class ResKVLlama:
             return None if t is None else t.data_ptr()
 
         def streamed(x, weight, n, mode, out, norm_weight=None):
-            """The library's own weight stream, for few rows; False where it does not take the sizes."""
-            if not lib.reskv_skinny_linear_fits(b, n, x.shape[-1], mode):
+            """The library's own weight stream, for few rows; False where it does not take the sizes or the tensors as
+            they are.  Asked while a step is captured only: a replay pays nothing for it."""
+            k = x.shape[-1]
+            if not (lib.reskv_skinny_linear_fits(b, n, k, mode) and _dense_half(x, (b, k), x.device)
+                    and _dense_half(weight, (2 * n if mode == 2 else n, k), x.device)
+                    and (norm_weight is None or _dense_half(norm_weight, (k,), x.device))):
                 return False
             check(lib.reskv_skinny_linear(x.data_ptr(), ptr(norm_weight), float(self.shape.rms_eps), weight.data_ptr(),
-                                          out.data_ptr(), b, n, x.shape[-1], mode, stream))
+                                          out.data_ptr(), b, n, k, mode, stream))
             return True
 
         def linear(x, weight, norm_weight):
