@@ -157,7 +157,16 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     return d;
 }
 
-// FAST: cluster sums on the tensor cores (needs padded <= 32), else exact integer accumulation.
+// Sixteen bytes from an address that is only on a 2-byte boundary.
+__device__ __forceinline__ uint4 load_halves(const uint4* p) {
+    const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __ldg(h + 2 * i) | static_cast<uint32_t>(__ldg(h + 2 * i + 1)) << 16;
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// FAST: cluster sums on the tensor cores (needs padded <= 32 and x on a 16-byte boundary), else exact integer accumulation.
 template <bool HILO, bool FAST>
 __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const KmeansParams p, int padded, int chunk) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -212,6 +221,7 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
     __syncthreads();
     const float cmax = cmax_s;
     const __half* xu = p.x + static_cast<size_t>(unit) * p.x_stride * kHeadDim;
+    const bool wide = FAST || (reinterpret_cast<uintptr_t>(xu) & 15u) == 0;  // a view may start anywhere
     // FAST: sums[cluster 16 mb + g (+8)][coordinate kstep_offset(ks, q) + 2 h + (0, 1)] of this warp's tokens,
     // n-block nb = 2 ks + h
     float acc_s[FAST ? 2 : 1][FAST ? 16 : 1][4];
@@ -253,7 +263,7 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint4* at = src + (k < 2 ? 0 : 8) + 2 * q + (k & 1);
-                    v[r][k] = row < t_end ? (FAST ? *at : __ldg(at)) : make_uint4(0, 0, 0, 0);
+                    v[r][k] = row >= t_end ? make_uint4(0, 0, 0, 0) : FAST ? *at : wide ? __ldg(at) : load_halves(at);
                 }
             }
             if constexpr (FAST) {
