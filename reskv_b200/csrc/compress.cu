@@ -116,12 +116,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) encode_compact_kernel(const
         const size_t orow = static_cast<size_t>(unit) * p.out_stride + t;
         if (lane < nwords) static_cast<int32_t*>(p.payload)[orow * nwords + lane] = static_cast<int32_t>(scratch[warp][lane]);
         if (lane == 0) {
-            uint4 bm;  // word w of the bitmap: coordinate d at bit 63 - d % 64
-            bm.y = __brev(vote[0]);
-            bm.x = __brev(vote[1]);
-            bm.w = __brev(vote[2]);
-            bm.z = __brev(vote[3]);
-            static_cast<uint4*>(p.meta)[orow] = bm;
+            // word w of the bitmap: coordinate d at bit 63 - d % 64; 64-bit stores, the rows need not be on 16-byte boundaries
+            unsigned long long* bm = static_cast<unsigned long long*>(p.meta) + 2 * orow;
+            bm[0] = static_cast<unsigned long long>(__brev(vote[0])) << 32 | __brev(vote[1]);
+            bm[1] = static_cast<unsigned long long>(__brev(vote[2])) << 32 | __brev(vote[3]);
             p.scale[orow] = hs;
         }
         __syncwarp();

@@ -41,3 +41,18 @@ def test_compressing_a_misaligned_prompt():
         given = ((side.centroids, side.cluster_ids),) * 2
         want = compress(x, x, cfg, clustering=given).key
         assert all(torch.equal(getattr(side, name), getattr(want, name)) for name in ("cluster_ids", "payload", "metadata", "scale"))
+
+
+@pytest.mark.parametrize("bits,nnz", [(4, 32), (4, 64), (2, 64)])
+def test_compact_bitmap_rows_on_eight_byte_boundaries(bits, nnz):
+    from reskv_b200._extension import _stream, check, library, load_extension
+    from reskv_b200.synthetic import gaussian, mixture
+
+    x, cen = mixture(1, 2, 77, seed=1, device=DEV), gaussian(1, 2, 16, 128, seed=2, device=DEV)
+    ids = torch.randint(16, (1, 2, 77), device=DEV, dtype=torch.int32)
+    words, bitmap, scale = load_extension("compression").compress_compact(x, cen, ids, nnz, bits)
+    buf = torch.zeros(bitmap.numel() + 1, dtype=torch.int64, device=DEV)
+    words2, scale2 = torch.empty_like(words), torch.empty_like(scale)
+    check(library().reskv_encode_compact(x.data_ptr(), cen.data_ptr(), ids.data_ptr(), 1, 2, 77, 77, 16, nnz, bits, words2.data_ptr(),
+                                         buf[1:].data_ptr(), scale2.data_ptr(), 77, _stream(x.device)))
+    assert torch.equal(buf[1:].view(bitmap.shape), bitmap) and torch.equal(words2, words) and torch.equal(scale2, scale)
