@@ -293,8 +293,11 @@ class CompressionOps(_Ops):
         centroids = torch.empty((b, h, count, 128), dtype=torch.float16, device=x.device)
         ids = torch.empty((b, h, t), dtype=torch.int32, device=x.device)
         flags = int(bool(value)) | (2 if exact else 0) | (4 if warp_mma else 0)
+        # one kernel for all iterations, or an initialisation and two kernels per iteration
+        together = not (exact or warp_mma) and count <= 32 and x.data_ptr() % 16 == 0
         check(self.lib.reskv_kmeans(x.data_ptr(), b, h, t, xs, count, iterations, flags, ws.data_ptr(), need,
-                                    centroids.data_ptr(), ids.data_ptr(), _stream(x.device)), launches=1 + 2 * iterations if exact or warp_mma or count > 32 else 1 + iterations)
+                                    centroids.data_ptr(), ids.data_ptr(), _stream(x.device)),
+              launches=1 if together else 1 + 2 * iterations)
         if return_status:
             word = ctypes.c_uint32(0xFFFFFFFF)
             check(self.lib.reskv_kmeans_status(ws.data_ptr(), b, h, count, ctypes.addressof(word), _stream(x.device)))
@@ -302,7 +305,7 @@ class CompressionOps(_Ops):
         return centroids, ids
 
     def kmeans_pair(self, key, value, count, iterations):
-        """``kmeans`` of K and of V in the same launches -> ``(centroids, int32 ids, int8 ids)`` of each; up to 32 centres,
+        """``kmeans`` of K and of V in the same launch -> ``(centroids, int32 ids, int8 ids)`` of each; up to 32 centres,
         at least as many tokens, 16-byte aligned inputs."""
         _same_device(self.device.index, key, value)
         return host().kmeans_pair(key, value, count, iterations)

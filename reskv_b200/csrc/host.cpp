@@ -476,7 +476,7 @@ PyObject* py_kmeans_pair(PyObject*, PyObject* const* o, Py_ssize_t n) {
                                     static_cast<int>(iterations), ws.data_ptr(), need, part[0][0].data_ptr(), part[1][0].data_ptr(),
                                     static_cast<int32_t*>(part[0][1].data_ptr()), static_cast<int32_t*>(part[1][1].data_ptr()),
                                     part[0][2].data_ptr(), part[1][2].data_ptr(), c10::cuda::getCurrentCUDAStream(dev).stream()));
-            g_launches += 1 + iterations;
+            ++g_launches;  // all iterations
         }
         PyObject* both = PyTuple_New(2);
         for (int i = 0; i < 2; ++i) {
@@ -816,7 +816,7 @@ PyMethodDef g_methods[] = {
     {"attention", FAST(py_attention), METH_FASTCALL, "decode attention on a compressed cache"},
     {"window_append", FAST(py_window_append), METH_FASTCALL, "append one token to the dense window"},
     {"encode", FAST(py_encode), METH_FASTCALL, "pack one side"},
-    {"kmeans_pair", FAST(py_kmeans_pair), METH_FASTCALL, "cluster K and V in the same launches"},
+    {"kmeans_pair", FAST(py_kmeans_pair), METH_FASTCALL, "cluster K and V in the same launch"},
     {"regrow", FAST(py_regrow), METH_FASTCALL, "larger buffers for a cache"},
     {"append_group", FAST(py_append_group), METH_FASTCALL, "cluster, pack and append one decode group"},
     {"window_fill", FAST(py_window_fill), METH_FASTCALL, "a prompt's dense tail into the window"},
