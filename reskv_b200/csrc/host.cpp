@@ -5,10 +5,12 @@
 // attribute reads, four allocations, a 30-argument ctypes call) took 65 us per call, so the GPU waited for the host
 // up to batch 8.  Nothing is kept between calls here: every pointer and size is read from the tensors of the call.
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <Python.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -101,6 +103,15 @@ const void* data(const at::Tensor& t) { return t.defined() && t.numel() ? t.cons
 void same_device(c10::DeviceIndex dev, const at::Tensor& t) {
     if (t.defined() && (!t.is_cuda() || t.get_device() != dev))
         value_error("all tensors of this call must live on cuda:" + std::to_string(static_cast<int>(dev)) + ", got one on " + t.device().str());
+}
+
+// A tensor whose memory a kernel may read behind the dispatcher's back: nothing that a tensor operation would do with it
+// besides is lost (a gradient or a forward-mode tangent, the wrappers of vmap, jvp and functionalisation, a subclass or a
+// mode that wants to see the operation, a trace being recorded), and it has memory at all.
+bool plain(PyObject* o, const at::Tensor& x) {
+    return THPVariable_CheckExact(o) && !at::isTensorSubclassLike(x) && x.unsafeGetTensorImpl()->has_storage() && !x._is_zerotensor() &&
+           !x.is_conj() && !x.is_neg() && !(c10::GradMode::is_enabled() && x.requires_grad()) && !x._fw_grad(0).defined() &&
+           !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer);
 }
 
 // Tokens between (sequence, head) units of x[B,H,T,128] when it is dense or a token slice of a dense
@@ -650,14 +661,14 @@ PyObject* py_window_fill(PyObject*, PyObject* const* o, Py_ssize_t n) {
         const at::Tensor window[3] = {tensor(o[0], "keys"), tensor(o[1], "raw keys"), tensor(o[2], "values")};
         const at::Tensor src[3] = {tensor(o[3], "key"), tensor(o[4], "raw key"), tensor(o[5], "value")};
         const int64_t slot = integer(o[6]), first = integer(o[7]), count = integer(o[8]);
+        for (int i = 0; i < 6; ++i)
+            if (!plain(o[i], i < 3 ? window[i] : src[i - 3])) return Py_NewRef(Py_False);
         const c10::DeviceIndex dev = window[0].get_device();
-        const bool grad = c10::GradMode::is_enabled();
         int64_t stride[3];
         for (int i = 0; i < 3; ++i) {
             const at::Tensor& x = src[i];
             if (!x.is_cuda() || x.get_device() != dev || x.scalar_type() != at::kHalf || window[i].scalar_type() != at::kHalf || x.dim() != 4 ||
-                x.size(0) != window[i].size(0) || x.size(1) != window[i].size(1) || x.size(2) < first + count || !window[i].is_contiguous() ||
-                (grad && x.requires_grad()) || x.is_conj() || x.is_neg())
+                x.size(0) != window[i].size(0) || x.size(1) != window[i].size(1) || x.size(2) < first + count || !window[i].is_contiguous())
                 return Py_NewRef(Py_False);
             stride[i] = token_stride_of(x);
             if (stride[i] < x.size(2) || !aligned16(x.const_data_ptr()) || !aligned16(window[i].const_data_ptr())) return Py_NewRef(Py_False);

@@ -62,3 +62,55 @@ def test_gradients_flow_through_the_window_as_before():
     keys, _ = cache.update(x, x, {"raw_keys": x})
     keys.float().sum().backward()
     assert torch.equal(x.grad, torch.ones_like(x))
+
+
+def test_tangents_flow_through_the_window_as_before():
+    import torch.autograd.forward_ad as fw
+    from reskv_b200 import ResKVKernelConfig
+    from reskv_b200.cache import ResKVLayerCache
+
+    x, t = (torch.randn(1, 2, 20, 128, device=DEV).half() for _ in range(2))
+    cache = ResKVLayerCache(ResKVKernelConfig())
+    with fw.dual_level():
+        dual = fw.make_dual(x, t)
+        for got in cache.update(dual, dual, {"raw_keys": dual}):
+            primal, tangent = fw.unpack_dual(got)
+            assert torch.equal(primal, x) and tangent is not None and torch.equal(tangent, t)
+
+
+def test_operations_are_seen_by_a_dispatch_mode_as_before():
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from reskv_b200 import ResKVKernelConfig
+    from reskv_b200.cache import ResKVLayerCache
+
+    class Count(TorchDispatchMode):
+        copies = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.copies += func is torch.ops.aten.copy_.default
+            return func(*args, **(kwargs or {}))
+
+    x = torch.randn(1, 2, 20, 128, device=DEV).half()
+    with Count() as seen:
+        keys, values = ResKVLayerCache(ResKVKernelConfig()).update(x, x + 1, {"raw_keys": x + 2})
+    assert torch.equal(keys, x) and torch.equal(values, x + 1) and seen.copies == 3
+
+
+def test_wrapped_tensors_of_a_transform_are_copied_as_before():
+    from reskv_b200 import ResKVKernelConfig
+    from reskv_b200.cache import ResKVLayerCache
+
+    x, t = (torch.randn(1, 2, 20, 128, device=DEV).half() for _ in range(2))
+    window = lambda k: ResKVLayerCache(ResKVKernelConfig()).update(k, k, {"raw_keys": k})[0]
+    primal, tangent = torch.func.jvp(window, (x,), (t,))
+    assert torch.equal(primal, x) and torch.equal(tangent, t)
+
+
+def test_a_tensor_without_memory_is_copied_as_before():
+    from reskv_b200 import ResKVKernelConfig
+    from reskv_b200.cache import ResKVLayerCache
+
+    x = torch.randn(1, 2, 20, 128, device=DEV).half()
+    zero = torch._efficientzerotensor((1, 2, 20, 128), dtype=torch.float16, device=DEV)
+    keys, values = ResKVLayerCache(ResKVKernelConfig()).update(x, zero, {"raw_keys": zero})
+    assert torch.equal(keys, x) and not values.any()
