@@ -74,6 +74,9 @@ __global__ void __launch_bounds__(kLinThreads, 1) skinny_linear_kernel(const Lin
         int slot = 0, round = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             for (int s = 0; s < steps; ++s) {
+                // the ring is full: nothing is given back before the kernel in front has ended, and however long that takes is
+                // no part of the bounded wait
+                if (round == 1 && slot == 0) wait_for_previous_launch();
                 if (round > 0) lost |= !mbar_wait(&bar_empty[slot], (round - 1) & 1);
                 if (lane == 0) {
                     mbar_arrive_expect_tx(&bar_full[slot], kLinStage);
