@@ -21,7 +21,9 @@ compressed cache goes through ``reskv_b200.compress`` / ``attention``.
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import gc
+import os
 import threading
 from dataclasses import dataclass
 
@@ -333,6 +335,19 @@ class ResKVLlama:
         return torch.stack(out, dim=1)
 
     # -- CUDA-graph decode ------------------------------------------------------------------------
+    # RESKV_CHECK_STATUS=1: every step is waited for, and a kernel's bounded wait that ran out (or a step state beyond its
+    # buffers) raises instead of leaving wrong logits
+    _check_status = os.environ.get("RESKV_CHECK_STATUS") == "1"
+
+    def _raise_on_status(self):
+        from .._extension import _stream, check
+
+        linear = ctypes.c_uint32(0)
+        check(self._native().reskv_skinny_linear_status(ctypes.addressof(linear), _stream(self.device)), launches=0)
+        decode = self._workspace[:4].view(torch.int32).item() if self.cache_kind == "reskv" else 0
+        if linear.value or decode:
+            raise RuntimeError(f"decode step: device status 0x{linear.value:x} (linear layers), 0x{decode:x} (attention)")
+
     # A decode step is ~20 small launches per layer; at small batch the GPU waits for Python.  The
     # step is therefore captured once per "epoch" (the 64 steps between two group compressions, in
     # which the compressed segment is fixed) and replayed: query position and window length live in
@@ -529,6 +544,8 @@ class ResKVLlama:
         if self._graph is None:
             self._capture_step()
         self._graph.replay()
+        if self._check_status:
+            self._raise_on_status()
         self.length += 1
         if self.cache_kind == "reskv":
             for cache in self.caches:

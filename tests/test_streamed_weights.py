@@ -1,6 +1,8 @@
 """Weights that a caller has assigned to a model: the captured step reads a weight by its address only where that is the whole
 truth about it (dense row-major FP16, aligned), and gives the logits of the eager step for every other one as well."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -92,3 +94,35 @@ def test_captured_step_with_an_expanded_head():
 
     for got, want in zip(*reversed(_step_logits(change, 2))):
         torch.testing.assert_close(got, want, atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["linear", "attention"])
+def test_a_step_whose_wait_ran_out_raises(which, monkeypatch):
+    """With RESKV_CHECK_STATUS=1; the status words are set by the host, no wait runs out here."""
+    from reskv_b200 import ResKVKernelConfig
+    from reskv_b200.models import LlamaShape, ResKVLlama
+
+    cfg = ResKVKernelConfig(num_clusters=4, max_clusters=8, group_size=16, recent_size=8, kmeans_iterations=2)
+    model = ResKVLlama(LlamaShape(hidden=512, layers=1, heads=4, kv_heads=1, ffn=1024, vocab=336), cfg, seed=3)
+    monkeypatch.setattr(ResKVLlama, "_check_status", True)
+    ids = torch.randint(0, 336, (2, 62), generator=torch.Generator().manual_seed(2)).cuda()
+    model.prefill(ids[:, :60], reserve=40)
+    model.begin_graph_decode(2)
+    model.decode_graph(ids[:, 60])
+    if which == "attention":
+        model._workspace[0] = 1
+    else:
+        library = model._native()
+
+        class Ran:
+            def __getattr__(self, name):
+                return getattr(library, name)
+
+            def reskv_skinny_linear_status(self, status, stream):
+                ctypes.c_uint32.from_address(status).value = 1
+                return 0
+
+        model._lib = Ran()
+    with pytest.raises(RuntimeError, match="device status"):
+        model.decode_graph(ids[:, 61])
