@@ -376,28 +376,31 @@ class ResKVLlama:
         def ptr(t):
             return None if t is None else t.data_ptr()
 
-        def streamed(x, weight, n, mode, out, norm_weight=None):
-            """The library's own weight stream, for few rows; False where it does not take the sizes or the tensors as
-            they are.  Asked while a step is captured only: a replay pays nothing for it."""
+        def streams(x, weight, n, mode, norm_weight=None):
+            """Whether the library's own weight stream, for few rows, takes the sizes, and the tensors as they are.  Asked
+            while a step is captured only: a replay pays nothing for it."""
             k = x.shape[-1]
-            if not (lib.reskv_skinny_linear_fits(b, n, k, mode) and _dense_half(x, (b, k), x.device)
+            return (lib.reskv_skinny_linear_fits(b, n, k, mode) and _dense_half(x, (b, k), x.device)
                     and _dense_half(weight, (2 * n if mode == 2 else n, k), x.device)
-                    and (norm_weight is None or _dense_half(norm_weight, (k,), x.device))):
-                return False
+                    and (norm_weight is None or _dense_half(norm_weight, (k,), x.device)))
+
+        def stream_weight(x, weight, mode, out, norm_weight=None):
             check(lib.reskv_skinny_linear(x.data_ptr(), ptr(norm_weight), float(self.shape.rms_eps), weight.data_ptr(),
-                                          out.data_ptr(), b, n, k, mode, stream))
-            return True
+                                          out.data_ptr(), b, out.shape[-1], x.shape[-1], mode, stream))
+            return out
 
         def linear(x, weight, norm_weight):
             """norm(x) @ weight^T"""
-            out = half(b, weight.shape[0])
-            return out if streamed(x, weight, weight.shape[0], 0, out, norm_weight) else F.linear(norm(x, norm_weight), weight)
+            n = weight.shape[0]
+            if streams(x, weight, n, 0, norm_weight):
+                return stream_weight(x, weight, 0, half(b, n), norm_weight)
+            return F.linear(norm(x, norm_weight), weight)
 
         def project(x, inp, weight):
             """x + inp @ weight^T, summed over the tensor-parallel group."""
             if self.tp == 1:
-                if streamed(inp, weight, d, 1, x):
-                    return x
+                if _dense_half(x, (b, d), inp.device) and streams(inp, weight, d, 1):
+                    return stream_weight(inp, weight, 1, x)
                 return x.addmm_(inp, weight.t())  # in place: no copy of x in front of the product
             return x + self._all_reduce(F.linear(inp, weight))
 
@@ -444,15 +447,18 @@ class ResKVLlama:
                 raise RuntimeError("graph decode of the dense baseline needs flash_attn")
             x = project(x, att, layer["wo"])
             act = half(b, self.ffn)
-            if not streamed(x, layer["w_gate_up"], self.ffn, 2, act, layer["norm2"]):
+            if streams(x, layer["w_gate_up"], self.ffn, 2, layer["norm2"]):
+                stream_weight(x, layer["w_gate_up"], 2, act, layer["norm2"])
+            else:
                 gate_up = F.linear(norm(x, layer["norm2"]), layer["w_gate_up"])
                 check(lib.reskv_silu_mul(gate_up.data_ptr(), act.data_ptr(), b, self.ffn, stream))
             x = project(x, act, layer["w_down"])
         if not reskv:
             self._seqlens += 1
-        logits = torch.empty((b, self.lm_head.shape[0]), dtype=torch.float32, device=self.device)
-        if streamed(x, self.lm_head, self.lm_head.shape[0], 3, logits, self.final_norm):
-            return logits
+        vocab = self.lm_head.shape[0]
+        if streams(x, self.lm_head, vocab, 3, self.final_norm):
+            logits = torch.empty((b, vocab), dtype=torch.float32, device=self.device)
+            return stream_weight(x, self.lm_head, 3, logits, self.final_norm)
         return F.linear(norm(x, self.final_norm), self.lm_head).float()
 
     @torch.no_grad()
