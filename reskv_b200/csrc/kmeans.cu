@@ -138,13 +138,6 @@ __device__ __forceinline__ void nearest(const float* cen_s, int clusters, const 
 constexpr int kCenHalfStride = 132;  // FP16 centre rows: stride = 2 banks mod 32, so B-fragment loads do not collide
 constexpr float kTieBound = 1.0f / 32768.0f;  // re-rank when (d2 - d1) <= kTieBound * (|x|^2 + max |c|^2)
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                        uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // Offset (in coordinates) of MMA k-step `ks` for quad lane `q`: a lane owns coordinates
 // [16 q, 16 q + 16) and [64 + 16 q, 64 + 16 q + 16), four per k-step.
 __device__ __forceinline__ int kstep_offset(int ks, int q) { return (ks < 4 ? 0 : 48) + 16 * q + 4 * ks; }
@@ -282,8 +275,8 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
             float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
-                mma_f16(s0, a[ks][0], a[ks][1], a[ks][2], a[ks][3], a[ks][0], a[ks][2]);
-                mma_f16(s1, a[ks][0], a[ks][1], a[ks][2], a[ks][3], a[ks][1], a[ks][3]);
+                mma_16816(s0, a[ks][0], a[ks][1], a[ks][2], a[ks][3], a[ks][0], a[ks][2]);
+                mma_16816(s1, a[ks][0], a[ks][1], a[ks][2], a[ks][3], a[ks][1], a[ks][3]);
             }
             // row g x token g sits in lane (g, g / 2), element g % 2; row g + 8 x token g + 8 likewise in s1[2..3]
             const float mine0 = (g & 1) ? s0[1] : s0[0], mine1 = (g & 1) ? s1[3] : s1[2];
@@ -311,13 +304,13 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 #pragma unroll
                 for (int h = 0; h < kChains; ++h) {
                     const uint2 bh = *reinterpret_cast<const uint2*>(hrow[h] + kstep_offset(ks, q));
-                    mma_f16(acc[h], a[ks][0], a[ks][1], a[ks][2], a[ks][3], bh.x, bh.y);
+                    mma_16816(acc[h], a[ks][0], a[ks][1], a[ks][2], a[ks][3], bh.x, bh.y);
                 }
                 if (HILO) {
 #pragma unroll
                     for (int h = 0; h < kChains; ++h) {
                         const uint2 bl = *reinterpret_cast<const uint2*>(lrow[h] + kstep_offset(ks, q));
-                        mma_f16(acc[h], a[ks][0], a[ks][1], a[ks][2], a[ks][3], bl.x, bl.y);
+                        mma_16816(acc[h], a[ks][0], a[ks][1], a[ks][2], a[ks][3], bl.x, bl.y);
                     }
                 }
             }
@@ -399,8 +392,8 @@ __global__ void __launch_bounds__(kThreads) kmeans_assign_mma_kernel(const Kmean
 #pragma unroll
                 for (int mb = 0; mb < 2; ++mb) {
                     if (16 * mb < padded) {
-                        mma_f16(acc_s[mb][2 * ks], oh[mb][0], oh[mb][1], oh[mb][2], oh[mb][3], b00, b01);
-                        mma_f16(acc_s[mb][2 * ks + 1], oh[mb][0], oh[mb][1], oh[mb][2], oh[mb][3], b10, b11);
+                        mma_16816(acc_s[mb][2 * ks], oh[mb][0], oh[mb][1], oh[mb][2], oh[mb][3], b00, b01);
+                        mma_16816(acc_s[mb][2 * ks + 1], oh[mb][0], oh[mb][1], oh[mb][2], oh[mb][3], b10, b11);
                     }
                 }
             }
@@ -773,62 +766,62 @@ __global__ void __launch_bounds__(kUThreads, 1) kmeans_assign_umma_kernel(const 
                     constexpr int kMakers = kUWorkers - 32;  // not the last worker warp, which may still announce the segment before
                     constexpr int kSteps = (32 * kHeadDim / 4 + kMakers - 1) / kMakers;
                     if (tid < kMakers) {
-                    float4 v[kSteps];
-                    CentreSums sums[kSteps];
-                    if (!first) {
+                        float4 v[kSteps];
+                        CentreSums sums[kSteps];
+                        if (!first) {
+#pragma unroll
+                            for (int k = 0; k < kSteps; ++k) {
+                                const int i4 = min(tid + k * kMakers, p.clusters * (kHeadDim / 4) - 1);
+                                sums[k] = load_sums(p, it - 1, row0 + i4 / (kHeadDim / 4), i4 % (kHeadDim / 4));
+                            }
+                        }
 #pragma unroll
                         for (int k = 0; k < kSteps; ++k) {
-                            const int i4 = min(tid + k * kMakers, p.clusters * (kHeadDim / 4) - 1);
-                            sums[k] = load_sums(p, it - 1, row0 + i4 / (kHeadDim / 4), i4 % (kHeadDim / 4));
+                            const int i4 = tid + k * kMakers;
+                            const int c = i4 / (kHeadDim / 4), d4 = i4 % (kHeadDim / 4);
+                            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (i4 >= 32 * kHeadDim / 4 || c >= p.clusters) continue;
+                            if (first) {
+                                const uint2 raw = __ldg(reinterpret_cast<const uint2*>(xu + static_cast<size_t>(p.init.idx[c]) * kHeadDim) + d4);
+                                const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+                                v[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                            } else {
+                                v[k] = new_centre(p, sums[k], it - 1, value, row0 + c, d4);
+                            }
+                            if (opens_unit) {
+                                reinterpret_cast<float4*>(p.centres[it & 1] + row0 * kHeadDim)[i4] = v[k];
+                                if (owned) continue;
+                                const longlong2 zero = make_longlong2(0, 0);
+                                longlong2* ahead = reinterpret_cast<longlong2*>(p.sums[(it + 1) % 3] + row0 * kHeadDim) + 2 * i4;
+                                ahead[0] = zero, ahead[1] = zero;
+                                if (d4 == 0) p.counts[(it + 1) % 3][row0 + c] = 0;
+                            }
                         }
-                    }
 #pragma unroll
-                    for (int k = 0; k < kSteps; ++k) {
-                        const int i4 = tid + k * kMakers;
-                        const int c = i4 / (kHeadDim / 4), d4 = i4 % (kHeadDim / 4);
-                        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (i4 >= 32 * kHeadDim / 4 || c >= p.clusters) continue;
-                        if (first) {
-                            const uint2 raw = __ldg(reinterpret_cast<const uint2*>(xu + static_cast<size_t>(p.init.idx[c]) * kHeadDim) + d4);
-                            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                            v[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
-                        } else {
-                            v[k] = new_centre(p, sums[k], it - 1, value, row0 + c, d4);
-                        }
-                        if (opens_unit) {
-                            reinterpret_cast<float4*>(p.centres[it & 1] + row0 * kHeadDim)[i4] = v[k];
-                            if (owned) continue;
-                            const longlong2 zero = make_longlong2(0, 0);
-                            longlong2* ahead = reinterpret_cast<longlong2*>(p.sums[(it + 1) % 3] + row0 * kHeadDim) + 2 * i4;
-                            ahead[0] = zero, ahead[1] = zero;
-                            if (d4 == 0) p.counts[(it + 1) % 3][row0 + c] = 0;
-                        }
-                    }
+                        for (int k = 0; k < kSteps; ++k) {
+                            const int i4 = tid + k * kMakers;
+                            if (i4 >= 32 * kHeadDim / 4) break;
+                            const int c = i4 / (kHeadDim / 4), d = (i4 % (kHeadDim / 4)) * 4;
+                            reinterpret_cast<float4*>(cen_s)[i4] = v[k];
+                            const __half2 h01 = __floats2half2_rn(v[k].x, v[k].y), h23 = __floats2half2_rn(v[k].z, v[k].w);
+                            unsigned char* at = cop + (d >> 6) * (kN * 128) + ((d & 7) << 1);
+                            *reinterpret_cast<uint2*>(at + sw128(c, (d & 63) >> 3)) =
+                                make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+                            float2 f01 = __half22float2(h01), f23 = __half22float2(h23);  // what the MMA sees: hi (+ lo)
+                            if (!value) {
+                                const __half2 l01 = __floats2half2_rn(v[k].x - f01.x, v[k].y - f01.y);
+                                const __half2 l23 = __floats2half2_rn(v[k].z - f23.x, v[k].w - f23.y);
+                                *reinterpret_cast<uint2*>(at + sw128(32 + c, (d & 63) >> 3)) =
+                                    make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
+                                const float2 g01 = __half22float2(l01), g23 = __half22float2(l23);
+                                f01.x += g01.x, f01.y += g01.y, f23.x += g23.x, f23.y += g23.y;
+                            }
+                            // |c|^2: the 32 threads of a warp hold one centre (the worker count is a multiple of 32)
+                            float sq = fmaf(f01.x, f01.x, fmaf(f01.y, f01.y, fmaf(f23.x, f23.x, f23.y * f23.y)));
 #pragma unroll
-                    for (int k = 0; k < kSteps; ++k) {
-                        const int i4 = tid + k * kMakers;
-                        if (i4 >= 32 * kHeadDim / 4) break;
-                        const int c = i4 / (kHeadDim / 4), d = (i4 % (kHeadDim / 4)) * 4;
-                        reinterpret_cast<float4*>(cen_s)[i4] = v[k];
-                        const __half2 h01 = __floats2half2_rn(v[k].x, v[k].y), h23 = __floats2half2_rn(v[k].z, v[k].w);
-                        unsigned char* at = cop + (d >> 6) * (kN * 128) + ((d & 7) << 1);
-                        *reinterpret_cast<uint2*>(at + sw128(c, (d & 63) >> 3)) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
-                        float2 f01 = __half22float2(h01), f23 = __half22float2(h23);  // what the MMA sees: hi (+ lo)
-                        if (!value) {
-                            const __half2 l01 = __floats2half2_rn(v[k].x - f01.x, v[k].y - f01.y);
-                            const __half2 l23 = __floats2half2_rn(v[k].z - f23.x, v[k].w - f23.y);
-                            *reinterpret_cast<uint2*>(at + sw128(32 + c, (d & 63) >> 3)) =
-                                make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
-                            const float2 g01 = __half22float2(l01), g23 = __half22float2(l23);
-                            f01.x += g01.x, f01.y += g01.y, f23.x += g23.x, f23.y += g23.y;
+                            for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(kFull, sq, off);
+                            if (lane == 0) cn_s[c] = c < p.clusters ? sq : INFINITY;
                         }
-                        // |c|^2: the 32 threads of a warp hold one centre (the worker count is a multiple of 32)
-                        float sq = fmaf(f01.x, f01.x, fmaf(f01.y, f01.y, fmaf(f23.x, f23.x, f23.y * f23.y)));
-#pragma unroll
-                        for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(kFull, sq, off);
-                        if (lane == 0) cn_s[c] = c < p.clusters ? sq : INFINITY;
-                    }
                     }
                 }
                 if (tid < (PAIRS ? 64 : 32)) cnt_s[tid] = 0;

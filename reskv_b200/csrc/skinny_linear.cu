@@ -44,13 +44,6 @@ struct LinearParams {
 
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLinWarps * 32) : "memory"); }
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 __global__ void __launch_bounds__(kLinThreads, 1) skinny_linear_kernel(const LinearParams p, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar_full[16], bar_empty[16], bar_x;
@@ -181,10 +174,10 @@ __global__ void __launch_bounds__(kLinThreads, 1) skinny_linear_kernel(const Lin
                     lo[j] = *reinterpret_cast<const uint4*>(at + 64 * j);
                     hi[j] = *reinterpret_cast<const uint4*>(at + 8 * (kLinBox * 2) + 64 * j);
                 }
-                mma_f16(c0, lo[0].x, hi[0].x, lo[0].y, hi[0].y, b[0].x, b[0].y);
-                mma_f16(c1, lo[0].z, hi[0].z, lo[0].w, hi[0].w, b[0].z, b[0].w);
-                mma_f16(c0, lo[1].x, hi[1].x, lo[1].y, hi[1].y, b[1].x, b[1].y);
-                mma_f16(c1, lo[1].z, hi[1].z, lo[1].w, hi[1].w, b[1].z, b[1].w);
+                mma_16816(c0, lo[0].x, hi[0].x, lo[0].y, hi[0].y, b[0].x, b[0].y);
+                mma_16816(c1, lo[0].z, hi[0].z, lo[0].w, hi[0].w, b[0].z, b[0].w);
+                mma_16816(c0, lo[1].x, hi[1].x, lo[1].y, hi[1].y, b[1].x, b[1].y);
+                mma_16816(c1, lo[1].z, hi[1].z, lo[1].w, hi[1].w, b[1].z, b[1].w);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bar_empty[slot]);
                 if (++slot == p.stages) slot = 0, ++round;
