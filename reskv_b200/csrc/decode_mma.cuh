@@ -874,9 +874,14 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                 const __half* qbuf = qf + ((it & 1) * 2 * kRows + g) * kQStride + 16 * qd;
                 constexpr int kLo = kRows * kQStride, kY = 8 * kQStride;  // offsets of the lo halves, of Y's heads (dual)
 
-                // two accumulators (hi.hi; hi.lo and lo.hi) keep the MMA dependency chains short; a third one costs registers (INT4,
-                // batch 8, 16320 tokens 102.0 instead of 100.8 us)
-                float sc2[4] = {0.f, 0.f, 0.f, 0.f};
+                // Two accumulators (hi.hi; hi.lo and lo.hi).  A third one for lo.hi makes the chains of MMAs shorter and costs
+                // registers; it pays at every size measured only with one head on tiled rows: 8 x 4000 tokens 46.4 -> 46.1 us,
+                // 16 x 8128 140.6 -> 139.5, 300 10.13 -> 10.07.  Elsewhere (us): INT4, 8 x 16320 tokens 100.8 -> 102.0; four heads,
+                // tiled 145.4 -> 147.2, bitmap 8 x 65536 419.0 -> 415.6 but 8128 tokens alone 18.2 -> 18.4; one head, bitmap
+                // 115.8 -> 117.5, 4:16 223.0 -> 224.4.
+                constexpr bool kThird = GQA == 1 && Field::kSlotwise && !ML::kPrefix && ML::kPayloadBytes == 128;
+                float sc2[4] = {0.f, 0.f, 0.f, 0.f}, third[kThird ? 4 : 1] = {};
+                float (&sc3)[4] = *reinterpret_cast<float (*)[4]>(kThird ? third : sc2);
                 float sy[kDual ? 4 : 1] = {}, sy2[kDual ? 4 : 1] = {};
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
@@ -935,11 +940,11 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     const uint2 qh_l = *reinterpret_cast<const uint2*>(qbuf + 4 * ks), ql_l = *reinterpret_cast<const uint2*>(qbuf + kLo + 4 * ks);
                     mma_16816(sc, hi_l[0], hi_l[1], hi_l[2], hi_l[3], qh_l.x, qh_l.y);
                     mma_16816(sc2, hi_l[0], hi_l[1], hi_l[2], hi_l[3], ql_l.x, ql_l.y);
-                    mma_16816(sc2, lo_l[0], lo_l[1], lo_l[2], lo_l[3], qh_l.x, qh_l.y);
+                    mma_16816(sc3, lo_l[0], lo_l[1], lo_l[2], lo_l[3], qh_l.x, qh_l.y);
                     const uint2 qh_h = *reinterpret_cast<const uint2*>(qbuf + 64 + 4 * ks), ql_h = *reinterpret_cast<const uint2*>(qbuf + kLo + 64 + 4 * ks);
                     mma_16816(sc, hi_h[0], hi_h[1], hi_h[2], hi_h[3], qh_h.x, qh_h.y);
                     mma_16816(sc2, hi_h[0], hi_h[1], hi_h[2], hi_h[3], ql_h.x, ql_h.y);
-                    mma_16816(sc2, lo_h[0], lo_h[1], lo_h[2], lo_h[3], qh_h.x, qh_h.y);
+                    mma_16816(sc3, lo_h[0], lo_h[1], lo_h[2], lo_h[3], qh_h.x, qh_h.y);
                     if constexpr (kDual) {
                         const uint2 yh_l = *reinterpret_cast<const uint2*>(qbuf + kY + 4 * ks), yl_l = *reinterpret_cast<const uint2*>(qbuf + kLo + kY + 4 * ks);
                         mma_16816(sy, hi_l[0], hi_l[1], hi_l[2], hi_l[3], yh_l.x, yh_l.y);
@@ -952,7 +957,7 @@ __global__ void __launch_bounds__(kThreadsM, 1) decode_mma_kernel(const DecodePa
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) sc[i] += sc2[i];
+                for (int i = 0; i < 4; ++i) sc[i] += kThird ? sc2[i] + sc3[i] : sc2[i];
                 if constexpr (kDual) sc[2] = sy[2] + sy2[2], sc[3] = sy[3] + sy2[3];  // Y's rows
                 // with shared columns only X's scores of columns 0..3 (q < 2) and Y's of columns 4..7 mean anything
                 if (!(okA && (kDual || qd < 2))) sc[0] = sc[1] = -INFINITY;
