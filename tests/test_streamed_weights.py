@@ -126,3 +126,12 @@ def test_a_step_whose_wait_ran_out_raises(which, monkeypatch):
         model._lib = Ran()
     with pytest.raises(RuntimeError, match="device status"):
         model.decode_graph(ids[:, 61])
+
+
+def test_rows_that_leave_room_for_the_stream():
+    """A ring of at least four stages beside the rows of x: any of the eight at 4096 columns, five at 14336."""
+    from reskv_b200._extension import library
+
+    for columns, most in ((512, 8), (4096, 8), (8192, 8), (14336, 5)):
+        for rows in range(1, 9):
+            assert bool(library().reskv_skinny_linear_fits(rows, 4096, columns, 1)) == (rows <= most), (rows, columns)
