@@ -417,7 +417,7 @@ int reskv_kmeans(const void* x, int batch, int kv_heads, int tokens, int64_t x_t
                  int iterations, int value, void* workspace, size_t workspace_bytes, void* centroids, int32_t* ids,
                  void* stream);
 
-/* Clustering of K (flavour 0) and of V (flavour 1) of one shape in the same launches, up to 32 centres and at least as
+/* Clustering of K (flavour 0) and of V (flavour 1) of one shape in the same launch, up to 32 centres and at least as
  * many tokens: what two calls of reskv_kmeans with value = 0 and 1 do, bit for bit.  The workspace is that of 2 * batch sequences.
  * k_ids8 / v_ids8 (i8 [B*KH,T], or NULL) also receive the ids as int8. */
 int reskv_kmeans_pair(const void* x_k, const void* x_v, int batch, int kv_heads, int tokens, int64_t k_tok_stride,

@@ -211,7 +211,7 @@ def compress(
 
     key, value = _dense_or_slice(key), _dense_or_slice(value)
     if previous is None and config.num_clusters <= min(32, key.shape[2]) and (key.data_ptr() | value.data_ptr()) % 16 == 0:
-        # K and V in the same launches: an iteration's fixed costs are paid once
+        # K and V in the same launch: an iteration's fixed costs are paid once
         sides = _ops(key).kmeans_pair(key, value, config.num_clusters, config.kmeans_iterations)
         return CompressedKV(*(_pack(x, centres, ids, plan, stored)
                               for x, (centres, ids, stored) in zip((key, value), sides)))

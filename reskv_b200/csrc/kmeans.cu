@@ -1231,9 +1231,11 @@ void place_state(UmmaParams& p, void* workspace, int units, int clusters) {
 }
 
 // Tiles per CTA of a call for one side, which is also where its tiles are cut.  One CTA per SM, every CTA an equal share of
-// all units' tiles, at least four.  A CTA pays about ten tile times per segment (pipeline drain, flush, new centre tables,
-// refill), so the share is chosen - between the even split and half as much again - for the shortest slowest CTA: a share
-// that divides the units evenly often beats the smallest one.
+// all units' tiles, at least four.  A segment is charged ten tile times (pipeline drain, flush, new centre tables, refill),
+// what it cost with a launch per iteration; in the present form, where runs, owned units and early requests have made it
+// cheaper, it was not measured again.  The share is chosen - between the even split and half as much again - for the
+// shortest slowest CTA under that charge: one that divides the units evenly often beats the smallest one, but may leave SMs
+// without work (64 units x 8128 tokens: 64 tiles on each of 128 CTAs, an even split would be 55.4 on 148).
 int side_share(int tiles_side, int tiles_unit) {
     constexpr int kLeast = 4, seg_max = kUChunkMax / kUTile;
     const int even = (tiles_side + sm_count() - 1) / sm_count();
@@ -1262,8 +1264,8 @@ int side_share(int tiles_side, int tiles_unit) {
 // Tiles per CTA when K and V share the launches.  They are cut as a call for one side cuts them, so that ids and centres
 // are those of two such calls bit for bit; only how many of the pieces a CTA takes is chosen here, again for the shortest
 // slowest CTA.  A segment of the unit whose tables a CTA already has is counted as four tile times, one of another unit as
-// ten; 7 and 1, 7 and 3, 14 and 2 choose shares of the same time, 8 units x 1152 to 64 x 8128 tokens.  About `kTries` shares
-// are looked at (host time).
+// ten, measured with a launch per iteration like side_share's (there 7 and 1, 7 and 3, 14 and 2 chose shares of the same
+// time, 8 units x 1152 to 64 x 8128 tokens).  About `kTries` shares are looked at (host time).
 int pair_share(const Cuts& c) {
     constexpr int kNewUnit = 10, kSameUnit = 4, kTries = 16, seg_max = kUChunkMax / kUTile;
     const int low = (c.tiles + sm_count() - 1) / sm_count();
@@ -1312,8 +1314,10 @@ int launch_umma(UmmaParams& p, void* centroids0, void* centroids1, cudaStream_t 
     const auto kern = pairs ? kmeans_assign_umma_kernel<true> : kmeans_assign_umma_kernel<false>;
     static std::atomic<unsigned long long> done[2];
     if (int rc = allow_smem(kern, smem, done[pairs], "cudaFuncSetAttribute(kmeans_assign_umma)")) return rc;
-    // cooperative: CTAs wait for one another between iterations, so all of them have to be resident.  A stream that has only
-    // a part of the SMs takes fewer CTAs with more pieces each; the cuts, and with them the results, stay.
+    // cooperative: CTAs wait for one another between iterations, so all of them have to be resident, and the launch starts
+    // only once every one of them has its place: beside a long kernel of another stream later than an ordinary launch, which
+    // could begin on the SMs that are free.  A context that has only a part of the SMs takes fewer CTAs with more pieces
+    // each; the cuts, and with them the results, stay.
     cudaLaunchConfig_t cfg{};
     cfg.blockDim = dim3(kUThreads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
     cudaLaunchAttribute attr{};

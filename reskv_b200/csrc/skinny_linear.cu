@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(kLinThreads, 1) skinny_linear_kernel(const Lin
 }
 
 // Taken: up to eight rows, the columns of one MMA (at eight rows still 12.3 and 38.9 us for the two with a norm, cuBLAS 12.7
-// and 39.1 without), as long as x leaves room for four stages: with fewer the stream waits for the copies' latency.
+// and 39.1 without), as long as the rows of x leave room for four stages: with fewer the stream waits for the copies'
+// latency.  14336 columns leave 11, 9, 8, 6 and 4 stages for one to five rows and are not taken for six to eight.
 // stages of the ring beside `rows` rows of x (0: they do not fit)
 int linear_stages(int rows, int k) {
     const int s = (kLinSmem - rows * (2 * k + 64)) / kLinStage;
@@ -243,7 +244,7 @@ extern "C" int reskv_skinny_linear(const void* x, const void* norm_weight, float
     for (const void* ptr : {x, norm_weight, weight, static_cast<const void*>(out)})
         if (reinterpret_cast<uintptr_t>(ptr) & 15u) return fail(RESKV_ERR_INVALID, "skinny_linear: pointers must be 16-byte aligned");
     LinearParams p{};
-    p.x = static_cast<const __half*>(x), p.norm = static_cast<const __half*>(norm_weight), 
+    p.x = static_cast<const __half*>(x), p.norm = static_cast<const __half*>(norm_weight);
     p.out = out, p.eps = eps, p.rows = rows, p.n = n, p.k = k, p.mode = mode, p.stages = linear_stages(rows, k);
     // weights as (column, row, gate or up): a unit's rows in one box
     const bool two = mode == kLinSiluMul;
